@@ -46,7 +46,9 @@ extern "C" {
 #define MSGPU_PREC_C64 1  /* precision form: complex64 vectors and H, FP64 reductions, expm and sums */
 
 /* Krylov recurrences. */
-#define MSGPU_REC_AUTO 0    /* Arnoldi for C128; for C64 Lanczos with scalar K, else Arnoldi */
+#define MSGPU_REC_AUTO 0    /* C128: Arnoldi; with a Hermitian H and scalar K, whose Arnoldi matrix
+                               is tridiagonal, by its three-term recurrence.  C64: Lanczos with
+                               scalar K, else Arnoldi */
 #define MSGPU_REC_ARNOLDI 1 /* Arnoldi on G = -iH - K (as SpinSpace::ArnoldiProcess).  C64
                                takes it when K acts on the electron pair only (K = I x K4,
                                e.g. unequal sinks on the pair's states: CGS2 with FP64 dots,
@@ -129,7 +131,7 @@ extern "C" {
                                         yields change only by FP64 summation order. */
 
 /* Execution forms (msgpu_set_form).  AUTO picks RESIDENT for small
- * dimensions (the whole time loop in one launch, one warp per trajectory,
+ * dimensions (the whole time loop in one launch, one CTA per trajectory,
  * Krylov basis in shared memory) and STREAMED otherwise (one kernel sequence
  * per step over the trajectory block, vectors in HBM). */
 #define MSGPU_FORM_AUTO 0

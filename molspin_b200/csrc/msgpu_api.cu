@@ -16,7 +16,7 @@
 #include "msgpu_dense.h"
 #include "msgpu_fused.cuh"
 #include "msgpu_kernels.cuh"
-#include "msgpu_resident.cuh"
+#include "msgpu_resident.h"
 #include "msgpu_spmm_tc.cuh"
 #include "msgpu_spmm_tm.cuh"
 
@@ -49,7 +49,10 @@ struct msgpu_ctx {
 
     // Hamiltonian
     int D = 0, nnz = 0;
-    DevBuf hrow, hcol, hval, hhi, hlo;
+    DevBuf hrow, hcol, hval, hhi;
+    int max_row = 0;   // most entries of a row of H
+    int hermitian = -1;  // H (every term of it) equals its conjugate transpose: 1, 0, or -1 (not yet checked)
+    DevBuf ell;        // resident form: H in padded column-major order, values then columns
     std::vector<int> h_rowptr, h_col;  // host copy for the quartet-block form
     std::vector<double> h_val;
     // quartet-block form of H for the current electron strides
@@ -106,7 +109,7 @@ struct msgpu_ctx {
     int q_variant = 0;               // autotuned kernel variant (kApplyVariants)
     // resident (one warp per trajectory, whole time loop per launch) form
     int form = MSGPU_FORM_AUTO;
-    DevBuf colbuf, trajval, times_d, pflip_d, sys_d, work_d, obs_d, dense_part;
+    DevBuf trajval, times_d, pflip_d, work_d, obs_d, dense_part;
     // dense tensor-core form
     msgpu::DenseState dense;
     std::vector<std::pair<void *, size_t>> dense_allocs;
@@ -336,12 +339,12 @@ void msgpu_destroy(msgpu_ctx *c)
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     collect_profile(c);
-    DevBuf *all[] = {&c->hrow, &c->hcol, &c->hval, &c->hhi, &c->hlo, &c->qrow, &c->qcolt, &c->qval, &c->qbase, &c->qval64,
+    DevBuf *all[] = {&c->hrow, &c->hcol, &c->hval, &c->hhi, &c->ell, &c->qrow, &c->qcolt, &c->qval, &c->qbase, &c->qval64,
                      &c->fblk, &c->fval, &c->frow, &c->fdsrc, &c->fdiag, &c->krow, &c->kcol, &c->kval, &c->bits,
                      &c->psi128, &c->basis, &c->wbuf, &c->zbuf, &c->ubuf, &c->part, &c->part2, &c->hess,
                      &c->tdiag, &c->toff, &c->coef, &c->mdim, &c->scale, &c->alpha, &c->beta0, &c->qpart_obs,
                      &c->qpart_nrm, &c->prev, &c->acc, &c->comp, &c->rates_d, &c->status, &c->values_d,
-                     &c->colbuf, &c->trajval, &c->times_d, &c->pflip_d, &c->sys_d, &c->work_d, &c->obs_d,
+                     &c->trajval, &c->times_d, &c->pflip_d, &c->work_d, &c->obs_d,
                      &c->dense_part, &c->hterms, &c->qsrc, &c->tc_src, &c->tc_tab, &c->tm_tab};
     for (DevBuf *b : all) release(c, *b);
     msgpu::dense_release(c->dense, dense_release_cb, c);  // its stream and events, then its buffers
@@ -444,15 +447,13 @@ int msgpu_upload_hamiltonian_csr(msgpu_ctx *c, int dim, const int *rowptr, const
     if (rowptr[0] != 0 || nnz < 0) return fail(c, MSGPU_ERR_INVALID, "Hamiltonian: malformed row pointer");
     for (int r = 0; r < dim; ++r)
         if (rowptr[r + 1] < rowptr[r]) return fail(c, MSGPU_ERR_INVALID, "Hamiltonian: row pointer not monotone");
-    std::vector<float> hi(2 * static_cast<size_t>(nnz)), lo(2 * static_cast<size_t>(nnz));
+    std::vector<float> hi(2 * static_cast<size_t>(nnz));
     for (int k = 0; k < nnz; ++k) {
         if (col[k] < 0 || col[k] >= dim) return fail(c, MSGPU_ERR_INVALID, "Hamiltonian: column index out of range");
         for (int p = 0; p < 2; ++p) {
             const double v = val[2 * k + p];
             if (!std::isfinite(v)) return fail(c, MSGPU_ERR_NONFINITE, "Hamiltonian: non-finite value");
-            const float h = static_cast<float>(v);
-            hi[2 * k + p] = h;
-            lo[2 * k + p] = static_cast<float>(v - static_cast<double>(h));
+            hi[2 * k + p] = static_cast<float>(v);
         }
     }
     if (c->D != 0 && c->D != dim) {
@@ -465,15 +466,13 @@ int msgpu_upload_hamiltonian_csr(msgpu_ctx *c, int dim, const int *rowptr, const
     if ((rc = ensure(c, c->hrow, sizeof(int) * (dim + 1), "H rowptr")) ||
         (rc = ensure(c, c->hcol, sizeof(int) * std::max(1, nnz), "H col")) ||
         (rc = ensure(c, c->hval, sizeof(double2) * std::max(1, nnz), "H val")) ||
-        (rc = ensure(c, c->hhi, sizeof(float2) * std::max(1, nnz), "H hi")) ||
-        (rc = ensure(c, c->hlo, sizeof(float2) * std::max(1, nnz), "H lo")))
+        (rc = ensure(c, c->hhi, sizeof(float2) * std::max(1, nnz), "H hi")))
         return rc;
     cudaError_t e;
     if ((e = cudaMemcpyAsync(c->hrow.p, rowptr, sizeof(int) * (dim + 1), cudaMemcpyHostToDevice, c->stream)) ||
         (e = cudaMemcpyAsync(c->hcol.p, col, sizeof(int) * nnz, cudaMemcpyHostToDevice, c->stream)) ||
         (e = cudaMemcpyAsync(c->hval.p, val, sizeof(double2) * nnz, cudaMemcpyHostToDevice, c->stream)) ||
-        (e = cudaMemcpyAsync(c->hhi.p, hi.data(), sizeof(float2) * nnz, cudaMemcpyHostToDevice, c->stream)) ||
-        (e = cudaMemcpyAsync(c->hlo.p, lo.data(), sizeof(float2) * nnz, cudaMemcpyHostToDevice, c->stream)))
+        (e = cudaMemcpyAsync(c->hhi.p, hi.data(), sizeof(float2) * nnz, cudaMemcpyHostToDevice, c->stream)))
         return cuda_fail(c, e, "Hamiltonian upload");
     if ((e = cudaStreamSynchronize(c->stream))) return cuda_fail(c, e, "Hamiltonian upload");
     c->D = dim;
@@ -482,6 +481,9 @@ int msgpu_upload_hamiltonian_csr(msgpu_ctx *c, int dim, const int *rowptr, const
     c->h_col.assign(col, col + nnz);
     c->h_val.assign(val, val + 2 * static_cast<size_t>(nnz));
     c->q_D = 0;  // quartet form must be rebuilt
+    c->max_row = 0;
+    for (int r = 0; r < dim; ++r) c->max_row = std::max(c->max_row, rowptr[r + 1] - rowptr[r]);
+    c->hermitian = -1;
     c->terms = false;
     c->dense.have_u = false;  // a cached dense propagator belongs to the old H
     return MSGPU_OK;
@@ -619,14 +621,13 @@ namespace msgpu {
 namespace {  // internal linkage, beside the other kernels
 
 // H = sum_k coef_k H_k on the common CSR pattern: complex128 values and
-// their FP32 hi/lo split; bit 2 of status on a non-finite value.
+// their FP32 copy; bit 2 of status on a non-finite value.
 struct TermCoef {
     double c[16];
 };
 
 __global__ void k_combine_terms(const double2 *__restrict__ terms, int nterms, TermCoef cf, int nnz,
-                                double2 *__restrict__ val, float2 *__restrict__ hi, float2 *__restrict__ lo,
-                                int *__restrict__ status)
+                                double2 *__restrict__ val, float2 *__restrict__ hi, int *__restrict__ status)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nnz) return;
@@ -638,10 +639,43 @@ __global__ void k_combine_terms(const double2 *__restrict__ terms, int nterms, T
     }
     if (!isfinite(v.x) || !isfinite(v.y)) atomicOr(status, 2);
     val[k] = v;
-    const float2 h = make_float2(static_cast<float>(v.x), static_cast<float>(v.y));
-    hi[k] = h;
-    lo[k] = make_float2(static_cast<float>(v.x - static_cast<double>(h.x)),
-                        static_cast<float>(v.y - static_cast<double>(h.y)));
+    hi[k] = make_float2(static_cast<float>(v.x), static_cast<float>(v.y));
+}
+
+// The resident form's copy of H: entry k of row r at r + k * D (values in the
+// vectors' precision, columns), so that a warp of consecutive rows reads it
+// coalesced; ecnt[r] entries.  kGen: of G = -iH - K (K a CSR operator, or
+// kappa I when krow is null), an entry of K merged into H's at the same column.
+template <typename T, bool kGen>
+__global__ void k_build_ell(const int *__restrict__ rowptr, const int *__restrict__ col, const double2 *__restrict__ val,
+                            const int *__restrict__ krow, const int *__restrict__ kcol, const double2 *__restrict__ kval,
+                            double kappa, int D, T *__restrict__ eval, int *__restrict__ ecol, int *__restrict__ ecnt)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= D) return;
+    const int b = rowptr[r];
+    int n = rowptr[r + 1] - b;
+    for (int k = 0; k < n; ++k) {
+        const size_t e = static_cast<size_t>(k) * D + r;
+        const double2 h = val[b + k];
+        st2(eval + e, kGen ? make_double2(h.y, -h.x) : h);
+        ecol[e] = col[b + k];
+    }
+    if (kGen) {
+        const int kb = krow ? krow[r] : 0, ke = krow ? krow[r + 1] : 1;
+        for (int q = kb; q < ke; ++q) {
+            const int c = krow ? kcol[q] : r;
+            const double2 kv = krow ? kval[q] : make_double2(kappa, 0.0);
+            int k = 0;
+            while (k < n && ecol[static_cast<size_t>(k) * D + r] != c) ++k;
+            const size_t e = static_cast<size_t>(k) * D + r;
+            const double2 g = k < n ? ld2(eval + e) : make_double2(0.0, 0.0);
+            st2(eval + e, csub(g, kv));
+            ecol[e] = c;
+            n = max(n, k + 1);
+        }
+    }
+    ecnt[r] = n;
 }
 
 // quartet value slot s (two FP32 per complex value, and its FP64 copy) <- the
@@ -899,27 +933,54 @@ int run_dense(msgpu_ctx *c, const msgpu_run_params *p)
     return MSGPU_OK;
 }
 
-// Warps per CTA of the resident form for this problem, 0 if it does not
-// apply (streamed form forced, dimension too large for the shared-memory
-// basis, Lanczos asked for with a non-scalar K).
+// Whether the resident form takes this problem (not when the streamed form is
+// forced, the dimension too large for the shared-memory basis, or Lanczos
+// needed with a non-scalar K).
 constexpr size_t kResidentSmemBudget = 200 * 1024;
 constexpr int kResidentMaxDim = 1024;
 
-int resident_warps(const msgpu_ctx *c, int prec, int m)
+bool resident_fits(const msgpu_ctx *c, int prec, int m)
 {
-    if (c->form == MSGPU_FORM_STREAMED || c->sched_steps) return 0;  // a schedule changes H between launches
-    if (prec == MSGPU_PREC_C64 && !c->k_scalar) return 0;
-    if (c->form == MSGPU_FORM_AUTO && c->D > kResidentMaxDim) return 0;
-    const size_t wb = resident_warp_bytes(c->D, m, prec == MSGPU_PREC_C128 ? 16 : 8);
-    // Warps never wait on one another, so a CTA's warp count only places them:
-    // while the block has fewer trajectories than 4 per SM, fewer warps per
-    // CTA spread them over more SMs (cfg1, 256 trajectories: 1.26M -> 1.41M
-    // traj-steps/s in complex128 with one warp per CTA instead of four).
-    int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess || sms < 1) sms = 1;
-    const int spread = std::max(1, c->M / sms);
-    const int w = static_cast<int>(std::min<size_t>(std::min(4, spread), kResidentSmemBudget / wb));
-    return w;
+    if (c->form == MSGPU_FORM_STREAMED || c->sched_steps) return false;  // a schedule changes H between launches
+    if (prec == MSGPU_PREC_C64 && !c->k_scalar) return false;
+    if (c->form == MSGPU_FORM_AUTO && c->D > kResidentMaxDim) return false;
+    return resident_bytes(c->D, m, prec == MSGPU_PREC_C128 ? 16 : 8) <= kResidentSmemBudget;
+}
+
+// Whether H's entries (CSR, duplicates not merged) equal their transposes'
+// conjugates to rounding: then, with K = kappa I, the Arnoldi matrix is
+// tridiagonal and the three-term recurrence gives the same Krylov step.
+bool is_hermitian(int dim, const int *rowptr, const int *col, const double *val)
+{
+    // rows are visited in order, so a sorted row's transposes come up in order too
+    std::vector<int> next(rowptr, rowptr + dim);
+    for (int r = 0; r < dim; ++r)
+        for (int k = rowptr[r]; k < rowptr[r + 1]; ++k) {
+            const int c = col[k];
+            const double re = val[2 * static_cast<size_t>(k)], im = val[2 * static_cast<size_t>(k) + 1];
+            const double tol = 4.0e-16 * (std::abs(re) + std::abs(im));
+            auto conj_at = [&](int l) {
+                return col[l] == r && std::abs(val[2 * static_cast<size_t>(l)] - re) <= tol &&
+                       std::abs(val[2 * static_cast<size_t>(l) + 1] + im) <= tol;
+            };
+            if (next[c] < rowptr[c + 1] && conj_at(next[c])) {
+                ++next[c];
+                continue;
+            }
+            bool found = false;
+            for (int l = rowptr[c]; l < rowptr[c + 1] && !found; ++l) found = conj_at(l);
+            if (!found) return false;
+        }
+    return true;
+}
+
+// complex128 runs whose recurrence is left to the library (MSGPU_REC_AUTO)
+// take the three-term recurrence when H is Hermitian and K = kappa I.
+bool lanczos128(msgpu_ctx *c, const msgpu_run_params *p)
+{
+    if (p->precision != MSGPU_PREC_C128 || p->recurrence != MSGPU_REC_AUTO || !c->k_scalar) return false;
+    if (c->hermitian < 0) c->hermitian = is_hermitian(c->D, c->h_rowptr.data(), c->h_col.data(), c->h_val.data());
+    return c->hermitian == 1;
 }
 
 // K as I (x) K4 on the electron pair (the 4 x 4 block in the pair index
@@ -964,12 +1025,9 @@ int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
 {
     const int D = c->D, ldm = c->ldm, M = c->M;
     const int nobs = static_cast<int>(c->obs.size());
-    const int warps = resident_warps(c, prec, m);
-    const size_t wb = resident_warp_bytes(D, m, prec == MSGPU_PREC_C128 ? 16 : 8);
     cudaStream_t st = c->stream;
     int rc;
     if ((rc = ensure_state(c, MSGPU_PREC_C128)) ||
-        (rc = ensure(c, c->colbuf, static_cast<size_t>(D) * M * sizeof(double2), "resident state")) ||
         (rc = ensure(c, c->acc, static_cast<size_t>(nobs) * ldm * sizeof(double), "yield acc")) ||
         (rc = ensure(c, c->comp, static_cast<size_t>(nobs) * ldm * sizeof(double), "yield comp")) ||
         (rc = ensure(c, c->prev, static_cast<size_t>(nobs) * ldm * sizeof(double), "yield prev")) ||
@@ -979,16 +1037,12 @@ int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
         (rc = ensure(c, c->trajval, static_cast<size_t>(p->ntimes) * M * nobs * sizeof(double), "values per trajectory")) ||
         (rc = ensure(c, c->times_d, static_cast<size_t>(p->ntimes) * sizeof(double), "times")) ||
         (rc = ensure(c, c->pflip_d, static_cast<size_t>(p->ntimes) * sizeof(double), "flip probabilities")) ||
-        (rc = ensure(c, c->sys_d, sizeof(ResidentSystem), "system")) ||
-        (rc = ensure(c, c->work_d, static_cast<size_t>(M) * sizeof(ResidentWork), "work list")) ||
         (rc = ensure(c, c->obs_d, 8 * 16 * sizeof(double2), "observables")))
         return rc;
     // flip probabilities and observables in the kernel's pair basis
     std::vector<double> pf(p->ntimes, 0.0);
     for (int s = 0; s + 1 < p->ntimes; ++s) pf[s] = flip_p(c->st_rate, 0.5 * (p->times[s + 1] - p->times[s]));
     const PairObs po = make_pair_obs(c);
-    std::vector<ResidentWork> work(M);
-    for (int t = 0; t < M; ++t) work[t] = ResidentWork{0, t};
     ResidentSystem S;
     std::memset(&S, 0, sizeof(S));
     S.rowptr = static_cast<const int *>(c->hrow.p);
@@ -1001,6 +1055,43 @@ int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
         S.kval = static_cast<const double2 *>(c->kval.p);
     }
     S.kappa = c->k_scalar ? c->kappa : 0.0;
+    const bool lanczos = prec == MSGPU_PREC_C64 || lanczos128(c, p);
+    // Coalesced copy of H (three-term recurrence) or G (Arnoldi), unless one long
+    // row would blow the padding up or the memory budget has no room for it; the
+    // kernel then walks the CSR rows.
+    int krow_max = 1;
+    if (!lanczos && !c->k_scalar)
+        for (int r = 0; r < D; ++r) krow_max = std::max(krow_max, c->k_hrow[r + 1] - c->k_hrow[r]);
+    S.kmax = c->max_row + (lanczos ? 0 : krow_max);
+    const size_t slots = static_cast<size_t>(D) * S.kmax;
+    const size_t esz = prec == MSGPU_PREC_C128 ? sizeof(double2) : sizeof(float2);
+    bool ell = slots > 0 && slots <= 2 * static_cast<size_t>(c->nnz) + 16 * static_cast<size_t>(D);
+    if (ell && ensure(c, c->ell, slots * (esz + sizeof(int)) + D * sizeof(int), "resident H") != MSGPU_OK) {
+        (void)cudaGetLastError();
+        c->err.clear();
+        ell = false;
+    }
+    if (ell) {
+        int *ecol = reinterpret_cast<int *>(static_cast<unsigned char *>(c->ell.p) + slots * esz);
+        int *ecnt = ecol + slots;
+        const int grid = ceil_div(D, 32);
+        ++c->launches;
+        if (!lanczos)
+            k_build_ell<double2, true><<<grid, 32, 0, st>>>(S.rowptr, S.col, S.val, S.krow, S.kcol, S.kval, S.kappa, D,
+                                                            static_cast<double2 *>(c->ell.p), ecol, ecnt);
+        else if (prec == MSGPU_PREC_C128)
+            k_build_ell<double2, false><<<grid, 32, 0, st>>>(S.rowptr, S.col, S.val, nullptr, nullptr, nullptr, 0.0, D,
+                                                             static_cast<double2 *>(c->ell.p), ecol, ecnt);
+        else
+            k_build_ell<float2, false><<<grid, 32, 0, st>>>(S.rowptr, S.col, S.val, nullptr, nullptr, nullptr, 0.0, D,
+                                                            static_cast<float2 *>(c->ell.p), ecol, ecnt);
+        S.col = ecol;
+        S.rowcnt = ecnt;
+        S.val = static_cast<const double2 *>(c->ell.p);
+        S.valf = static_cast<const float2 *>(c->ell.p);
+        S.kstride = D;
+        S.generator = !lanczos;
+    }
     S.D = D;
     S.M = M;
     S.acc_ld = ldm;  // acc/comp/prev share the streamed layout [nobs][ldm]
@@ -1015,7 +1106,9 @@ int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
     S.nz.bits_steps = c->bits_steps;
     S.nz.M = c->noise_mode == MSGPU_NOISE_REPLAY ? c->bits_ntraj : M;
     S.nz.seed = c->seed;
-    S.psi = c->colbuf.p;
+    S.psi = S.psi_out = c->psi128.p;
+    S.rs = ldm;
+    S.ts = 1;
     S.acc = static_cast<double *>(c->acc.p);
     S.comp = static_cast<double *>(c->comp.p);
     S.prev = static_cast<double *>(c->prev.p);
@@ -1030,52 +1123,20 @@ int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
         (e = cudaMemcpyAsync(c->obs_d.p, po.op, sizeof(double2) * 16 * nobs, cudaMemcpyHostToDevice, st)) ||
         (e = cudaMemcpyAsync(c->times_d.p, p->times, sizeof(double) * p->ntimes, cudaMemcpyHostToDevice, st)) ||
         (e = cudaMemcpyAsync(c->pflip_d.p, pf.data(), sizeof(double) * p->ntimes, cudaMemcpyHostToDevice, st)) ||
-        (e = cudaMemcpyAsync(c->sys_d.p, &S, sizeof(S), cudaMemcpyHostToDevice, st)) ||
-        (e = cudaMemcpyAsync(c->work_d.p, work.data(), sizeof(ResidentWork) * M, cudaMemcpyHostToDevice, st)) ||
         (e = cudaMemsetAsync(c->status.p, 0, sizeof(int), st)))
         return cuda_fail(c, e, "resident setup");
-    // column-major state for the warps (complex64: narrowed through zbuf)
-    const size_t ne = static_cast<size_t>(D) * M;
-    double2 *col128 = static_cast<double2 *>(c->colbuf.p);
-    if (prec == MSGPU_PREC_C64)
-        if (int rc2 = ensure(c, c->zbuf, ne * sizeof(double2), "resident staging")) return rc2;
-    double2 *stage = prec == MSGPU_PREC_C64 ? static_cast<double2 *>(c->zbuf.p) : col128;
-    {
-        Timed tm(c, KC_COMBINE);
-        dim3 grid(ceil_div(D, 32), ldm / 32), block(32, 8);
-        k_interleaved_to_cols<double2><<<grid, block, 0, st>>>(stage, static_cast<const double2 *>(c->psi128.p), D, M, ldm);
-        if (prec == MSGPU_PREC_C64)
-            k_convert<float2, double2><<<ceil_div(ne, 256), 256, 0, st>>>(reinterpret_cast<float2 *>(col128), stage, ne);
-    }
-    const size_t smem = static_cast<size_t>(warps) * wb;
-    const int blocks = ceil_div(M, warps);
+    const ResidentShape shape =
+        prec == MSGPU_PREC_C64 ? resident_shape_c64(D, m) : resident_shape_c128(D, m, lanczos);
     {
         Timed tm(c, KC_APPLY);
-        if (prec == MSGPU_PREC_C128) {
-            if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_resident<double2, false>), static_cast<int>(smem))))
-                return cuda_fail(c, e, "resident shared memory");
-            k_resident<double2, false><<<blocks, 32 * warps, smem, st>>>(
-                static_cast<const ResidentSystem *>(c->sys_d.p), static_cast<const ResidentWork *>(c->work_d.p), M, wb,
-                static_cast<int *>(c->status.p));
-        } else {
-            if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_resident<float2, true>), static_cast<int>(smem))))
-                return cuda_fail(c, e, "resident shared memory");
-            k_resident<float2, true><<<blocks, 32 * warps, smem, st>>>(
-                static_cast<const ResidentSystem *>(c->sys_d.p), static_cast<const ResidentWork *>(c->work_d.p), M, wb,
-                static_cast<int *>(c->status.p));
-        }
+        if ((e = raise_smem_limit(reinterpret_cast<const void *>(shape.fn), static_cast<int>(shape.smem))))
+            return cuda_fail(c, e, "resident shared memory");
+        shape.fn<<<M, 32 * shape.warps, shape.smem, st>>>(S, static_cast<int *>(c->status.p));
     }
     {
         Timed tm(c, KC_YIELD);
         k_resident_values<<<p->ntimes, 256, 0, st>>>(static_cast<const double *>(c->trajval.p), M, nobs,
                                                       static_cast<double *>(c->values_d.p));
-    }
-    {
-        Timed tm(c, KC_COMBINE);
-        if (prec == MSGPU_PREC_C64)
-            k_convert<double2, float2><<<ceil_div(ne, 256), 256, 0, st>>>(stage, reinterpret_cast<const float2 *>(col128), ne);
-        dim3 grid(ceil_div(D, 32), ldm / 32), block(32, 8);
-        k_cols_to_interleaved<double2><<<grid, block, 0, st>>>(static_cast<double2 *>(c->psi128.p), stage, D, M, ldm);
     }
     int status = 0;
     c->last_values.assign(static_cast<size_t>(p->ntimes) * nobs, 0.0);
@@ -1840,6 +1901,9 @@ int msgpu_upload_hamiltonian_terms(msgpu_ctx *c, int dim, const int *rowptr, con
         return cuda_fail(c, e, "Hamiltonian terms upload");
     c->terms = true;
     c->nterms = nterms;
+    c->hermitian = 1;
+    for (int t = 0; t < nterms && c->hermitian == 1; ++t)
+        c->hermitian = is_hermitian(dim, rowptr, col, vals + 2 * static_cast<size_t>(t) * nnz);
     return msgpu_set_hamiltonian_coefficients(c, coef);
 }
 
@@ -1861,7 +1925,7 @@ int msgpu_set_hamiltonian_coefficients(msgpu_ctx *c, const double *coef)
     if ((e = cudaMemsetAsync(c->status.p, 0, sizeof(int), c->stream))) return cuda_fail(c, e, "Hamiltonian update");
     k_combine_terms<<<ceil_div(std::max(1, c->nnz), 256), 256, 0, c->stream>>>(
         static_cast<const double2 *>(c->hterms.p), c->nterms, cf, c->nnz, static_cast<double2 *>(c->hval.p),
-        static_cast<float2 *>(c->hhi.p), static_cast<float2 *>(c->hlo.p), static_cast<int *>(c->status.p));
+        static_cast<float2 *>(c->hhi.p), static_cast<int *>(c->status.p));
     if ((e = cudaGetLastError())) return cuda_fail(c, e, "Hamiltonian update");
     // the quartet form keeps its structure; only its values follow H
     if (c->q_D == c->D)
@@ -2021,7 +2085,7 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
     const int D = c->D, ldm = c->ldm, M = c->M;
     const int m = (taylor || rk4) ? 1 : std::min(p->krylov_dim, D);  // no Krylov basis (RK4 uses slot 0 as its sum)
     const int prec = p->precision;
-    if (!taylor && !rk4 && resident_warps(c, prec, m) > 0) return run_resident(c, p, prec, m);
+    if (!taylor && !rk4 && resident_fits(c, prec, m)) return run_resident(c, p, prec, m);
     if (c->form == MSGPU_FORM_RESIDENT)
         return fail(c, MSGPU_ERR_INVALID, "run: the resident form does not fit this dimension / recurrence / propagator");
     const int nobs = static_cast<int>(c->obs.size());
@@ -2183,7 +2247,7 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
             }
             k_combine_terms<<<ceil_div(std::max(1, c->nnz), 256), 256, 0, st>>>(
                 static_cast<const double2 *>(c->hterms.p), c->nterms, cf, c->nnz, static_cast<double2 *>(c->hval.p),
-                static_cast<float2 *>(c->hhi.p), static_cast<float2 *>(c->hlo.p), static_cast<int *>(c->status.p));
+                static_cast<float2 *>(c->hhi.p), static_cast<int *>(c->status.p));
             if (prec == MSGPU_PREC_C64 || quartet128)
                 if (int rc = refresh_quartet_values(c)) return rc;
             if (taylor) taylor_shift(hs);
@@ -2241,7 +2305,7 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                     k_combine_terms<<<ceil_div(std::max(1, c->nnz), 256), 256, 0, st>>>(
                         static_cast<const double2 *>(c->hterms.p), c->nterms, cf, c->nnz,
                         static_cast<double2 *>(c->hval.p), static_cast<float2 *>(c->hhi.p),
-                        static_cast<float2 *>(c->hlo.p), static_cast<int *>(c->status.p));
+                        static_cast<int *>(c->status.p));
                 }
                 Timed tm(c, KC_APPLY);
                 k_rk4_stage<<<tgrid, tblock, 0, st>>>(Hd, Kd, kappa, in[stage], psi, out[stage], acc, cs[stage],
@@ -2657,6 +2721,42 @@ extern "C" int msgpu_krylov_step_noalloc(int dim, const int *rowptr, const int *
     int *status = cv.take<int>(1);
 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (resident_bytes(D, m, 16) <= kResidentSmemBudget && D <= kResidentMaxDim) {
+        // One launch of the resident form (a CTA per trajectory, basis in shared
+        // memory) instead of the 8 m + 5 kernels below, whose launches and serial
+        // reductions set the time: 61 against 785 us at D = 64, 64 trajectories,
+        // m = 16.
+        ResidentSystem S;
+        std::memset(&S, 0, sizeof(S));
+        S.rowptr = rowptr;
+        S.col = col;
+        S.val = reinterpret_cast<const double2 *>(val);
+        S.kmax = D;  // row lengths stay on the device
+        S.kappa = kappa;
+        S.D = D;
+        S.M = S.acc_ld = ntraj;
+        S.m = m;
+        S.s1 = D / 2;  // any two spin-1/2 strides partition the rows into quartets
+        S.s2 = D / 4;
+        S.psi = psi_in;
+        S.psi_out = psi_out;
+        S.rs = 1;
+        S.ts = D;
+        S.dt0 = dt;
+        S.ntimes = 2;
+        S.check_start = 1;
+        const ResidentShape shape = resident_shape_c128(D, m, false);
+        int h_status = 0;
+        if (raise_smem_limit(reinterpret_cast<const void *>(shape.fn), static_cast<int>(shape.smem)) != cudaSuccess ||
+            cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess)
+            return MSGPU_ERR_CUDA;
+        shape.fn<<<ntraj, 32 * shape.warps, shape.smem, st>>>(S, status);
+        if (cudaGetLastError() != cudaSuccess ||
+            cudaMemcpyAsync(&h_status, status, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess)
+            return MSGPU_ERR_CUDA;
+        return h_status & 2 ? MSGPU_ERR_NONFINITE : h_status & 1 ? MSGPU_ERR_EXPM : MSGPU_OK;
+    }
     // Contents left by the previous call are stale: clear what must start at zero.
     if (cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess ||
         cudaMemsetAsync(mdim, 0, ldm * sizeof(int), st) != cudaSuccess)

@@ -147,7 +147,7 @@ int prepare(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_of
         S.nz.mode = s.st_rate > 0.0 ? MSGPU_NOISE_PHILOX : MSGPU_NOISE_NONE;
         S.nz.M = s.M;
         S.nz.seed = s.seed;
-        S.psi = s.psi.p;
+        S.psi = S.psi_out = s.psi.p;
         S.acc = static_cast<double *>(s.acc.p);
         S.comp = static_cast<double *>(s.comp.p);
         S.prev = static_cast<double *>(s.prev.p);

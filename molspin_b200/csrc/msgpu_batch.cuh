@@ -122,7 +122,7 @@ __device__ void team_propagate(const Team &tm, const ResidentSystem &S, int t, f
     double2 *Hm = ex;  // alpha in .x, beta in .y (m entries)
     double2 *A = Hm + m, *X = A + static_cast<size_t>(m) * m, *N = X + static_cast<size_t>(m) * m;
     double2 *Dm = N + static_cast<size_t>(m) * m, *y = Dm + static_cast<size_t>(m) * m;
-    float2 *col = reinterpret_cast<float2 *>(S.psi) + static_cast<size_t>(t) * D;
+    float2 *col = static_cast<float2 *>(S.psi_out) + static_cast<size_t>(t) * D;
     for (int r = tm.rank(); r < D; r += tm.size()) z[r] = col[r];
     tm.sync();
     double accv[8], compv[8], prevv[8], vals[8];

@@ -52,6 +52,14 @@ __device__ __forceinline__ double2 cconjmul(double2 a, double2 b)  // conj(a)*b
 {
     return make_double2(fma(a.x, b.x, a.y * b.y), fma(a.x, b.y, -a.y * b.x));
 }
+__device__ __forceinline__ double2 cconjfma(double2 a, double2 b, double2 c)  // conj(a)*b + c
+{
+    return make_double2(fma(a.x, b.x, fma(a.y, b.y, c.x)), fma(a.x, b.y, fma(-a.y, b.x, c.y)));
+}
+__device__ __forceinline__ double2 cnfma(double2 a, double2 b, double2 c)  // c - a*b
+{
+    return make_double2(fma(-a.x, b.x, fma(a.y, b.y, c.x)), fma(-a.x, b.y, fma(-a.y, b.x, c.y)));
+}
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
@@ -61,6 +69,19 @@ __device__ __forceinline__ float2 cfmaf(float2 a, float2 b, float2 c)
 {
     return make_float2(fmaf(a.x, b.x, fmaf(-a.y, b.y, c.x)), fmaf(a.x, b.y, fmaf(a.y, b.x, c.y)));
 }
+
+// element access in FP64 whatever the storage
+__device__ __forceinline__ double2 ld2(const double2 *p) { return *p; }
+__device__ __forceinline__ double2 ld2(const float2 *p) { const float2 v = *p; return make_double2(v.x, v.y); }
+__device__ __forceinline__ void st2(double2 *p, double2 v) { *p = v; }
+__device__ __forceinline__ void st2(float2 *p, double2 v) { *p = make_float2(static_cast<float>(v.x), static_cast<float>(v.y)); }
+
+// A value that is the same on every lane, told to the compiler: branches and
+// loops on it are then compiled as warp-uniform.  A shuffle result or
+// threadIdx.x >> 5 is not known to be, and every warp-wide operation under a
+// branch on one costs an extra reconvergence (the resident step at D = 64 took
+// 30 us instead of 15 with one such branch around its series).
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 
 // ------------------------------------------------------------ warp reductions
 __device__ __forceinline__ double warp_sum(double v)
@@ -102,38 +123,71 @@ __device__ __forceinline__ int quartet_base(int q, int s1, int s2)
 // 4 x kTridiagMaxSubsteps.
 constexpr int kTridiagMaxSubsteps = 1 << 14;
 
+// 1 / k and 1 / k!, 0 <= k <= 64: an FP64 division per Taylor term would cost
+// more than the rest of the term.
+struct TaylorTable {
+    double inv[65], ifact[65];
+    constexpr TaylorTable() : inv(), ifact()
+    {
+        inv[0] = ifact[0] = 1.0;
+        for (int k = 1; k < 65; ++k) {
+            inv[k] = 1.0 / k;
+            ifact[k] = ifact[k - 1] / k;
+        }
+    }
+};
+static __constant__ TaylorTable c_taylor{};
+
+// Smallest Taylor degree K with theta^(K+1) / (K+1)! < 1e-17 (in FP32, with a
+// margin above its rounding: the choice only has to be safe, and an FP64
+// division per candidate took longer than the series).
+__device__ __forceinline__ int taylor_degree(double theta)
+{
+    const float th = static_cast<float>(theta);
+    int K = 1;
+    for (float rem = 0.5f * th * th; rem >= 0.999e-17f && K < 64; ++K) rem *= th * static_cast<float>(c_taylor.inv[K + 2 < 65 ? K + 2 : 64]);
+    return K;
+}
+
 __device__ inline bool warp_tridiag_expm_e1(int n, double diag, double lo, double hi, double kappa, double dt,
                                             double2 &y)
 {
     const int lane = threadIdx.x & 31;
     const bool live = lane < n;
+    const double sk = exp(-kappa * dt);  // ahead of the series, whose latency hides it
     const double d = live ? -dt * diag : 0.0;
     const double l = (live && lane > 0) ? -dt * lo : 0.0;
     const double h = (lane + 1 < n) ? -dt * hi : 0.0;
     const double nrm = warp_max(fabs(d) + fabs(l) + fabs(h));
     y = make_double2(lane == 0 ? 1.0 : 0.0, 0.0);
-    if (!(isfinite(nrm) && nrm <= 4.0 * kTridiagMaxSubsteps)) return false;
-    const int r = max(1, static_cast<int>(ceil(nrm / 4.0)));
-    const double theta = nrm / r, inv_r = 1.0 / r;
-    int K = 1;
-    for (double rem = theta * theta / 2.0; rem >= 1e-17 && K < 64; ++K) rem *= theta / (K + 2);
-    const double ds = d * inv_r, ls = l * inv_r, hs = h * inv_r;
+    if (__any_sync(0xffffffffu, !(isfinite(nrm) && nrm <= 4.0 * kTridiagMaxSubsteps))) return false;
+    const int r = warp_uniform(max(1, static_cast<int>(ceil(nrm * 0.25))));
+    double theta = nrm, ds = d, ls = l, hs = h;
+    if (r > 1) {
+        const double inv_r = 1.0 / r;
+        theta = nrm * inv_r;
+        ds *= inv_r;
+        ls *= inv_r;
+        hs *= inv_r;
+    }
+    const int K = warp_uniform(taylor_degree(theta));
     for (int rep = 0; rep < r; ++rep) {
-        double2 term = y, acc = y;
+        // t = B^k y unscaled (|B| <= 4, k <= 64: no overflow); acc += t / k!, off
+        // the dependent chain, which is one shuffle and two FMAs a term
+        double2 t = y, acc = y;
         for (int k = 1; k <= K; ++k) {
-            // (B term)_i = i (l term_{i-1} + d term_i + h term_{i+1})
-            const double pr = __shfl_up_sync(0xffffffffu, term.x, 1), pi = __shfl_up_sync(0xffffffffu, term.y, 1);
-            const double nr = __shfl_down_sync(0xffffffffu, term.x, 1), ni = __shfl_down_sync(0xffffffffu, term.y, 1);
-            const double re = ls * pr + ds * term.x + hs * nr;
-            const double im = ls * pi + ds * term.y + hs * ni;
-            const double inv = 1.0 / k;
-            term = live ? make_double2(-im * inv, re * inv) : make_double2(0.0, 0.0);  // times i / k
-            acc.x += term.x;
-            acc.y += term.y;
+            // (B t)_i = i (l t_{i-1} + d t_i + h t_{i+1})
+            const double pr = __shfl_up_sync(0xffffffffu, t.x, 1), pi = __shfl_up_sync(0xffffffffu, t.y, 1);
+            const double nr = __shfl_down_sync(0xffffffffu, t.x, 1), ni = __shfl_down_sync(0xffffffffu, t.y, 1);
+            const double re = fma(hs, nr, fma(ls, pr, ds * t.x));
+            const double im = fma(hs, ni, fma(ls, pi, ds * t.y));
+            t = make_double2(-im, re);  // times i; rows >= n stay zero (their coefficients are)
+            const double c = c_taylor.ifact[k];
+            acc.x = fma(c, t.x, acc.x);
+            acc.y = fma(c, t.y, acc.y);
         }
         y = acc;
     }
-    const double sk = exp(-kappa * dt);
     y = make_double2(y.x * sk, y.y * sk);
     return __all_sync(0xffffffffu, isfinite(y.x) && isfinite(y.y));
 }

@@ -20,6 +20,7 @@
 #include <utility>
 
 #include "msgpu_device.cuh"
+#include "msgpu_resident.h"
 
 namespace msgpu {
 // Kernels defined in these headers have internal linkage: every translation
@@ -1208,18 +1209,7 @@ k_lanczos_expm(const double *__restrict__ tdiag, const double *__restrict__ toff
     if (!ok && b0 > 0.0 && lane == 0 && t < M) atomicOr(status, 1);
 }
 
-// Flip bit for trajectory t at (global step, half): replay bits (layout
-// ((step*2+half)*M + t)) or Philox.
-struct Noise {
-    int mode;                // 0 none, 1 replay bits, 2 philox
-    const uint8_t *bits;     // replay
-    long long bits_steps;    // number of steps covered by bits
-    int M;                   // trajectories in the bit layout
-    uint64_t seed;           // philox
-    uint32_t traj_offset;    // added to the launch's trajectory index (a trajectory group's first)
-    double p_full;           // flip probability for a half step of the current step
-};
-
+// Flip bit of one half step (struct Noise: msgpu_resident.h).
 __device__ __forceinline__ int noise_bit(const Noise &nz, int t, long long step, int half, double p)
 {
     if (step < 0) return 0;
@@ -1553,17 +1543,26 @@ k_yield_values(const double *__restrict__ prev, int nobs, int ldm, int M, double
     }
 }
 
-template <typename Dst, typename Src>
-__global__ void k_convert(Dst *__restrict__ out, const Src *__restrict__ in, size_t n)
+// values[s][o] = sum over trajectories of traj_values[s][t][o] (fixed order);
+// one block per time point.
+__global__ void k_resident_values(const double *__restrict__ traj_values, int M, int nobs, double *__restrict__ values)
 {
-    const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    Dst o;
-    o.x = in[i].x;
-    o.y = in[i].y;
-    out[i] = o;
+    __shared__ double red[8][32];
+    const int s = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int t = threadIdx.x; t < M; t += blockDim.x)
+        for (int o = 0; o < nobs; ++o) acc[o] += traj_values[(static_cast<size_t>(s) * M + t) * nobs + o];
+    for (int o = 0; o < nobs; ++o) {
+        const double v = warp_sum(acc[o]);
+        if (lane == 0) red[o][warp] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < nobs) {
+        double v = 0.0;
+        for (int w = 0; w < (blockDim.x >> 5); ++w) v += red[threadIdx.x][w];
+        values[static_cast<size_t>(s) * nobs + threadIdx.x] = v;
+    }
 }
-
 
 // Column-major D x M (one trajectory per column, as HSPreparedState factors)
 // <-> trajectory-interleaved (row r, trajectory t at r*ldm + t), through 32x32

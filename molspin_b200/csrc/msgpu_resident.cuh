@@ -1,22 +1,27 @@
 // msgpu_resident.cuh -- "resident" form for small Hilbert dimensions.
 //
-// One warp owns one trajectory for the whole time loop: its Krylov basis,
-// Hessenberg matrix and expm scratch live in shared memory, the trajectory is
-// read from and written back to its column of the reference's column-major
-// D x M factor block once per launch, and every time step (evaluation, ST
-// flips, Krylov step, trapezoid) runs inside one kernel launch.  For small D
-// (the radical pair with a handful of nuclei) this removes the per-step
-// launches of the streamed path; the arithmetic is FP64-latency bound.
+// One CTA owns one trajectory for the whole time loop: its Krylov basis lives
+// in shared memory, the trajectory is read from and written back to the state
+// once per launch, and every time step (evaluation, ST flips, Krylov step,
+// trapezoid) runs inside one kernel launch.  A step is a serial chain of m
+// products with H and their reductions, so the chain's latency sets the time:
+// rows are spread over the warps of the CTA (RPT rows a thread), a Krylov
+// iteration has two barriers, and the small exponential is a Taylor series on
+// a vector in one warp.
+//
+// What bounds it: dependent FP64 latency and, at few warps an SM, the
+// instructions of a warp.  B200, us per time step of the whole block:
+//   D = 64, 256 trajectories, m = 16, complex128: 14 (186 with a warp per
+//     trajectory, Arnoldi and Pade); complex64: 14.3 (36), at 4096 trajectories 66;
+//   D = 96, 100 trajectories, unequal sinks: 35 (220);
+//   D = 1024, 256 trajectories, complex64: 280 (1570).
 //
 // Recurrences:
-//   complex128: Arnoldi with modified Gram-Schmidt in the order of
-//     SpinSpace::ArnoldiProcess (SpinSpace_operators.cpp:1352-1408), on
-//     G = -iH - K, breakdown below 1e-14;
-//   complex64: Lanczos on H (K = kappa I) with FP32 vectors and SpMV, FP64
-//     dot products, norms, tridiagonal and expm.
-//
-// Work items are (system, trajectory) pairs so that one launch can serve
-// several systems of different dimension (the batching form).
+//   Lanczos on H (Hermitian, K = kappa I), complex64 or complex128 vectors,
+//     FP64 dot products, norms, tridiagonal and expm;
+//   Arnoldi on G = -iH - K (SpinSpace::ArnoldiProcess,
+//     SpinSpace_operators.cpp:1352-1408) for any other operator, complex128,
+//     with classical Gram-Schmidt applied twice; breakdown below 1e-14.
 #pragma once
 
 #include "msgpu_kernels.cuh"
@@ -24,323 +29,694 @@
 namespace msgpu {
 namespace {  // internal linkage (see msgpu_kernels.cuh)
 
-struct ResidentSystem {
-    // H (rad/ns) as CSR; values complex128 and complex64 copies
-    const int *rowptr;
-    const int *col;
-    const double2 *val;
-    const float2 *valf;
-    // K: CSR (krow != null) or kappa * I
-    const int *krow;
-    const int *kcol;
-    const double2 *kval;
-    double kappa;
-    int D, M, m;       // dimension, trajectories, Krylov dimension
-    int acc_ld;        // stride of acc/comp/prev (>= M)
-    int s1, s2;        // electron-pair strides (s1 > s2)
-    int nobs;
-    const double2 *obs;   // nobs x 16 (row-major 4x4, kernel pair basis)
-    const double *rates;  // nobs
-    Noise nz;             // flip stream (replay bits indexed by this system's M)
-    void *psi;            // D x M column-major, double2 or float2
-    double *acc, *comp, *prev;  // nobs x M (observable-major)
-    double *traj_values;        // (ntimes) x M x nobs, or null
-    const double *times;        // ntimes
-    const double *pflip;        // per step flip probability of a half step
-    int ntimes;
-    long long step_offset;
-    int accumulate;
+// Carves a team's shared memory (the same sequence sizes it on the host).
+struct SmemCarve {
+    unsigned char *p;
+    size_t off;
+    template <typename U>
+    __host__ __device__ U *take(size_t n)
+    {
+        U *q = reinterpret_cast<U *>(p + off);
+        off += (n * sizeof(U) + 15) / 16 * 16;
+        return q;
+    }
 };
 
-struct ResidentWork {
-    int sys;
-    int traj;
+// Pair observables as upper-triangle coefficients over a quartet's (a <= c)
+// pairs: Re <x|O|x> = sum Cr Re(x_a* x_c) - Ci Im(x_a* x_c), C_ac = O_ac +
+// conj(O_ca) (a < c), C_aa = Re O_aa.  Bit k of re / im: some observable has a
+// real / imaginary part in pair k (the four pair-state projectors: 5 of 10 and
+// none).
+struct ObsTable {
+    double2 c[10][8];
+    unsigned re, im;
 };
 
 template <typename T>
-struct ResidentSmem;
+struct ResidentSmem {
+    T *V;               // w_0 (the state) .. w_{m-1}; Arnoldi: padded columns, then the vector being orthogonalised
+    double2 *Hm;        // Arnoldi: Hessenberg, column-major; Lanczos: alpha_j, beta_{j+1} in .x, .y
+    double2 *A;         // 4 m^2 + m: small exponential scratch
+    double *sc;         // 1 / |w_j|
+    double2 *cf;        // combination coefficients
+    double *red;        // 2 x W reduction buffers
+    double *rede;       // W x 9 (evaluation)
+    double2 *hp;        // Arnoldi: partial dots of warps 1.., W x 32; row 0: the coefficients
+    ObsTable *obs;
+    int *flags;         // [0] flip of the coming evaluation, [1] Krylov dimension for the combination
+    size_t bytes;
+};
 
-__device__ __forceinline__ double2 ld2(const double2 *p) { return *p; }
-__device__ __forceinline__ double2 ld2(const float2 *p) { const float2 v = *p; return make_double2(v.x, v.y); }
-__device__ __forceinline__ void st2(double2 *p, double2 v) { *p = v; }
-__device__ __forceinline__ void st2(float2 *p, double2 v) { *p = make_float2(static_cast<float>(v.x), static_cast<float>(v.y)); }
-
-// Bytes of shared memory one warp needs.
-__host__ __device__ inline size_t resident_warp_bytes(int D, int m, int elem)
+template <typename T, bool kLanczos>
+__host__ __device__ inline ResidentSmem<T> resident_carve(unsigned char *base, int D, int m, int W)
 {
-    // basis m*D + work vector D (elements), then FP64 Hessenberg/tridiagonal
-    // (m*m complex) and expm scratch (4 m*m + m complex)
-    size_t b = static_cast<size_t>(elem) * D * (m + 1);
-    b = (b + 15) / 16 * 16;
-    b += sizeof(double2) * (static_cast<size_t>(m) * m + 4 * static_cast<size_t>(m) * m + m);
-    return b;
+    SmemCarve c{base, 0};
+    ResidentSmem<T> s;
+    s.V = c.take<T>(kLanczos ? static_cast<size_t>(D) * m : static_cast<size_t>(D + 1) * (m + 1));
+    s.Hm = c.take<double2>(kLanczos ? m : static_cast<size_t>(m) * m);
+    // complex64 Lanczos has no Pade fallback
+    s.A = c.take<double2>(kLanczos && sizeof(T) == 8 ? m : 4 * static_cast<size_t>(m) * m + m);
+    s.sc = c.take<double>(m);
+    s.cf = c.take<double2>(m);
+    s.red = c.take<double>(2 * W);
+    s.rede = c.take<double>(9 * W);
+    s.hp = c.take<double2>(kLanczos ? 1 : 32 * W);
+    s.obs = c.take<ObsTable>(1);
+    s.flags = c.take<int>(2);
+    s.bytes = c.off;
+    return s;
 }
 
-// Evaluate the pair observables of the trajectory held in x (shared), apply
-// the flip first; returns per-lane partials summed over the warp.
-template <typename T>
-__device__ void resident_epilogue(T *x, const ResidentSystem &S, int flip, double *vals, double &nrm)
+// One CTA of W warps working on one trajectory.
+template <int W>
+struct Team {
+    __device__ static void sync()
+    {
+        if constexpr (W == 1) __syncwarp();
+        else __syncthreads();
+    }
+    // sum over the team, the same bits on every thread; also orders the team's
+    // shared-memory writes before it.  red: W doubles, not reused before the
+    // next team barrier.
+    __device__ static double sum(double v, double *red)
+    {
+        v = warp_sum(v);
+        if constexpr (W == 1) {
+            __syncwarp();
+            return v;
+        } else {
+            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+            __syncthreads();
+            if constexpr (W <= 8) {
+                double s = red[0];
+#pragma unroll
+                for (int w = 1; w < W; ++w) s += red[w];
+                return s;
+            } else {
+                const int lane = threadIdx.x & 31;
+                return warp_sum(lane < W ? red[lane] : 0.0);
+            }
+        }
+    }
+};
+
+// A thread's rows of H.  With one row a thread, the row's first kRowRegs
+// entries stay in registers for the whole time loop (absent ones: value 0 on
+// the row itself), so a product costs one round of shared-memory gathers;
+// entries beyond them, and every entry with more rows a thread, are read again
+// from the cached copy of H on each product (about 100 cycles a round).
+template <typename T, int RPT>
+constexpr int row_regs() { return RPT == 1 ? kRowRegs : 0; }
+
+template <typename T, int RPT>
+struct Rows {
+    static constexpr int KR = row_regs<T, RPT>();
+    int base[RPT], cnt[RPT], stride;
+    T h[RPT][KR ? KR : 1];
+    int c[RPT][KR ? KR : 1];
+
+    __device__ static T value(const ResidentSystem &S, int e)
+    {
+        if constexpr (sizeof(T) == sizeof(double2)) return __ldg(S.val + e);
+        else return __ldg(S.valf + e);
+    }
+    __device__ static T mac(T h, T x, T a)
+    {
+        if constexpr (sizeof(T) == sizeof(double2)) return cfma(h, x, a);
+        else return cfmaf(h, x, a);
+    }
+    __device__ void load(const ResidentSystem &S, int tid, int nt)
+    {
+        stride = S.kstride > 0 ? S.kstride : 1;
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            const int r = tid + nt * i;
+            const bool in = r < S.D;
+            const int b = in ? (S.kstride > 0 ? r : __ldg(S.rowptr + r)) : 0;
+            cnt[i] = !in ? 0 : S.kstride > 0 ? __ldg(S.rowcnt + r) : __ldg(S.rowptr + r + 1) - b;
+            base[i] = b;
+#pragma unroll
+            for (int k = 0; k < KR; ++k) {
+                h[i][k].x = h[i][k].y = 0;
+                c[i][k] = in ? r : 0;
+                if (k < cnt[i]) {
+                    h[i][k] = value(S, base[i] + k * stride);
+                    c[i][k] = __ldg(S.col + base[i] + k * stride);
+                }
+            }
+        }
+    }
+    // (H v)_r of row i in the vector's own precision; kmax: the longest row
+    __device__ double2 apply(const ResidentSystem &S, int i, int kmax, const T *v) const
+    {
+        T a0, a1;
+        a0.x = a0.y = a1.x = a1.y = 0;
+#pragma unroll
+        for (int k = 0; k < KR; k += 4) {
+            if (k >= kmax) break;
+            T x[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) x[q] = v[c[i][k + q]];
+            a0 = mac(h[i][k], x[0], a0);
+            a1 = mac(h[i][k + 1], x[1], a1);
+            a0 = mac(h[i][k + 2], x[2], a0);
+            a1 = mac(h[i][k + 3], x[3], a1);
+        }
+        if (KR == 0 || kmax > KR) {
+#pragma unroll 4
+            for (int k = KR; k < cnt[i]; ++k) {
+                const int e = base[i] + k * stride;
+                a0 = mac(value(S, e), v[__ldg(S.col + e)], a0);
+            }
+        }
+        a0.x += a1.x;
+        a0.y += a1.y;
+        return make_double2(a0.x, a0.y);
+    }
+};
+
+// Flips (if set), norm and pair observables of the state x, one quartet per
+// thread; val on thread o < nobs (its observable, times the rate), the norm on
+// every thread.  NO: 4 or 8 observable slots.
+template <typename T, int W, int NO>
+__device__ __forceinline__ void resident_evaluate(const ResidentSystem &S, const ResidentSmem<T> &sm, T *x, int flip,
+                                                  double &val, double &nrm)
 {
-    const int lane = threadIdx.x & 31;
-    const int Q = S.D / 4;
-    double obs[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    double nn = 0.0;
-    for (int q = lane; q < Q; q += 32) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, Q = S.D / 4;
+    double v[NO + 1];  // observables, then the squared norm
+#pragma unroll
+    for (int o = 0; o <= NO; ++o) v[o] = 0.0;
+    const unsigned mre = sm.obs->re, mim = sm.obs->im;
+    for (int q = threadIdx.x; q < Q; q += 32 * W) {
         const int base = quartet_base(q, S.s1, S.s2);
         const int r[4] = {base, base + S.s2, base + S.s1, base + S.s1 + S.s2};
-        double2 v[4];
+        double2 z[4];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) v[a] = ld2(x + r[a]);
+        for (int a = 0; a < 4; ++a) z[a] = ld2(x + r[a]);
         if (flip) {  // U = PS - PT on the pair
-            const double2 b = v[1];
-            v[0] = make_double2(-v[0].x, -v[0].y);
-            v[1] = make_double2(-v[2].x, -v[2].y);
-            v[2] = make_double2(-b.x, -b.y);
-            v[3] = make_double2(-v[3].x, -v[3].y);
+            const double2 b = z[1];
+            z[0] = make_double2(-z[0].x, -z[0].y);
+            z[1] = make_double2(-z[2].x, -z[2].y);
+            z[2] = make_double2(-b.x, -b.y);
+            z[3] = make_double2(-z[3].x, -z[3].y);
+#pragma unroll
+            for (int a = 0; a < 4; ++a) st2(x + r[a], z[a]);
         }
-        nn += cabs2(v[0]) + cabs2(v[1]) + cabs2(v[2]) + cabs2(v[3]);
-        for (int o = 0; o < S.nobs; ++o) {
-            const double2 *op = S.obs + o * 16;
-            double sum = 0.0;
+        v[NO] += (cabs2(z[0]) + cabs2(z[1])) + (cabs2(z[2]) + cabs2(z[3]));
+        int k = 0;
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                double2 ox = make_double2(0.0, 0.0);
+        for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) ox = cfma(__ldg(op + a * 4 + b), v[b], ox);
-                sum += v[a].x * ox.x + v[a].y * ox.y;
+            for (int c = a; c < 4; ++c, ++k) {
+                if ((mre >> k) & 1u) {
+                    const double p = fma(z[a].x, z[c].x, z[a].y * z[c].y);
+#pragma unroll
+                    for (int o = 0; o < NO; ++o) v[o] = fma(sm.obs->c[k][o].x, p, v[o]);
+                }
+                if ((mim >> k) & 1u) {
+                    const double p = fma(z[a].x, z[c].y, -z[a].y * z[c].x);
+#pragma unroll
+                    for (int o = 0; o < NO; ++o) v[o] = fma(-sm.obs->c[k][o].y, p, v[o]);
+                }
             }
-            obs[o] += sum;
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a) st2(x + r[a], v[a]);
     }
-    for (int o = 0; o < S.nobs; ++o) vals[o] = warp_sum(obs[o]) * S.rates[o];
-    nrm = warp_sum(nn);
-    __syncwarp();
+    // all values through the warp together (their shuffles overlap), one barrier
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+        for (int o = 0; o <= NO; ++o) v[o] += __shfl_xor_sync(0xffffffffu, v[o], off);
+    if (lane == 0) {
+#pragma unroll
+        for (int o = 0; o < NO; ++o) sm.rede[9 * warp + o] = v[o];
+        sm.rede[9 * warp + 8] = v[NO];
+    }
+    Team<W>::sync();
+    nrm = sm.rede[8];
+#pragma unroll
+    for (int w = 1; w < W; ++w) nrm += sm.rede[9 * w + 8];
+    val = 0.0;
+    if (static_cast<int>(threadIdx.x) < S.nobs) {
+        for (int w = 0; w < W; ++w) val += sm.rede[9 * w + threadIdx.x];
+        val *= S.rates[threadIdx.x];
+    }
 }
 
-// y = G v (complex128, G = -iH - K) or y = H v (complex64 Lanczos) for the
-// rows owned by this lane; v, y in shared memory.
-template <typename T>
-__device__ __forceinline__ void resident_apply(const ResidentSystem &S, const T *v, T *y, bool lanczos)
+template <typename T, int W>
+__device__ __forceinline__ void resident_epilogue(const ResidentSystem &S, const ResidentSmem<T> &sm, T *x, int flip,
+                                                  double &val, double &nrm)
+{
+    if (S.nobs <= 4) resident_evaluate<T, W, 4>(S, sm, x, flip, val, nrm);
+    else resident_evaluate<T, W, 8>(S, sm, x, flip, val, nrm);
+}
+
+// The Pade form as a call: it is hardly ever taken and large.
+__device__ __noinline__ bool warp_expm_col0_cold(int n, double2 *A, double2 *X, double2 *N, double2 *Dm, double2 *y)
+{
+    return warp_expm_col0(n, A, X, N, Dm, y);
+}
+
+// exp(A) e1 for the n x n matrix A (column-major, n <= 32) in shared memory,
+// by one warp; y in shared memory.  Taylor series on the vector over r equal
+// sub-steps of norm theta <= 2 (the same truncation rule as
+// warp_tridiag_expm_e1): about 20 products with A where the Pade approximant
+// costs 6 to 10 matrix-matrix products and an LU solve (at n = 16: 26 us to
+// under 3 us).  For norms beyond 64 the squarings of the Pade form win, and
+// warp_expm_col0 runs (A, X, N, Dm: n x n each).
+__device__ inline bool warp_expm_e1(int n, double2 *A, double2 *X, double2 *N, double2 *Dm, double2 *y)
 {
     const int lane = threadIdx.x & 31;
-    for (int r = lane; r < S.D; r += 32) {
-        const int kb = __ldg(S.rowptr + r), ke = __ldg(S.rowptr + r + 1);
-        double2 acc = make_double2(0.0, 0.0);
-        if (sizeof(T) == sizeof(double2)) {
-            for (int k = kb; k < ke; ++k) acc = cfma(__ldg(S.val + k), ld2(v + __ldg(S.col + k)), acc);
-        } else {
-            float2 a = make_float2(0.f, 0.f);
-            for (int k = kb; k < ke; ++k) {
-                const float2 h = __ldg(S.valf + k);
-                const double2 xv = ld2(v + __ldg(S.col + k));
-                a = cfmaf(h, make_float2(static_cast<float>(xv.x), static_cast<float>(xv.y)), a);
+    double rs = 0.0;
+    if (lane < n)
+        for (int j = 0; j < n; ++j) rs += sqrt(cabs2(A[lane + j * n]));
+    const double nrm = warp_max(rs);
+    if (__any_sync(0xffffffffu, !isfinite(nrm))) return false;
+    if (__any_sync(0xffffffffu, nrm > 64.0)) return warp_expm_col0_cold(n, A, X, N, Dm, y);
+    const int r = warp_uniform(max(1, static_cast<int>(ceil(nrm * 0.5))));
+    const double theta = nrm / r, inv_r = 1.0 / r;
+    const int K = warp_uniform(taylor_degree(theta));
+    // n <= 16: both half-warps share a row's columns
+    const bool split = n <= 16;
+    const int i = split ? (lane & 15) : lane;
+    const int k0 = split && lane >= 16 ? n / 2 : 0, k1 = split && lane < 16 ? n / 2 : n;
+    const bool live = i < n;
+    double2 yv = make_double2(i == 0 ? 1.0 : 0.0, 0.0);
+    for (int rep = 0; rep < r; ++rep) {
+        double2 term = yv;
+        for (int k = 1; k <= K; ++k) {
+            if (live && (!split || lane < 16)) y[i] = term;
+            __syncwarp();
+            double2 s = make_double2(0.0, 0.0), s2 = make_double2(0.0, 0.0);
+            if (live) {
+                int c = k0;
+#pragma unroll 2
+                for (; c + 1 < k1; c += 2) {
+                    s = cfma(A[i + c * n], y[c], s);
+                    s2 = cfma(A[i + (c + 1) * n], y[c + 1], s2);
+                }
+                if (c < k1) s = cfma(A[i + c * n], y[c], s);
             }
-            acc = make_double2(a.x, a.y);
-        }
-        if (lanczos) {
-            st2(y + r, acc);
-        } else {
-            double2 g = make_double2(acc.y, -acc.x);  // -i * (H v)
-            if (S.krow) {
-                double2 ka = make_double2(0.0, 0.0);
-                for (int k = __ldg(S.krow + r); k < __ldg(S.krow + r + 1); ++k)
-                    ka = cfma(__ldg(S.kval + k), ld2(v + __ldg(S.kcol + k)), ka);
-                g = csub(g, ka);
-            } else {
-                g = csub(g, cscale(ld2(v + r), S.kappa));
+            s = cadd(s, s2);
+            if (split) {
+                s.x += __shfl_xor_sync(0xffffffffu, s.x, 16);
+                s.y += __shfl_xor_sync(0xffffffffu, s.y, 16);
             }
-            st2(y + r, g);
+            term = cscale(s, inv_r * c_taylor.inv[k]);
+            yv = cadd(yv, term);
+            __syncwarp();
         }
     }
+    if (live && (!split || lane < 16)) y[i] = yv;
     __syncwarp();
+    return __all_sync(0xffffffffu, !live || (isfinite(yv.x) && isfinite(yv.y)));
 }
 
-template <typename T>
-__device__ double resident_dot_re(const T *a, const T *b, int D, double2 *cplx)
+// Lanczos factorisation of the state sm.V (= w_0, |w_0|^2 = nrm2): w_j
+// unnormalised in slot j with scale sm.sc[j], alpha and beta in sm.Hm.
+// Returns the Krylov dimension.  Two team barriers per iteration: the one of
+// alpha, and the one of |w_{j+1}|^2, which also publishes w_{j+1} for the next
+// product (hence stored before it is normalised).
+template <typename T, int W, int RPT>
+__device__ __forceinline__ int resident_lanczos(const ResidentSystem &S, const ResidentSmem<T> &sm, const Rows<T, RPT> &H,
+                                                int kmax, double inv0)
 {
-    const int lane = threadIdx.x & 31;
-    double2 s = make_double2(0.0, 0.0);
-    for (int r = lane; r < D; r += 32) s = cadd(s, cconjmul(ld2(a + r), ld2(b + r)));
-    s.x = warp_sum(s.x);
-    s.y = warp_sum(s.y);
-    if (cplx) *cplx = s;
-    return s.x;
+    const int D = S.D, m = S.m, tid = threadIdx.x;
+    constexpr int NT = 32 * W;
+    double2 vc[RPT], vp[RPT], u[RPT];
+    double s = inv0, bprev = 0.0;
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+        vp[i] = u[i] = make_double2(0.0, 0.0);
+        const int r = tid + NT * i;
+        vc[i] = r < D ? cscale(ld2(sm.V + r), s) : make_double2(0.0, 0.0);
+    }
+    if (tid == 0) sm.sc[0] = s;
+    int n = m;
+    for (int j = 0; j < m; ++j) {
+        const T *wj = sm.V + static_cast<size_t>(j) * D;
+        double pa = 0.0;
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            if (tid + NT * i < D) {
+                u[i] = cscale(H.apply(S, i, kmax, wj), s);
+                pa = fma(vc[i].x, u[i].x, fma(vc[i].y, u[i].y, pa));
+            }
+        }
+        const double alpha = Team<W>::sum(pa, sm.red);
+        if (j == m - 1) {  // T_m is complete; w_m is never used
+            if (tid == 0) sm.Hm[j] = make_double2(alpha, 0.0);
+            break;
+        }
+        double pn = 0.0;
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            const int r = tid + NT * i;
+            if (r < D) {
+                double2 w = make_double2(fma(-bprev, vp[i].x, u[i].x), fma(-bprev, vp[i].y, u[i].y));
+                w = make_double2(fma(-alpha, vc[i].x, w.x), fma(-alpha, vc[i].y, w.y));
+                T wr;
+                st2(&wr, w);
+                sm.V[static_cast<size_t>(j + 1) * D + r] = wr;
+                u[i] = ld2(&wr);  // the stored (rounded) vector is the one the norm and the next product see
+                pn += cabs2(u[i]);
+            }
+        }
+        const double nn = Team<W>::sum(pn, sm.red + W);
+        s = rsqrt(nn);
+        const double bn = nn > 0.0 ? nn * s : 0.0;
+        if (tid == 0) {
+            sm.Hm[j] = make_double2(alpha, bn);
+            sm.sc[j + 1] = s;
+        }
+        if (__any_sync(0xffffffffu, bn < 1e-14)) { n = j + 1; break; }
+        bprev = bn;
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            vp[i] = vc[i];
+            vc[i] = cscale(u[i], s);
+        }
+    }
+    return n;
 }
 
-// One launch = the whole time loop for every work item (one warp each).
-template <typename T, bool kLanczos>
-__global__ void k_resident(const ResidentSystem *__restrict__ systems, const ResidentWork *__restrict__ work,
-                           int nwork, size_t warp_bytes, int *__restrict__ status)
+// Below this ratio of |w| after to before orthogonalisation a second
+// Gram-Schmidt pass runs.  One pass leaves w orthogonal to the basis to about
+// rounding / ratio; at 0.3 the basis stays closer to orthonormal than modified
+// Gram-Schmidt keeps it, and few iterations ask for the second pass.
+constexpr double kReorthRatio2 = 0.3 * 0.3;
+
+// Dots of z with the first nv basis vectors (nv <= 32), and |z|^2 when kNorm:
+// a warp takes every W-th row, its lanes one basis vector each (two rows at a
+// time while 16 lanes suffice), so no shuffles; then the warps' sums.  Columns
+// are D + 1 apart, which keeps both this access and a thread's own rows free
+// of bank conflicts.  Lane i < nv of warp 0 returns w_i^H z, lane nv |z|^2.
+template <int W, bool kNorm>
+__device__ __forceinline__ double2 resident_dots(const double2 *V, const double2 *z, int D, int nv, double2 *hp)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wi = blockIdx.x * (blockDim.x >> 5) + warp;
-    if (wi >= nwork) return;
-    const ResidentWork w = work[wi];
-    const ResidentSystem &S = systems[w.sys];
-    const int D = S.D, m = S.m, t = w.traj;
-    unsigned char *base = smem_raw + static_cast<size_t>(warp) * warp_bytes;
-    T *V = reinterpret_cast<T *>(base);               // m x D basis
-    T *z = V + static_cast<size_t>(m) * D;            // work vector / state
-    size_t off = (sizeof(T) * static_cast<size_t>(D) * (m + 1) + 15) / 16 * 16;
-    double2 *Hm = reinterpret_cast<double2 *>(base + off);  // m x m, column-major
-    double2 *A = Hm + static_cast<size_t>(m) * m;
-    double2 *X = A + static_cast<size_t>(m) * m, *N = X + static_cast<size_t>(m) * m;
-    double2 *Dm = N + static_cast<size_t>(m) * m, *y = Dm + static_cast<size_t>(m) * m;
+    const int lane = threadIdx.x & 31, warp = warp_uniform(threadIdx.x >> 5);
+    const int nd = kNorm ? nv + 1 : nv;
+    const bool split = nd <= 16;
+    const int i = split ? (lane & 15) : lane;
+    double2 a = make_double2(0.0, 0.0), b = make_double2(0.0, 0.0);
+    const double2 *vi = i < nv ? V + static_cast<size_t>(i) * (D + 1) : z;  // lanes beyond nv repeat |z|^2
+    const int step = split ? 2 * W : W;
+    int r = split ? 2 * warp + (lane >> 4) : warp;
+#pragma unroll 2
+    for (; r + step < D; r += 2 * step) {
+        a = cconjfma(vi[r], z[r], a);
+        b = cconjfma(vi[r + step], z[r + step], b);
+    }
+    if (r < D) a = cconjfma(vi[r], z[r], a);
+    a = cadd(a, b);
+    if (split) {
+        a.x += __shfl_xor_sync(0xffffffffu, a.x, 16);
+        a.y += __shfl_xor_sync(0xffffffffu, a.y, 16);
+    }
+    if constexpr (W > 1) {
+        if (warp > 0) hp[32 * warp + lane] = a;
+        __syncthreads();
+        if (warp == 0) {
+#pragma unroll
+            for (int w = 1; w < W; ++w) a = cadd(a, hp[32 * w + lane]);
+        }
+    }
+    return a;
+}
 
-    T *col = reinterpret_cast<T *>(S.psi) + static_cast<size_t>(t) * D;
-    for (int r = lane; r < D; r += 32) z[r] = col[r];
-    __syncwarp();
+// Arnoldi factorisation of the state (slot 0 of sm.V) on G = -iH - K: w_j
+// unnormalised in slot j with scale sm.sc[j], H_m in sm.Hm.  Classical
+// Gram-Schmidt: one round of dots per iteration, where modified Gram-Schmidt
+// serialises j + 1 of them; a second pass when the first cancelled
+// (kReorthRatio2).  Returns the Krylov dimension.
+template <int W, int RPT>
+__device__ __forceinline__ int resident_arnoldi(const ResidentSystem &S, const ResidentSmem<double2> &sm,
+                                                const Rows<double2, RPT> &H, int kmax, double inv0)
+{
+    const int D = S.D, m = S.m, tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5);
+    constexpr int NT = 32 * W;
+    const size_t ld = static_cast<size_t>(D) + 1;
+    double2 *V = sm.V, *z = sm.V + static_cast<size_t>(m) * ld, *h = sm.hp;  // h: coefficients of the w_i, then |z|^2
+    double2 u[RPT];
+    double s = inv0;
+    if (tid == 0) sm.sc[0] = s;
+    int n = m;
+    for (int j = 0; j < m; ++j) {
+        const double2 *wj = V + j * ld;
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            const int r = tid + NT * i;
+            if (r >= D) continue;
+            double2 g = H.apply(S, i, kmax, wj);
+            if (!S.generator) {
+                g = make_double2(g.y, -g.x);  // -i (H w)_r
+                if (S.krow) {
+                    double2 ka = make_double2(0.0, 0.0);
+                    for (int k = __ldg(S.krow + r); k < __ldg(S.krow + r + 1); ++k)
+                        ka = cfma(__ldg(S.kval + k), wj[__ldg(S.kcol + k)], ka);
+                    g = csub(g, ka);
+                } else {
+                    g = csub(g, cscale(wj[r], S.kappa));
+                }
+            }
+            u[i] = cscale(g, s);
+            z[r] = u[i];
+        }
+        Team<W>::sync();
+        double nn = 0.0;
+        for (int pass = 0; pass < 2; ++pass) {
+            // the column of H_m is complete after its dots when it is the last
+            const bool last = j == m - 1;
+            const double2 d = pass == 0 && !last ? resident_dots<W, true>(V, z, D, j + 1, sm.hp)
+                                                 : resident_dots<W, false>(V, z, D, j + 1, sm.hp);
+            if (warp == 0) {
+                if (lane <= j) {
+                    const double2 t = cscale(d, sm.sc[lane]);
+                    double2 *hm = sm.Hm + lane + j * m;
+                    *hm = pass ? cadd(*hm, t) : t;
+                    h[lane] = cscale(t, sm.sc[lane]);
+                } else if (lane == j + 1) {
+                    h[lane] = d;
+                }
+            }
+            Team<W>::sync();
+            if (last) break;
+            double pn = 0.0;
+#pragma unroll
+            for (int i = 0; i < RPT; ++i) {
+                const int r = tid + NT * i;
+                if (r >= D) continue;
+                double2 w = u[i], w2 = make_double2(0.0, 0.0);
+                const double2 *col = V + r;
+                int k = 0;
+#pragma unroll 2
+                for (; k < j; k += 2) {
+                    w = cnfma(h[k], col[k * ld], w);
+                    w2 = cnfma(h[k + 1], col[(k + 1) * ld], w2);
+                }
+                if (k <= j) w = cnfma(h[k], col[k * ld], w);
+                u[i] = cadd(w, w2);
+                V[(j + 1) * ld + r] = u[i];
+                if (pass == 0) z[r] = u[i];
+                pn += cabs2(u[i]);
+            }
+            const double before = h[j + 1].x;
+            nn = Team<W>::sum(pn, sm.red + pass * W);
+            if (pass == 0 && !__any_sync(0xffffffffu, nn < kReorthRatio2 * before)) break;
+        }
+        if (j == m - 1) break;
+        s = rsqrt(nn);
+        const double bn = nn > 0.0 ? nn * s : 0.0;
+        if (tid == 0) {
+            sm.Hm[(j + 1) + j * m] = make_double2(bn, 0.0);
+            sm.sc[j + 1] = s;
+        }
+        if (__any_sync(0xffffffffu, bn < 1e-14)) { n = j + 1; break; }
+    }
+    return n;
+}
 
-    double accv[8], compv[8], prevv[8], vals[8];
-    for (int o = 0; o < S.nobs; ++o) {
-        accv[o] = S.accumulate ? S.acc[static_cast<size_t>(o) * S.acc_ld + t] : 0.0;
-        compv[o] = S.accumulate ? S.comp[static_cast<size_t>(o) * S.acc_ld + t] : 0.0;
+// Whole time loop of trajectory t of system S by one CTA of W warps, RPT rows
+// a thread (32 W RPT >= D).  TS: the state's type in memory.
+template <typename T, typename TS, int W, int RPT, bool kLanczos>
+__device__ __forceinline__ void resident_propagate(const ResidentSystem &S, int t, unsigned char *smem,
+                                                   int *__restrict__ status)
+{
+    constexpr int NT = 32 * W;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5);
+    const int D = S.D, m = S.m;
+    const ResidentSmem<T> sm = resident_carve<T, kLanczos>(smem, D, m, W);
+    T *x = sm.V;  // the state
+    const size_t ld = kLanczos ? D : D + 1;
+    const TS *in = static_cast<const TS *>(S.psi) + static_cast<size_t>(t) * S.ts;
+    Rows<T, RPT> H;
+    H.load(S, tid, NT);
+    const int kmax = S.kmax;
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+        const int r = tid + NT * i;
+        if (r < D) st2(x + r, ld2(in + static_cast<size_t>(r) * S.rs));
+    }
+    // observables in upper-triangle form, lane o < 8: observable o
+    if (warp == 0) {
+        unsigned mre = 0, mim = 0;
+        if (lane < 8) {
+            int k = 0;
+            for (int a = 0; a < 4; ++a)
+                for (int c = a; c < 4; ++c, ++k) {
+                    double2 cc = make_double2(0.0, 0.0);
+                    if (lane < S.nobs) {
+                        const double2 p = S.obs[16 * lane + 4 * a + c], q = S.obs[16 * lane + 4 * c + a];
+                        cc = a == c ? make_double2(p.x, 0.0) : make_double2(p.x + q.x, p.y - q.y);
+                    }
+                    sm.obs->c[k][lane] = cc;
+                    if (cc.x != 0.0) mre |= 1u << k;
+                    if (cc.y != 0.0) mim |= 1u << k;
+                }
+        }
+        mre = __reduce_or_sync(0xffffffffu, mre);
+        mim = __reduce_or_sync(0xffffffffu, mim);
+        if (lane == 0) {
+            sm.obs->re = mre;
+            sm.obs->im = mim;
+        }
     }
     const int steps = S.ntimes - 1;
     const long long g0 = S.step_offset;
-    double nrm2 = 0.0;
+    const bool noisy = S.nz.mode != 0;
+    if (tid == 0) sm.flags[0] = noisy && steps > 0 ? noise_bit(S.nz, t, g0, 0, S.pflip[0]) : 0;
+    // thread o < nobs keeps observable o's trapezoid
+    const bool own = tid < S.nobs;
+    const size_t ak = static_cast<size_t>(tid) * S.acc_ld + t;
+    double acc = 0.0, comp = 0.0, prev = 0.0, val = 0.0, nrm2 = 0.0;
+    if (own && S.accumulate) {
+        acc = S.acc[ak];
+        comp = S.comp[ak];
+    }
     bool bad = false;
-    // first time point: evaluate, then the first half-step flip of step 0
-    {
-        const int f = steps > 0 ? noise_bit(S.nz, t, g0, 0, S.pflip[0]) : 0;
-        resident_epilogue(z, S, f, vals, nrm2);
-        for (int o = 0; o < S.nobs; ++o) prevv[o] = vals[o];
-        if (S.traj_values && lane == 0)
-            for (int o = 0; o < S.nobs; ++o) S.traj_values[static_cast<size_t>(t) * S.nobs + o] = vals[o];
-    }
+    Team<W>::sync();
+    resident_epilogue<T, W>(S, sm, x, sm.flags[0], val, nrm2);
+    prev = val;
+    if (S.traj_values && own) S.traj_values[static_cast<size_t>(t) * S.nobs + tid] = val;
+    if (S.check_start && !isfinite(nrm2)) bad = true;
     for (int s = 0; s < steps; ++s) {
-        const double dt = S.times[s + 1] - S.times[s];
-        const double beta0 = sqrt(nrm2);
-        int n = m;
+        const double dt = S.times ? S.times[s + 1] - S.times[s] : S.dt0;
+        const double inv0 = rsqrt(nrm2), beta0 = nrm2 > 0.0 ? nrm2 * inv0 : 0.0;
+        // second half flip of step s and first half flip of step s + 1, by the
+        // last warp while the first one exponentiates
+        auto draw_flip = [&]() {
+            if (warp == W - 1 && lane == 0) {
+                int f = 0;
+                if (noisy) {
+                    f = noise_bit(S.nz, t, g0 + s, 1, S.pflip[s]);
+                    if (s + 1 < steps) f ^= noise_bit(S.nz, t, g0 + s + 1, 0, S.pflip[s + 1]);
+                }
+                sm.flags[0] = f;
+            }
+        };
         if (beta0 > 0.0) {
-            const double inv = 1.0 / beta0;
-            for (int r = lane; r < D; r += 32) st2(V + r, cscale(ld2(z + r), inv));
-            __syncwarp();
-            if (!kLanczos) {
-                // Arnoldi with modified Gram-Schmidt (reference order)
-                for (int j = 0; j < m; ++j) {
-                    resident_apply(S, V + static_cast<size_t>(j) * D, z, false);
-                    for (int i = 0; i <= j; ++i) {
-                        double2 h;
-                        resident_dot_re(V + static_cast<size_t>(i) * D, z, D, &h);
-                        for (int r = lane; r < D; r += 32)
-                            st2(z + r, csub(ld2(z + r), cmul(h, ld2(V + static_cast<size_t>(i) * D + r))));
-                        if (lane == 0) Hm[i + j * m] = h;
+            int n;
+            if constexpr (kLanczos) n = resident_lanczos<T, W, RPT>(S, sm, H, kmax, inv0);
+            else n = resident_arnoldi<W, RPT>(S, sm, H, kmax, inv0);
+            if (warp == 0) {
+                bool ok;
+                double2 c = make_double2(0.0, 0.0);
+                __syncwarp();
+                if constexpr (kLanczos) {
+                    const double d = lane < n ? sm.Hm[lane].x : 0.0;
+                    const double lo = (lane < n && lane > 0) ? sm.Hm[lane - 1].y : 0.0;
+                    const double hi = lane + 1 < n ? sm.Hm[lane].y : 0.0;
+                    bool taylor = true;
+                    if constexpr (sizeof(T) == sizeof(double2))
+                        taylor = !__any_sync(0xffffffffu, fabs(dt) * (fabs(d) + fabs(lo) + fabs(hi)) > 256.0);
+                    if (taylor) {
+                        ok = warp_tridiag_expm_e1(n, d, lo, hi, S.kappa, dt, c);
+                    } else {
+                        // the reference's Pade form on the same matrix
+                        double2 *A = sm.A, *X = A + m * m, *N = X + m * m, *Dm = N + m * m, *y = Dm + m * m;
+                        if (lane < n)
+                            for (int i = 0; i < n; ++i) {
+                                double2 e = make_double2(0.0, 0.0);
+                                if (i == lane) e = make_double2(-S.kappa, -d);
+                                else if (i == lane + 1) e = make_double2(0.0, -hi);
+                                else if (i + 1 == lane) e = make_double2(0.0, -lo);
+                                A[i + lane * n] = cscale(e, dt);
+                            }
                         __syncwarp();
+                        ok = warp_expm_col0_cold(n, A, X, N, Dm, y);
+                        if (lane < n) c = y[lane];
                     }
-                    const double zn = sqrt(resident_dot_re(z, z, D, nullptr));
-                    if (j == m - 1) break;
-                    if (lane == 0) Hm[(j + 1) + j * m] = make_double2(zn, 0.0);
-                    if (zn < 1e-14) { n = j + 1; break; }
-                    const double zi = 1.0 / zn;
-                    for (int r = lane; r < D; r += 32)
-                        st2(V + static_cast<size_t>(j + 1) * D + r, cscale(ld2(z + r), zi));
+                } else {
+                    double2 *A = sm.A, *X = A + m * m, *N = X + m * m, *Dm = N + m * m, *y = Dm + m * m;
+                    // upper Hessenberg part only; entries below the subdiagonal are never written
+                    if (lane < n)
+                        for (int i = 0; i < n; ++i)
+                            A[i + lane * n] = i <= lane + 1 ? cscale(sm.Hm[i + lane * m], dt) : make_double2(0.0, 0.0);
                     __syncwarp();
+                    ok = warp_expm_e1(n, A, X, N, Dm, y);
+                    if (lane < n) c = y[lane];
                 }
-                __syncwarp();
-                // upper Hessenberg part only; entries below the subdiagonal are never written
-                if (lane < n)
-                    for (int i = 0; i < n; ++i)
-                        A[i + lane * n] = i <= lane + 1 ? cscale(Hm[i + lane * m], dt) : make_double2(0.0, 0.0);
-            } else {
-                // Lanczos on H: alpha on Hm[j] .x, beta_{j+1} on Hm[j] .y
-                double bprev = 0.0;
-                for (int j = 0; j < m; ++j) {
-                    T *vj = V + static_cast<size_t>(j) * D;
-                    resident_apply(S, vj, z, true);
-                    const double alpha = resident_dot_re(vj, z, D, nullptr);
-                    for (int r = lane; r < D; r += 32) {
-                        double2 u = csub(ld2(z + r), cscale(ld2(vj + r), alpha));
-                        if (j > 0) u = csub(u, cscale(ld2(vj - D + r), bprev));
-                        st2(z + r, u);
-                    }
-                    __syncwarp();
-                    const double bn = sqrt(resident_dot_re(z, z, D, nullptr));
-                    if (lane == 0) Hm[j] = make_double2(alpha, bn);
-                    if (j == m - 1) break;
-                    if (bn < 1e-14) { n = j + 1; break; }
-                    const double bi = 1.0 / bn;
-                    for (int r = lane; r < D; r += 32) st2(vj + D + r, cscale(ld2(z + r), bi));
-                    bprev = bn;
-                    __syncwarp();
-                }
-                __syncwarp();
+                if (lane < n) c = cscale(c, beta0 * sm.sc[lane]);
+                if (!ok && lane == 0) atomicOr(status, 1);
+                if (lane < n) sm.cf[lane] = ok ? c : make_double2(0.0, 0.0);
             }
-            __syncwarp();
-            bool ok;
-            if (kLanczos) {
-                // tridiagonal: alpha on Hm[i].x, beta_{i+1} on Hm[i].y
-                const double d = lane < n ? Hm[lane].x : 0.0;
-                const double lo = (lane < n && lane > 0) ? Hm[lane - 1].y : 0.0;
-                const double hi = lane + 1 < n ? Hm[lane].y : 0.0;
-                double2 yl;
-                ok = warp_tridiag_expm_e1(n, d, lo, hi, S.kappa, dt, yl);
-                if (lane < n) y[lane] = yl;
-                __syncwarp();
-            } else {
-                ok = warp_expm_col0(n, A, X, N, Dm, y);
+            draw_flip();
+            Team<W>::sync();
+#pragma unroll
+            for (int i = 0; i < RPT; ++i) {
+                const int r = tid + NT * i;
+                if (r >= D) continue;
+                double2 a[4];  // partial sums: the dependent FMA chain, not the loads, sets the time
+#pragma unroll
+                for (int k = 0; k < 4; ++k) a[k] = make_double2(0.0, 0.0);
+                int j = 0;
+                for (; j + 3 < n; j += 4)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) a[k] = cfma(sm.cf[j + k], ld2(sm.V + (j + k) * ld + r), a[k]);
+                for (; j < n; ++j) a[0] = cfma(sm.cf[j], ld2(sm.V + j * ld + r), a[0]);
+                st2(x + r, cadd(cadd(a[0], a[1]), cadd(a[2], a[3])));
             }
-            if (!ok) {
-                if (lane == 0) atomicOr(status, 1);
-                n = 0;
-            }
-            for (int r = lane; r < D; r += 32) {
-                double2 sacc = make_double2(0.0, 0.0);
-                for (int j = 0; j < n; ++j) sacc = cfma(y[j], ld2(V + static_cast<size_t>(j) * D + r), sacc);
-                st2(z + r, cscale(sacc, beta0));
-            }
-            __syncwarp();
+        } else {
+            draw_flip();
         }
-        // second half flip of step s, first half flip of step s+1, evaluation
-        const long long g = g0 + s;
-        int f = noise_bit(S.nz, t, g, 1, S.pflip[s]);
-        if (s + 1 < steps) f ^= noise_bit(S.nz, t, g + 1, 0, S.pflip[s + 1]);
-        resident_epilogue(z, S, f, vals, nrm2);
-        for (int o = 0; o < S.nobs; ++o) {
-            const double term = 0.5 * dt * (prevv[o] + vals[o]) - compv[o];
-            const double sum = accv[o] + term;
-            compv[o] = (sum - accv[o]) - term;
-            accv[o] = sum;
-            prevv[o] = vals[o];
-            if (!isfinite(vals[o])) bad = true;
+        Team<W>::sync();
+        resident_epilogue<T, W>(S, sm, x, sm.flags[0], val, nrm2);
+        if (own) {
+            const double term = 0.5 * dt * (prev + val) - comp;
+            const double sum = acc + term;
+            comp = (sum - acc) - term;
+            acc = sum;
+            prev = val;
+            if (!isfinite(val)) bad = true;
+            if (S.traj_values) S.traj_values[(static_cast<size_t>(s + 1) * S.M + t) * S.nobs + tid] = val;
         }
-        if (S.traj_values && lane == 0)
-            for (int o = 0; o < S.nobs; ++o)
-                S.traj_values[(static_cast<size_t>(s + 1) * S.M + t) * S.nobs + o] = vals[o];
     }
-    for (int r = lane; r < D; r += 32) col[r] = z[r];
-    if (lane == 0) {
-        for (int o = 0; o < S.nobs; ++o) {
-            S.acc[static_cast<size_t>(o) * S.acc_ld + t] = accv[o];
-            S.comp[static_cast<size_t>(o) * S.acc_ld + t] = compv[o];
-            S.prev[static_cast<size_t>(o) * S.acc_ld + t] = prevv[o];
-        }
-        if (bad) atomicOr(status, 2);
+    TS *out = static_cast<TS *>(S.psi_out) + static_cast<size_t>(t) * S.ts;
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+        const int r = tid + NT * i;
+        if (r < D) st2(out + static_cast<size_t>(r) * S.rs, ld2(x + r));
     }
+    if (own) {
+        S.acc[ak] = acc;
+        S.comp[ak] = comp;
+        S.prev[ak] = prev;
+    }
+    if (bad) atomicOr(status, 2);
 }
 
-// values[s][o] = sum over trajectories of traj_values[s][t][o] (fixed order);
-// one block per time point.
-__global__ void k_resident_values(const double *__restrict__ traj_values, int M, int nobs, double *__restrict__ values)
+// CTAs per SM the register allocation must allow.  complex64 keeps 16 warps on
+// an SM (128 registers a thread): with 133 registers a scheduler holds three
+// warps, not four, and 1024 trajectories of D = 64 took 27 instead of 18 us a
+// step.
+template <typename T>
+constexpr int resident_min_ctas(int W) { return sizeof(T) == sizeof(float2) && W <= 16 ? 16 / W : 1; }
+
+// One launch = the whole time loop of every trajectory (one CTA each).
+template <typename T, int W, int RPT, bool kLanczos>
+__global__ void __launch_bounds__(32 * W, resident_min_ctas<T>(W))
+k_resident(const __grid_constant__ ResidentSystem S, int *__restrict__ status)
 {
-    __shared__ double red[8][32];
-    const int s = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int t = threadIdx.x; t < M; t += blockDim.x)
-        for (int o = 0; o < nobs; ++o) acc[o] += traj_values[(static_cast<size_t>(s) * M + t) * nobs + o];
-    for (int o = 0; o < nobs; ++o) {
-        const double v = warp_sum(acc[o]);
-        if (lane == 0) red[o][warp] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < nobs) {
-        double v = 0.0;
-        for (int w = 0; w < (blockDim.x >> 5); ++w) v += red[threadIdx.x][w];
-        values[static_cast<size_t>(s) * nobs + threadIdx.x] = v;
-    }
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    resident_propagate<T, double2, W, RPT, kLanczos>(S, blockIdx.x, smem_raw, status);
 }
 
 }  // namespace
