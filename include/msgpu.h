@@ -117,7 +117,7 @@ extern "C" {
                                         Same results to FP32 rounding; at D=16384 with 1024
                                         trajectories on a B200 it is the slower of the two
                                         (latency-bound at one 512-thread CTA per SM) */
-#define MSGPU_OPT_TRAJ_GROUPS 5       /* complex64 streamed form: 0 (default) splits a block of
+#define MSGPU_OPT_TRAJ_GROUPS 5       /* streamed three-term recurrence: 0 (default) splits a block of
                                         512 or more trajectories into 2 groups whose step
                                         sequences run on two streams, so that one group's SpMM
                                         (held by the SM's load pipe) overlaps the other's

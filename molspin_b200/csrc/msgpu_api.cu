@@ -51,6 +51,8 @@ struct msgpu_ctx {
     int D = 0, nnz = 0;
     DevBuf hrow, hcol, hval, hhi;
     int max_row = 0;   // most entries of a row of H
+    double h_norm1 = 0.0;            // largest absolute row sum of H (of one term)
+    std::vector<double> term_norm1;  // the same of each term (msgpu_upload_hamiltonian_terms)
     int hermitian = -1;  // H (every term of it) equals its conjugate transpose: 1, 0, or -1 (not yet checked)
     DevBuf ell;        // resident form: H in padded column-major order, values then columns
     std::vector<int> h_rowptr, h_col;  // host copy for the quartet-block form
@@ -272,7 +274,7 @@ void collect_profile(msgpu_ctx *c)
 
 inline int ceil_div(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
 
-// Trajectory groups of the complex64 streamed step (MSGPU_OPT_TRAJ_GROUPS).
+// Trajectory groups of the streamed three-term step (MSGPU_OPT_TRAJ_GROUPS).
 // Each group is a multiple of 128 trajectories, the width of the widest SpMM
 // variant's CTA; auto takes two groups from 512 trajectories up.
 int traj_groups(const msgpu_ctx *c)
@@ -291,6 +293,27 @@ int pick_rows_per_tile(int D)
     R = std::max(8, std::min(512, R));
     R = (R + 7) / 8 * 8;
     return R;
+}
+
+// largest absolute row sum of a CSR matrix (interleaved complex values)
+double row_sum_norm(int dim, const int *rowptr, const double *val)
+{
+    double mx = 0.0;
+    for (int r = 0; r < dim; ++r) {
+        double s = 0.0;
+        for (int k = rowptr[r]; k < rowptr[r + 1]; ++k)
+            s += std::abs(val[2 * static_cast<size_t>(k)]) + std::abs(val[2 * static_cast<size_t>(k) + 1]);
+        mx = std::max(mx, s);
+    }
+    return mx;
+}
+
+// Quartets per CTA of k_lanczos_apply_d: 16, or 8 while 16 leaves under 8 CTAs
+// an SM (D = 16384, us per launch: 512 trajectories 176 with 8 or 16, 185 with
+// 32, 223 with 64).
+int quartet_tile_d(int Q, int width)
+{
+    return static_cast<long long>(Q) / 16 * (width / 32) >= 8 * 148 ? 16 : 8;
 }
 
 PairObs make_pair_obs(const msgpu_ctx *c)
@@ -483,6 +506,7 @@ int msgpu_upload_hamiltonian_csr(msgpu_ctx *c, int dim, const int *rowptr, const
     c->q_D = 0;  // quartet form must be rebuilt
     c->max_row = 0;
     for (int r = 0; r < dim; ++r) c->max_row = std::max(c->max_row, rowptr[r + 1] - rowptr[r]);
+    c->h_norm1 = row_sum_norm(dim, rowptr, val);
     c->hermitian = -1;
     c->terms = false;
     c->dense.have_u = false;  // a cached dense propagator belongs to the old H
@@ -1901,6 +1925,9 @@ int msgpu_upload_hamiltonian_terms(msgpu_ctx *c, int dim, const int *rowptr, con
         return cuda_fail(c, e, "Hamiltonian terms upload");
     c->terms = true;
     c->nterms = nterms;
+    c->term_norm1.clear();
+    for (int t = 0; t < nterms; ++t)
+        c->term_norm1.push_back(row_sum_norm(dim, rowptr, vals + 2 * static_cast<size_t>(t) * nnz));
     c->hermitian = 1;
     for (int t = 0; t < nterms && c->hermitian == 1; ++t)
         c->hermitian = is_hermitian(dim, rowptr, col, vals + 2 * static_cast<size_t>(t) * nnz);
@@ -2156,7 +2183,7 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
         const long long sB = -1;
         if (prec == MSGPU_PREC_C128)
             k_combine<double2, false><<<qgrid, qblock, 0, st>>>(
-                static_cast<double2 *>(c->psi128.p), nullptr, 0, nullptr, nullptr, mws, c->s1, c->s2, Q, ldm, QR, nz,
+                static_cast<double2 *>(c->psi128.p), nullptr, nullptr, 0, nullptr, nullptr, mws, c->s1, c->s2, Q, ldm, QR, nz,
                 steps > 0 ? g0 : -1, 0, pstep(0), sB, 0, 0.0, po, static_cast<double *>(c->qpart_obs.p),
                 static_cast<double *>(c->qpart_nrm.p));
         else
@@ -2170,6 +2197,7 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
     const bool arn64 = prec == MSGPU_PREC_C64 && rec == MSGPU_REC_ARNOLDI;
     // the complex128 Arnoldi apply runs over quartet blocks when K = kappa I
     const bool quartet128 = prec == MSGPU_PREC_C128 && !taylor && !rk4 && c->k_scalar;
+    const bool three_term = quartet128 && lanczos128(c, p);
     if (quartet128)
         if (int rc = build_quartet(c)) return rc;
     if (prec == MSGPU_PREC_C64) {
@@ -2226,6 +2254,35 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
         taylor_shift(hs);
         if (!std::isfinite(tnorm)) return fail(c, MSGPU_ERR_NONFINITE, "run: non-finite Hamiltonian norm");
     }
+    // Trajectory groups: the step's kernels work on columns [t0, t0 + width)
+    // through offset pointers with the row stride ldm, so the groups share the
+    // buffers.  With overlap each group has its own stream (group 0 the
+    // context's) and one group's SpMM runs beside another's update and combine;
+    // profiled steps run the groups back to back so that each launch is timed
+    // alone.
+    auto for_groups = [&](int G, auto body) -> int {
+        const int width = ldm / G;
+        const bool timed_step = c->prof == 1 || (c->prof == 2 && c->prof_tick % kProfileEvery == 0);
+        const bool overlap = G > 1 && !timed_step;
+        const int nside = overlap ? G - 1 : 0;
+        cudaError_t ge;
+        if (overlap) {
+            if (!c->gfork && (ge = cudaEventCreateWithFlags(&c->gfork, cudaEventDisableTiming)))
+                return cuda_fail(c, ge, "trajectory group stream");
+            for (int k = 0; k < nside; ++k)
+                if (!c->gside[k] && ((ge = cudaStreamCreateWithFlags(&c->gside[k], cudaStreamNonBlocking)) ||
+                                     (ge = cudaEventCreateWithFlags(&c->gjoin[k], cudaEventDisableTiming))))
+                    return cuda_fail(c, ge, "trajectory group stream");
+            if ((ge = cudaEventRecord(c->gfork, st))) return cuda_fail(c, ge, "trajectory group fork");
+            for (int k = 0; k < nside; ++k)
+                if ((ge = cudaStreamWaitEvent(c->gside[k], c->gfork, 0))) return cuda_fail(c, ge, "trajectory group fork");
+        }
+        for (int gi = 0; gi < G; ++gi) body(gi * width, width, overlap && gi > 0 ? c->gside[gi - 1] : st);
+        for (int k = 0; k < nside; ++k)
+            if ((ge = cudaEventRecord(c->gjoin[k], c->gside[k])) || (ge = cudaStreamWaitEvent(st, c->gjoin[k], 0)))
+                return cuda_fail(c, ge, "trajectory group join");
+        return MSGPU_OK;
+    };
     for (int s = 0; s < steps; ++s) {
         c->prof_tick = s;
         const double dt = p->times[s + 1] - p->times[s];
@@ -2281,7 +2338,7 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
             {
                 Timed tm(c, KC_COMBINE);
                 k_combine<double2, false><<<qgrid, qblock, 0, st>>>(
-                    F, nullptr, 0, nullptr, nullptr, mws, c->s1, c->s2, Q, ldm, QR, nz, g, 1, pstep(s),
+                    F, nullptr, nullptr, 0, nullptr, nullptr, mws, c->s1, c->s2, Q, ldm, QR, nz, g, 1, pstep(s),
                     s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po, static_cast<double *>(c->qpart_obs.p),
                     static_cast<double *>(c->qpart_nrm.p));
             }
@@ -2314,10 +2371,81 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
             {
                 Timed tm(c, KC_COMBINE);
                 k_combine<double2, false><<<qgrid, qblock, 0, st>>>(
-                    psi, nullptr, 0, nullptr, nullptr, mws, c->s1, c->s2, Q, ldm, QR, nz, g, 1, pstep(s),
+                    psi, nullptr, nullptr, 0, nullptr, nullptr, mws, c->s1, c->s2, Q, ldm, QR, nz, g, 1, pstep(s),
                     s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po, static_cast<double *>(c->qpart_obs.p),
                     static_cast<double *>(c->qpart_nrm.p));
             }
+        } else if (three_term) {
+            // slot 0 of the basis is the state itself, w_j (j >= 1) at basis + (j - 1) n
+            double2 *psi = static_cast<double2 *>(c->psi128.p), *Wb = static_cast<double2 *>(c->basis.p);
+            double2 *U = static_cast<double2 *>(c->wbuf.p);
+            double *part = static_cast<double *>(c->part.p), *alpha = static_cast<double *>(c->part2.p);
+            double *td = static_cast<double *>(c->hess.p), *to = td + static_cast<size_t>(ldm) * mws;
+            int *mdim = static_cast<int *>(c->mdim.p);
+            double2 *coef = static_cast<double2 *>(c->coef.p);
+            auto slot = [&](int j) { return j == 0 ? psi : Wb + static_cast<size_t>(j - 1) * n; };
+            const QuartetD Hq{static_cast<const int *>(c->qrow.p), static_cast<const int2 *>(c->qcolt.p),
+                              static_cast<const double2 *>(c->qval64.p), static_cast<const int *>(c->qbase.p)};
+            // dt |T| is below dt |H|: past 128 the squarings of the Pade form take
+            // fewer steps than the sub-steps of the Taylor series
+            double hn = c->h_norm1;
+            if (c->terms) {
+                hn = 0.0;
+                const double *row = c->sched_steps ? sched_row(c, g, 1) : c->hcoef.data();
+                for (int k = 0; k < c->nterms; ++k) hn += std::abs(row[k]) * c->term_norm1[k];
+            }
+            const int rc = for_groups(traj_groups(c), [&](int t0, int width, cudaStream_t gs) {
+                const size_t tm0 = static_cast<size_t>(t0) * mws;  // offset into the [t][m] T arrays
+                const int QT = quartet_tile_d(Q, width), nqt = ceil_div(Q, QT);
+                for (int j = 0; j < m; ++j) {
+                    const double *sj = sc + static_cast<size_t>(j) * ldm + t0;
+                    {
+                        Timed tm(c, KC_APPLY, gs);
+                        k_lanczos_apply_d<<<dim3(nqt, width / 32), kThreads, 0, gs>>>(Hq, slot(j) + t0, sj, U + t0, part + t0, Q,
+                                                                                      c->s1, c->s2, ldm, QT);
+                    }
+                    {
+                        Timed tm(c, KC_REDUCE, gs);
+                        k_lanczos_reduce<<<width / 32, dim3(32, kRedRows), 0, gs>>>(part + t0, nqt, ldm, 0, j, mws, alpha + t0,
+                                                                                    td + tm0, to + tm0, mdim + t0);
+                    }
+                    if (j == m - 1) break;  // T_m is complete; w_m is never used
+                    {
+                        Timed tm(c, KC_ORTH, gs);
+                        k_lanczos_update_d<<<dim3(nt, width / 32), kThreads, 0, gs>>>(
+                            U + t0, slot(j) + t0, j > 0 ? slot(j - 1) + t0 : nullptr, sj, j > 0 ? sj - ldm : nullptr, alpha + t0,
+                            slot(j + 1) + t0, part + t0, D, ldm, R);
+                    }
+                    {
+                        Timed tm(c, KC_REDUCE, gs);
+                        k_lanczos_reduce<<<width / 32, dim3(32, kRedRows), 0, gs>>>(
+                            part + t0, nt, ldm, 1, j, mws, sc + static_cast<size_t>(j + 1) * ldm + t0, td + tm0, to + tm0,
+                            mdim + t0);
+                    }
+                }
+                {
+                    Timed tm(c, KC_EXPM, gs);
+                    const int live = std::max(0, std::min(M - t0, width));
+                    int *status = static_cast<int *>(c->status.p);
+                    if (dt * hn <= 128.0)
+                        k_lanczos_expm<<<ceil_div(width, 8), 256, 0, gs>>>(td + tm0, to + tm0, kappa, mdim + t0, beta0 + t0,
+                                                                           sc + t0, mws, ldm, live, dt, coef + t0, status, width);
+                    else
+                        k_krylov_expm<<<ceil_div(width, expm_warps), 32 * expm_warps, expm_warps * expm_smem_warp, gs>>>(
+                            nullptr, td + tm0, to + tm0, kappa, mdim + t0, beta0 + t0, sc + t0, mws, ldm, live, dt, coef + t0,
+                            status, width);
+                }
+                {
+                    Timed tm(c, KC_COMBINE, gs);
+                    Noise gnz = nz;
+                    gnz.traj_offset = static_cast<uint32_t>(t0);
+                    k_combine<double2, true><<<dim3(qt, width / 32), qblock, 0, gs>>>(
+                        psi + t0, psi + t0, Wb + t0, n, coef + t0, mdim + t0, mws, c->s1, c->s2, Q, ldm, QR, gnz, g, 1, pstep(s),
+                        s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po, static_cast<double *>(c->qpart_obs.p) + t0,
+                        static_cast<double *>(c->qpart_nrm.p) + t0);
+                }
+            });
+            if (rc) return rc;
         } else if (prec == MSGPU_PREC_C128) {
             double2 *V = static_cast<double2 *>(c->basis.p);
             double2 *bufA = static_cast<double2 *>(c->wbuf.p), *bufB = static_cast<double2 *>(c->zbuf.p);
@@ -2373,12 +2501,12 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                 Timed tm(c, KC_EXPM);
                 k_krylov_expm<<<ceil_div(ldm, expm_warps), 32 * expm_warps, expm_warps * expm_smem_warp, st>>>(
                     static_cast<double2 *>(c->hess.p), nullptr, nullptr, 0.0, static_cast<int *>(c->mdim.p), beta0,
-                    nullptr, mws, ldm, M, dt, static_cast<double2 *>(c->coef.p), static_cast<int *>(c->status.p));
+                    nullptr, mws, ldm, M, dt, static_cast<double2 *>(c->coef.p), static_cast<int *>(c->status.p), ldm);
             }
             {
                 Timed tm(c, KC_COMBINE);
                 k_combine<double2, true><<<qgrid, qblock, 0, st>>>(
-                    static_cast<double2 *>(c->psi128.p), V, n, static_cast<double2 *>(c->coef.p),
+                    static_cast<double2 *>(c->psi128.p), V, V + n, n, static_cast<double2 *>(c->coef.p),
                     static_cast<int *>(c->mdim.p), mws, c->s1, c->s2, Q, ldm, QR, nz, g, 1, pstep(s),
                     s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po, static_cast<double *>(c->qpart_obs.p),
                     static_cast<double *>(c->qpart_nrm.p));
@@ -2419,7 +2547,7 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                 Timed tm(c, KC_EXPM);
                 k_krylov_expm<<<ceil_div(ldm, expm_warps), 32 * expm_warps, expm_warps * expm_smem_warp, st>>>(
                     static_cast<double2 *>(c->hess.p), nullptr, nullptr, 0.0, static_cast<int *>(c->mdim.p), beta0, sc,
-                    mws, ldm, M, dt, static_cast<double2 *>(c->coef.p), static_cast<int *>(c->status.p));
+                    mws, ldm, M, dt, static_cast<double2 *>(c->coef.p), static_cast<int *>(c->status.p), ldm);
             }
             {
                 Timed tm(c, KC_COMBINE);
@@ -2442,31 +2570,8 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                 Timed tm(c, KC_LANCZOS);
                 if (int rc = launch_fused(c, fused_c, Wb, n, sc, td, to, mdim, m)) return rc;
             }
-            // Trajectory groups: every kernel below works on columns [t0, t0 + width)
-            // through offset pointers with the row stride ldm, so the groups share
-            // the buffers. With overlap, odd groups run on the second stream and
-            // one group's SpMM runs beside another's update and combine; profiled
-            // steps run the groups back to back so that each launch is timed alone.
-            const int G = fused_c ? 1 : traj_groups(c), width = ldm / G;
-            const bool timed_step = c->prof == 1 || (c->prof == 2 && c->prof_tick % kProfileEvery == 0);
-            const bool overlap = G > 1 && !timed_step;
-            // each group on its own stream (group 0 on the context stream)
-            const int nside = overlap ? G - 1 : 0;
-            if (overlap) {
-                if (!c->gfork && (e = cudaEventCreateWithFlags(&c->gfork, cudaEventDisableTiming)))
-                    return cuda_fail(c, e, "trajectory group stream");
-                for (int k = 0; k < nside; ++k)
-                    if (!c->gside[k] && ((e = cudaStreamCreateWithFlags(&c->gside[k], cudaStreamNonBlocking)) ||
-                                         (e = cudaEventCreateWithFlags(&c->gjoin[k], cudaEventDisableTiming))))
-                        return cuda_fail(c, e, "trajectory group stream");
-                if ((e = cudaEventRecord(c->gfork, st))) return cuda_fail(c, e, "trajectory group fork");
-                for (int k = 0; k < nside; ++k)
-                    if ((e = cudaStreamWaitEvent(c->gside[k], c->gfork, 0))) return cuda_fail(c, e, "trajectory group fork");
-            }
-            for (int gi = 0; gi < G; ++gi) {
-                const int t0 = gi * width;
+            const int rc = for_groups(fused_c ? 1 : traj_groups(c), [&](int t0, int width, cudaStream_t gs) {
                 const size_t tm0 = static_cast<size_t>(t0) * mws;  // offset into the [t][m] T arrays
-                cudaStream_t gs = (overlap && gi > 0) ? c->gside[gi - 1] : st;
                 dim3 grid(nt, width / 64);
                 for (int j = 0; j < (fused_c ? 0 : m); ++j) {
                     {
@@ -2498,7 +2603,7 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                     Timed tm(c, KC_EXPM, gs);
                     k_lanczos_expm<<<ceil_div(width, 8), 256, 0, gs>>>(
                         td + tm0, to + tm0, kappa, mdim + t0, beta0 + t0, sc + t0, mws, ldm,
-                        std::max(0, std::min(M - t0, width)), dt, coef + t0, static_cast<int *>(c->status.p));
+                        std::max(0, std::min(M - t0, width)), dt, coef + t0, static_cast<int *>(c->status.p), width);
                 }
                 {
                     Timed tm(c, KC_COMBINE, gs);
@@ -2508,10 +2613,8 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                         Wb + t0, Wb + t0, n, coef + t0, mdim + t0, c->s1, c->s2, Q, ldm, QR, gnz, g, 1, pstep(s),
                         s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po, qobs + t0, qnrm + t0);
                 }
-            }
-            for (int k = 0; k < nside; ++k)
-                if ((e = cudaEventRecord(c->gjoin[k], c->gside[k])) || (e = cudaStreamWaitEvent(st, c->gjoin[k], 0)))
-                    return cuda_fail(c, e, "trajectory group join");
+            });
+            if (rc) return rc;
         }
         yield_update(dt, 0, s + 1);
         if ((e = cudaGetLastError())) return cuda_fail(c, e, "step launch");
@@ -2774,7 +2877,7 @@ extern "C" int msgpu_krylov_step_noalloc(int dim, const int *rowptr, const int *
     // any two spin-1/2 digit strides partition the rows into quartets; without
     // observables or flips only the norms are read from the quartet pass
     const int s1 = D / 2, s2 = D / 4;
-    k_combine<double2, false><<<qgrid, qblock, 0, st>>>(psi, nullptr, 0, nullptr, nullptr, m, s1, s2, Q, ldm, QR, nz,
+    k_combine<double2, false><<<qgrid, qblock, 0, st>>>(psi, nullptr, nullptr, 0, nullptr, nullptr, m, s1, s2, Q, ldm, QR, nz,
                                                         -1, 0, 0.0, -1, 0, 0.0, po, qobs, qnrm);
     k_yield_update<<<1, 1024, 0, st>>>(qobs, qnrm, qt, 0, ldm, ntraj, nullptr, 0.0, 1, nullptr, nullptr, nullptr,
                                        beta0, sc, nullptr, status);
@@ -2801,8 +2904,8 @@ extern "C" int msgpu_krylov_step_noalloc(int dim, const int *rowptr, const int *
     if (raise_smem_limit(reinterpret_cast<const void *>(k_krylov_expm), static_cast<int>(warps * smem_warp)) != cudaSuccess)
         return MSGPU_ERR_CUDA;
     k_krylov_expm<<<ceil_div(ldm, warps), 32 * warps, warps * smem_warp, st>>>(hess, nullptr, nullptr, 0.0, mdim, beta0,
-                                                                              nullptr, m, ldm, ntraj, dt, coef, status);
-    k_combine<double2, true><<<qgrid, qblock, 0, st>>>(psi, V, n, coef, mdim, m, s1, s2, Q, ldm, QR, nz, -1, 0, 0.0,
+                                                                              nullptr, m, ldm, ntraj, dt, coef, status, ldm);
+    k_combine<double2, true><<<qgrid, qblock, 0, st>>>(psi, V, V + n, n, coef, mdim, m, s1, s2, Q, ldm, QR, nz, -1, 0, 0.0,
                                                        -1, 0, 0.0, po, qobs, qnrm);
     {
         dim3 g(ceil_div(D, 32), ldm / 32), b(32, 8);

@@ -212,6 +212,105 @@ k_arnoldi_apply_q(QuartetD H, double kappa, const double2 *__restrict__ src, con
     }
 }
 
+// Three-term recurrence for a Hermitian H with K = kappa I, complex128: the
+// Arnoldi matrix of G = -iH - kappa I is then -iT - kappa I with T real
+// tridiagonal, so an iteration reads three vectors where Gram-Schmidt reads
+// the basis three times.  w_j unnormalised with scale s_j = 1 / |w_j|, as in
+// the complex64 form.  D = 16384, 512 trajectories, m = 20: 5.4 ms a time step
+// in two groups, against 22.2 ms for CGS2 over the whole basis.
+//
+// U = s_j H w_j over quartet blocks, and the tile's partial alpha_j = <v_j, U>.
+// Grid (ceil(Q / QT), width / 32): a warp per output quartet, a lane per
+// trajectory.
+// Bound by the gathers (13 quartet rows per output quartet at D = 16384, L2 to
+// L1) and FP64 issue, about 60 us each per launch of 512 trajectories; measured
+// 176 us, 1.5 TB/s.  Four CTAs an SM (64 registers) beat loading a block ahead
+// at three (214 us) or two (240 us): more warps in flight hide more than more
+// loads per warp do.
+__global__ void __launch_bounds__(kThreads, 4)
+k_lanczos_apply_d(QuartetD H, const double2 *__restrict__ wj, const double *__restrict__ sj, double2 *__restrict__ U,
+                  double *__restrict__ part, int Q, int s1, int s2, int ldm, int QT)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t = blockIdx.y * 32 + lane;
+    const int q0 = blockIdx.x * QT;
+    const double sc = sj[t];
+    const int off[4] = {0, s2, s1, s1 + s2};
+    double alpha = 0.0;
+    for (int q = q0 + warp; q < min(q0 + QT, Q); q += kWarps) {
+        double2 o[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) o[a] = make_double2(0.0, 0.0);
+        double2 x[4];
+        int last = -1;
+        const int kb = __ldg(H.rowptr + q), ke = __ldg(H.rowptr + q + 1);
+        for (int kk = kb; kk < ke; ++kk) {
+            const int2 cur = __ldg(H.blk + kk);
+            last = cur.x >> 3;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) x[b] = wj[static_cast<size_t>(last + off[b]) * ldm + t];
+            quartet_block_d(o, cur.x & 7, H.val + 2 * static_cast<size_t>(cur.y), x);
+        }
+        // the quartet's own block comes last: its gathered rows are w_j here
+        const int base = __ldg(H.base + q);
+        const bool own = last == base;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const size_t e = static_cast<size_t>(base + off[a]) * ldm + t;
+            const double2 v = own ? x[a] : wj[e];
+            const double2 u = cscale(o[a], sc);
+            U[e] = u;
+            alpha = fma(v.x, u.x, fma(v.y, u.y, alpha));
+        }
+    }
+    __shared__ double sm[kWarps][32];
+    sm[warp][lane] = alpha * sc;
+    __syncthreads();
+    if (warp == 0) {
+        double s = sm[0][lane];
+#pragma unroll
+        for (int w = 1; w < kWarps; ++w) s += sm[w][lane];
+        part[static_cast<size_t>(blockIdx.x) * ldm + t] = s;
+    }
+}
+
+// w_{j+1} = U - alpha_j v_j - beta_j v_{j-1}; partial |w_{j+1}|^2.  Grid
+// (row tiles, width / 32).
+__global__ void __launch_bounds__(kThreads)
+k_lanczos_update_d(const double2 *__restrict__ U, const double2 *__restrict__ wj, const double2 *__restrict__ wjm1,
+                   const double *__restrict__ sj, const double *__restrict__ sjm1, const double *__restrict__ alpha,
+                   double2 *__restrict__ wn, double *__restrict__ part, int D, int ldm, int R)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t = blockIdx.y * 32 + lane;
+    const int r0 = blockIdx.x * R;
+    // alpha s_j and beta_j s_{j-1} where beta_j = 1 / s_j
+    const double ca = alpha[t] * sj[t];
+    const double cb = wjm1 && sj[t] > 0.0 ? sjm1[t] / sj[t] : 0.0;
+    double n = 0.0;
+#pragma unroll 2
+    for (int r = r0 + warp; r < min(r0 + R, D); r += kWarps) {
+        const size_t e = static_cast<size_t>(r) * ldm + t;
+        const double2 u = U[e], v = wj[e];
+        double2 o = make_double2(fma(-ca, v.x, u.x), fma(-ca, v.y, u.y));
+        if (wjm1) {
+            const double2 p = wjm1[e];
+            o = make_double2(fma(-cb, p.x, o.x), fma(-cb, p.y, o.y));
+        }
+        wn[e] = o;
+        n = fma(o.x, o.x, fma(o.y, o.y, n));
+    }
+    __shared__ double sm[kWarps][32];
+    sm[warp][lane] = n;
+    __syncthreads();
+    if (warp == 0) {
+        double s = sm[0][lane];
+#pragma unroll
+        for (int w = 1; w < kWarps; ++w) s += sm[w][lane];
+        part[static_cast<size_t>(blockIdx.x) * ldm + t] = s;
+    }
+}
+
 // Partial dots <V_i, W>, i <= j (the first Gram-Schmidt pass; W unchanged,
 // h unused).  Each V_i is used once and the compiler keeps every load of a
 // row in flight; two CTAs per SM bound its registers.
@@ -1023,12 +1122,13 @@ k_lanczos_reduce(const double *__restrict__ part, int ntiles, int ldm, int mode,
 __global__ void k_krylov_expm(const double2 *__restrict__ hess, const double *__restrict__ tdiag,
                               const double *__restrict__ toff, double kappa, const int *__restrict__ mdim,
                               const double *__restrict__ beta0, const double *__restrict__ vscale, int m,
-                              int ldm, int M, double dt, double2 *__restrict__ coef, int *__restrict__ status)
+                              int ldm, int M, double dt, double2 *__restrict__ coef, int *__restrict__ status,
+                              int width)
 {
     extern __shared__ double2 smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + warp;
-    if (t >= ldm) return;
+    if (t >= width) return;  // width: trajectories of this launch
     double2 *A = smem + static_cast<size_t>(warp) * (4 * m * m + m);
     double2 *X = A + m * m, *N = X + m * m, *Dm = N + m * m, *y = Dm + m * m;
     const int n = max(1, mdim[t]);
@@ -1185,11 +1285,11 @@ __global__ void __launch_bounds__(256) k_g_stats(CsrD H, int D, double *__restri
 __global__ void __launch_bounds__(256)
 k_lanczos_expm(const double *__restrict__ tdiag, const double *__restrict__ toff, double kappa,
                const int *__restrict__ mdim, const double *__restrict__ beta0, const double *__restrict__ vscale,
-               int m, int ldm, int M, double dt, double2 *__restrict__ coef, int *__restrict__ status)
+               int m, int ldm, int M, double dt, double2 *__restrict__ coef, int *__restrict__ status, int width)
 {
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (t >= ldm) return;  // whole warps leave together
+    if (t >= width) return;  // whole warps leave together
     const int n = max(1, mdim[t]);
     const double b0 = beta0[t];
     const bool live = lane < n;
@@ -1258,11 +1358,12 @@ __device__ __forceinline__ void quartet_epilogue(double2 x[4], int flip, const P
 
 // psi = sum_{j<n_t} coef[t][j] V_j at the four rows of each quartet, then the
 // combined flip of this half step pair, observables and norm partials.
-// kBasis=false evaluates psi itself (start of a run: flip of the first half
-// step only, no Krylov combination).
+// V_0 is at V0 (may be psi itself: a thread reads its elements before it
+// writes them), V_j at V + (j - 1) vstride.  kBasis=false evaluates psi itself
+// (start of a run: flip of the first half step only, no Krylov combination).
 template <typename T, bool kBasis>
 __global__ void __launch_bounds__(256)
-k_combine(T *__restrict__ psi, const T *__restrict__ V, size_t vstride, const double2 *__restrict__ coef,
+k_combine(T *psi, const T *V0, const T *__restrict__ V, size_t vstride, const double2 *__restrict__ coef,
           const int *__restrict__ mdim, int m, int s1, int s2, int Q, int ldm, int QR, Noise nz, long long stepA,
           int halfA, double pA, long long stepB, int halfB, double pB, PairObs po, double *__restrict__ part_obs,
           double *__restrict__ part_nrm)
@@ -1286,11 +1387,19 @@ k_combine(T *__restrict__ psi, const T *__restrict__ V, size_t vstride, const do
         if (kBasis) {
 #pragma unroll
             for (int a = 0; a < 4; ++a) x[a] = make_double2(0.0, 0.0);
-            for (int jj = 0; jj < n; ++jj) {
+            {
+                const double2 c = coef[t];
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    const T v = V0[e[a]];
+                    x[a] = cfma(c, make_double2(v.x, v.y), x[a]);
+                }
+            }
+            for (int jj = 1; jj < n; ++jj) {
                 const double2 c = coef[static_cast<size_t>(jj) * ldm + t];
 #pragma unroll
                 for (int a = 0; a < 4; ++a) {
-                    const T v = V[jj * vstride + e[a]];
+                    const T v = V[(jj - 1) * vstride + e[a]];
                     x[a] = cfma(c, make_double2(v.x, v.y), x[a]);
                 }
             }
