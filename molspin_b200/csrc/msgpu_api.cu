@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 
+#include "msgpu_arnoldi.h"
 #include "msgpu_dense.h"
 #include "msgpu_fused.cuh"
 #include "msgpu_kernels.cuh"
@@ -1011,7 +1012,7 @@ bool lanczos128(msgpu_ctx *c, const msgpu_run_params *p)
 // a = 2 a1 + a2, a1 the digit of stride s1): true when every quartet's rows
 // couple only to the same quartet, with the same block (to 1e-12 of the
 // largest entry).  A scalar K is kappa I.
-bool pair_reaction(const msgpu_ctx *c, PairK *out)
+bool pair_reaction(const msgpu_ctx *c, ArnoldiPairK *out)
 {
     for (int i = 0; i < 16; ++i) out->k[i] = make_double2(0.0, 0.0);
     if (c->k_scalar) {
@@ -2094,7 +2095,7 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
         rec = (p->precision == MSGPU_PREC_C64 && c->k_scalar) ? MSGPU_REC_LANCZOS : MSGPU_REC_ARNOLDI;
     if (rec == MSGPU_REC_LANCZOS && !c->k_scalar)
         return fail(c, MSGPU_ERR_INVALID, "run: Lanczos requires a scalar reaction operator K");
-    PairK pair_k{};  // K on the electron pair, for the complex64 Arnoldi form
+    ArnoldiPairK pair_k{};  // K on the electron pair, for the complex64 Arnoldi form
     if (p->precision == MSGPU_PREC_C64 && rec == MSGPU_REC_ARNOLDI && !pair_reaction(c, &pair_k))
         return fail(c, MSGPU_ERR_INVALID,
                     "run: the complex64 Arnoldi form needs K acting on the electron pair only (K = I x K4, e.g. "
@@ -2253,6 +2254,15 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
             return cuda_fail(c, e, "Taylor statistics");
         taylor_shift(hs);
         if (!std::isfinite(tnorm)) return fail(c, MSGPU_ERR_NONFINITE, "run: non-finite Hamiltonian norm");
+    }
+    ArnoldiScratch arn{};
+    if (arn64 || (prec == MSGPU_PREC_C128 && !taylor && !rk4 && !three_term)) {
+        arn.QT = arnoldi_quartet_tile(Q, ldm, c->ntiles);
+        arn.scale = sc;
+        arn.part = static_cast<double2 *>(arn64 ? c->wbuf.p : c->part.p);
+        arn.hess = static_cast<double2 *>(c->hess.p);
+        arn.mdim = static_cast<int *>(c->mdim.p);
+        if ((e = arnoldi_scratch(arn, c->part2.p, m, ldm, st))) return cuda_fail(c, e, "Arnoldi scratch");
     }
     // Trajectory groups: the step's kernels work on columns [t0, t0 + width)
     // through offset pointers with the row stride ldm, so the groups share the
@@ -2447,101 +2457,53 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
             });
             if (rc) return rc;
         } else if (prec == MSGPU_PREC_C128) {
-            double2 *V = static_cast<double2 *>(c->basis.p);
-            double2 *bufA = static_cast<double2 *>(c->wbuf.p), *bufB = static_cast<double2 *>(c->zbuf.p);
-            double2 *dots = static_cast<double2 *>(c->part2.p);  // [3][m+1][ldm]: h1, h2, norm
-            double2 *h1 = dots, *h2 = dots + static_cast<size_t>(m + 1) * ldm, *nr = dots + 2 * static_cast<size_t>(m + 1) * ldm;
-            const double2 *src = static_cast<const double2 *>(c->psi128.p);
-            double2 *W = bufA;
+            // w_0 is the state, w_j (j >= 1) at basis + (j - 1) n
+            double2 *psi = static_cast<double2 *>(c->psi128.p), *Wb = static_cast<double2 *>(c->basis.p);
+            const ArnoldiVectors<double2> B{psi, Wb, n, Q, c->s1, c->s2, ldm};
             dim3 grid(nt, ldm / 32);
             for (int j = 0; j < m; ++j) {
                 {
                     Timed tm(c, KC_APPLY);
+                    const double *sj = sc + static_cast<size_t>(j) * ldm;
                     if (quartet128)
                         k_arnoldi_apply_q<<<dim3(ceil_div(Q, kWarps), ldm / 32), kThreads, 0, st>>>(
                             QuartetD{static_cast<const int *>(c->qrow.p), static_cast<const int2 *>(c->qcolt.p),
                                      static_cast<const double2 *>(c->qval64.p), static_cast<const int *>(c->qbase.p)},
-                            kappa, src, j == 0 ? sc : sc + ldm, V + j * n, W, Q, c->s1, c->s2, ldm);
+                            kappa, B.slot(j), sj, B.slot(j + 1), Q, c->s1, c->s2, ldm);
                     else
-                        k_arnoldi_apply<<<grid, kThreads, 0, st>>>(Hd, Kd, kappa, src, j == 0 ? sc : sc + ldm, V + j * n,
-                                                                   W, D, ldm, R);
-                    arnoldi_orth_fn(j, 0)<<<grid, kThreads, 0, st>>>(W, V, n, nullptr, static_cast<double2 *>(c->part.p), D,
-                                                                     ldm, R);
+                        k_arnoldi_apply<<<grid, kThreads, 0, st>>>(Hd, Kd, kappa, B.slot(j), sj, B.slot(j + 1), D, ldm, R);
                 }
-                {
-                    Timed tm(c, KC_REDUCE);
-                    k_reduce_partials<<<dim3(ldm / 32, j + 1), dim3(32, 8), 0, st>>>(
-                        static_cast<double2 *>(c->part.p), nt, j + 1, ldm, h1);
-                }
-                {
-                    Timed tm(c, KC_ORTH);
-                    arnoldi_orth_fn(j, 1)<<<grid, kThreads, 0, st>>>(W, V, n, h1, static_cast<double2 *>(c->part.p), D, ldm, R);
-                }
-                {
-                    Timed tm(c, KC_REDUCE);
-                    k_reduce_partials<<<dim3(ldm / 32, j + 1), dim3(32, 8), 0, st>>>(
-                        static_cast<double2 *>(c->part.p), nt, j + 1, ldm, h2);
-                }
-                {
-                    Timed tm(c, KC_ORTH);
-                    arnoldi_orth_fn(j, 2)<<<grid, kThreads, 0, st>>>(W, V, n, h2, static_cast<double2 *>(c->part.p), D, ldm, R);
-                }
-                {
-                    Timed tm(c, KC_REDUCE);
-                    k_reduce_partials<<<dim3(ldm / 32, 1), dim3(32, 8), 0, st>>>(static_cast<double2 *>(c->part.p), nt, 1, ldm, nr);
-                    k_arnoldi_finalize<<<ceil_div(ldm, 256), 256, 0, st>>>(h1, h2, nr, j, mws, ldm,
-                                                                           static_cast<double2 *>(c->hess.p),
-                                                                           static_cast<int *>(c->mdim.p), sc + ldm);
-                }
-                // next iteration reads W scaled by 1/beta; write into the other buffer
-                src = W;
-                W = (W == bufA) ? bufB : bufA;
+                Timed tm(c, KC_ORTH);
+                c->launches += arnoldi_orthogonalise(B, arn, j, st) - 1;
             }
             {
                 Timed tm(c, KC_EXPM);
                 k_krylov_expm<<<ceil_div(ldm, expm_warps), 32 * expm_warps, expm_warps * expm_smem_warp, st>>>(
-                    static_cast<double2 *>(c->hess.p), nullptr, nullptr, 0.0, static_cast<int *>(c->mdim.p), beta0,
-                    nullptr, mws, ldm, M, dt, static_cast<double2 *>(c->coef.p), static_cast<int *>(c->status.p), ldm);
+                    static_cast<double2 *>(c->hess.p), nullptr, nullptr, 0.0, static_cast<int *>(c->mdim.p), beta0, sc, mws,
+                    ldm, M, dt, static_cast<double2 *>(c->coef.p), static_cast<int *>(c->status.p), ldm);
             }
             {
                 Timed tm(c, KC_COMBINE);
                 k_combine<double2, true><<<qgrid, qblock, 0, st>>>(
-                    static_cast<double2 *>(c->psi128.p), V, V + n, n, static_cast<double2 *>(c->coef.p),
+                    psi, psi, Wb, n, static_cast<double2 *>(c->coef.p),
                     static_cast<int *>(c->mdim.p), mws, c->s1, c->s2, Q, ldm, QR, nz, g, 1, pstep(s),
                     s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po, static_cast<double *>(c->qpart_obs.p),
                     static_cast<double *>(c->qpart_nrm.p));
             }
         } else if (arn64) {
-            // complex64 Arnoldi (CGS2) for K = I (x) K4: basis slot j holds w_j with
-            // scale sc[j] = 1/|w_j|, as the Lanczos form; one trajectory group
+            // complex64 Arnoldi for K = I (x) K4; one trajectory group
             float2 *Wb = static_cast<float2 *>(c->basis.p);
             float2 *U = static_cast<float2 *>(c->ubuf.p);
-            double2 *dots = static_cast<double2 *>(c->part2.p);  // [3][m+1][ldm]: h1, h2, norm
-            double2 *h1 = dots, *h2 = dots + static_cast<size_t>(m + 1) * ldm, *nr = dots + 2 * static_cast<size_t>(m + 1) * ldm;
-            double2 *apart = static_cast<double2 *>(c->wbuf.p);  // Gram-Schmidt partials [tile][i][t]
+            const ArnoldiVectors<float2> B{Wb, Wb + n, n, Q, c->s1, c->s2, ldm};
             const int QT = c->q_tile;
-            const dim3 ogrid(nt, ldm / 32);
             for (int j = 0; j < m; ++j) {
-                float2 *Wn = Wb + static_cast<size_t>(j + 1) * n;
                 {
                     Timed tm(c, KC_APPLY);
-                    launch_apply(c, c->q_variant, QT, dim3(ceil_div(Q, std::max(1, QT))), st, Wb + j * n,
+                    launch_apply(c, c->q_variant, QT, dim3(ceil_div(Q, std::max(1, QT))), st, B.slot(j),
                                  sc + static_cast<size_t>(j) * ldm, U, static_cast<double *>(c->part.p), ldm);
-                    k_arn64_apply<<<dim3(ceil_div(Q, kWarps), ldm / 64), kThreads, 0, st>>>(
-                        pair_k, U, Wb + j * n, sc + static_cast<size_t>(j) * ldm, Wn, Q, c->s1, c->s2, ldm);
                 }
-                {
-                    Timed tm(c, KC_ORTH);
-                    arn64_orth_fn(j, 0)<<<ogrid, kThreads, 0, st>>>(Wn, Wb, n, sc, nullptr, apart, D, ldm, R);
-                    k_reduce_partials<<<dim3(ldm / 32, j + 1), dim3(32, 8), 0, st>>>(apart, nt, j + 1, ldm, h1);
-                    arn64_orth_fn(j, 1)<<<ogrid, kThreads, 0, st>>>(Wn, Wb, n, sc, h1, apart, D, ldm, R);
-                    k_reduce_partials<<<dim3(ldm / 32, j + 1), dim3(32, 8), 0, st>>>(apart, nt, j + 1, ldm, h2);
-                    arn64_orth_fn(j, 2)<<<ogrid, kThreads, 0, st>>>(Wn, Wb, n, sc, h2, apart, D, ldm, R);
-                    k_reduce_partials<<<dim3(ldm / 32, 1), dim3(32, 8), 0, st>>>(apart, nt, 1, ldm, nr);
-                    k_arnoldi_finalize<<<ceil_div(ldm, 256), 256, 0, st>>>(
-                        h1, h2, nr, j, mws, ldm, static_cast<double2 *>(c->hess.p), static_cast<int *>(c->mdim.p),
-                        sc + static_cast<size_t>(j + 1) * ldm);
-                }
+                Timed tm(c, KC_ORTH);
+                c->launches += arnoldi_orthogonalise(B, pair_k, U, arn, j, st) - 1;
             }
             {
                 Timed tm(c, KC_EXPM);
@@ -2791,8 +2753,7 @@ extern "C" int msgpu_krylov_step_noalloc(int dim, const int *rowptr, const int *
     Carve probe{nullptr};
     probe.take<double2>(n);                                  // interleaved state
     probe.take<double2>(n * m);                              // Krylov basis
-    probe.take<double2>(n);                                  // W
-    probe.take<double2>(n);                                  // Z
+    probe.take<double2>(2 * n);                              // (held free: the capacity rule counts them)
     probe.take<double2>(static_cast<size_t>(nt) * (m + 1) * ldm);  // partials
     probe.take<double2>(static_cast<size_t>(3) * (m + 1) * ldm);   // dots
     probe.take<double2>(static_cast<size_t>(ldm) * m * m);   // Hessenberg
@@ -2810,8 +2771,7 @@ extern "C" int msgpu_krylov_step_noalloc(int dim, const int *rowptr, const int *
     Carve cv{static_cast<unsigned char *>(base)};
     double2 *psi = cv.take<double2>(n);
     double2 *V = cv.take<double2>(n * m);
-    double2 *bufA = cv.take<double2>(n);
-    double2 *bufB = cv.take<double2>(n);
+    cv.take<double2>(2 * n);
     double2 *part = cv.take<double2>(static_cast<size_t>(nt) * (m + 1) * ldm);
     double2 *dots = cv.take<double2>(static_cast<size_t>(3) * (m + 1) * ldm);
     double2 *hess = cv.take<double2>(static_cast<size_t>(ldm) * m * m);
@@ -2883,29 +2843,27 @@ extern "C" int msgpu_krylov_step_noalloc(int dim, const int *rowptr, const int *
                                        beta0, sc, nullptr, status);
     CsrD Hd{rowptr, col, reinterpret_cast<const double2 *>(val)};
     CsrD Kd{nullptr, nullptr, nullptr};
-    double2 *h1 = dots, *h2 = dots + static_cast<size_t>(m + 1) * ldm, *nr = dots + 2 * static_cast<size_t>(m + 1) * ldm;
-    const double2 *src = psi;
-    double2 *W = bufA;
+    const ArnoldiVectors<double2> B{psi, V, n, Q, s1, s2, ldm};
+    ArnoldiScratch arn{};
+    arn.QT = arnoldi_quartet_tile(Q, ldm, nt);
+    arn.scale = sc;
+    arn.part = part;
+    arn.hess = hess;
+    arn.mdim = mdim;
+    if (arnoldi_scratch(arn, dots, m, ldm, st) != cudaSuccess) return MSGPU_ERR_CUDA;
     dim3 grid(nt, ldm / 32);
     for (int j = 0; j < m; ++j) {
-        k_arnoldi_apply<<<grid, kThreads, 0, st>>>(Hd, Kd, kappa, src, j == 0 ? sc : sc + ldm, V + j * n, W, D, ldm, R);
-        arnoldi_orth_fn(j, 0)<<<grid, kThreads, 0, st>>>(W, V, n, nullptr, part, D, ldm, R);
-        k_reduce_partials<<<dim3(ldm / 32, j + 1), dim3(32, 8), 0, st>>>(part, nt, j + 1, ldm, h1);
-        arnoldi_orth_fn(j, 1)<<<grid, kThreads, 0, st>>>(W, V, n, h1, part, D, ldm, R);
-        k_reduce_partials<<<dim3(ldm / 32, j + 1), dim3(32, 8), 0, st>>>(part, nt, j + 1, ldm, h2);
-        arnoldi_orth_fn(j, 2)<<<grid, kThreads, 0, st>>>(W, V, n, h2, part, D, ldm, R);
-        k_reduce_partials<<<dim3(ldm / 32, 1), dim3(32, 8), 0, st>>>(part, nt, 1, ldm, nr);
-        k_arnoldi_finalize<<<ceil_div(ldm, 256), 256, 0, st>>>(h1, h2, nr, j, m, ldm, hess, mdim, sc + ldm);
-        src = W;
-        W = (W == bufA) ? bufB : bufA;
+        k_arnoldi_apply<<<grid, kThreads, 0, st>>>(Hd, Kd, kappa, B.slot(j), sc + static_cast<size_t>(j) * ldm, B.slot(j + 1), D,
+                                                   ldm, R);
+        arnoldi_orthogonalise(B, arn, j, st);
     }
     const size_t smem_warp = (4 * static_cast<size_t>(m) * m + m) * sizeof(double2);
     const int warps = std::max(1, std::min(8, static_cast<int>(160 * 1024 / smem_warp)));
     if (raise_smem_limit(reinterpret_cast<const void *>(k_krylov_expm), static_cast<int>(warps * smem_warp)) != cudaSuccess)
         return MSGPU_ERR_CUDA;
     k_krylov_expm<<<ceil_div(ldm, warps), 32 * warps, warps * smem_warp, st>>>(hess, nullptr, nullptr, 0.0, mdim, beta0,
-                                                                              nullptr, m, ldm, ntraj, dt, coef, status, ldm);
-    k_combine<double2, true><<<qgrid, qblock, 0, st>>>(psi, V, V + n, n, coef, mdim, m, s1, s2, Q, ldm, QR, nz, -1, 0, 0.0,
+                                                                              sc, m, ldm, ntraj, dt, coef, status, ldm);
+    k_combine<double2, true><<<qgrid, qblock, 0, st>>>(psi, psi, V, n, coef, mdim, m, s1, s2, Q, ldm, QR, nz, -1, 0, 0.0,
                                                        -1, 0, 0.0, po, qobs, qnrm);
     {
         dim3 g(ceil_div(D, 32), ldm / 32), b(32, 8);

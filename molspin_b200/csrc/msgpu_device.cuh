@@ -313,4 +313,65 @@ __device__ inline bool warp_expm_col0(int n, double2 *A, double2 *X, double2 *N,
     return true;
 }
 
+// The Pade form as a call: it is hardly ever taken and large.
+static __device__ __noinline__ bool warp_expm_col0_cold(int n, double2 *A, double2 *X, double2 *N, double2 *Dm, double2 *y)
+{
+    return warp_expm_col0(n, A, X, N, Dm, y);
+}
+
+// exp(A) e1 for the n x n matrix A (column-major, n <= 32) in shared memory,
+// by one warp; y in shared memory.  Taylor series on the vector over r equal
+// sub-steps of norm theta <= 2 (the same truncation rule as
+// warp_tridiag_expm_e1): about 20 products with A where the Pade approximant
+// costs 6 to 10 matrix-matrix products and an LU solve (at n = 16: 26 us to
+// under 3 us).  For norms beyond 64 the squarings of the Pade form win, and
+// warp_expm_col0 runs (A, X, N, Dm: n x n each).
+__device__ inline bool warp_expm_e1(int n, double2 *A, double2 *X, double2 *N, double2 *Dm, double2 *y)
+{
+    const int lane = threadIdx.x & 31;
+    double rs = 0.0;
+    if (lane < n)
+        for (int j = 0; j < n; ++j) rs += sqrt(cabs2(A[lane + j * n]));
+    const double nrm = warp_max(rs);
+    if (__any_sync(0xffffffffu, !isfinite(nrm))) return false;
+    if (__any_sync(0xffffffffu, nrm > 64.0)) return warp_expm_col0_cold(n, A, X, N, Dm, y);
+    const int r = warp_uniform(max(1, static_cast<int>(ceil(nrm * 0.5))));
+    const double theta = nrm / r, inv_r = 1.0 / r;
+    const int K = warp_uniform(taylor_degree(theta));
+    // n <= 16: both half-warps share a row's columns
+    const bool split = n <= 16;
+    const int i = split ? (lane & 15) : lane;
+    const int k0 = split && lane >= 16 ? n / 2 : 0, k1 = split && lane < 16 ? n / 2 : n;
+    const bool live = i < n;
+    double2 yv = make_double2(i == 0 ? 1.0 : 0.0, 0.0);
+    for (int rep = 0; rep < r; ++rep) {
+        double2 term = yv;
+        for (int k = 1; k <= K; ++k) {
+            if (live && (!split || lane < 16)) y[i] = term;
+            __syncwarp();
+            double2 s = make_double2(0.0, 0.0), s2 = make_double2(0.0, 0.0);
+            if (live) {
+                int c = k0;
+#pragma unroll 2
+                for (; c + 1 < k1; c += 2) {
+                    s = cfma(A[i + c * n], y[c], s);
+                    s2 = cfma(A[i + (c + 1) * n], y[c + 1], s2);
+                }
+                if (c < k1) s = cfma(A[i + c * n], y[c], s);
+            }
+            s = cadd(s, s2);
+            if (split) {
+                s.x += __shfl_xor_sync(0xffffffffu, s.x, 16);
+                s.y += __shfl_xor_sync(0xffffffffu, s.y, 16);
+            }
+            term = cscale(s, inv_r * c_taylor.inv[k]);
+            yv = cadd(yv, term);
+            __syncwarp();
+        }
+    }
+    if (live && (!split || lane < 16)) y[i] = yv;
+    __syncwarp();
+    return __all_sync(0xffffffffu, !live || (isfinite(yv.x) && isfinite(yv.y)));
+}
+
 }  // namespace msgpu

@@ -44,24 +44,13 @@ struct CsrF {
 };
 
 // ===================================================================== c128
-// Arnoldi on G = -iH - K with classical Gram-Schmidt applied twice (CGS2),
-// trajectory tile of 32 (one trajectory per lane, 16-byte loads).
+// Arnoldi on G = -iH - K, one trajectory per lane (16-byte loads); the
+// Gram-Schmidt passes are in msgpu_arnoldi.cuh.
 
-// The Krylov index j is a template parameter (J) of k_arnoldi_dots and
-// k_arnoldi_orth, so that the per-trajectory arrays over i <= j (dot
-// accumulators, a row of every V_i) have static indices and live in
-// registers: with a runtime j they sat in local memory, whose traffic spilled
-// to DRAM (more bytes written by the Gram-Schmidt pass than the vector it
-// updates).  The host picks the instantiation from a table
-// (arnoldi_orth_fn); the arithmetic and its order are those of one generic
-// loop over i.
-
-// W = G * v_j where v_j = src * scale[t]; also stores v_j into Vj.  The
-// first-pass dots <V_i, W> are k_arnoldi_dots: fused here they held
-// this kernel (whose CSR gathers want occupancy) to two CTAs per SM.
+// W = G v_j where v_j = src * scale[t].
 __global__ void __launch_bounds__(kThreads)
 k_arnoldi_apply(CsrD H, CsrD K, double kappa, const double2 *__restrict__ src, const double *__restrict__ scale,
-                double2 *__restrict__ Vj, double2 *__restrict__ W, int D, int ldm, int R)
+                double2 *__restrict__ W, int D, int ldm, int R)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.y * 32 + lane;
@@ -98,9 +87,7 @@ k_arnoldi_apply(CsrD H, CsrD K, double kappa, const double2 *__restrict__ src, c
         } else {
             g = csub(g, cscale(vr, kappa));
         }
-        const size_t e = static_cast<size_t>(r) * ldm + t;
-        Vj[e] = vr;
-        W[e] = g;
+        W[static_cast<size_t>(r) * ldm + t] = g;
     }
 }
 
@@ -178,7 +165,7 @@ __device__ __forceinline__ void quartet_block_d(double2 o[4], int type, const do
 // for its four rows.  Summation runs in block order, not CSR order.
 __global__ void __launch_bounds__(kThreads)
 k_arnoldi_apply_q(QuartetD H, double kappa, const double2 *__restrict__ src, const double *__restrict__ scale,
-                  double2 *__restrict__ Vj, double2 *__restrict__ W, int Q, int s1, int s2, int ldm)
+                  double2 *__restrict__ W, int Q, int s1, int s2, int ldm)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.y * 32 + lane;
@@ -207,7 +194,6 @@ k_arnoldi_apply_q(QuartetD H, double kappa, const double2 *__restrict__ src, con
         const size_t e = static_cast<size_t>(base + off[a]) * ldm + t;
         const double2 vr = cscale(own ? x[a] : src[e], sc);
         const double2 acc = cscale(o[a], sc);
-        Vj[e] = vr;
         W[e] = csub(make_double2(acc.y, -acc.x), cscale(vr, kappa));  // -i H v - kappa v
     }
 }
@@ -309,287 +295,6 @@ k_lanczos_update_d(const double2 *__restrict__ U, const double2 *__restrict__ wj
         for (int w = 1; w < kWarps; ++w) s += sm[w][lane];
         part[static_cast<size_t>(blockIdx.x) * ldm + t] = s;
     }
-}
-
-// Partial dots <V_i, W>, i <= j (the first Gram-Schmidt pass; W unchanged,
-// h unused).  Each V_i is used once and the compiler keeps every load of a
-// row in flight; two CTAs per SM bound its registers.
-template <int J>
-__global__ void __launch_bounds__(kThreads, 2)
-k_arnoldi_dots(double2 *__restrict__ W, const double2 *__restrict__ V, size_t vstride,
-               const double2 *__restrict__ h, double2 *__restrict__ part, int D, int ldm, int R)
-{
-    (void)h;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int t = blockIdx.y * 32 + lane;
-    const int r0 = blockIdx.x * R;
-    double2 dacc[J + 1];
-#pragma unroll
-    for (int i = 0; i <= J; ++i) dacc[i] = make_double2(0.0, 0.0);
-    for (int r = r0 + warp; r < min(r0 + R, D); r += kWarps) {
-        const size_t e = static_cast<size_t>(r) * ldm + t;
-        const double2 w = W[e];
-#pragma unroll
-        for (int i = 0; i <= J; ++i) dacc[i] = cadd(dacc[i], cconjmul(__ldg(V + i * vstride + e), w));
-    }
-    __shared__ double2 sm[kWarps][32];
-#pragma unroll  // static indices keep dacc in registers
-    for (int i = 0; i <= J; ++i) {
-        sm[warp][lane] = dacc[i];
-        __syncthreads();
-        if (warp == 0) {
-            double2 s = sm[0][lane];
-            for (int w = 1; w < kWarps; ++w) s = cadd(s, sm[w][lane]);
-            part[(static_cast<size_t>(blockIdx.x) * (J + 1) + i) * ldm + t] = s;
-        }
-        __syncthreads();
-    }
-}
-
-// W -= sum_{i<=j} h[i][t] V_i; then partial dots <V_i, W> (MODE 1) or the
-// partial squared norm |W|^2 (MODE 2, stored in .x).  The coefficients sit in
-// shared memory; a row's V_i are all loaded before the first is used.
-template <int J, int MODE>
-__global__ void __launch_bounds__(kThreads)
-k_arnoldi_orth(double2 *__restrict__ W, const double2 *__restrict__ V, size_t vstride,
-               const double2 *__restrict__ h, double2 *__restrict__ part, int D, int ldm, int R)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int t = blockIdx.y * 32 + lane;
-    const int r0 = blockIdx.x * R;
-    __shared__ double2 hc[J + 1][32];
-    for (int k = threadIdx.x; k < (J + 1) * 32; k += kThreads)
-        hc[k >> 5][k & 31] = h[static_cast<size_t>(k >> 5) * ldm + blockIdx.y * 32 + (k & 31)];
-    __syncthreads();
-    constexpr int ND = MODE == 1 ? J + 1 : 1;
-    double2 dacc[ND];
-#pragma unroll
-    for (int i = 0; i < ND; ++i) dacc[i] = make_double2(0.0, 0.0);
-    for (int r = r0 + warp; r < min(r0 + R, D); r += kWarps) {
-        const size_t e = static_cast<size_t>(r) * ldm + t;
-        double2 w = W[e];
-        double2 vi[J + 1];  // every load of the row in flight before the first use
-#pragma unroll
-        for (int i = 0; i <= J; ++i) vi[i] = __ldg(V + i * vstride + e);
-#pragma unroll
-        for (int i = 0; i <= J; ++i) w = csub(w, cmul(hc[i][lane], vi[i]));
-        W[e] = w;
-        if (MODE == 1) {
-#pragma unroll
-            for (int i = 0; i <= J; ++i) dacc[i] = cadd(dacc[i], cconjmul(vi[i], w));
-        } else {
-            dacc[0].x += cabs2(w);
-        }
-    }
-    __shared__ double2 sm[kWarps][32];
-#pragma unroll  // static indices keep dacc in registers
-    for (int i = 0; i < ND; ++i) {
-        sm[warp][lane] = dacc[i];
-        __syncthreads();
-        if (warp == 0) {
-            double2 s = sm[0][lane];
-            for (int w = 1; w < kWarps; ++w) s = cadd(s, sm[w][lane]);
-            part[(static_cast<size_t>(blockIdx.x) * ND + i) * ldm + t] = s;
-        }
-        __syncthreads();
-    }
-}
-
-// ------------------------------------------------ complex64 Arnoldi (general K on the pair)
-// The complex64 form for a reaction operator K = I (x) K4 that acts on the
-// electron pair only (unequal sinks: K = sum_c k_c/2 P_c).  Basis slot j holds
-// w_j unnormalised in the pair-planar layout, with the per-trajectory scale
-// s_j = 1 / |w_j| (v_j = s_j w_j), as in the Lanczos form; the quartet SpMM
-// gives U = H v_j.  Arithmetic in FP64 (FP32 storage), one trajectory per lane:
-// a lane reads its trajectory's re and im words of the pair's 16 bytes.
-
-struct PairK {
-    double2 k[16];  // K4, row-major in the pair index a = 2 a1 + a2
-};
-
-// W = -i U - K4 v_j per quartet, stored as w_{j+1} (before orthogonalisation).
-// Grid (ceil(Q / 8), ldm / 64), 256 threads: a warp per quartet, a lane per
-// trajectory pair.
-__global__ void __launch_bounds__(kThreads)
-k_arn64_apply(PairK K, const float2 *__restrict__ U, const float2 *__restrict__ wj, const double *__restrict__ sj,
-              float2 *__restrict__ W, int Q, int s1, int s2, int ldm)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int t = blockIdx.y * 64 + 2 * lane;
-    const int q = blockIdx.x * kWarps + warp;
-    if (q >= Q) return;
-    const int base = quartet_base(q, s1, s2);
-    const int off[4] = {0, s2, s1, s1 + s2};
-    const double sc0 = sj[t], sc1 = sj[t + 1];
-    double2 v[2][4], u[2][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const size_t e = static_cast<size_t>(base + off[a]) * ldm + t;
-        const float4 x = *reinterpret_cast<const float4 *>(wj + e);
-        const float4 h = *reinterpret_cast<const float4 *>(U + e);
-        v[0][a] = make_double2(x.x * sc0, x.z * sc0);
-        v[1][a] = make_double2(x.y * sc1, x.w * sc1);
-        u[0][a] = make_double2(h.x, h.z);
-        u[1][a] = make_double2(h.y, h.w);
-    }
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        double2 g[2];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            double2 kv = make_double2(0.0, 0.0);
-#pragma unroll
-            for (int b = 0; b < 4; ++b) kv = cfma(K.k[4 * a + b], v[k][b], kv);
-            g[k] = csub(make_double2(u[k][a].y, -u[k][a].x), kv);  // -i U - K v
-        }
-        *reinterpret_cast<float4 *>(W + static_cast<size_t>(base + off[a]) * ldm + t) =
-            make_float4(static_cast<float>(g[0].x), static_cast<float>(g[1].x), static_cast<float>(g[0].y),
-                        static_cast<float>(g[1].y));
-    }
-}
-
-// MODE 0: partial dots <v_i, W>, i <= J; MODE 1: W -= sum_i h_i v_i, then the
-// dots again; MODE 2: W -= sum_i h_i v_i, then |W|^2 (in .x).  v_i = s_i w_i
-// from the basis slots: the update uses h_i s_i and the dots scale by s_i once
-// at the end, so the per-element work is that of the complex128 kernels.
-// Grid (ntiles, ldm / 32), a lane per trajectory (its re and im words of the
-// pair's 16 bytes).  Partials go to part[tile][i][t] (the layout of the
-// complex128 kernels).
-template <int J, int MODE>
-__global__ void __launch_bounds__(kThreads)
-k_arn64_orth(float2 *__restrict__ W, const float2 *__restrict__ V, size_t vstride, const double *__restrict__ sc,
-             const double2 *__restrict__ h, double2 *__restrict__ part, int D, int ldm, int R)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int t = blockIdx.y * 32 + lane;
-    const int r0 = blockIdx.x * R;
-    // per-trajectory h_i s_i and s_i, once per CTA
-    __shared__ double2 hs[J + 1][32];
-    __shared__ double si[J + 1][32];
-    for (int k = threadIdx.x; k < (J + 1) * 32; k += kThreads) {
-        const size_t e = static_cast<size_t>(k >> 5) * ldm + blockIdx.y * 32 + (k & 31);
-        si[k >> 5][k & 31] = sc[e];
-        hs[k >> 5][k & 31] = MODE == 0 ? make_double2(0.0, 0.0) : cscale(h[e], sc[e]);
-    }
-    __syncthreads();
-    constexpr int ND = MODE == 2 ? 1 : J + 1;
-    double2 dacc[ND];
-#pragma unroll
-    for (int i = 0; i < ND; ++i) dacc[i] = make_double2(0.0, 0.0);
-    auto ld = [&](const float2 *x, int r) {
-        const float *f = reinterpret_cast<const float *>(x + static_cast<size_t>(r) * ldm + (t & ~1)) + (t & 1);
-        return make_double2(f[0], f[2]);
-    };
-    for (int r = r0 + warp; r < min(r0 + R, D); r += kWarps) {
-        double2 w = ld(W, r);
-        if (MODE != 0) {
-#pragma unroll
-            for (int i = 0; i <= J; ++i) w = csub(w, cmul(hs[i][lane], ld(V + i * vstride, r)));
-            float *f = reinterpret_cast<float *>(W + static_cast<size_t>(r) * ldm + (t & ~1)) + (t & 1);
-            f[0] = static_cast<float>(w.x);
-            f[2] = static_cast<float>(w.y);
-            w = make_double2(f[0], f[2]);  // the stored (rounded) vector is the one the next pass sees
-        }
-        if (MODE != 2) {
-#pragma unroll
-            for (int i = 0; i <= J; ++i) dacc[i] = cadd(dacc[i], cconjmul(ld(V + i * vstride, r), w));
-        } else {
-            dacc[0].x += cabs2(w);
-        }
-    }
-    __shared__ double2 sm[kWarps][32];
-#pragma unroll  // static indices keep dacc in registers
-    for (int i = 0; i < ND; ++i) {
-        sm[warp][lane] = MODE == 2 ? dacc[i] : cscale(dacc[i], si[i][lane]);
-        __syncthreads();
-        if (warp == 0) {
-            double2 s = sm[0][lane];
-            for (int w2 = 1; w2 < kWarps; ++w2) s = cadd(s, sm[w2][lane]);
-            part[(static_cast<size_t>(blockIdx.x) * ND + i) * ldm + t] = s;
-        }
-        __syncthreads();
-    }
-}
-
-using Arn64Fn = void (*)(float2 *, const float2 *, size_t, const double *, const double2 *, double2 *, int, int, int);
-template <int J, int MODE>
-constexpr Arn64Fn arn64_kernel() { return &k_arn64_orth<J, MODE>; }
-template <int MODE, int... J>
-Arn64Fn arn64_pick(int j, std::integer_sequence<int, J...>)
-{
-    static constexpr Arn64Fn table[] = {arn64_kernel<J, MODE>()...};
-    return table[j];
-}
-// The complex64 Gram-Schmidt kernel of iteration j (0 <= j < kMaxKrylov), mode 0, 1 or 2.
-inline Arn64Fn arn64_orth_fn(int j, int mode)
-{
-    constexpr auto js = std::make_integer_sequence<int, kMaxKrylov>{};
-    return mode == 0 ? arn64_pick<0>(j, js) : mode == 1 ? arn64_pick<1>(j, js) : arn64_pick<2>(j, js);
-}
-
-using ArnoldiOrthFn = void (*)(double2 *, const double2 *, size_t, const double2 *, double2 *, int, int, int);
-
-template <int J, int MODE>
-constexpr ArnoldiOrthFn arnoldi_kernel()
-{
-    if constexpr (MODE == 0) return &k_arnoldi_dots<J>;
-    else return &k_arnoldi_orth<J, MODE>;
-}
-template <int MODE, int... J>
-ArnoldiOrthFn arnoldi_orth_pick(int j, std::integer_sequence<int, J...>)
-{
-    static constexpr ArnoldiOrthFn table[] = {arnoldi_kernel<J, MODE>()...};
-    return table[j];
-}
-// The kernel of iteration j, 0 <= j < kMaxKrylov: mode 0 k_arnoldi_dots,
-// modes 1 and 2 k_arnoldi_orth.
-inline ArnoldiOrthFn arnoldi_orth_fn(int j, int mode)
-{
-    constexpr auto js = std::make_integer_sequence<int, kMaxKrylov>{};
-    return mode == 0 ? arnoldi_orth_pick<0>(j, js) : mode == 1 ? arnoldi_orth_pick<1>(j, js) : arnoldi_orth_pick<2>(j, js);
-}
-
-// out[i][t] = sum over tiles of part[tile][i][t] (fixed order).
-// Launch with blockDim (32, 8) and (ldm/32, ni) blocks; fixed summation order.
-__global__ void k_reduce_partials(const double2 *__restrict__ part, int ntiles, int ni, int ldm,
-                                  double2 *__restrict__ out)
-{
-    __shared__ double2 red[8][33];
-    const int t = blockIdx.x * 32 + threadIdx.x, i = blockIdx.y;
-    double2 ps = make_double2(0.0, 0.0);
-    for (int tile = threadIdx.y; tile < ntiles; tile += 8)
-        ps = cadd(ps, part[(static_cast<size_t>(tile) * ni + i) * ldm + t]);
-    red[threadIdx.y][threadIdx.x] = ps;
-    __syncthreads();
-    if (threadIdx.y != 0) return;
-    double2 s = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int y = 0; y < 8; ++y) s = cadd(s, red[y][threadIdx.x]);
-    out[static_cast<size_t>(i) * ldm + t] = s;
-}
-
-// Per-trajectory Arnoldi bookkeeping after CGS2 of iteration j:
-// H_m[i][j] = h1[i] + h2[i]; beta = |W|; H_m[j+1][j] = beta; scale = 1/beta;
-// a trajectory whose beta falls below 1e-14 (breakdown, as the reference) or
-// that reached the last iteration keeps dimension j+1.
-__global__ void k_arnoldi_finalize(const double2 *__restrict__ h1, const double2 *__restrict__ h2,
-                                   const double2 *__restrict__ nrm, int j, int m, int ldm,
-                                   double2 *__restrict__ hess, int *__restrict__ mdim, double *__restrict__ scale)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ldm) return;
-    const bool active = mdim[t] == 0;
-    double2 *Ht = hess + static_cast<size_t>(t) * m * m;  // column-major m x m
-    for (int i = 0; i <= j; ++i) {
-        const double2 v = cadd(h1[static_cast<size_t>(i) * ldm + t], h2[static_cast<size_t>(i) * ldm + t]);
-        if (active) Ht[i + j * m] = v;
-    }
-    const double beta = sqrt(nrm[t].x);
-    if (!active) { scale[t] = 0.0; return; }
-    if (j == m - 1) { mdim[t] = m; scale[t] = 0.0; return; }
-    Ht[(j + 1) + j * m] = make_double2(beta, 0.0);
-    if (beta < 1e-14) { mdim[t] = j + 1; scale[t] = 0.0; return; }
-    scale[t] = 1.0 / beta;
 }
 
 // ===================================================================== c64
@@ -1131,7 +836,7 @@ __global__ void k_krylov_expm(const double2 *__restrict__ hess, const double *__
     if (t >= width) return;  // width: trajectories of this launch
     double2 *A = smem + static_cast<size_t>(warp) * (4 * m * m + m);
     double2 *X = A + m * m, *N = X + m * m, *Dm = N + m * m, *y = Dm + m * m;
-    const int n = max(1, mdim[t]);
+    const int n = warp_uniform(max(1, mdim[t]));
     const double b0 = beta0[t];
     if (lane < n) {
         for (int i = 0; i < n; ++i) {
@@ -1150,7 +855,7 @@ __global__ void k_krylov_expm(const double2 *__restrict__ hess, const double *__
     }
     __syncwarp();
     bool ok = true;
-    if (b0 > 0.0) ok = warp_expm_col0(n, A, X, N, Dm, y);
+    if (__any_sync(0xffffffffu, b0 > 0.0)) ok = warp_expm_e1(n, A, X, N, Dm, y);
     if (lane < m) {
         double2 c = make_double2(0.0, 0.0);
         if (b0 > 0.0 && ok && lane < n) {
