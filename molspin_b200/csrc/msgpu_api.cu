@@ -796,7 +796,7 @@ int ensure_workspace(msgpu_ctx *c, int prec, int m)
         (rc = ensure(c, c->acc, static_cast<size_t>(nobs) * ldm * sizeof(double), "yield acc")) ||
         (rc = ensure(c, c->comp, static_cast<size_t>(nobs) * ldm * sizeof(double), "yield comp")) ||
         (rc = ensure(c, c->rates_d, 8 * sizeof(double), "rates")) ||
-        (rc = ensure(c, c->status, sizeof(int), "status")))
+        (rc = ensure(c, c->status, 2 * sizeof(int), "status")))
         return rc;
     c->ws_prec = prec;
     c->ws_m = m;
@@ -872,7 +872,7 @@ int run_dense(msgpu_ctx *c, const msgpu_run_params *p)
         (rc = ensure(c, c->comp, static_cast<size_t>(nobs) * ldm * sizeof(double), "yield comp")) ||
         (rc = ensure(c, c->prev, static_cast<size_t>(nobs) * ldm * sizeof(double), "yield prev")) ||
         (rc = ensure(c, c->rates_d, 8 * sizeof(double), "rates")) ||
-        (rc = ensure(c, c->status, sizeof(int), "status")) ||
+        (rc = ensure(c, c->status, 2 * sizeof(int), "status")) ||
         (rc = ensure(c, c->values_d, static_cast<size_t>(p->ntimes) * nobs * sizeof(double), "values")) ||
         (rc = ensure(c, c->obs_d, 8 * 16 * sizeof(double2), "observables")) ||
         (rc = ensure(c, c->dense_part, 2 * static_cast<size_t>(p->ntimes) * nobs * sizeof(double), "dense values")))
@@ -881,7 +881,7 @@ int run_dense(msgpu_ctx *c, const msgpu_run_params *p)
     cudaError_t e;
     if ((e = cudaMemcpyAsync(c->rates_d.p, c->rates.data(), nobs * sizeof(double), cudaMemcpyHostToDevice, st)) ||
         (e = cudaMemcpyAsync(c->obs_d.p, po.op, sizeof(double2) * 16 * nobs, cudaMemcpyHostToDevice, st)) ||
-        (e = cudaMemsetAsync(c->status.p, 0, sizeof(int), st)))
+        (e = cudaMemsetAsync(c->status.p, 0, 2 * sizeof(int), st)))
         return cuda_fail(c, e, "dense setup");
     if (!p->accumulate) {
         if ((e = cudaMemsetAsync(c->acc.p, 0, static_cast<size_t>(nobs) * ldm * sizeof(double), st)) ||
@@ -1010,9 +1010,9 @@ bool lanczos128(msgpu_ctx *c, const msgpu_run_params *p)
 
 // K as I (x) K4 on the electron pair (the 4 x 4 block in the pair index
 // a = 2 a1 + a2, a1 the digit of stride s1): true when every quartet's rows
-// couple only to the same quartet, with the same block (to 1e-12 of the
+// couple only to the same quartet, with the same block (to rel_tol of the
 // largest entry).  A scalar K is kappa I.
-bool pair_reaction(const msgpu_ctx *c, ArnoldiPairK *out)
+bool pair_reaction(const msgpu_ctx *c, ArnoldiPairK *out, double rel_tol = 1e-12)
 {
     for (int i = 0; i < 16; ++i) out->k[i] = make_double2(0.0, 0.0);
     if (c->k_scalar) {
@@ -1023,7 +1023,7 @@ bool pair_reaction(const msgpu_ctx *c, ArnoldiPairK *out)
     if (static_cast<int>(c->k_hrow.size()) != D + 1 || s1 <= 0 || s2 <= 0) return false;
     double kmax = 0.0;
     for (size_t k = 0; k < c->k_hcol.size(); ++k) kmax = std::max(kmax, std::hypot(c->k_hval[2 * k], c->k_hval[2 * k + 1]));
-    const double tol = 1e-12 * kmax;
+    const double tol = rel_tol * kmax;
     bool have[4] = {false, false, false, false};
     for (int r = 0; r < D; ++r) {
         const int a1 = (r / s1) & 1, a2 = (r / s2) & 1, a = 2 * a1 + a2;
@@ -1057,7 +1057,7 @@ int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
         (rc = ensure(c, c->comp, static_cast<size_t>(nobs) * ldm * sizeof(double), "yield comp")) ||
         (rc = ensure(c, c->prev, static_cast<size_t>(nobs) * ldm * sizeof(double), "yield prev")) ||
         (rc = ensure(c, c->rates_d, 8 * sizeof(double), "rates")) ||
-        (rc = ensure(c, c->status, sizeof(int), "status")) ||
+        (rc = ensure(c, c->status, 2 * sizeof(int), "status")) ||
         (rc = ensure(c, c->values_d, static_cast<size_t>(p->ntimes) * nobs * sizeof(double), "values")) ||
         (rc = ensure(c, c->trajval, static_cast<size_t>(p->ntimes) * M * nobs * sizeof(double), "values per trajectory")) ||
         (rc = ensure(c, c->times_d, static_cast<size_t>(p->ntimes) * sizeof(double), "times")) ||
@@ -1148,7 +1148,7 @@ int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
         (e = cudaMemcpyAsync(c->obs_d.p, po.op, sizeof(double2) * 16 * nobs, cudaMemcpyHostToDevice, st)) ||
         (e = cudaMemcpyAsync(c->times_d.p, p->times, sizeof(double) * p->ntimes, cudaMemcpyHostToDevice, st)) ||
         (e = cudaMemcpyAsync(c->pflip_d.p, pf.data(), sizeof(double) * p->ntimes, cudaMemcpyHostToDevice, st)) ||
-        (e = cudaMemsetAsync(c->status.p, 0, sizeof(int), st)))
+        (e = cudaMemsetAsync(c->status.p, 0, 2 * sizeof(int), st)))
         return cuda_fail(c, e, "resident setup");
     const ResidentShape shape =
         prec == MSGPU_PREC_C64 ? resident_shape_c64(D, m) : resident_shape_c128(D, m, lanczos);
@@ -1215,93 +1215,96 @@ int build_quartet(msgpu_ctx *c)
     std::vector<int2> blks;
     std::vector<float> vals;
     std::vector<double> vals64;  // the same values in FP64
-    std::vector<std::pair<int, std::array<double, 32>>> blocks;  // (neighbour base, 16 complex)
-    std::vector<std::array<int, 16>> bsrc;                        // CSR index of each block entry
-    std::vector<int> src;                                         // CSR index per stored value slot
+    std::vector<int> src;        // CSR index per stored value slot
+    blks.reserve(c->nnz / 6 + Q);
+    vals.reserve(2 * static_cast<size_t>(c->nnz));
+    vals64.reserve(2 * static_cast<size_t>(c->nnz));
+    if (c->terms) src.reserve(c->nnz);
+    struct Block {
+        int base;
+        double z[32];  // 16 complex, row-major in the pair index
+        int src[16];   // CSR index of each entry
+    };
+    std::vector<Block> blocks;
+    std::vector<int> ord;
+    // storage order (4 a + b) of each block type, see QuartetC
+    static const int kOrder[6][16] = {{0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15},
+                                      {0, 2, 8, 10, 5, 7, 13, 15},
+                                      {0, 1, 4, 5, 10, 11, 14, 15},
+                                      {0, 5, 10, 15},
+                                      {0, 2, 8, 10},
+                                      {0, 1, 4, 5}};
+    static const int kCount[6] = {16, 8, 8, 4, 4, 4};
     for (int q = 0; q < Q; ++q) {
         const int lo = q % s2, mid = (q / s2) % (s1 / (2 * s2)), hi = q / (s1 / 2);
         const int b = hi * (2 * s1) + mid * (2 * s2) + lo;
         base[q] = b;
-        blocks.clear();
-        bsrc.clear();
+        size_t nblk = 0;
         for (int a = 0; a < 4; ++a) {
             const int r = b + off[a];
+            size_t at = 0;  // rows meet their neighbours in a similar order
             for (int k = c->h_rowptr[r]; k < c->h_rowptr[r + 1]; ++k) {
                 const int col = c->h_col[k];
                 const int a1 = (col / s1) & 1, a2 = (col / s2) & 1;
                 const int cb = col - a1 * s1 - a2 * s2, bi = 2 * a1 + a2;
-                size_t slot = 0;
-                while (slot < blocks.size() && blocks[slot].first != cb) ++slot;
-                if (slot == blocks.size()) {
-                    std::array<double, 32> z;
-                    z.fill(0.0);
-                    blocks.push_back({cb, z});
-                    std::array<int, 16> none;
-                    none.fill(-1);
-                    bsrc.push_back(none);
+                size_t slot = at;
+                while (slot < nblk && blocks[slot].base != cb) ++slot;
+                if (slot == nblk) {
+                    slot = 0;
+                    while (slot < at && blocks[slot].base != cb) ++slot;
+                    if (slot == at) slot = nblk;
                 }
-                bsrc[slot][a * 4 + bi] = k;
-                blocks[slot].second[2 * (a * 4 + bi)] += c->h_val[2 * static_cast<size_t>(k)];
-                blocks[slot].second[2 * (a * 4 + bi) + 1] += c->h_val[2 * static_cast<size_t>(k) + 1];
+                if (slot == nblk) {
+                    if (blocks.size() == nblk) blocks.emplace_back();
+                    Block &z = blocks[nblk++];
+                    z.base = cb;
+                    std::fill(z.z, z.z + 32, 0.0);
+                    std::fill(z.src, z.src + 16, -1);
+                }
+                at = slot;
+                Block &z = blocks[slot];
+                z.src[a * 4 + bi] = k;
+                z.z[2 * (a * 4 + bi)] += c->h_val[2 * static_cast<size_t>(k)];
+                z.z[2 * (a * 4 + bi) + 1] += c->h_val[2 * static_cast<size_t>(k) + 1];
             }
         }
-        std::vector<size_t> ord(blocks.size());
-        for (size_t i = 0; i < ord.size(); ++i) ord[i] = i;
         // by neighbour base, the quartet's own block last (the SpMM reuses its
         // gathered rows for the alpha partial)
-        std::sort(ord.begin(), ord.end(), [&](size_t x, size_t y) {
-            const bool ox = blocks[x].first == b, oy = blocks[y].first == b;
-            return ox != oy ? oy : blocks[x].first < blocks[y].first;
+        ord.resize(nblk);
+        for (size_t i = 0; i < nblk; ++i) ord[i] = static_cast<int>(i);
+        std::sort(ord.begin(), ord.end(), [&](int x, int y) {
+            const bool ox = blocks[x].base == b, oy = blocks[y].base == b;
+            return ox != oy ? oy : blocks[x].base < blocks[y].base;
         });
-        for (size_t oi : ord) {
-            const auto &blk = blocks[oi];
-            const auto &B = blk.second;  // 16 complex, row-major in the pair index
-            auto re = [&](int a, int b) { return B[2 * (a * 4 + b)]; };
-            auto im = [&](int a, int b) { return B[2 * (a * 4 + b) + 1]; };
+        for (int oi : ord) {
+            const Block &blk = blocks[oi];
+            const double *B = blk.z;
             double bmax = 0.0;
             bool e1only = true, e2only = true;
             for (int a = 0; a < 4; ++a)
                 for (int bb = 0; bb < 4; ++bb) {
-                    bmax = std::max(bmax, std::abs(re(a, bb)) + std::abs(im(a, bb)));
-                    const bool nz = re(a, bb) != 0.0 || im(a, bb) != 0.0;
-                    if (!nz) continue;
+                    const double re = B[2 * (a * 4 + bb)], im = B[2 * (a * 4 + bb) + 1];
+                    if (re == 0.0 && im == 0.0) continue;
+                    bmax = std::max(bmax, std::abs(re) + std::abs(im));
                     if ((a & 1) != (bb & 1)) e1only = false;  // couples different second digits
                     if ((a & 2) != (bb & 2)) e2only = false;  // couples different first digits
                 }
-            auto same = [&](int a, int b, int a2, int b2) {
-                return std::abs(re(a, b) - re(a2, b2)) + std::abs(im(a, b) - im(a2, b2)) <= 1e-13 * bmax;
+            auto same = [&](int x, int y) {
+                return std::abs(B[2 * x] - B[2 * y]) + std::abs(B[2 * x + 1] - B[2 * y + 1]) <= 1e-13 * bmax;
             };
-            // emit (a, b) pairs of the block in the storage order of its type
-            std::vector<std::pair<int, int>> order;
-            int type;
-            if (e1only && e2only) {
-                type = 3;
-                for (int a = 0; a < 4; ++a) order.push_back({a, a});
-            } else if (e1only) {
-                // acts on the first digit; A (x) I when both second-digit halves agree
-                const bool kron = same(0, 0, 1, 1) && same(0, 2, 1, 3) && same(2, 0, 3, 1) && same(2, 2, 3, 3);
-                type = kron ? 4 : 1;
-                for (int a2 = 0; a2 < (kron ? 1 : 2); ++a2)
-                    for (int a1 = 0; a1 < 2; ++a1)
-                        for (int b1 = 0; b1 < 2; ++b1) order.push_back({2 * a1 + a2, 2 * b1 + a2});
-            } else if (e2only) {
-                const bool kron = same(0, 0, 2, 2) && same(0, 1, 2, 3) && same(1, 0, 3, 2) && same(1, 1, 3, 3);
-                type = kron ? 5 : 2;
-                for (int a1 = 0; a1 < (kron ? 1 : 2); ++a1)
-                    for (int a2 = 0; a2 < 2; ++a2)
-                        for (int b2 = 0; b2 < 2; ++b2) order.push_back({2 * a1 + a2, 2 * a1 + b2});
-            } else {
-                type = 0;
-                for (int a = 0; a < 4; ++a)
-                    for (int bb = 0; bb < 4; ++bb) order.push_back({a, bb});
-            }
-            blks.push_back({(blk.first << 3) | type, static_cast<int>(vals.size() / 4)});
-            for (auto &ab : order) {
-                vals.push_back(static_cast<float>(re(ab.first, ab.second)));
-                vals.push_back(static_cast<float>(im(ab.first, ab.second)));
-                vals64.push_back(re(ab.first, ab.second));
-                vals64.push_back(im(ab.first, ab.second));
-                src.push_back(bsrc[oi][ab.first * 4 + ab.second]);
+            int type = 0;
+            if (e1only && e2only) type = 3;
+            // acts on one digit; A (x) I when both halves of the other digit agree
+            else if (e1only) type = same(0, 5) && same(2, 7) && same(8, 13) && same(10, 15) ? 4 : 1;
+            else if (e2only) type = same(0, 10) && same(1, 11) && same(4, 14) && same(5, 15) ? 5 : 2;
+            blks.push_back({(blk.base << 3) | type, static_cast<int>(vals.size() / 4)});
+            for (int k = 0; k < kCount[type]; ++k) {
+                const int x = kOrder[type][k];
+                vals.push_back(static_cast<float>(B[2 * x]));
+                vals.push_back(static_cast<float>(B[2 * x + 1]));
+                vals64.push_back(B[2 * x]);
+                vals64.push_back(B[2 * x + 1]);
+                if (c->terms) src.push_back(blk.src[x]);
             }
         }
         rowptr[q + 1] = static_cast<int>(blks.size());
@@ -1948,9 +1951,9 @@ int msgpu_set_hamiltonian_coefficients(msgpu_ctx *c, const double *coef)
         cf.c[t] = coef[t];
         c->hcoef[t] = coef[t];
     }
-    if (int rc = ensure(c, c->status, sizeof(int), "status")) return rc;
+    if (int rc = ensure(c, c->status, 2 * sizeof(int), "status")) return rc;
     cudaError_t e;
-    if ((e = cudaMemsetAsync(c->status.p, 0, sizeof(int), c->stream))) return cuda_fail(c, e, "Hamiltonian update");
+    if ((e = cudaMemsetAsync(c->status.p, 0, 2 * sizeof(int), c->stream))) return cuda_fail(c, e, "Hamiltonian update");
     k_combine_terms<<<ceil_div(std::max(1, c->nnz), 256), 256, 0, c->stream>>>(
         static_cast<const double2 *>(c->hterms.p), c->nterms, cf, c->nnz, static_cast<double2 *>(c->hval.p),
         static_cast<float2 *>(c->hhi.p), static_cast<int *>(c->status.p));
@@ -2139,7 +2142,7 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
     cudaError_t e;
     cudaStream_t st = c->stream;
     if ((e = cudaMemcpyAsync(c->rates_d.p, c->rates.data(), nobs * sizeof(double), cudaMemcpyHostToDevice, st)) ||
-        (e = cudaMemsetAsync(c->status.p, 0, sizeof(int), st)))
+        (e = cudaMemsetAsync(c->status.p, 0, 2 * sizeof(int), st)))
         return cuda_fail(c, e, "run setup");
     if (!p->accumulate) {
         if ((e = cudaMemsetAsync(c->acc.p, 0, static_cast<size_t>(nobs) * ldm * sizeof(double), st)) ||
@@ -2168,14 +2171,11 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
     double *beta0 = static_cast<double *>(c->beta0.p);
     auto yield_update = [&](double dt, int init, int row) {
         Timed tm(c, KC_YIELD);
-        ++c->launches;  // two kernels: per trajectory, then the ensemble value
-        k_yield_traj<<<dim3(ceil_div(ldm, 128), nobs + 1), 128, 0, st>>>(
-            static_cast<double *>(c->qpart_obs.p), static_cast<double *>(c->qpart_nrm.p), qt, nobs, ldm,
+        k_yield<<<dim3(ldm / 32, nobs + 1), dim3(32, 32), 0, st>>>(
+            static_cast<double *>(c->qpart_obs.p), static_cast<double *>(c->qpart_nrm.p), qt, nobs, ldm, M,
             static_cast<double *>(c->rates_d.p), dt, init, static_cast<double *>(c->prev.p),
             static_cast<double *>(c->acc.p), static_cast<double *>(c->comp.p), beta0, sc,
-            static_cast<int *>(c->status.p));
-        k_yield_values<<<1, 1024, 0, st>>>(static_cast<double *>(c->prev.p), nobs, ldm, M,
-                                           values + static_cast<size_t>(row) * nobs);
+            values + static_cast<size_t>(row) * nobs, static_cast<int *>(c->status.p) + 1, static_cast<int *>(c->status.p));
     };
 
     // Evaluate the first time point and apply the first half-step flip.
@@ -2201,6 +2201,28 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
     const bool three_term = quartet128 && lanczos128(c, p);
     if (quartet128)
         if (int rc = build_quartet(c)) return rc;
+    // Taylor and RK4 with K on the electron pair run over quartet blocks (a
+    // budget without room for them keeps the CSR kernels)
+    PairGenerator pg{};
+    bool quartet_gen = false;
+    if (taylor || rk4) {
+        quartet_gen = c->k_scalar || pair_reaction(c, &pg.K, 0.0);
+        pg.pair = !c->k_scalar;
+        if (quartet_gen && build_quartet(c) != MSGPU_OK) {
+            (void)cudaGetLastError();
+            c->err.clear();
+            quartet_gen = false;
+        }
+        if (quartet_gen) {
+            pg.H = QuartetD{static_cast<const int *>(c->qrow.p), static_cast<const int2 *>(c->qcolt.p),
+                            static_cast<const double2 *>(c->qval64.p), static_cast<const int *>(c->qbase.p)};
+            pg.kappa = c->k_scalar ? c->kappa : 0.0;
+            pg.Q = Q;
+            pg.s1 = c->s1;
+            pg.s2 = c->s2;
+            pg.ldm = ldm;
+        }
+    }
     if (prec == MSGPU_PREC_C64) {
         if (int rc = build_quartet(c)) return rc;
         if (int rc = build_tc(c)) return rc;
@@ -2315,7 +2337,7 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
             k_combine_terms<<<ceil_div(std::max(1, c->nnz), 256), 256, 0, st>>>(
                 static_cast<const double2 *>(c->hterms.p), c->nterms, cf, c->nnz, static_cast<double2 *>(c->hval.p),
                 static_cast<float2 *>(c->hhi.p), static_cast<int *>(c->status.p));
-            if (prec == MSGPU_PREC_C64 || quartet128)
+            if (prec == MSGPU_PREC_C64 || quartet128 || quartet_gen)
                 if (int rc = refresh_quartet_values(c)) return rc;
             if (taylor) taylor_shift(hs);
         }
@@ -2333,17 +2355,30 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                 rem *= theta / (mt + 2);
             const double er = std::exp(dt * tmu.x / nsub), ea = dt * tmu.y / nsub;
             const double2 eta = make_double2(er * std::cos(ea), er * std::sin(ea));
-            if ((e = cudaMemcpyAsync(cur, F, n * sizeof(double2), cudaMemcpyDeviceToDevice, st)))
-                return cuda_fail(c, e, "Taylor step");
-            dim3 tgrid(ceil_div(D, 8), ldm / 32), tblock(32, 8);
-            for (int sub = 0; sub < nsub; ++sub) {
-                for (int k = 1; k <= mt; ++k) {
-                    Timed tm(c, KC_APPLY);
-                    k_taylor_term<<<tgrid, tblock, 0, st>>>(Hd, Kd, kappa, tmu, cur, nxt, F, dt / (nsub * k), D, ldm);
-                    std::swap(cur, nxt);
+            const dim3 gq(ceil_div(Q, kWarps), ldm / 32);
+            if (quartet_gen) {
+                mt = std::max(mt, 2);  // the last term must not write the state that it gathers from
+                for (int sub = 0; sub < nsub; ++sub)
+                    for (int k = 1; k <= mt; ++k) {
+                        const bool end = k == mt;
+                        const int what = (end ? kTaylorEnd : kTaylorOut) | (k % 2 == 0 ? kTaylorBoth : end ? kTaylorAdd : 0);
+                        Timed tm(c, KC_APPLY);
+                        k_taylor_term_q<<<gq, kThreads, 0, st>>>(pg, tmu, k == 1 ? F : cur, nxt, F, dt / (nsub * k), eta, what);
+                        std::swap(cur, nxt);
+                    }
+            } else {
+                if ((e = cudaMemcpyAsync(cur, F, n * sizeof(double2), cudaMemcpyDeviceToDevice, st)))
+                    return cuda_fail(c, e, "Taylor step");
+                dim3 tgrid(ceil_div(D, 8), ldm / 32), tblock(32, 8);
+                for (int sub = 0; sub < nsub; ++sub) {
+                    for (int k = 1; k <= mt; ++k) {
+                        Timed tm(c, KC_APPLY);
+                        k_taylor_term<<<tgrid, tblock, 0, st>>>(Hd, Kd, kappa, tmu, cur, nxt, F, dt / (nsub * k), D, ldm);
+                        std::swap(cur, nxt);
+                    }
+                    Timed tm(c, KC_ORTH);
+                    k_taylor_rescale<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(F, cur, eta, n);
                 }
-                Timed tm(c, KC_ORTH);
-                k_taylor_rescale<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(F, cur, eta, n);
             }
             {
                 Timed tm(c, KC_COMBINE);
@@ -2374,9 +2409,15 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                         static_cast<double2 *>(c->hval.p), static_cast<float2 *>(c->hhi.p),
                         static_cast<int *>(c->status.p));
                 }
+                if (c->sched_steps && quartet_gen && stage != 2)
+                    if (int rc = refresh_quartet_values(c)) return rc;
                 Timed tm(c, KC_APPLY);
-                k_rk4_stage<<<tgrid, tblock, 0, st>>>(Hd, Kd, kappa, in[stage], psi, out[stage], acc, cs[stage],
-                                                      ws[stage], stage + 1, D, ldm);
+                if (quartet_gen)
+                    k_rk4_stage_q<<<dim3(ceil_div(Q, kWarps), ldm / 32), kThreads, 0, st>>>(
+                        pg, in[stage], psi, out[stage], acc, cs[stage], ws[stage], stage + 1);
+                else
+                    k_rk4_stage<<<tgrid, tblock, 0, st>>>(Hd, Kd, kappa, in[stage], psi, out[stage], acc, cs[stage],
+                                                          ws[stage], stage + 1, D, ldm);
             }
             {
                 Timed tm(c, KC_COMBINE);

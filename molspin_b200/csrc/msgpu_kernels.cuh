@@ -19,6 +19,7 @@
 
 #include <utility>
 
+#include "msgpu_arnoldi.h"
 #include "msgpu_device.cuh"
 #include "msgpu_resident.h"
 
@@ -947,6 +948,114 @@ __global__ void k_taylor_rescale(double2 *__restrict__ F, double2 *__restrict__ 
     B[i] = f;
 }
 
+// ---------------------------------------------------------------- quartet forms of both
+// For K on the electron pair (K = I x K4, kappa I among them) a warp takes a
+// quartet and a lane a trajectory, as in k_arnoldi_apply_q: 10 quartet rows
+// per row at D = 2048 where the CSR gathers 21 entries.
+struct PairGenerator {
+    QuartetD H;
+    ArnoldiPairK K;
+    int pair;      // K4 in K; else kappa I
+    double kappa;
+    int Q, s1, s2, ldm;
+};
+
+// g = (-i H - K) x at quartet q and trajectory t; x: the quartet's own rows
+// (read again only if its own block is absent), e: their elements.  Loading the
+// next block's rows before this block's arithmetic was slower at every size
+// (16 to 20 us a term at D = 2048, 256 trajectories; 165 to 236 at D = 16384,
+// 512): the registers cost more warps than the loads hide.
+__device__ __forceinline__ void pair_generator(const PairGenerator &G, int q, int t, const double2 *__restrict__ in,
+                                               double2 g[4], double2 x[4], size_t e[4])
+{
+    const int off[4] = {0, G.s2, G.s1, G.s1 + G.s2};
+    double2 o[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) o[a] = make_double2(0.0, 0.0);
+    int last = -1;
+    const int kb = __ldg(G.H.rowptr + q), ke = __ldg(G.H.rowptr + q + 1);
+    for (int kk = kb; kk < ke; ++kk) {
+        const int2 cur = __ldg(G.H.blk + kk);
+        last = cur.x >> 3;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) x[b] = in[static_cast<size_t>(last + off[b]) * G.ldm + t];
+        quartet_block_d(o, cur.x & 7, G.H.val + 2 * static_cast<size_t>(cur.y), x);
+    }
+    const int base = __ldg(G.H.base + q);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        e[a] = static_cast<size_t>(base + off[a]) * G.ldm + t;
+        if (last != base) x[a] = in[e[a]];
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        g[a] = make_double2(o[a].y, -o[a].x);  // -i H x
+        if (G.pair) {
+#pragma unroll
+            for (int b = 0; b < 4; ++b) g[a] = cnfma(G.K.k[4 * a + b], x[b], g[a]);
+        } else {
+            g[a] = csub(g[a], cscale(x[a], G.kappa));
+        }
+    }
+}
+
+// What a Taylor term does with the sum F besides out = scale (G - mu I) in.
+constexpr int kTaylorOut = 1;   // write out (not on the last term)
+constexpr int kTaylorAdd = 2;   // F += out
+constexpr int kTaylorBoth = 4;  // F += in + out: the term before left its own addition to this one
+constexpr int kTaylorEnd = 8;   // F *= eta, the end of a sub-step
+
+// The sum is touched on every second term only, and the first term reads the
+// state itself, so a sub-step needs no copy and no rescaling pass.  Bound by
+// the gathers from L2 (84 MB a launch at D = 2048, 256 trajectories, in 14 us);
+// five steps of 19 terms there: 1.48 ms, 2.05 with k_taylor_term.
+__global__ void __launch_bounds__(kThreads, 4)
+k_taylor_term_q(PairGenerator G, double2 mu, const double2 *in, double2 *out, double2 *F, double scale, double2 eta, int what)
+{
+    const int t = blockIdx.y * 32 + (threadIdx.x & 31);
+    const int q = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    if (q >= G.Q) return;
+    double2 g[4], x[4];
+    size_t e[4];
+    pair_generator(G, q, t, in, g, x, e);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const double2 o = cscale(cnfma(mu, x[a], g[a]), scale);
+        if (what & kTaylorOut) out[e[a]] = o;
+        if (what & (kTaylorAdd | kTaylorBoth)) {
+            double2 f = F[e[a]];
+            if (what & kTaylorBoth) f = cadd(f, x[a]);
+            f = cadd(f, o);
+            F[e[a]] = what & kTaylorEnd ? cmul(eta, f) : f;
+        }
+    }
+}
+
+// k_rk4_stage over quartets.
+__global__ void __launch_bounds__(kThreads, 4)
+k_rk4_stage_q(PairGenerator G, const double2 *y_in, double2 *psi, double2 *__restrict__ y_out, double2 *__restrict__ acc,
+              double c, double w, int stage)
+{
+    const int t = blockIdx.y * 32 + (threadIdx.x & 31);
+    const int q = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    if (q >= G.Q) return;
+    double2 g[4], x[4];
+    size_t e[4];
+    pair_generator(G, q, t, y_in, g, x, e);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (stage == 4) {
+            const double2 a = acc[e[i]];
+            psi[e[i]] = make_double2(a.x + w * g[i].x, a.y + w * g[i].y);
+            continue;
+        }
+        const double2 p = psi[e[i]];
+        y_out[e[i]] = make_double2(p.x + c * g[i].x, p.y + c * g[i].y);
+        const double2 a = stage == 1 ? p : acc[e[i]];
+        acc[e[i]] = make_double2(a.x + w * g[i].x, a.y + w * g[i].y);
+    }
+}
+
 // trace(H) and max_r sum_k |H_rk| (= the 1-norm of a Hermitian H) in a fixed
 // order: one block; out = {tr.re, tr.im, max row sum}.
 __global__ void __launch_bounds__(256) k_g_stats(CsrD H, int D, double *__restrict__ out)
@@ -1291,70 +1400,75 @@ __global__ void k_yield_update(const double *__restrict__ part_obs, const double
     }
 }
 
-// The per-trajectory part of k_yield_update spread over the GPU: thread t of
-// grid row o sums the tile partials of observable o (o == nobs: the squared
-// norm) in tile order, exactly as k_yield_update does, so the results are the
-// same bits.  One 1024-thread CTA reads 5 x 64 partials per thread serially
-// and took about 120 us per time step at 1024 trajectories; this form takes a
-// few microseconds.  Grid (ceil(ldm / 128), nobs + 1), 128 threads.
-__global__ void __launch_bounds__(128)
-k_yield_traj(const double *__restrict__ part_obs, const double *__restrict__ part_nrm, int ntiles, int nobs, int ldm,
-             const double *__restrict__ rates, double dt, int init, double *__restrict__ prev,
-             double *__restrict__ acc, double *__restrict__ comp, double *__restrict__ beta0,
-             double *__restrict__ inv0, int *__restrict__ status)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int o = blockIdx.y;
-    if (t >= ldm) return;
-    bool bad = false;
-    if (o < nobs) {
-        double v = 0.0;
-#pragma unroll 8
-        for (int tile = 0; tile < ntiles; ++tile) v += part_obs[(static_cast<size_t>(tile) * nobs + o) * ldm + t];
-        v *= rates[o];
-        const size_t k = static_cast<size_t>(o) * ldm + t;
-        if (!init) {
-            const double term = 0.5 * dt * (prev[k] + v) - comp[k];
-            const double s = acc[k] + term;
-            comp[k] = (s - acc[k]) - term;
-            acc[k] = s;
-        }
-        prev[k] = v;
-        if (!isfinite(v)) bad = true;
-    } else {
-        double nn = 0.0;
-#pragma unroll 8
-        for (int tile = 0; tile < ntiles; ++tile) nn += part_nrm[static_cast<size_t>(tile) * ldm + t];
-        const double b = sqrt(nn);
-        beta0[t] = b;
-        inv0[t] = b > 0.0 ? 1.0 / b : 0.0;
-        if (!isfinite(b)) bad = true;
-    }
-    if (bad) atomicOr(status, 2);
-}
-
-// Ensemble value of this time point, values_out[o] = sum over trajectories
-// t < M of prev[o][t], summed in k_yield_update's order (thread-strided, then
-// warps, then the warp totals).  One CTA of 1024 threads.
+// k_yield_update over many CTAs: CTA (x, o) sums the tile partials of
+// observable o (o == nobs: the squared norm) for 32 trajectories, 32 threads a
+// trajectory over the tiles and then their sums in order.  The CTA that
+// finishes last sums the ensemble value of this time point over the
+// trajectories t < M (thread-strided, then warps, then the warp totals).  Grid
+// (ldm / 32, nobs + 1), (32, 32) threads; *count is zero between launches.
 __global__ void __launch_bounds__(1024)
-k_yield_values(const double *__restrict__ prev, int nobs, int ldm, int M, double *__restrict__ values_out)
+k_yield(const double *__restrict__ part_obs, const double *__restrict__ part_nrm, int ntiles, int nobs, int ldm, int M,
+        const double *__restrict__ rates, double dt, int init, double *prev, double *__restrict__ acc,
+        double *__restrict__ comp, double *__restrict__ beta0, double *__restrict__ inv0, double *__restrict__ values_out,
+        int *__restrict__ count, int *__restrict__ status)
 {
-    __shared__ double red[8][32];
-    double ens[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int t = threadIdx.x; t < ldm; t += blockDim.x)
-        for (int o = 0; o < nobs; ++o)
-            if (t < M) ens[o] += prev[static_cast<size_t>(o) * ldm + t];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int o = 0; o < nobs; ++o) {
-        double v = warp_sum(ens[o]);
-        if (lane == 0) red[o][warp] = v;
+    __shared__ double red[32][33];
+    __shared__ int last;
+    const int t = blockIdx.x * 32 + threadIdx.x, y = threadIdx.y;
+    const int o = blockIdx.y;
+    double ps = 0.0;
+    if (o < nobs) {
+        for (int tile = y; tile < ntiles; tile += 32) ps += part_obs[(static_cast<size_t>(tile) * nobs + o) * ldm + t];
+    } else {
+        for (int tile = y; tile < ntiles; tile += 32) ps += part_nrm[static_cast<size_t>(tile) * ldm + t];
+    }
+    red[y][threadIdx.x] = ps;
+    __syncthreads();
+    if (y == 0) {
+        double v = 0.0;
+#pragma unroll
+        for (int k = 0; k < 32; ++k) v += red[k][threadIdx.x];
+        if (o < nobs) {
+            v *= rates[o];
+            const size_t k = static_cast<size_t>(o) * ldm + t;
+            if (!init) {
+                const double term = 0.5 * dt * (prev[k] + v) - comp[k];
+                const double s = acc[k] + term;
+                comp[k] = (s - acc[k]) - term;
+                acc[k] = s;
+            }
+            prev[k] = v;
+        } else {
+            v = sqrt(v);
+            beta0[t] = v;
+            inv0[t] = v > 0.0 ? 1.0 / v : 0.0;
+        }
+        if (!isfinite(v)) atomicOr(status, 2);
+        __threadfence();
     }
     __syncthreads();
-    if (threadIdx.x < nobs) {
-        double s = 0.0;
-        for (int w = 0; w < (blockDim.x >> 5); ++w) s += red[threadIdx.x][w];
-        values_out[threadIdx.x] = s;
+    if (threadIdx.x == 0 && y == 0) last = atomicAdd(count, 1) == static_cast<int>(gridDim.x * gridDim.y) - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int tid = y * 32 + threadIdx.x;
+    double ens[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int k = tid; k < M; k += 1024)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (i < nobs) ens[i] += __ldcg(prev + static_cast<size_t>(i) * ldm + k);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const double v = warp_sum(ens[i]);
+        if (threadIdx.x == 0) red[i][y] = v;
     }
+    __syncthreads();
+    if (tid < nobs) {
+        double s = 0.0;
+        for (int w = 0; w < 32; ++w) s += red[tid][w];
+        values_out[tid] = s;
+    }
+    if (tid == 0) *count = 0;
 }
 
 // values[s][o] = sum over trajectories of traj_values[s][t][o] (fixed order);
