@@ -1227,6 +1227,7 @@ int build_quartet(msgpu_ctx *c)
     };
     std::vector<Block> blocks;
     std::vector<int> ord;
+    std::map<std::array<double, 9>, int> shared;  // values of a block of type 4 or 5 -> their offset
     // storage order (4 a + b) of each block type, see QuartetC
     static const int kOrder[6][16] = {{0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15},
                                       {0, 2, 8, 10, 5, 7, 13, 15},
@@ -1297,6 +1298,22 @@ int build_quartet(msgpu_ctx *c)
             // acts on one digit; A (x) I when both halves of the other digit agree
             else if (e1only) type = same(0, 5) && same(2, 7) && same(8, 13) && same(10, 15) ? 4 : 1;
             else if (e2only) type = same(0, 10) && same(1, 11) && same(4, 14) && same(5, 15) ? 5 : 2;
+            // blocks A (x) I with the same four values share them: a nucleus' flip
+            // block takes two values over all quartets, so they stay in L1 (D =
+            // 16384, 1024 trajectories complex64: 101.6 to 99.2 ms for 20 steps)
+            if (type >= 4) {
+                std::array<double, 9> key;
+                key[8] = type;
+                for (int k = 0; k < 4; ++k) {
+                    key[2 * k] = B[2 * kOrder[type][k]];
+                    key[2 * k + 1] = B[2 * kOrder[type][k] + 1];
+                }
+                const auto at = shared.emplace(key, static_cast<int>(vals.size() / 4));
+                if (!at.second) {
+                    blks.push_back({(blk.base << 3) | type, at.first->second});
+                    continue;
+                }
+            }
             blks.push_back({(blk.base << 3) | type, static_cast<int>(vals.size() / 4)});
             for (int k = 0; k < kCount[type]; ++k) {
                 const int x = kOrder[type][k];
