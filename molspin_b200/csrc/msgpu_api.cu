@@ -17,6 +17,7 @@
 #include "msgpu_dense.h"
 #include "msgpu_fused.cuh"
 #include "msgpu_kernels.cuh"
+#include "msgpu_quartet.h"
 #include "msgpu_resident.h"
 #include "msgpu_spmm_tc.cuh"
 #include "msgpu_spmm_tm.cuh"
@@ -61,7 +62,8 @@ struct msgpu_ctx {
     // quartet-block form of H for the current electron strides
     DevBuf qrow, qcolt, qval, qbase;
     DevBuf qval64;  // the quartet values in FP64 (complex128 Arnoldi apply)
-    int q_s1 = 0, q_s2 = 0, q_D = 0, q_nblocks = 0;
+    int q_s1 = 0, q_s2 = 0, q_D = 0, q_nblocks = 0, q_neighbours = 0;
+    DevBuf rqbuf;                     // ResidentQuartets of the resident form
     long long q_build = 0;            // counts quartet-form builds
     std::vector<int> q_hrow;          // host copies of the quartet form
     std::vector<int2> q_hblk;
@@ -363,7 +365,7 @@ void msgpu_destroy(msgpu_ctx *c)
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     collect_profile(c);
-    DevBuf *all[] = {&c->hrow, &c->hcol, &c->hval, &c->hhi, &c->ell, &c->qrow, &c->qcolt, &c->qval, &c->qbase, &c->qval64,
+    DevBuf *all[] = {&c->hrow, &c->hcol, &c->hval, &c->hhi, &c->ell, &c->rqbuf, &c->qrow, &c->qcolt, &c->qval, &c->qbase, &c->qval64,
                      &c->fblk, &c->fval, &c->frow, &c->fdsrc, &c->fdiag, &c->krow, &c->kcol, &c->kval, &c->bits,
                      &c->psi128, &c->basis, &c->wbuf, &c->zbuf, &c->ubuf, &c->part, &c->part2, &c->hess,
                      &c->tdiag, &c->toff, &c->coef, &c->mdim, &c->scale, &c->alpha, &c->beta0, &c->qpart_obs,
@@ -1046,6 +1048,81 @@ bool pair_reaction(const msgpu_ctx *c, ArnoldiPairK *out, double rel_tol = 1e-12
     return true;
 }
 
+// Quartet-block form of H for the current electron strides (see QuartetC).
+// B-operand tables of the tensor-core SpMM from the current quartet values.
+int tc_tables(msgpu_ctx *c)
+{
+    if (!c->tc_ok) return MSGPU_OK;
+    k_tc_tables<<<c->tc_entries, 128, 0, c->stream>>>(static_cast<const int2 *>(c->tc_src.p), c->tc_entries,
+                                                      static_cast<const float4 *>(c->qval.p),
+                                                      static_cast<unsigned char *>(c->tc_tab.p));
+    k_tm_tables<<<ceil_div(8 * c->tc_entries, 256), 256, 0, c->stream>>>(
+        static_cast<const int2 *>(c->tc_src.p), 2 * c->tc_P, c->tc_entries, static_cast<const float4 *>(c->qval.p),
+        static_cast<float4 *>(c->tm_tab.p));
+    const cudaError_t e = cudaGetLastError();
+    return e ? cuda_fail(c, e, "tensor-core SpMM tables") : MSGPU_OK;
+}
+
+int refresh_quartet_values(msgpu_ctx *c)
+{
+    if (!c->q_nslots) return MSGPU_OK;
+    k_quartet_refresh<<<static_cast<unsigned>((c->q_nslots + 255) / 256), 256, 0, c->stream>>>(
+        static_cast<const int *>(c->qsrc.p), c->q_nslots, static_cast<const double2 *>(c->hval.p),
+        static_cast<float2 *>(c->qval.p), static_cast<double2 *>(c->qval64.p));
+    const cudaError_t e = cudaGetLastError();
+    if (e) return cuda_fail(c, e, "quartet value refresh");
+    return c->tc_build == c->q_build ? tc_tables(c) : MSGPU_OK;
+}
+
+int build_quartet(msgpu_ctx *c)
+{
+    if (c->q_D == c->D && c->q_s1 == c->s1 && c->q_s2 == c->s2) return MSGPU_OK;
+    const int D = c->D, s1 = c->s1, s2 = c->s2, Q = D / 4;
+    QuartetForm f = quartet_form(D, s1, s2, c->h_rowptr.data(), c->h_col.data(), c->h_val.data(), c->terms);
+    std::vector<int> &rowptr = f.rowptr, &base = f.base, &src = f.src;
+    std::vector<int2> &blks = f.blk;
+    std::vector<float> &vals = f.val;
+    std::vector<double> &vals64 = f.val64;
+    const int nb = static_cast<int>(blks.size());
+    int rc;
+    if ((rc = ensure(c, c->qrow, sizeof(int) * (Q + 1), "quartet rowptr")) ||
+        (rc = ensure(c, c->qcolt, sizeof(int2) * std::max(1, nb), "quartet blocks")) ||
+        (rc = ensure(c, c->qval, sizeof(float) * std::max<size_t>(4, vals.size()), "quartet values")) ||
+        (rc = ensure(c, c->qval64, sizeof(double) * std::max<size_t>(4, vals64.size()), "quartet values (FP64)")) ||
+        (rc = ensure(c, c->qbase, sizeof(int) * Q, "quartet bases")))
+        return rc;
+    cudaError_t e;
+    if ((e = cudaMemcpyAsync(c->qrow.p, rowptr.data(), sizeof(int) * (Q + 1), cudaMemcpyHostToDevice, c->stream)) ||
+        (e = cudaMemcpyAsync(c->qcolt.p, blks.data(), sizeof(int2) * nb, cudaMemcpyHostToDevice, c->stream)) ||
+        (e = cudaMemcpyAsync(c->qval.p, vals.data(), sizeof(float) * vals.size(), cudaMemcpyHostToDevice, c->stream)) ||
+        (e = cudaMemcpyAsync(c->qval64.p, vals64.data(), sizeof(double) * vals64.size(), cudaMemcpyHostToDevice,
+                             c->stream)) ||
+        (e = cudaMemcpyAsync(c->qbase.p, base.data(), sizeof(int) * Q, cudaMemcpyHostToDevice, c->stream)) ||
+        (e = cudaStreamSynchronize(c->stream)))
+        return cuda_fail(c, e, "quartet upload");
+    c->q_D = D;
+    c->q_s1 = s1;
+    c->q_s2 = s2;
+    c->q_nblocks = nb;
+    c->q_neighbours = f.neighbours;
+    ++c->q_build;
+    c->q_hrow = std::move(rowptr);
+    c->q_hblk = std::move(blks);
+    c->q_hval = std::move(vals);
+    c->q_tile = 0;
+    c->q_nslots = src.size();
+    if (c->terms) {
+        // the structure came from a generic combination of the terms; the
+        // values of the current coefficients come from the device CSR
+        if ((rc = ensure(c, c->qsrc, sizeof(int) * std::max<size_t>(1, src.size()), "quartet value map")))
+            return rc;
+        if ((e = cudaMemcpyAsync(c->qsrc.p, src.data(), sizeof(int) * src.size(), cudaMemcpyHostToDevice, c->stream)))
+            return cuda_fail(c, e, "quartet value map");
+        if ((rc = refresh_quartet_values(c))) return rc;
+    }
+    return MSGPU_OK;
+}
+
 int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
 {
     const int D = c->D, ldm = c->ldm, M = c->M;
@@ -1081,6 +1158,22 @@ int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
     }
     S.kappa = c->k_scalar ? c->kappa : 0.0;
     const bool lanczos = prec == MSGPU_PREC_C64 || lanczos128(c, p);
+    // complex64 above the row form's range: H by quartets
+    bool quartets = prec == MSGPU_PREC_C64 && resident_q_takes(D);
+    if (quartets) {
+        const bool ok = build_quartet(c) == MSGPU_OK &&
+                        ensure(c, c->rqbuf, resident_q_bytes(D / 4, c->q_neighbours), "resident quartets") == MSGPU_OK;
+        if (ok) {
+            ++c->launches;
+            S.rq = resident_q_build(c->rqbuf.p, D / 4, c->s1, c->s2, c->q_neighbours, static_cast<const int *>(c->qrow.p),
+                                    static_cast<const int2 *>(c->qcolt.p), static_cast<const float4 *>(c->qval.p),
+                                    static_cast<const int *>(c->qbase.p), st);
+        } else {  // no room in the memory budget: the row form
+            (void)cudaGetLastError();
+            c->err.clear();
+            quartets = false;
+        }
+    }
     // Coalesced copy of H (three-term recurrence) or G (Arnoldi), unless one long
     // row would blow the padding up or the memory budget has no room for it; the
     // kernel then walks the CSR rows.
@@ -1090,7 +1183,7 @@ int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
     S.kmax = c->max_row + (lanczos ? 0 : krow_max);
     const size_t slots = static_cast<size_t>(D) * S.kmax;
     const size_t esz = prec == MSGPU_PREC_C128 ? sizeof(double2) : sizeof(float2);
-    bool ell = slots > 0 && slots <= 2 * static_cast<size_t>(c->nnz) + 16 * static_cast<size_t>(D);
+    bool ell = !quartets && slots > 0 && slots <= 2 * static_cast<size_t>(c->nnz) + 16 * static_cast<size_t>(D);
     if (ell && ensure(c, c->ell, slots * (esz + sizeof(int)) + D * sizeof(int), "resident H") != MSGPU_OK) {
         (void)cudaGetLastError();
         c->err.clear();
@@ -1151,7 +1244,8 @@ int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
         (e = cudaMemsetAsync(c->status.p, 0, 2 * sizeof(int), st)))
         return cuda_fail(c, e, "resident setup");
     const ResidentShape shape =
-        prec == MSGPU_PREC_C64 ? resident_shape_c64(D, m) : resident_shape_c128(D, m, lanczos);
+        quartets ? resident_shape_q(D, m)
+                 : prec == MSGPU_PREC_C64 ? resident_shape_c64(D, m) : resident_shape_c128(D, m, lanczos);
     {
         Timed tm(c, KC_APPLY);
         if ((e = raise_smem_limit(reinterpret_cast<const void *>(shape.fn), static_cast<int>(shape.smem))))
@@ -1177,191 +1271,6 @@ int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
     c->have_integrals = true;
     if (status & 2) return fail(c, MSGPU_ERR_NONFINITE, "run: non-finite observable or norm on the device");
     if (status & 1) return fail(c, MSGPU_ERR_EXPM, "run: small matrix exponential failed");
-    return MSGPU_OK;
-}
-
-// Quartet-block form of H for the current electron strides (see QuartetC).
-// B-operand tables of the tensor-core SpMM from the current quartet values.
-int tc_tables(msgpu_ctx *c)
-{
-    if (!c->tc_ok) return MSGPU_OK;
-    k_tc_tables<<<c->tc_entries, 128, 0, c->stream>>>(static_cast<const int2 *>(c->tc_src.p), c->tc_entries,
-                                                      static_cast<const float4 *>(c->qval.p),
-                                                      static_cast<unsigned char *>(c->tc_tab.p));
-    k_tm_tables<<<ceil_div(8 * c->tc_entries, 256), 256, 0, c->stream>>>(
-        static_cast<const int2 *>(c->tc_src.p), 2 * c->tc_P, c->tc_entries, static_cast<const float4 *>(c->qval.p),
-        static_cast<float4 *>(c->tm_tab.p));
-    const cudaError_t e = cudaGetLastError();
-    return e ? cuda_fail(c, e, "tensor-core SpMM tables") : MSGPU_OK;
-}
-
-int refresh_quartet_values(msgpu_ctx *c)
-{
-    if (!c->q_nslots) return MSGPU_OK;
-    k_quartet_refresh<<<static_cast<unsigned>((c->q_nslots + 255) / 256), 256, 0, c->stream>>>(
-        static_cast<const int *>(c->qsrc.p), c->q_nslots, static_cast<const double2 *>(c->hval.p),
-        static_cast<float2 *>(c->qval.p), static_cast<double2 *>(c->qval64.p));
-    const cudaError_t e = cudaGetLastError();
-    if (e) return cuda_fail(c, e, "quartet value refresh");
-    return c->tc_build == c->q_build ? tc_tables(c) : MSGPU_OK;
-}
-
-int build_quartet(msgpu_ctx *c)
-{
-    if (c->q_D == c->D && c->q_s1 == c->s1 && c->q_s2 == c->s2) return MSGPU_OK;
-    const int D = c->D, s1 = c->s1, s2 = c->s2, Q = D / 4;
-    const int off[4] = {0, s2, s1, s1 + s2};
-    std::vector<int> rowptr(Q + 1, 0), base(Q);
-    std::vector<int2> blks;
-    std::vector<float> vals;
-    std::vector<double> vals64;  // the same values in FP64
-    std::vector<int> src;        // CSR index per stored value slot
-    blks.reserve(c->nnz / 6 + Q);
-    vals.reserve(2 * static_cast<size_t>(c->nnz));
-    vals64.reserve(2 * static_cast<size_t>(c->nnz));
-    if (c->terms) src.reserve(c->nnz);
-    struct Block {
-        int base;
-        double z[32];  // 16 complex, row-major in the pair index
-        int src[16];   // CSR index of each entry
-    };
-    std::vector<Block> blocks;
-    std::vector<int> ord;
-    std::map<std::array<double, 9>, int> shared;  // values of a block of type 4 or 5 -> their offset
-    // storage order (4 a + b) of each block type, see QuartetC
-    static const int kOrder[6][16] = {{0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15},
-                                      {0, 2, 8, 10, 5, 7, 13, 15},
-                                      {0, 1, 4, 5, 10, 11, 14, 15},
-                                      {0, 5, 10, 15},
-                                      {0, 2, 8, 10},
-                                      {0, 1, 4, 5}};
-    static const int kCount[6] = {16, 8, 8, 4, 4, 4};
-    for (int q = 0; q < Q; ++q) {
-        const int lo = q % s2, mid = (q / s2) % (s1 / (2 * s2)), hi = q / (s1 / 2);
-        const int b = hi * (2 * s1) + mid * (2 * s2) + lo;
-        base[q] = b;
-        size_t nblk = 0;
-        for (int a = 0; a < 4; ++a) {
-            const int r = b + off[a];
-            size_t at = 0;  // rows meet their neighbours in a similar order
-            for (int k = c->h_rowptr[r]; k < c->h_rowptr[r + 1]; ++k) {
-                const int col = c->h_col[k];
-                const int a1 = (col / s1) & 1, a2 = (col / s2) & 1;
-                const int cb = col - a1 * s1 - a2 * s2, bi = 2 * a1 + a2;
-                size_t slot = at;
-                while (slot < nblk && blocks[slot].base != cb) ++slot;
-                if (slot == nblk) {
-                    slot = 0;
-                    while (slot < at && blocks[slot].base != cb) ++slot;
-                    if (slot == at) slot = nblk;
-                }
-                if (slot == nblk) {
-                    if (blocks.size() == nblk) blocks.emplace_back();
-                    Block &z = blocks[nblk++];
-                    z.base = cb;
-                    std::fill(z.z, z.z + 32, 0.0);
-                    std::fill(z.src, z.src + 16, -1);
-                }
-                at = slot;
-                Block &z = blocks[slot];
-                z.src[a * 4 + bi] = k;
-                z.z[2 * (a * 4 + bi)] += c->h_val[2 * static_cast<size_t>(k)];
-                z.z[2 * (a * 4 + bi) + 1] += c->h_val[2 * static_cast<size_t>(k) + 1];
-            }
-        }
-        // by neighbour base, the quartet's own block last (the SpMM reuses its
-        // gathered rows for the alpha partial)
-        ord.resize(nblk);
-        for (size_t i = 0; i < nblk; ++i) ord[i] = static_cast<int>(i);
-        std::sort(ord.begin(), ord.end(), [&](int x, int y) {
-            const bool ox = blocks[x].base == b, oy = blocks[y].base == b;
-            return ox != oy ? oy : blocks[x].base < blocks[y].base;
-        });
-        for (int oi : ord) {
-            const Block &blk = blocks[oi];
-            const double *B = blk.z;
-            double bmax = 0.0;
-            bool e1only = true, e2only = true;
-            for (int a = 0; a < 4; ++a)
-                for (int bb = 0; bb < 4; ++bb) {
-                    const double re = B[2 * (a * 4 + bb)], im = B[2 * (a * 4 + bb) + 1];
-                    if (re == 0.0 && im == 0.0) continue;
-                    bmax = std::max(bmax, std::abs(re) + std::abs(im));
-                    if ((a & 1) != (bb & 1)) e1only = false;  // couples different second digits
-                    if ((a & 2) != (bb & 2)) e2only = false;  // couples different first digits
-                }
-            auto same = [&](int x, int y) {
-                return std::abs(B[2 * x] - B[2 * y]) + std::abs(B[2 * x + 1] - B[2 * y + 1]) <= 1e-13 * bmax;
-            };
-            int type = 0;
-            if (e1only && e2only) type = 3;
-            // acts on one digit; A (x) I when both halves of the other digit agree
-            else if (e1only) type = same(0, 5) && same(2, 7) && same(8, 13) && same(10, 15) ? 4 : 1;
-            else if (e2only) type = same(0, 10) && same(1, 11) && same(4, 14) && same(5, 15) ? 5 : 2;
-            // blocks A (x) I with the same four values share them: a nucleus' flip
-            // block takes two values over all quartets, so they stay in L1 (D =
-            // 16384, 1024 trajectories complex64: 101.6 to 99.2 ms for 20 steps)
-            if (type >= 4) {
-                std::array<double, 9> key;
-                key[8] = type;
-                for (int k = 0; k < 4; ++k) {
-                    key[2 * k] = B[2 * kOrder[type][k]];
-                    key[2 * k + 1] = B[2 * kOrder[type][k] + 1];
-                }
-                const auto at = shared.emplace(key, static_cast<int>(vals.size() / 4));
-                if (!at.second) {
-                    blks.push_back({(blk.base << 3) | type, at.first->second});
-                    continue;
-                }
-            }
-            blks.push_back({(blk.base << 3) | type, static_cast<int>(vals.size() / 4)});
-            for (int k = 0; k < kCount[type]; ++k) {
-                const int x = kOrder[type][k];
-                vals.push_back(static_cast<float>(B[2 * x]));
-                vals.push_back(static_cast<float>(B[2 * x + 1]));
-                vals64.push_back(B[2 * x]);
-                vals64.push_back(B[2 * x + 1]);
-                if (c->terms) src.push_back(blk.src[x]);
-            }
-        }
-        rowptr[q + 1] = static_cast<int>(blks.size());
-    }
-    const int nb = static_cast<int>(blks.size());
-    int rc;
-    if ((rc = ensure(c, c->qrow, sizeof(int) * (Q + 1), "quartet rowptr")) ||
-        (rc = ensure(c, c->qcolt, sizeof(int2) * std::max(1, nb), "quartet blocks")) ||
-        (rc = ensure(c, c->qval, sizeof(float) * std::max<size_t>(4, vals.size()), "quartet values")) ||
-        (rc = ensure(c, c->qval64, sizeof(double) * std::max<size_t>(4, vals64.size()), "quartet values (FP64)")) ||
-        (rc = ensure(c, c->qbase, sizeof(int) * Q, "quartet bases")))
-        return rc;
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(c->qrow.p, rowptr.data(), sizeof(int) * (Q + 1), cudaMemcpyHostToDevice, c->stream)) ||
-        (e = cudaMemcpyAsync(c->qcolt.p, blks.data(), sizeof(int2) * nb, cudaMemcpyHostToDevice, c->stream)) ||
-        (e = cudaMemcpyAsync(c->qval.p, vals.data(), sizeof(float) * vals.size(), cudaMemcpyHostToDevice, c->stream)) ||
-        (e = cudaMemcpyAsync(c->qval64.p, vals64.data(), sizeof(double) * vals64.size(), cudaMemcpyHostToDevice,
-                             c->stream)) ||
-        (e = cudaMemcpyAsync(c->qbase.p, base.data(), sizeof(int) * Q, cudaMemcpyHostToDevice, c->stream)) ||
-        (e = cudaStreamSynchronize(c->stream)))
-        return cuda_fail(c, e, "quartet upload");
-    c->q_D = D;
-    c->q_s1 = s1;
-    c->q_s2 = s2;
-    c->q_nblocks = nb;
-    ++c->q_build;
-    c->q_hrow = std::move(rowptr);
-    c->q_hblk = std::move(blks);
-    c->q_hval = std::move(vals);
-    c->q_tile = 0;
-    c->q_nslots = src.size();
-    if (c->terms) {
-        // the structure came from a generic combination of the terms; the
-        // values of the current coefficients come from the device CSR
-        if ((rc = ensure(c, c->qsrc, sizeof(int) * std::max<size_t>(1, src.size()), "quartet value map")))
-            return rc;
-        if ((e = cudaMemcpyAsync(c->qsrc.p, src.data(), sizeof(int) * src.size(), cudaMemcpyHostToDevice, c->stream)))
-            return cuda_fail(c, e, "quartet value map");
-        if ((rc = refresh_quartet_values(c))) return rc;
-    }
     return MSGPU_OK;
 }
 

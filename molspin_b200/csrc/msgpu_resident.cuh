@@ -196,9 +196,85 @@ struct Rows {
     }
 };
 
+// The observables' table, by one warp (lane o < 8: observable o).
+__device__ __forceinline__ void fill_observables(const ResidentSystem &S, ObsTable &tab, int lane)
+{
+    unsigned mre = 0, mim = 0;
+    if (lane < 8) {
+        int k = 0;
+        for (int a = 0; a < 4; ++a)
+            for (int c = a; c < 4; ++c, ++k) {
+                double2 cc = make_double2(0.0, 0.0);
+                if (lane < S.nobs) {
+                    const double2 p = S.obs[16 * lane + 4 * a + c], q = S.obs[16 * lane + 4 * c + a];
+                    cc = a == c ? make_double2(p.x, 0.0) : make_double2(p.x + q.x, p.y - q.y);
+                }
+                tab.c[k][lane] = cc;
+                if (cc.x != 0.0) mre |= 1u << k;
+                if (cc.y != 0.0) mim |= 1u << k;
+            }
+    }
+    mre = __reduce_or_sync(0xffffffffu, mre);
+    mim = __reduce_or_sync(0xffffffffu, mim);
+    if (lane == 0) {
+        tab.re = mre;
+        tab.im = mim;
+    }
+}
+
+// Adds the quartet z's observables to v[0 .. NO) and its squared norm to v[NO].
+template <int NO>
+__device__ __forceinline__ void pair_observables(const ObsTable &tab, const double2 (&z)[4], double (&v)[NO + 1])
+{
+    const unsigned mre = tab.re, mim = tab.im;
+    v[NO] += (cabs2(z[0]) + cabs2(z[1])) + (cabs2(z[2]) + cabs2(z[3]));
+    int k = 0;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int c = a; c < 4; ++c, ++k) {
+            if ((mre >> k) & 1u) {
+                const double p = fma(z[a].x, z[c].x, z[a].y * z[c].y);
+#pragma unroll
+                for (int o = 0; o < NO; ++o) v[o] = fma(tab.c[k][o].x, p, v[o]);
+            }
+            if ((mim >> k) & 1u) {
+                const double p = fma(z[a].x, z[c].y, -z[a].y * z[c].x);
+#pragma unroll
+                for (int o = 0; o < NO; ++o) v[o] = fma(-tab.c[k][o].y, p, v[o]);
+            }
+        }
+}
+
+// Sums v over the team: val on thread o < nobs (its observable, times the
+// rate), the norm on every thread.  All values go through the warp together
+// (their shuffles overlap), then one barrier.
+template <int W, int NO>
+__device__ __forceinline__ void team_reduce_values(const ResidentSystem &S, double *rede, double (&v)[NO + 1], int lane,
+                                                   int warp, double &val, double &nrm)
+{
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+        for (int o = 0; o <= NO; ++o) v[o] += __shfl_xor_sync(0xffffffffu, v[o], off);
+    if (lane == 0) {
+#pragma unroll
+        for (int o = 0; o < NO; ++o) rede[9 * warp + o] = v[o];
+        rede[9 * warp + 8] = v[NO];
+    }
+    Team<W>::sync();
+    nrm = rede[8];
+#pragma unroll
+    for (int w = 1; w < W; ++w) nrm += rede[9 * w + 8];
+    val = 0.0;
+    if (static_cast<int>(threadIdx.x) < S.nobs) {
+        for (int w = 0; w < W; ++w) val += rede[9 * w + threadIdx.x];
+        val *= S.rates[threadIdx.x];
+    }
+}
+
 // Flips (if set), norm and pair observables of the state x, one quartet per
-// thread; val on thread o < nobs (its observable, times the rate), the norm on
-// every thread.  NO: 4 or 8 observable slots.
+// thread.  NO: 4 or 8 observable slots.
 template <typename T, int W, int NO>
 __device__ __forceinline__ void resident_evaluate(const ResidentSystem &S, const ResidentSmem<T> &sm, T *x, int flip,
                                                   double &val, double &nrm)
@@ -207,7 +283,6 @@ __device__ __forceinline__ void resident_evaluate(const ResidentSystem &S, const
     double v[NO + 1];  // observables, then the squared norm
 #pragma unroll
     for (int o = 0; o <= NO; ++o) v[o] = 0.0;
-    const unsigned mre = sm.obs->re, mim = sm.obs->im;
     for (int q = threadIdx.x; q < Q; q += 32 * W) {
         const int base = quartet_base(q, S.s1, S.s2);
         const int r[4] = {base, base + S.s2, base + S.s1, base + S.s1 + S.s2};
@@ -223,43 +298,9 @@ __device__ __forceinline__ void resident_evaluate(const ResidentSystem &S, const
 #pragma unroll
             for (int a = 0; a < 4; ++a) st2(x + r[a], z[a]);
         }
-        v[NO] += (cabs2(z[0]) + cabs2(z[1])) + (cabs2(z[2]) + cabs2(z[3]));
-        int k = 0;
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int c = a; c < 4; ++c, ++k) {
-                if ((mre >> k) & 1u) {
-                    const double p = fma(z[a].x, z[c].x, z[a].y * z[c].y);
-#pragma unroll
-                    for (int o = 0; o < NO; ++o) v[o] = fma(sm.obs->c[k][o].x, p, v[o]);
-                }
-                if ((mim >> k) & 1u) {
-                    const double p = fma(z[a].x, z[c].y, -z[a].y * z[c].x);
-#pragma unroll
-                    for (int o = 0; o < NO; ++o) v[o] = fma(-sm.obs->c[k][o].y, p, v[o]);
-                }
-            }
+        pair_observables<NO>(*sm.obs, z, v);
     }
-    // all values through the warp together (their shuffles overlap), one barrier
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-        for (int o = 0; o <= NO; ++o) v[o] += __shfl_xor_sync(0xffffffffu, v[o], off);
-    if (lane == 0) {
-#pragma unroll
-        for (int o = 0; o < NO; ++o) sm.rede[9 * warp + o] = v[o];
-        sm.rede[9 * warp + 8] = v[NO];
-    }
-    Team<W>::sync();
-    nrm = sm.rede[8];
-#pragma unroll
-    for (int w = 1; w < W; ++w) nrm += sm.rede[9 * w + 8];
-    val = 0.0;
-    if (static_cast<int>(threadIdx.x) < S.nobs) {
-        for (int w = 0; w < W; ++w) val += sm.rede[9 * w + threadIdx.x];
-        val *= S.rates[threadIdx.x];
-    }
+    team_reduce_values<W, NO>(S, sm.rede, v, lane, warp, val, nrm);
 }
 
 template <typename T, int W>
@@ -489,30 +530,7 @@ __device__ __forceinline__ void resident_propagate(const ResidentSystem &S, int 
         const int r = tid + NT * i;
         if (r < D) st2(x + r, ld2(in + static_cast<size_t>(r) * S.rs));
     }
-    // observables in upper-triangle form, lane o < 8: observable o
-    if (warp == 0) {
-        unsigned mre = 0, mim = 0;
-        if (lane < 8) {
-            int k = 0;
-            for (int a = 0; a < 4; ++a)
-                for (int c = a; c < 4; ++c, ++k) {
-                    double2 cc = make_double2(0.0, 0.0);
-                    if (lane < S.nobs) {
-                        const double2 p = S.obs[16 * lane + 4 * a + c], q = S.obs[16 * lane + 4 * c + a];
-                        cc = a == c ? make_double2(p.x, 0.0) : make_double2(p.x + q.x, p.y - q.y);
-                    }
-                    sm.obs->c[k][lane] = cc;
-                    if (cc.x != 0.0) mre |= 1u << k;
-                    if (cc.y != 0.0) mim |= 1u << k;
-                }
-        }
-        mre = __reduce_or_sync(0xffffffffu, mre);
-        mim = __reduce_or_sync(0xffffffffu, mim);
-        if (lane == 0) {
-            sm.obs->re = mre;
-            sm.obs->im = mim;
-        }
-    }
+    if (warp == 0) fill_observables(S, *sm.obs, lane);
     const int steps = S.ntimes - 1;
     const long long g0 = S.step_offset;
     const bool noisy = S.nz.mode != 0;

@@ -23,6 +23,15 @@ struct Noise {
 // Entries of a row of H that a one-row thread of the resident form keeps in registers.
 constexpr int kRowRegs = 16;
 
+// H by quartets (msgpu_resident_q.cuh), or null pointers.
+struct ResidentQuartets {
+    const int *nblk;     // [Q]: neighbour blocks of a quartet
+    const int2 *blk;     // [kmax][Q]: {neighbour quartet << 3 | type, value offset}
+    const float4 *val;   // the quartet form's values
+    const float4 *own;   // [8][Q]: own block, columns b as re, im of the four rows
+    int Q, kmax;
+};
+
 struct ResidentSystem {
     // H (rad/ns): row r has rowptr[r + 1] - rowptr[r] entries at rowptr[r] + k
     // (CSR); with kstride > 0 it has rowcnt[r] entries at r + k * kstride (the
@@ -36,6 +45,7 @@ struct ResidentSystem {
     int kstride;
     int kmax;          // longest row
     int generator;
+    ResidentQuartets rq;
     // K: CSR (krow != null) or kappa * I
     const int *krow;
     const int *kcol;
@@ -92,5 +102,13 @@ struct ResidentShape {
 // complex128 (three-term recurrence or Arnoldi), complex64 (three-term).
 ResidentShape resident_shape_c128(int D, int m, bool lanczos);
 ResidentShape resident_shape_c64(int D, int m);
+// complex64 over quartets (msgpu_resident_q.cu): dimensions it takes, its shape,
+// the device bytes of a system's ResidentQuartets (kmax: most neighbour blocks
+// of a quartet) and their set-up in buf from the quartet form's arrays.
+bool resident_q_takes(int D);
+ResidentShape resident_shape_q(int D, int m);
+size_t resident_q_bytes(int Q, int kmax);
+ResidentQuartets resident_q_build(void *buf, int Q, int s1, int s2, int kmax, const int *rowptr, const int2 *blk,
+                                  const float4 *val, const int *base, cudaStream_t st);
 
 }  // namespace msgpu

@@ -1,0 +1,438 @@
+// msgpu_resident_q.cuh -- resident form over quartets, complex64 (D > 128).
+//
+// As msgpu_resident.cuh (one CTA per trajectory for the whole time loop,
+// three-term recurrence), with a thread per quartet instead of per row: a
+// nucleus' flip block is 4 values for 16 matrix entries and one gather serves
+// four rows, and a thread's whole part of H -- its own 4x4 block and up to KF
+// flip blocks -- stays in registers for the whole time loop, so a product
+// reads nothing but the vector in shared memory.  At D = 1024 the row form
+// reads 233 KB of H a product through L2, which sets its time: a step of 256
+// trajectories takes 280 us there against KQTIME here (B200, m = 16).
+//
+// A vector is kept in two planes, re and im, of one float4 a quartet (the
+// quartet's four rows), so that packed FP32 pairs need no shuffling:
+// A (x) I blocks pair the rows of one first digit with broadcast values,
+// I (x) A blocks and the own block pair values with broadcast rows.
+#pragma once
+
+#include "msgpu_resident.cuh"
+
+namespace msgpu {
+namespace {  // internal linkage (see msgpu_kernels.cuh)
+
+// Own block of quartet q to full 4 x 4, columns b: re and im of the four rows.
+__device__ inline void quartet_expand(int type, const float2 *v, float4 (&re)[4], float4 (&im)[4])
+{
+    float r[4][4], i[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int a1 = a >> 1, a2 = a & 1, b1 = b >> 1, b2 = b & 1;
+            float2 z = make_float2(0.f, 0.f);
+            if (type == 0) z = v[4 * a + b];
+            else if (type == 1 && a2 == b2) z = v[(2 * a2 + a1) * 2 + b1];
+            else if (type == 2 && a1 == b1) z = v[(2 * a1 + a2) * 2 + b2];
+            else if (type == 3 && a == b) z = v[a];
+            else if (type == 4 && a2 == b2) z = v[2 * a1 + b1];
+            else if (type == 5 && a1 == b1) z = v[2 * a2 + b2];
+            r[a][b] = z.x;
+            i[a][b] = z.y;
+        }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        re[b] = make_float4(r[0][b], r[1][b], r[2][b], r[3][b]);
+        im[b] = make_float4(i[0][b], i[1][b], i[2][b], i[3][b]);
+    }
+}
+
+// The resident layout from the quartet form (QuartetC): per quartet its
+// neighbour blocks, those of type 4 and 5 first and by distance (a slot then
+// belongs to one nucleus and a warp's lanes meet the same type), and its own
+// block expanded.
+__global__ void k_build_resident_quartets(QuartetC H, int Q, int s1, int s2, int kmax, int *__restrict__ nblk,
+                                          int2 *__restrict__ blk, float4 *__restrict__ own)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= Q) return;
+    const int base = H.base[q];
+    const float2 *val = reinterpret_cast<const float2 *>(H.val);
+    float4 re[4], im[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) re[b] = im[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+    int n = 0;
+    auto key = [&](int2 x) { return (static_cast<long long>((x.x & 7) < 4) << 32) + abs((x.x >> 3) - q); };
+    for (int k = H.rowptr[q]; k < H.rowptr[q + 1]; ++k) {
+        const int2 c = H.blk[k];
+        const int cb = c.x >> 3, type = c.x & 7;
+        if (cb == base) {
+            quartet_expand(type, val + 2 * static_cast<size_t>(c.y), re, im);
+            continue;
+        }
+        const int qn = (cb / (2 * s1)) * (s1 / 2) + ((cb / (2 * s2)) % (s1 / (2 * s2))) * s2 + cb % s2;
+        const int2 x = make_int2((qn << 3) | type, c.y);
+        int at = n++;
+        for (; at > 0 && key(blk[static_cast<size_t>(at - 1) * Q + q]) > key(x); --at)
+            blk[static_cast<size_t>(at) * Q + q] = blk[static_cast<size_t>(at - 1) * Q + q];
+        blk[static_cast<size_t>(at) * Q + q] = x;
+    }
+    nblk[q] = n;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        own[static_cast<size_t>(2 * b) * Q + q] = re[b];
+        own[static_cast<size_t>(2 * b + 1) * Q + q] = im[b];
+    }
+}
+
+struct QuartetAcc {
+    float2 re01, re23, im01, im23;  // rows (0, 1) and (2, 3)
+};
+
+__device__ __forceinline__ float2 bc(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 neg2(float2 x) { return make_float2(-x.x, -x.y); }
+
+// o += A x for a pair of rows, A broadcast
+__device__ __forceinline__ void mac_bcast(float2 &ore, float2 &oim, float2 A, float2 xre, float2 xim)
+{
+    ore = __ffma2_rn(bc(A.x), xre, ore);
+    ore = __ffma2_rn(bc(-A.y), xim, ore);
+    oim = __ffma2_rn(bc(A.x), xim, oim);
+    oim = __ffma2_rn(bc(A.y), xre, oim);
+}
+// o += (c_0 x, c_1 x) for a pair of rows, x broadcast
+__device__ __forceinline__ void mac_pair(float2 &ore, float2 &oim, float2 cre, float2 cim, float xre, float xim)
+{
+    ore = __ffma2_rn(cre, bc(xre), ore);
+    ore = __ffma2_rn(neg2(cim), bc(xim), ore);
+    oim = __ffma2_rn(cre, bc(xim), oim);
+    oim = __ffma2_rn(cim, bc(xre), oim);
+}
+
+// One flip block, values A00 A01 | A10 A11 as two float4.
+__device__ __forceinline__ void flip_mac(QuartetAcc &o, bool second, float4 p, float4 q, float4 xr, float4 xi)
+{
+    if (!second) {  // A (x) I: acts on the first digit
+        const float2 r01 = make_float2(xr.x, xr.y), r23 = make_float2(xr.z, xr.w);
+        const float2 i01 = make_float2(xi.x, xi.y), i23 = make_float2(xi.z, xi.w);
+        mac_bcast(o.re01, o.im01, make_float2(p.x, p.y), r01, i01);
+        mac_bcast(o.re01, o.im01, make_float2(p.z, p.w), r23, i23);
+        mac_bcast(o.re23, o.im23, make_float2(q.x, q.y), r01, i01);
+        mac_bcast(o.re23, o.im23, make_float2(q.z, q.w), r23, i23);
+    } else {  // I (x) A: acts on the second digit
+        const float2 c0r = make_float2(p.x, q.x), c0i = make_float2(p.y, q.y);
+        const float2 c1r = make_float2(p.z, q.z), c1i = make_float2(p.w, q.w);
+        mac_pair(o.re01, o.im01, c0r, c0i, xr.x, xi.x);
+        mac_pair(o.re01, o.im01, c1r, c1i, xr.y, xi.y);
+        mac_pair(o.re23, o.im23, c0r, c0i, xr.z, xi.z);
+        mac_pair(o.re23, o.im23, c1r, c1i, xr.w, xi.w);
+    }
+}
+
+// o += B x, B full with columns (re[b], im[b])
+__device__ __forceinline__ void full_mac(QuartetAcc &o, const float4 (&re)[4], const float4 (&im)[4], float4 xr, float4 xi)
+{
+    const float x[4] = {xr.x, xr.y, xr.z, xr.w}, y[4] = {xi.x, xi.y, xi.z, xi.w};
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        mac_pair(o.re01, o.im01, make_float2(re[b].x, re[b].y), make_float2(im[b].x, im[b].y), x[b], y[b]);
+        mac_pair(o.re23, o.im23, make_float2(re[b].z, re[b].w), make_float2(im[b].z, im[b].w), x[b], y[b]);
+    }
+}
+
+// A thread's quartet of H: its own block and the first KF flip blocks in
+// registers (absent ones: value 0 on the quartet itself); further blocks and
+// types other than 4 and 5 are read on each product.
+template <int KF>
+struct QuartetRow {
+    int q, n, nreg;     // quartet, neighbour blocks, those of them in registers
+    int nb[KF];
+    unsigned second;    // bit k: block k acts on the second digit
+    float4 p[KF], r[KF];
+    float4 ore[4], oim[4];
+
+    __device__ void load(const ResidentQuartets &H, int q_, bool live)
+    {
+        q = live ? q_ : 0;
+        n = live ? __ldg(H.nblk + q) : 0;
+        nreg = 0;
+        second = 0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            ore[b] = live ? __ldg(H.own + static_cast<size_t>(2 * b) * H.Q + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+            oim[b] = live ? __ldg(H.own + static_cast<size_t>(2 * b + 1) * H.Q + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int k = 0; k < KF; ++k) {
+            nb[k] = q;
+            p[k] = r[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (k < n) {
+                const int2 x = __ldg(H.blk + static_cast<size_t>(k) * H.Q + q);
+                const int type = x.x & 7;
+                if (type >= 4) {
+                    nb[k] = x.x >> 3;
+                    p[k] = __ldg(H.val + x.y);
+                    r[k] = __ldg(H.val + x.y + 1);
+                    if (type == 5) second |= 1u << k;
+                    nreg = k + 1;
+                }
+            }
+        }
+    }
+    // H x at the quartet; xr, xi: its own rows; re, im: the vector's planes
+    __device__ QuartetAcc apply(const ResidentQuartets &H, const float4 *re, const float4 *im, float4 xr, float4 xi) const
+    {
+        QuartetAcc o;
+        o.re01 = o.re23 = o.im01 = o.im23 = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < KF; ++k) {
+            if (k >= H.kmax) break;
+            flip_mac(o, (second >> k) & 1u, p[k], r[k], re[nb[k]], im[nb[k]]);
+        }
+        full_mac(o, ore, oim, xr, xi);
+        for (int k = nreg; k < n; ++k) {
+            const int2 x = __ldg(H.blk + static_cast<size_t>(k) * H.Q + q);
+            const int type = x.x & 7, m = x.x >> 3;
+            if (type >= 4) {
+                flip_mac(o, type == 5, __ldg(H.val + x.y), __ldg(H.val + x.y + 1), re[m], im[m]);
+            } else {
+                float4 br[4], bi[4];
+                quartet_expand(type, reinterpret_cast<const float2 *>(H.val) + 2 * static_cast<size_t>(x.y), br, bi);
+                full_mac(o, br, bi, re[m], im[m]);
+            }
+        }
+        return o;
+    }
+};
+
+struct QuartetSmem {
+    float4 *V;          // slot j: re plane at V + 2 j Q, im plane Q further; slot 0 is the state
+    double2 *Hm;        // alpha_j, beta_{j+1}
+    double *sc;         // 1 / |w_j|
+    double2 *cf;        // combination coefficients
+    double *red, *rede;
+    ObsTable *obs;
+    int *flags;
+    size_t bytes;
+};
+
+__host__ __device__ inline QuartetSmem quartet_carve(unsigned char *base, int Q, int m, int W)
+{
+    SmemCarve c{base, 0};
+    QuartetSmem s;
+    s.V = c.take<float4>(2 * static_cast<size_t>(Q) * m);
+    s.Hm = c.take<double2>(m);
+    s.sc = c.take<double>(m);
+    s.cf = c.take<double2>(m);
+    s.red = c.take<double>(2 * W);
+    s.rede = c.take<double>(9 * W);
+    s.obs = c.take<ObsTable>(1);
+    s.flags = c.take<int>(2);
+    s.bytes = c.off;
+    return s;
+}
+
+// Flip, norm and observables of the thread's quartet z, which is written back
+// to the state when it flipped.
+template <int W, int NO>
+__device__ __forceinline__ void quartet_evaluate(const ResidentSystem &S, const QuartetSmem &sm, bool live, int flip,
+                                                 double2 (&z)[4], double &val, double &nrm)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double v[NO + 1];
+#pragma unroll
+    for (int o = 0; o <= NO; ++o) v[o] = 0.0;
+    if (live) {
+        if (flip) {  // U = PS - PT on the pair
+            const double2 b = z[1];
+            z[0] = make_double2(-z[0].x, -z[0].y);
+            z[1] = make_double2(-z[2].x, -z[2].y);
+            z[2] = make_double2(-b.x, -b.y);
+            z[3] = make_double2(-z[3].x, -z[3].y);
+        }
+        pair_observables<NO>(*sm.obs, z, v);
+    }
+    team_reduce_values<W, NO>(S, sm.rede, v, lane, warp, val, nrm);
+}
+
+template <typename TS, int W, int KF>
+__device__ __forceinline__ void resident_quartet_propagate(const ResidentSystem &S, int t, unsigned char *smem,
+                                                           int *__restrict__ status)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_uniform(tid >> 5);
+    const int Q = S.D / 4, m = S.m;
+    const bool live = tid < Q;
+    const QuartetSmem sm = quartet_carve(smem, Q, m, W);
+    float4 *Vre = sm.V, *Vim = sm.V + Q;
+    QuartetRow<KF> H;
+    H.load(S.rq, tid, live);
+    const TS *in = static_cast<const TS *>(S.psi) + static_cast<size_t>(t) * S.ts;
+    size_t row[4];
+    {
+        const int base = live ? quartet_base(tid, S.s1, S.s2) : 0;
+        row[0] = static_cast<size_t>(base) * S.rs;
+        row[1] = static_cast<size_t>(base + S.s2) * S.rs;
+        row[2] = static_cast<size_t>(base + S.s1) * S.rs;
+        row[3] = static_cast<size_t>(base + S.s1 + S.s2) * S.rs;
+    }
+    double2 z[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        z[a] = live ? ld2(in + row[a]) : make_double2(0.0, 0.0);
+        z[a] = make_double2(static_cast<float>(z[a].x), static_cast<float>(z[a].y));
+    }
+    auto store = [&](int slot, const double2 (&w)[4]) {
+        if (!live) return;
+        Vre[2 * slot * Q + tid] = make_float4(static_cast<float>(w[0].x), static_cast<float>(w[1].x),
+                                              static_cast<float>(w[2].x), static_cast<float>(w[3].x));
+        Vim[2 * slot * Q + tid] = make_float4(static_cast<float>(w[0].y), static_cast<float>(w[1].y),
+                                              static_cast<float>(w[2].y), static_cast<float>(w[3].y));
+    };
+    if (warp == 0) fill_observables(S, *sm.obs, lane);
+    const int steps = S.ntimes - 1;
+    const long long g0 = S.step_offset;
+    const bool noisy = S.nz.mode != 0;
+    if (tid == 0) sm.flags[0] = noisy && steps > 0 ? noise_bit(S.nz, t, g0, 0, S.pflip[0]) : 0;
+    const bool own = tid < S.nobs;  // thread o < nobs keeps observable o's trapezoid
+    const size_t ak = static_cast<size_t>(tid) * S.acc_ld + t;
+    double acc = 0.0, comp = 0.0, prev = 0.0, val = 0.0, nrm2 = 0.0;
+    if (own && S.accumulate) {
+        acc = S.acc[ak];
+        comp = S.comp[ak];
+    }
+    bool bad = false;
+    Team<W>::sync();
+    auto evaluate = [&]() {
+        if (S.nobs <= 4) quartet_evaluate<W, 4>(S, sm, live, sm.flags[0], z, val, nrm2);
+        else quartet_evaluate<W, 8>(S, sm, live, sm.flags[0], z, val, nrm2);
+    };
+    evaluate();
+    prev = val;
+    if (S.traj_values && own) S.traj_values[static_cast<size_t>(t) * S.nobs + tid] = val;
+    for (int s = 0; s < steps; ++s) {
+        const double dt = S.times ? S.times[s + 1] - S.times[s] : S.dt0;
+        const double inv0 = rsqrt(nrm2), beta0 = nrm2 > 0.0 ? nrm2 * inv0 : 0.0;
+        auto draw_flip = [&]() {
+            if (warp == W - 1 && lane == 0) {
+                int f = 0;
+                if (noisy) {
+                    f = noise_bit(S.nz, t, g0 + s, 1, S.pflip[s]);
+                    if (s + 1 < steps) f ^= noise_bit(S.nz, t, g0 + s + 1, 0, S.pflip[s + 1]);
+                }
+                sm.flags[0] = f;
+            }
+        };
+        if (beta0 > 0.0) {
+            // three-term recurrence, as resident_lanczos
+            store(0, z);
+            double sj = inv0, bprev = 0.0;
+            double2 vc[4], vp[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                vc[a] = cscale(z[a], sj);
+                vp[a] = make_double2(0.0, 0.0);
+            }
+            if (tid == 0) sm.sc[0] = sj;
+            Team<W>::sync();
+            int n = m;
+            for (int j = 0; j < m; ++j) {
+                const float4 *re = Vre + 2 * j * Q, *im = Vim + 2 * j * Q;
+                double2 u[4];
+                {
+                    const float4 xr = re[H.q], xi = im[H.q];
+                    const QuartetAcc o = H.apply(S.rq, re, im, xr, xi);
+                    u[0] = make_double2(o.re01.x * sj, o.im01.x * sj);
+                    u[1] = make_double2(o.re01.y * sj, o.im01.y * sj);
+                    u[2] = make_double2(o.re23.x * sj, o.im23.x * sj);
+                    u[3] = make_double2(o.re23.y * sj, o.im23.y * sj);
+                }
+                double pa = 0.0, pb = 0.0;
+                if (live) {
+                    pa = fma(vc[0].x, u[0].x, fma(vc[0].y, u[0].y, fma(vc[1].x, u[1].x, vc[1].y * u[1].y)));
+                    pb = fma(vc[2].x, u[2].x, fma(vc[2].y, u[2].y, fma(vc[3].x, u[3].x, vc[3].y * u[3].y)));
+                }
+                const double alpha = Team<W>::sum(pa + pb, sm.red);
+                if (j == m - 1) {  // T_m is complete; w_m is never used
+                    if (tid == 0) sm.Hm[j] = make_double2(alpha, 0.0);
+                    break;
+                }
+                double pn = 0.0;
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    double2 w = make_double2(fma(-bprev, vp[a].x, u[a].x), fma(-bprev, vp[a].y, u[a].y));
+                    w = make_double2(fma(-alpha, vc[a].x, w.x), fma(-alpha, vc[a].y, w.y));
+                    // the stored (rounded) vector is the one the norm and the next product see
+                    u[a] = make_double2(static_cast<float>(w.x), static_cast<float>(w.y));
+                    pn += cabs2(u[a]);
+                }
+                store(j + 1, u);
+                const double nn = Team<W>::sum(live ? pn : 0.0, sm.red + W);
+                sj = rsqrt(nn);
+                const double bn = nn > 0.0 ? nn * sj : 0.0;
+                if (tid == 0) {
+                    sm.Hm[j] = make_double2(alpha, bn);
+                    sm.sc[j + 1] = sj;
+                }
+                if (__any_sync(0xffffffffu, bn < 1e-14)) { n = j + 1; break; }
+                bprev = bn;
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    vp[a] = vc[a];
+                    vc[a] = cscale(u[a], sj);
+                }
+            }
+            if (warp == 0) {
+                __syncwarp();
+                const double d = lane < n ? sm.Hm[lane].x : 0.0;
+                const double lo = (lane < n && lane > 0) ? sm.Hm[lane - 1].y : 0.0;
+                const double hi = lane + 1 < n ? sm.Hm[lane].y : 0.0;
+                double2 c;
+                const bool ok = warp_tridiag_expm_e1(n, d, lo, hi, S.kappa, dt, c);
+                if (!ok && lane == 0) atomicOr(status, 1);
+                if (lane < n) sm.cf[lane] = ok ? cscale(c, beta0 * sm.sc[lane]) : make_double2(0.0, 0.0);
+            }
+            draw_flip();
+            Team<W>::sync();
+#pragma unroll
+            for (int a = 0; a < 4; ++a) z[a] = make_double2(0.0, 0.0);
+            if (live) {
+#pragma unroll 2
+                for (int j = 0; j < n; ++j) {
+                    const double2 c = sm.cf[j];
+                    const float4 xr = Vre[2 * j * Q + tid], xi = Vim[2 * j * Q + tid];
+                    z[0] = cfma(c, make_double2(xr.x, xi.x), z[0]);
+                    z[1] = cfma(c, make_double2(xr.y, xi.y), z[1]);
+                    z[2] = cfma(c, make_double2(xr.z, xi.z), z[2]);
+                    z[3] = cfma(c, make_double2(xr.w, xi.w), z[3]);
+                }
+#pragma unroll
+                for (int a = 0; a < 4; ++a) z[a] = make_double2(static_cast<float>(z[a].x), static_cast<float>(z[a].y));
+            }
+        } else {
+            draw_flip();
+            Team<W>::sync();
+        }
+        evaluate();
+        if (own) {
+            const double term = 0.5 * dt * (prev + val) - comp;
+            const double sum = acc + term;
+            comp = (sum - acc) - term;
+            acc = sum;
+            prev = val;
+            if (!isfinite(val)) bad = true;
+            if (S.traj_values) S.traj_values[(static_cast<size_t>(s + 1) * S.M + t) * S.nobs + tid] = val;
+        }
+    }
+    TS *out = static_cast<TS *>(S.psi_out) + static_cast<size_t>(t) * S.ts;
+    if (live)
+#pragma unroll
+        for (int a = 0; a < 4; ++a) st2(out + row[a], z[a]);
+    if (own) {
+        S.acc[ak] = acc;
+        S.comp[ak] = comp;
+        S.prev[ak] = prev;
+    }
+    if (bad) atomicOr(status, 2);
+}
+
+}  // namespace
+}  // namespace msgpu
