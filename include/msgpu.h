@@ -279,20 +279,22 @@ int msgpu_set_option(msgpu_ctx *ctx, int key, double value);
 int msgpu_get_option(msgpu_ctx *ctx, int key, double *value);
 
 /* ---------------------------------------------------------------- batching
- * Many spin systems of uneven dimension and trajectory count propagated by
- * ONE persistent launch (replayed from a CUDA graph): the loop over
- * orientations / field values / systems of a powder or sweep run
- * (TaskHSGeneral.cpp:347 orientation loop, RunSection::Step sweeps) with each
- * system's HSGeneral time loop inside the launch.  Precision form
+ * Many spin systems of uneven dimension and trajectory count propagated
+ * together: the loop over orientations / field values / systems of a powder or
+ * sweep run (TaskHSGeneral.cpp:347 orientation loop, RunSection::Step sweeps)
+ * with each system's HSGeneral time loop on the device.  Precision form
  * (complex64 vectors, FP64 reductions and yield sums), Lanczos recurrence,
  * K = kappa I, Philox noise keyed by (seed, trajectory, step, half).
- * Systems with dimension >= the team threshold get a whole CTA per
- * trajectory, smaller ones a warp; msgpu_batch_tune picks the threshold and
- * the persistent grid size by timing the batch itself.  Systems of dimension
- * >= 2048 instead run the streamed single-system path (all trajectories in
- * lockstep through the quartet-block SpMM) on their own context and stream,
- * concurrently with the persistent launch; msgpu_batch_run returns when all
- * are done and its stats report the wall time of the whole run. */
+ * Systems of dimension below 2048 whose Krylov basis fits shared memory run
+ * the resident kernels, one launch per system, all at once; the others below
+ * 2048 share one persistent launch (replayed from a CUDA graph) in which
+ * systems with dimension >= the team threshold get a whole CTA per trajectory,
+ * smaller ones a warp.  msgpu_batch_tune picks that threshold and the
+ * persistent grid size by timing the batch itself.  Systems of dimension
+ * >= 2048 run the streamed single-system path (all trajectories in lockstep
+ * through the quartet-block SpMM) on their own context and stream,
+ * concurrently; msgpu_batch_run returns when all are done and its stats report
+ * the wall time of the whole run. */
 typedef struct msgpu_batch msgpu_batch;
 msgpu_batch *msgpu_batch_create(int device, size_t hbm_budget_bytes);
 void msgpu_batch_destroy(msgpu_batch *batch);

@@ -1,17 +1,17 @@
-"""Batching form: many spin systems in one persistent launch.
+"""Batching form: many spin systems propagated together.
 
 The reference propagates the systems of a powder average or parameter sweep
 one after another: the orientation loop of ``TaskHSGeneral::RunLocal``
 (RunSection/General/HS/TaskHSGeneral.cpp:347) and the RunSection step loop
 (main.cpp:651-678) each re-run the whole HSGeneral time loop.  Here every
-(system, trajectory) pair of a system below the streamed-route dimension
-(2048) advances inside ONE persistent kernel launch (msgpu_batch_* in
-include/msgpu.h), replayed from a CUDA graph, with the team threshold and
-grid size chosen by an autotuner on the batch.  Systems at or above that
+system below the streamed-route dimension (2048) runs a resident kernel, a CTA
+per trajectory with the Krylov basis in shared memory, all systems at once
+(msgpu_batch_* in include/msgpu.h); one whose basis does not fit shared memory
+joins a persistent launch, replayed from a CUDA graph, with the team threshold
+and grid size chosen by an autotuner on the batch.  Systems at or above that
 dimension run the streamed precision form (quartet SpMM over the whole
 trajectory block) on their own contexts and streams, concurrently with the
-persistent launch: a persistent team propagates one trajectory at a time
-and re-reads H per trajectory, which loses to the lockstep SpMM there.
+rest: a trajectory of that size no longer fits one CTA's shared memory.
 """
 from __future__ import annotations
 

@@ -62,7 +62,8 @@ struct msgpu_ctx {
     // quartet-block form of H for the current electron strides
     DevBuf qrow, qcolt, qval, qbase;
     DevBuf qval64;  // the quartet values in FP64 (complex128 Arnoldi apply)
-    int q_s1 = 0, q_s2 = 0, q_D = 0, q_nblocks = 0, q_neighbours = 0;
+    int q_s1 = 0, q_s2 = 0, q_D = 0, q_nblocks = 0;
+    msgpu::QuartetSlots q_slots;      // slots of the resident quartet form
     DevBuf rqbuf;                     // ResidentQuartets of the resident form
     long long q_build = 0;            // counts quartet-form builds
     std::vector<int> q_hrow;          // host copies of the quartet form
@@ -1104,7 +1105,7 @@ int build_quartet(msgpu_ctx *c)
     c->q_s1 = s1;
     c->q_s2 = s2;
     c->q_nblocks = nb;
-    c->q_neighbours = f.neighbours;
+    if (resident_q_takes(D)) c->q_slots = quartet_slots(f, s1, s2);
     ++c->q_build;
     c->q_hrow = std::move(rowptr);
     c->q_hblk = std::move(blks);
@@ -1162,10 +1163,10 @@ int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
     bool quartets = prec == MSGPU_PREC_C64 && resident_q_takes(D);
     if (quartets) {
         const bool ok = build_quartet(c) == MSGPU_OK &&
-                        ensure(c, c->rqbuf, resident_q_bytes(D / 4, c->q_neighbours), "resident quartets") == MSGPU_OK;
+                        ensure(c, c->rqbuf, resident_q_bytes(D / 4, c->q_slots), "resident quartets") == MSGPU_OK;
         if (ok) {
             ++c->launches;
-            S.rq = resident_q_build(c->rqbuf.p, D / 4, c->s1, c->s2, c->q_neighbours, static_cast<const int *>(c->qrow.p),
+            S.rq = resident_q_build(c->rqbuf.p, D / 4, c->s1, c->s2, c->q_slots, static_cast<const int *>(c->qrow.p),
                                     static_cast<const int2 *>(c->qcolt.p), static_cast<const float4 *>(c->qval.p),
                                     static_cast<const int *>(c->qbase.p), st);
         } else {  // no room in the memory budget: the row form

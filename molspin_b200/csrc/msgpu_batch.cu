@@ -1,9 +1,12 @@
 // msgpu_batch.cu -- C ABI of the batching form (include/msgpu.h,
 // msgpu_batch_*): many radical-pair systems of uneven dimension and
-// trajectory count propagated together.  Systems below kStreamDim run in
-// one persistent launch (k_batch), replayed from a CUDA graph, with the team
-// threshold and the persistent grid size picked by an autotuner on the batch
-// itself.  A large system is better served by the streamed single-system
+// trajectory count propagated together.  Systems below kStreamDim run the
+// resident kernels (msgpu_resident.cuh, msgpu_resident_q.cuh), a CTA per
+// trajectory with the Krylov basis in shared memory, one launch per system, all
+// launches at once on a few streams.  A system whose basis does not fit shared
+// memory joins the persistent launch k_batch instead, replayed from a CUDA
+// graph, with the team threshold and the grid size picked by an autotuner.  A
+// large system is better served by the streamed single-system
 // path, which advances all its trajectories in lockstep through the
 // quartet-block SpMM (one read of H per 64 trajectories instead of one per
 // trajectory): those systems get their own context and stream and run
@@ -22,6 +25,7 @@
 #include <vector>
 
 #include "msgpu_batch.cuh"
+#include "msgpu_quartet.h"
 
 using namespace msgpu;
 
@@ -43,6 +47,15 @@ struct BatchSystem {
     double kappa = 0.0, st_rate = 0.0;
     unsigned long long seed = 0;
     Buf rowptr, col, valf, obs, rates, psi, acc, comp, prev, pflip;
+    // resident kernels: H in padded row order (ell: values, columns, lengths) up
+    // to D = 128, by quartets (quart) above; kind 0: neither
+    Buf ell, quart;
+    int kind = 0, kmax = 0;
+    ResidentQuartets rq{};
+    // CSR of a system on the quartet kernels, uploaded if a Krylov dimension ever
+    // needs the persistent launch
+    std::vector<int> h_rowptr, h_col;
+    std::vector<float> h_valf;
     msgpu_ctx *ctx = nullptr;  // streamed single-system path (D >= kStreamDim)
 };
 
@@ -64,7 +77,9 @@ struct msgpu_batch {
     size_t graph_key = 0;
     float last_ms = 0.f;
     int m = 0;
-    long long launches = 0;  // persistent launches (tuning probes included)
+    long long launches = 0;  // kernels launched here (tuning probes included)
+    cudaStream_t side[8] = {};  // the resident launches' streams, made on first use
+    cudaEvent_t fork = nullptr, join[8] = {};
 };
 
 namespace {
@@ -119,10 +134,60 @@ void drop_graph(msgpu_batch *b)
 
 double flip_prob(double st_rate, double h) { return -0.5 * std::expm1(-2.0 * (0.5 * st_rate) * h); }
 
-// Descriptors, work items and scratch for the given schedule; returns the
-// grid size through *grid.
+// One system's launch of a resident kernel (a CTA per trajectory).
+struct ResidentLaunch {
+    ResidentSystem S;
+    ResidentShape shape;
+    double cost;  // of one trajectory
+};
+constexpr size_t kResidentSmemMax = 227 * 1024;
+
+// Queues the resident launches, longest trajectories first, over the side
+// streams between two events on the batch's stream.
+int launch_resident(msgpu_batch *b, std::vector<ResidentLaunch> &runs)
+{
+    if (runs.empty()) return MSGPU_OK;
+    std::stable_sort(runs.begin(), runs.end(), [](const ResidentLaunch &x, const ResidentLaunch &y) { return x.cost > y.cost; });
+    const int ns = std::min<int>(8, static_cast<int>(runs.size()));
+    cudaError_t e = cudaSuccess;
+    if (!b->fork) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
+    for (int k = 0; k < ns && !e; ++k)
+        if (!b->side[k] && !(e = cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking)))
+            e = cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming);
+    if (!e) e = cudaEventRecord(b->fork, b->stream);
+    for (int k = 0; k < ns && !e; ++k) e = cudaStreamWaitEvent(b->side[k], b->fork, 0);
+    for (size_t i = 0; i < runs.size() && !e; ++i) {
+        const ResidentLaunch &r = runs[i];
+        if ((e = raise_smem_limit(reinterpret_cast<const void *>(r.shape.fn), static_cast<int>(r.shape.smem)))) break;
+        r.shape.fn<<<r.S.M, 32 * r.shape.warps, r.shape.smem, b->side[i % ns]>>>(r.S, static_cast<int *>(b->status_d.p));
+        ++b->launches;
+        e = cudaGetLastError();
+    }
+    for (int k = 0; k < ns && b->join[k]; ++k) {  // joined even after an error: nothing is left running behind it
+        const cudaError_t je = cudaEventRecord(b->join[k], b->side[k]);
+        const cudaError_t we = cudaStreamWaitEvent(b->stream, b->join[k], 0);
+        if (!e) e = je ? je : we;
+    }
+    return e ? bfail(b, MSGPU_ERR_CUDA, std::string("batch: resident launch: ") + cudaGetErrorString(e)) : MSGPU_OK;
+}
+
+// The CSR arrays that the persistent launch reads.
+int upload_csr(msgpu_batch *b, BatchSystem &s, const int *rowptr, const int *col, const std::vector<float> &val)
+{
+    const int nnz = rowptr[s.D];
+    int rc;
+    if ((rc = upload(b, s.rowptr, rowptr, sizeof(int) * (s.D + 1), "rowptr")) ||
+        (nnz > 0 && (rc = upload(b, s.col, col, sizeof(int) * nnz, "col"))) ||
+        (nnz > 0 && (rc = upload(b, s.valf, val.data(), sizeof(float) * val.size(), "values"))))
+        return rc;
+    return MSGPU_OK;
+}
+
+// Descriptors, work items and scratch for the given schedule, and the resident
+// launches; returns the grid size through *grid.
 int prepare(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_offset, int threshold,
-            int ctas_per_sm, int *grid, size_t *slice, size_t *smem, int *nlarge, int *nitems)
+            int ctas_per_sm, int *grid, size_t *slice, size_t *smem, int *nlarge, int *nitems,
+            std::vector<ResidentLaunch> *resident)
 {
     std::vector<ResidentSystem> desc(b->sys.size());
     std::vector<ResidentWork> large, small;
@@ -148,6 +213,8 @@ int prepare(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_of
         S.nz.M = s.M;
         S.nz.seed = s.seed;
         S.psi = S.psi_out = s.psi.p;
+        S.rs = 1;
+        S.ts = s.D;
         S.acc = static_cast<double *>(s.acc.p);
         S.comp = static_cast<double *>(s.comp.p);
         S.prev = static_cast<double *>(s.prev.p);
@@ -159,6 +226,33 @@ int prepare(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_of
         S.accumulate = accumulate;
         desc[i] = S;
         if (s.ctx) continue;  // streamed path: no work items here
+        if (s.kind) {
+            ResidentShape shape = s.kind == 1 ? resident_shape_c64_state(s.D, S.m) : resident_shape_q_state(s.D, S.m);
+            if (shape.fn && shape.smem <= kResidentSmemMax) {
+                if (s.kind == 1) {
+                    const size_t slots = static_cast<size_t>(s.D) * s.kmax;
+                    S.valf = static_cast<const float2 *>(s.ell.p);
+                    S.col = reinterpret_cast<const int *>(S.valf + slots);
+                    S.rowcnt = S.col + slots;
+                    S.kstride = s.D;
+                    S.kmax = s.kmax;
+                } else {
+                    S.rq = s.rq;
+                }
+                resident->push_back(ResidentLaunch{S, shape, static_cast<double>(s.D) * S.m});
+                continue;
+            }
+        }
+        if (s.kind && !s.h_rowptr.empty()) {
+            if (int rc = upload_csr(b, s, s.h_rowptr.data(), s.h_col.data(), s.h_valf)) return rc;
+            if (cudaStreamSynchronize(b->stream) != cudaSuccess)
+                return bfail(b, MSGPU_ERR_CUDA, "batch: Hamiltonian upload failed");
+            s.h_rowptr.clear();
+            S.rowptr = static_cast<const int *>(s.rowptr.p);
+            S.col = static_cast<const int *>(s.col.p);
+            S.valf = static_cast<const float2 *>(s.valf.p);
+            desc[i] = S;
+        }
         auto &dst = s.D >= threshold ? large : small;
         for (int t = 0; t < s.M; ++t) dst.push_back(ResidentWork{static_cast<int>(i), t});
         if (s.D >= threshold) dmax_large = std::max(dmax_large, s.D);
@@ -179,11 +273,15 @@ int prepare(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_of
     *slice = (std::max(per_large, per_small) + 63) / 64 * 64;
     *grid = std::max(1, b->sm_count * ctas_per_sm);
     *smem = sizeof(double2) * kBatchWarps * batch_expm_words(m);
+    // the Krylov dimensions that the persistent launch takes, on every route
+    if ((!items.empty() || !resident->empty()) && *smem > kResidentSmemMax)
+        return bfail(b, MSGPU_ERR_CUDA, std::string("batch: shared memory: ") + cudaGetErrorString(cudaErrorInvalidValue));
     int rc;
+    if ((rc = bensure(b, b->status_d, sizeof(int), "status"))) return rc;
+    if (items.empty()) return MSGPU_OK;
     if ((rc = upload(b, b->sys_d, desc.data(), sizeof(ResidentSystem) * desc.size(), "descriptors")) ||
-        (rc = upload(b, b->items_d, items.data(), sizeof(ResidentWork) * std::max<size_t>(1, items.size()), "items")) ||
+        (rc = upload(b, b->items_d, items.data(), sizeof(ResidentWork) * items.size(), "items")) ||
         (rc = bensure(b, b->queue_d, 2 * sizeof(int), "queue")) ||
-        (rc = bensure(b, b->status_d, sizeof(int), "status")) ||
         (rc = bensure(b, b->scratch, sizeof(float2) * *slice * *grid, "scratch")))
         return rc;
     return MSGPU_OK;
@@ -200,7 +298,6 @@ int launch(msgpu_batch *b, int grid, size_t slice, size_t smem, int nlarge, int 
                        (reinterpret_cast<size_t>(b->queue_d.p) << 3) ^ (reinterpret_cast<size_t>(b->status_d.p) << 4);
     auto enqueue = [&]() {
         cudaMemsetAsync(b->queue_d.p, 0, 2 * sizeof(int), b->stream);
-        cudaMemsetAsync(b->status_d.p, 0, sizeof(int), b->stream);
         k_batch<<<grid, kBatchThreads, smem, b->stream>>>(
             static_cast<const ResidentSystem *>(b->sys_d.p), static_cast<const ResidentWork *>(b->items_d.p), nlarge,
             nitems, static_cast<int *>(b->queue_d.p), static_cast<float2 *>(b->scratch.p), slice, m,
@@ -229,6 +326,62 @@ int launch(msgpu_batch *b, int grid, size_t slice, size_t smem, int nlarge, int 
     return MSGPU_OK;
 }
 
+// The resident kernels' forms of a system's H.  Without room for them in the
+// memory budget the system takes the persistent launch (kind stays 0).
+void build_rows(msgpu_batch *b, BatchSystem &s, const int *rowptr, const int *col, const std::vector<float> &val, int max_row)
+{
+    const int D = s.D;
+    const size_t slots = static_cast<size_t>(D) * max_row;
+    if (slots == 0) return;
+    std::vector<unsigned char> buf(slots * (sizeof(float2) + sizeof(int)) + D * sizeof(int), 0);
+    float *v = reinterpret_cast<float *>(buf.data());
+    int *c = reinterpret_cast<int *>(buf.data() + slots * sizeof(float2)), *n = c + slots;
+    for (int r = 0; r < D; ++r) {
+        n[r] = rowptr[r + 1] - rowptr[r];
+        for (int k = 0; k < n[r]; ++k) {
+            const size_t e = static_cast<size_t>(k) * D + r, from = rowptr[r] + k;
+            v[2 * e] = val[2 * from];
+            v[2 * e + 1] = val[2 * from + 1];
+            c[e] = col[from];
+        }
+    }
+    if (upload(b, s.ell, buf.data(), buf.size(), "rows") != MSGPU_OK) {
+        (void)cudaGetLastError();
+        b->err.clear();
+        return;
+    }
+    s.kind = 1;
+    s.kmax = max_row;
+}
+
+void build_quartets(msgpu_batch *b, BatchSystem &s, const int *rowptr, const int *col, const double *val)
+{
+    const int Q = s.D / 4;
+    const QuartetForm f = quartet_form(s.D, s.s1, s.s2, rowptr, col, val, false);
+    const QuartetSlots slots = quartet_slots(f, s.s1, s.s2);
+    // one buffer: values (16-byte aligned), the resident arrays, blocks, row pointers, bases
+    auto up = [](size_t n) { return (n + 15) / 16 * 16; };
+    const size_t nval = up(f.val.size() * sizeof(float)), nrq = up(resident_q_bytes(Q, slots));
+    const size_t nblk = up(f.blk.size() * sizeof(int2)), nrow = up(f.rowptr.size() * sizeof(int)), nbase = up(Q * sizeof(int));
+    std::vector<unsigned char> buf(nval + nrq + nblk + nrow + nbase, 0);
+    std::memcpy(buf.data(), f.val.data(), f.val.size() * sizeof(float));
+    std::memcpy(buf.data() + nval + nrq, f.blk.data(), f.blk.size() * sizeof(int2));
+    std::memcpy(buf.data() + nval + nrq + nblk, f.rowptr.data(), f.rowptr.size() * sizeof(int));
+    std::memcpy(buf.data() + nval + nrq + nblk + nrow, f.base.data(), Q * sizeof(int));
+    if (upload(b, s.quart, buf.data(), buf.size(), "quartets") != MSGPU_OK) {
+        (void)cudaGetLastError();
+        b->err.clear();
+        return;
+    }
+    unsigned char *p = static_cast<unsigned char *>(s.quart.p);
+    s.rq = resident_q_build(p + nval, Q, s.s1, s.s2, slots, reinterpret_cast<const int *>(p + nval + nrq + nblk),
+                            reinterpret_cast<const int2 *>(p + nval + nrq), reinterpret_cast<const float4 *>(p),
+                            reinterpret_cast<const int *>(p + nval + nrq + nblk + nrow), b->stream);
+    if (cudaGetLastError() != cudaSuccess) return;
+    ++b->launches;
+    s.kind = 2;
+}
+
 int set_times(msgpu_batch *b, const double *times, int ntimes)
 {
     for (int s = 0; s < ntimes; ++s)
@@ -249,15 +402,22 @@ int run_once(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_o
 {
     int grid, nlarge, nitems;
     size_t slice, smem;
-    if (int rc = prepare(b, ntimes, m, accumulate, step_offset, threshold, cps, &grid, &slice, &smem, &nlarge, &nitems))
+    std::vector<ResidentLaunch> resident;
+    if (int rc = prepare(b, ntimes, m, accumulate, step_offset, threshold, cps, &grid, &slice, &smem, &nlarge, &nitems,
+                         &resident))
         return rc;
+    const bool here = nitems > 0 || !resident.empty();
     const auto w0 = std::chrono::steady_clock::now();
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, b->stream);
-    int rc = nitems > 0 ? launch(b, grid, slice, smem, nlarge, nitems, m, graph) : MSGPU_OK;
-    if (nitems > 0) b->launches += graph ? 1 : 3;  // a replay of the captured graph, or memsets + kernel
+    int rc = MSGPU_OK;
+    if (here && cudaMemsetAsync(b->status_d.p, 0, sizeof(int), b->stream) != cudaSuccess)
+        rc = bfail(b, MSGPU_ERR_CUDA, "batch: status reset failed");
+    if (!rc) rc = launch_resident(b, resident);
+    if (!rc && nitems > 0) rc = launch(b, grid, slice, smem, nlarge, nitems, m, graph);
+    if (nitems > 0) b->launches += graph ? 1 : 2;  // a replay of the captured graph, or memset + kernel
     cudaEventRecord(e1, b->stream);
     // streamed systems (times given: a real run, not a tuning probe), each on
     // its own context and stream, while the persistent launch runs
@@ -299,7 +459,7 @@ int run_once(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_o
             return bfail(b, rcs[k], "batch: system " + std::to_string(routed[k]) + ": " +
                                         msgpu_last_error(b->sys[routed[k]].ctx));
     int status = 0;
-    if (nitems > 0 && (e = cudaMemcpy(&status, b->status_d.p, sizeof(int), cudaMemcpyDeviceToHost)))
+    if (here && (e = cudaMemcpy(&status, b->status_d.p, sizeof(int), cudaMemcpyDeviceToHost)))
         return bfail(b, MSGPU_ERR_CUDA, std::string("batch: status: ") + cudaGetErrorString(e));
     if (status & 2) return bfail(b, MSGPU_ERR_NONFINITE, "batch: non-finite observable on the device");
     if (status & 1) return bfail(b, MSGPU_ERR_EXPM, "batch: small matrix exponential failed");
@@ -337,12 +497,17 @@ void msgpu_batch_destroy(msgpu_batch *b)
     drop_graph(b);
     for (auto *list : {&b->sys, &b->spare})
         for (auto &s : *list) {
-            Buf *all[] = {&s.rowptr, &s.col, &s.valf, &s.obs, &s.rates, &s.psi, &s.acc, &s.comp, &s.prev, &s.pflip};
+            Buf *all[] = {&s.rowptr, &s.col, &s.valf, &s.obs, &s.rates, &s.psi, &s.acc, &s.comp, &s.prev, &s.pflip, &s.ell, &s.quart};
             for (Buf *x : all) brelease(b, *x);
             if (s.ctx) msgpu_destroy(s.ctx);
         }
     Buf *all[] = {&b->sys_d, &b->items_d, &b->queue_d, &b->status_d, &b->scratch, &b->times_d, &b->backup};
     for (Buf *x : all) brelease(b, *x);
+    for (int k = 0; k < 8; ++k) {
+        if (b->join[k]) cudaEventDestroy(b->join[k]);
+        if (b->side[k]) cudaStreamDestroy(b->side[k]);
+    }
+    if (b->fork) cudaEventDestroy(b->fork);
     cudaStreamDestroy(b->stream);
     delete b;
 }
@@ -446,13 +611,23 @@ int msgpu_batch_add_system(msgpu_batch *b, int dim, const int *rowptr, const int
                 op[o * 32 + 2 * (a * 4 + c)] = ops[o * 32 + 2 * (ua * 4 + uc)];
                 op[o * 32 + 2 * (a * 4 + c) + 1] = ops[o * 32 + 2 * (ua * 4 + uc) + 1];
             }
+    s.kind = 0;
+    int max_row = 0;
+    for (int r = 0; r < dim; ++r) max_row = std::max(max_row, rowptr[r + 1] - rowptr[r]);
+    if (dim <= 128) build_rows(b, s, rowptr, col, vf, max_row);
+    else if (resident_q_takes(dim)) build_quartets(b, s, rowptr, col, val);
     std::vector<float> psi(2 * static_cast<size_t>(dim) * ntraj);
     for (size_t i = 0; i < psi.size(); ++i) psi[i] = static_cast<float>(factors[i]);
     std::vector<double> zeros(static_cast<size_t>(nobs) * ntraj, 0.0);
     int rc;
-    if ((rc = upload(b, s.rowptr, rowptr, sizeof(int) * (dim + 1), "rowptr")) ||
-        (rc = upload(b, s.col, col, sizeof(int) * std::max(1, nnz), "col")) ||
-        (rc = upload(b, s.valf, vf.data(), sizeof(float) * std::max<size_t>(2, vf.size()), "values")) ||
+    s.h_rowptr.clear();
+    if (s.kind == 2) {
+        s.h_rowptr.assign(rowptr, rowptr + dim + 1);
+        s.h_col.assign(col, col + nnz);
+        s.h_valf = vf;
+    }
+    // up to D = 128 a basis of any Krylov dimension fits shared memory
+    if ((s.kind == 0 && (rc = upload_csr(b, s, rowptr, col, vf))) ||
         (rc = upload(b, s.obs, op.data(), sizeof(double) * op.size(), "observables")) ||
         (rc = upload(b, s.rates, rates, sizeof(double) * nobs, "rates")) ||
         (rc = upload(b, s.psi, psi.data(), sizeof(float) * psi.size(), "factors")) ||
@@ -492,8 +667,15 @@ int msgpu_batch_tune(msgpu_batch *b, const double *times, int ntimes, int krylov
     const int thresholds[] = {256, 512, 1024, 2048};
     const int cps[] = {1, 2, 3, 4};
     float best = 1e30f;
+    bool persistent = false;  // any system on the persistent launch, which these parameters shape
+    for (auto &s : b->sys) {
+        const int m = std::min(krylov_dim, s.D);
+        persistent = persistent || (!s.ctx && !(s.kind && (s.kind == 1 ? resident_shape_c64_state(s.D, m).smem
+                                                                       : resident_shape_q_state(s.D, m).smem) <= kResidentSmemMax));
+    }
     for (int th : thresholds)
         for (int c : cps) {
+            if (!persistent) break;
             float ms = 0.f;
             if (int rc = run_once(b, ntimes, krylov_dim, 0, 0, th, c, false, &ms)) return rc;
             if (ms < best) {

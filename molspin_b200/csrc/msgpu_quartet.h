@@ -19,8 +19,74 @@ struct QuartetForm {
     std::vector<double> val64;  // the same in FP64
     std::vector<int> base;      // first row of each quartet
     std::vector<int> src;       // CSR index per value slot (want_src)
-    int neighbours = 0;         // most blocks of a quartet beside its own
 };
+
+// Slots of the resident form: neighbour blocks by their distance in quartets,
+// d and -d in one slot when no quartet has both (a spin-1/2 nucleus; a spin-1
+// nucleus takes two).  Only distances whose blocks are all of type 4, or all of
+// type 5, get one; `left` is the most blocks of a quartet without a slot.
+constexpr int kQuartetSlots = 8;
+struct QuartetSlots {
+    int n = 0, left = 0;
+    int delta[kQuartetSlots] = {0};    // distance of slot k
+    unsigned shared = 0, second = 0;   // bit k: -delta too; type 5
+};
+
+inline QuartetSlots quartet_slots(const QuartetForm &f, int s1, int s2)
+{
+    const int Q = static_cast<int>(f.base.size());
+    auto index = [&](int cb) { return (cb / (2 * s1)) * (s1 / 2) + ((cb / (2 * s2)) % (s1 / (2 * s2))) * s2 + cb % s2; };
+    struct Seen {
+        bool uniform = true, both = false;
+        int type = -1;
+        long long count = 0;
+    };
+    std::map<int, Seen> seen;  // by signed distance
+    for (int q = 0; q < Q; ++q)
+        for (int k = f.rowptr[q]; k < f.rowptr[q + 1]; ++k) {
+            const int cb = f.blk[k].x >> 3, type = f.blk[k].x & 7;
+            if (cb == f.base[q]) continue;
+            Seen &s = seen[index(cb) - q];
+            s.uniform = s.uniform && type >= 4 && (s.type < 0 || s.type == type);
+            s.type = type;
+            ++s.count;
+        }
+    for (int q = 0; q < Q; ++q)  // quartets with both d and -d
+        for (int k = f.rowptr[q]; k < f.rowptr[q + 1]; ++k)
+            for (int l = k + 1; l < f.rowptr[q + 1]; ++l) {
+                const int d = index(f.blk[k].x >> 3) - q, e = index(f.blk[l].x >> 3) - q;
+                if (d != 0 && d == -e) seen[d].both = seen[e].both = true;
+            }
+    // the most used first, should there be more than fit
+    std::vector<std::pair<long long, std::pair<int, bool>>> cand;
+    for (auto &x : seen) {
+        auto neg = seen.find(-x.first);
+        const bool pair = neg != seen.end() && !x.second.both && x.second.uniform && neg->second.uniform &&
+                          x.second.type == neg->second.type;
+        if (!x.second.uniform || (pair && x.first < 0)) continue;
+        cand.push_back({-(x.second.count + (pair ? neg->second.count : 0)), {x.first, pair}});
+    }
+    std::sort(cand.begin(), cand.end());
+    QuartetSlots out;
+    for (auto &c : cand) {
+        if (out.n == kQuartetSlots) break;
+        out.delta[out.n] = c.second.first;
+        if (c.second.second) out.shared |= 1u << out.n;
+        if (seen[c.second.first].type == 5) out.second |= 1u << out.n;
+        ++out.n;
+    }
+    for (int q = 0; q < Q; ++q) {
+        int left = 0;
+        for (int k = f.rowptr[q]; k < f.rowptr[q + 1]; ++k) {
+            const int d = index(f.blk[k].x >> 3) - q;
+            bool in = d == 0;
+            for (int i = 0; i < out.n; ++i) in = in || d == out.delta[i] || (((out.shared >> i) & 1u) && d == -out.delta[i]);
+            if (!in) ++left;
+        }
+        out.left = std::max(out.left, left);
+    }
+    return out;
+}
 
 inline QuartetForm quartet_form(int D, int s1, int s2, const int *h_rowptr, const int *h_col, const double *h_val,
                                 bool want_src)
@@ -143,9 +209,6 @@ inline QuartetForm quartet_form(int D, int s1, int s2, const int *h_rowptr, cons
             }
         }
         rowptr[q + 1] = static_cast<int>(blks.size());
-        bool own = false;
-        for (size_t i = 0; i < nblk; ++i) own = own || blocks[i].base == b;
-        f.neighbours = std::max(f.neighbours, static_cast<int>(nblk) - (own ? 1 : 0));
     }
     return f;
 }

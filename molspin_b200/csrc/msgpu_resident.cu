@@ -34,4 +34,13 @@ ResidentShape resident_shape_c128(int D, int m, bool lanczos)
 
 ResidentShape resident_shape_c64(int D, int m) { return resident_shape<float2, true>(D, m); }
 
+ResidentShape resident_shape_c64_state(int D, int m)
+{
+    auto make = [&](ResidentFn fn, int w) { return ResidentShape{fn, w, resident_carve<float2, true>(nullptr, D, m, w).bytes}; };
+    if (D <= 32) return make(&k_resident<float2, 1, 1, true, float2>, 1);
+    if (D <= 64) return make(&k_resident<float2, 2, 1, true, float2>, 2);
+    if (D <= 128) return make(&k_resident<float2, 4, 1, true, float2>, 4);
+    return make(nullptr, 0);
+}
+
 }  // namespace msgpu

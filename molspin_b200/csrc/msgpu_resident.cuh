@@ -663,12 +663,12 @@ template <typename T>
 constexpr int resident_min_ctas(int W) { return sizeof(T) == sizeof(float2) && W <= 16 ? 16 / W : 1; }
 
 // One launch = the whole time loop of every trajectory (one CTA each).
-template <typename T, int W, int RPT, bool kLanczos>
+template <typename T, int W, int RPT, bool kLanczos, typename TS = double2>
 __global__ void __launch_bounds__(32 * W, resident_min_ctas<T>(W))
 k_resident(const __grid_constant__ ResidentSystem S, int *__restrict__ status)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    resident_propagate<T, double2, W, RPT, kLanczos>(S, blockIdx.x, smem_raw, status);
+    resident_propagate<T, TS, W, RPT, kLanczos>(S, blockIdx.x, smem_raw, status);
 }
 
 }  // namespace

@@ -25,11 +25,13 @@ constexpr int kRowRegs = 16;
 
 // H by quartets (msgpu_resident_q.cuh), or null pointers.
 struct ResidentQuartets {
-    const int *nblk;     // [Q]: neighbour blocks of a quartet
-    const int2 *blk;     // [kmax][Q]: {neighbour quartet << 3 | type, value offset}
-    const float4 *val;   // the quartet form's values
     const float4 *own;   // [8][Q]: own block, columns b as re, im of the four rows
-    int Q, kmax;
+    const int2 *slot;    // [nslot][Q]: {neighbour quartet, value offset; the quartet itself and -1 if absent}
+    const int2 *blk;     // [left][Q]: blocks without a slot, {neighbour quartet << 3 | type, value offset}
+    const int *nblk;     // [Q]: their number
+    const float4 *val;   // the quartet form's values
+    int Q, nslot;
+    unsigned second;     // bit k: slot k acts on the second digit
 };
 
 struct ResidentSystem {
@@ -102,13 +104,17 @@ struct ResidentShape {
 // complex128 (three-term recurrence or Arnoldi), complex64 (three-term).
 ResidentShape resident_shape_c128(int D, int m, bool lanczos);
 ResidentShape resident_shape_c64(int D, int m);
+// complex64 on a complex64 state (the batching form); fn null when no shape takes it.
+ResidentShape resident_shape_c64_state(int D, int m);
 // complex64 over quartets (msgpu_resident_q.cu): dimensions it takes, its shape,
-// the device bytes of a system's ResidentQuartets (kmax: most neighbour blocks
-// of a quartet) and their set-up in buf from the quartet form's arrays.
+// the device bytes of a system's ResidentQuartets and their set-up in buf from
+// the quartet form's arrays.
+struct QuartetSlots;
 bool resident_q_takes(int D);
 ResidentShape resident_shape_q(int D, int m);
-size_t resident_q_bytes(int Q, int kmax);
-ResidentQuartets resident_q_build(void *buf, int Q, int s1, int s2, int kmax, const int *rowptr, const int2 *blk,
-                                  const float4 *val, const int *base, cudaStream_t st);
+ResidentShape resident_shape_q_state(int D, int m);  // on a complex64 state
+size_t resident_q_bytes(int Q, const QuartetSlots &slots);
+ResidentQuartets resident_q_build(void *buf, int Q, int s1, int s2, const QuartetSlots &slots, const int *rowptr,
+                                  const int2 *blk, const float4 *val, const int *base, cudaStream_t st);
 
 }  // namespace msgpu

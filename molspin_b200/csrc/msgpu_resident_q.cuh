@@ -3,18 +3,19 @@
 // As msgpu_resident.cuh (one CTA per trajectory for the whole time loop,
 // three-term recurrence), with a thread per quartet instead of per row: a
 // nucleus' flip block is 4 values for 16 matrix entries and one gather serves
-// four rows, and a thread's whole part of H -- its own 4x4 block and up to KF
-// flip blocks -- stays in registers for the whole time loop, so a product
+// four rows, and a thread's whole part of H -- its own 4x4 block and up to
+// eight flip blocks, one slot per nucleus -- stays in registers for the whole time loop, so a product
 // reads nothing but the vector in shared memory.  At D = 1024 the row form
 // reads 233 KB of H a product through L2, which sets its time: a step of 256
-// trajectories takes 280 us there against KQTIME here (B200, m = 16).
+// trajectories takes 280 us there against 65 here (B200, m = 16; 1570 with a
+// warp per trajectory).  A product is then about 1900 of an iteration's 3700
+// cycles (FMA issue of two warps a scheduler), its two reductions 800.
 //
 // A vector is kept in two planes, re and im, of one float4 a quartet (the
-// quartet's four rows), so that packed FP32 pairs need no shuffling:
-// A (x) I blocks pair the rows of one first digit with broadcast values,
-// I (x) A blocks and the own block pair values with broadcast rows.
+// quartet's four rows): 16-byte accesses without bank conflicts.
 #pragma once
 
+#include "msgpu_quartet.h"
 #include "msgpu_resident.cuh"
 
 namespace msgpu {
@@ -46,12 +47,9 @@ __device__ inline void quartet_expand(int type, const float2 *v, float4 (&re)[4]
     }
 }
 
-// The resident layout from the quartet form (QuartetC): per quartet its
-// neighbour blocks, those of type 4 and 5 first and by distance (a slot then
-// belongs to one nucleus and a warp's lanes meet the same type), and its own
-// block expanded.
-__global__ void k_build_resident_quartets(QuartetC H, int Q, int s1, int s2, int kmax, int *__restrict__ nblk,
-                                          int2 *__restrict__ blk, float4 *__restrict__ own)
+// The resident layout from the quartet form (QuartetC).
+__global__ void k_build_resident_quartets(QuartetC H, int Q, int s1, int s2, QuartetSlots S, float4 *__restrict__ own,
+                                          int2 *__restrict__ slot, int2 *__restrict__ blk, int *__restrict__ nblk)
 {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= Q) return;
@@ -60,8 +58,8 @@ __global__ void k_build_resident_quartets(QuartetC H, int Q, int s1, int s2, int
     float4 re[4], im[4];
 #pragma unroll
     for (int b = 0; b < 4; ++b) re[b] = im[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < S.n; ++k) slot[static_cast<size_t>(k) * Q + q] = make_int2(q, -1);
     int n = 0;
-    auto key = [&](int2 x) { return (static_cast<long long>((x.x & 7) < 4) << 32) + abs((x.x >> 3) - q); };
     for (int k = H.rowptr[q]; k < H.rowptr[q + 1]; ++k) {
         const int2 c = H.blk[k];
         const int cb = c.x >> 3, type = c.x & 7;
@@ -70,11 +68,11 @@ __global__ void k_build_resident_quartets(QuartetC H, int Q, int s1, int s2, int
             continue;
         }
         const int qn = (cb / (2 * s1)) * (s1 / 2) + ((cb / (2 * s2)) % (s1 / (2 * s2))) * s2 + cb % s2;
-        const int2 x = make_int2((qn << 3) | type, c.y);
-        int at = n++;
-        for (; at > 0 && key(blk[static_cast<size_t>(at - 1) * Q + q]) > key(x); --at)
-            blk[static_cast<size_t>(at) * Q + q] = blk[static_cast<size_t>(at - 1) * Q + q];
-        blk[static_cast<size_t>(at) * Q + q] = x;
+        int at = -1;
+        for (int i = 0; i < S.n; ++i)
+            if (qn - q == S.delta[i] || (((S.shared >> i) & 1u) && q - qn == S.delta[i])) at = i;
+        if (at >= 0) slot[static_cast<size_t>(at) * Q + q] = make_int2(qn, c.y);
+        else if (n < S.left) blk[static_cast<size_t>(n++) * Q + q] = make_int2((qn << 3) | type, c.y);
     }
     nblk[q] = n;
 #pragma unroll
@@ -85,46 +83,36 @@ __global__ void k_build_resident_quartets(QuartetC H, int Q, int s1, int s2, int
 }
 
 struct QuartetAcc {
-    float2 re01, re23, im01, im23;  // rows (0, 1) and (2, 3)
+    float re[4], im[4];
 };
 
-__device__ __forceinline__ float2 bc(float x) { return make_float2(x, x); }
-__device__ __forceinline__ float2 neg2(float2 x) { return make_float2(-x.x, -x.y); }
-
-// o += A x for a pair of rows, A broadcast
-__device__ __forceinline__ void mac_bcast(float2 &ore, float2 &oim, float2 A, float2 xre, float2 xim)
+__device__ __forceinline__ void acc_mac(QuartetAcc &o, int a, float br, float bi, float xr, float xi)
 {
-    ore = __ffma2_rn(bc(A.x), xre, ore);
-    ore = __ffma2_rn(bc(-A.y), xim, ore);
-    oim = __ffma2_rn(bc(A.x), xim, oim);
-    oim = __ffma2_rn(bc(A.y), xre, oim);
-}
-// o += (c_0 x, c_1 x) for a pair of rows, x broadcast
-__device__ __forceinline__ void mac_pair(float2 &ore, float2 &oim, float2 cre, float2 cim, float xre, float xim)
-{
-    ore = __ffma2_rn(cre, bc(xre), ore);
-    ore = __ffma2_rn(neg2(cim), bc(xim), ore);
-    oim = __ffma2_rn(cre, bc(xim), oim);
-    oim = __ffma2_rn(cim, bc(xre), oim);
+    o.re[a] = fmaf(br, xr, o.re[a]);
+    o.re[a] = fmaf(-bi, xi, o.re[a]);
+    o.im[a] = fmaf(br, xi, o.im[a]);
+    o.im[a] = fmaf(bi, xr, o.im[a]);
 }
 
-// One flip block, values A00 A01 | A10 A11 as two float4.
-__device__ __forceinline__ void flip_mac(QuartetAcc &o, bool second, float4 p, float4 q, float4 xr, float4 xi)
+// One flip block, values p = A00 A01, r = A10 A11, on the first digit (A (x) I)
+// or the second (I (x) A).  Plain FMAs: packed ones need every broadcast value
+// or row twice in registers, and the copies cost what they save.
+__device__ __forceinline__ void flip_mac(QuartetAcc &o, bool second, float4 p, float4 r, float4 xr, float4 xi)
 {
-    if (!second) {  // A (x) I: acts on the first digit
-        const float2 r01 = make_float2(xr.x, xr.y), r23 = make_float2(xr.z, xr.w);
-        const float2 i01 = make_float2(xi.x, xi.y), i23 = make_float2(xi.z, xi.w);
-        mac_bcast(o.re01, o.im01, make_float2(p.x, p.y), r01, i01);
-        mac_bcast(o.re01, o.im01, make_float2(p.z, p.w), r23, i23);
-        mac_bcast(o.re23, o.im23, make_float2(q.x, q.y), r01, i01);
-        mac_bcast(o.re23, o.im23, make_float2(q.z, q.w), r23, i23);
-    } else {  // I (x) A: acts on the second digit
-        const float2 c0r = make_float2(p.x, q.x), c0i = make_float2(p.y, q.y);
-        const float2 c1r = make_float2(p.z, q.z), c1i = make_float2(p.w, q.w);
-        mac_pair(o.re01, o.im01, c0r, c0i, xr.x, xi.x);
-        mac_pair(o.re01, o.im01, c1r, c1i, xr.y, xi.y);
-        mac_pair(o.re23, o.im23, c0r, c0i, xr.z, xi.z);
-        mac_pair(o.re23, o.im23, c1r, c1i, xr.w, xi.w);
+    const float x[4] = {xr.x, xr.y, xr.z, xr.w}, y[4] = {xi.x, xi.y, xi.z, xi.w};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (!second) {
+            acc_mac(o, h, p.x, p.y, x[h], y[h]);
+            acc_mac(o, 2 + h, r.x, r.y, x[h], y[h]);
+            acc_mac(o, h, p.z, p.w, x[2 + h], y[2 + h]);
+            acc_mac(o, 2 + h, r.z, r.w, x[2 + h], y[2 + h]);
+        } else {
+            acc_mac(o, 2 * h, p.x, p.y, x[2 * h], y[2 * h]);
+            acc_mac(o, 2 * h + 1, r.x, r.y, x[2 * h], y[2 * h]);
+            acc_mac(o, 2 * h, p.z, p.w, x[2 * h + 1], y[2 * h + 1]);
+            acc_mac(o, 2 * h + 1, r.z, r.w, x[2 * h + 1], y[2 * h + 1]);
+        }
     }
 }
 
@@ -134,46 +122,42 @@ __device__ __forceinline__ void full_mac(QuartetAcc &o, const float4 (&re)[4], c
     const float x[4] = {xr.x, xr.y, xr.z, xr.w}, y[4] = {xi.x, xi.y, xi.z, xi.w};
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-        mac_pair(o.re01, o.im01, make_float2(re[b].x, re[b].y), make_float2(im[b].x, im[b].y), x[b], y[b]);
-        mac_pair(o.re23, o.im23, make_float2(re[b].z, re[b].w), make_float2(im[b].z, im[b].w), x[b], y[b]);
+        acc_mac(o, 0, re[b].x, im[b].x, x[b], y[b]);
+        acc_mac(o, 1, re[b].y, im[b].y, x[b], y[b]);
+        acc_mac(o, 2, re[b].z, im[b].z, x[b], y[b]);
+        acc_mac(o, 3, re[b].w, im[b].w, x[b], y[b]);
     }
 }
 
-// A thread's quartet of H: its own block and the first KF flip blocks in
-// registers (absent ones: value 0 on the quartet itself); further blocks and
-// types other than 4 and 5 are read on each product.
-template <int KF>
+// A thread's quartet of H: its own block and its slots' blocks in registers
+// (absent ones: value 0 on the quartet itself); other blocks are read on each
+// product.
 struct QuartetRow {
-    int q, n, nreg;     // quartet, neighbour blocks, those of them in registers
-    int nb[KF];
-    unsigned second;    // bit k: block k acts on the second digit
-    float4 p[KF], r[KF];
+    int q, n;           // quartet, blocks without a slot
+    int nb[kQuartetSlots];
+    float4 p[kQuartetSlots], r[kQuartetSlots];
     float4 ore[4], oim[4];
 
     __device__ void load(const ResidentQuartets &H, int q_, bool live)
     {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
         q = live ? q_ : 0;
         n = live ? __ldg(H.nblk + q) : 0;
-        nreg = 0;
-        second = 0;
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            ore[b] = live ? __ldg(H.own + static_cast<size_t>(2 * b) * H.Q + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-            oim[b] = live ? __ldg(H.own + static_cast<size_t>(2 * b + 1) * H.Q + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+            ore[b] = live ? __ldg(H.own + static_cast<size_t>(2 * b) * H.Q + q) : zero;
+            oim[b] = live ? __ldg(H.own + static_cast<size_t>(2 * b + 1) * H.Q + q) : zero;
         }
 #pragma unroll
-        for (int k = 0; k < KF; ++k) {
+        for (int k = 0; k < kQuartetSlots; ++k) {
             nb[k] = q;
-            p[k] = r[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (k < n) {
-                const int2 x = __ldg(H.blk + static_cast<size_t>(k) * H.Q + q);
-                const int type = x.x & 7;
-                if (type >= 4) {
-                    nb[k] = x.x >> 3;
+            p[k] = r[k] = zero;
+            if (k < H.nslot && live) {
+                const int2 x = __ldg(H.slot + static_cast<size_t>(k) * H.Q + q);
+                nb[k] = x.x;
+                if (x.y >= 0) {
                     p[k] = __ldg(H.val + x.y);
                     r[k] = __ldg(H.val + x.y + 1);
-                    if (type == 5) second |= 1u << k;
-                    nreg = k + 1;
                 }
             }
         }
@@ -182,23 +166,20 @@ struct QuartetRow {
     __device__ QuartetAcc apply(const ResidentQuartets &H, const float4 *re, const float4 *im, float4 xr, float4 xi) const
     {
         QuartetAcc o;
-        o.re01 = o.re23 = o.im01 = o.im23 = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int k = 0; k < KF; ++k) {
-            if (k >= H.kmax) break;
-            flip_mac(o, (second >> k) & 1u, p[k], r[k], re[nb[k]], im[nb[k]]);
+        for (int a = 0; a < 4; ++a) o.re[a] = o.im[a] = 0.f;
+#pragma unroll
+        for (int k = 0; k < kQuartetSlots; ++k) {
+            if (k >= H.nslot) break;
+            flip_mac(o, (H.second >> k) & 1u, p[k], r[k], re[nb[k]], im[nb[k]]);
         }
         full_mac(o, ore, oim, xr, xi);
-        for (int k = nreg; k < n; ++k) {
+        for (int k = 0; k < n; ++k) {
             const int2 x = __ldg(H.blk + static_cast<size_t>(k) * H.Q + q);
             const int type = x.x & 7, m = x.x >> 3;
-            if (type >= 4) {
-                flip_mac(o, type == 5, __ldg(H.val + x.y), __ldg(H.val + x.y + 1), re[m], im[m]);
-            } else {
-                float4 br[4], bi[4];
-                quartet_expand(type, reinterpret_cast<const float2 *>(H.val) + 2 * static_cast<size_t>(x.y), br, bi);
-                full_mac(o, br, bi, re[m], im[m]);
-            }
+            float4 br[4], bi[4];
+            quartet_expand(type, reinterpret_cast<const float2 *>(H.val) + 2 * static_cast<size_t>(x.y), br, bi);
+            full_mac(o, br, bi, re[m], im[m]);
         }
         return o;
     }
@@ -254,7 +235,7 @@ __device__ __forceinline__ void quartet_evaluate(const ResidentSystem &S, const 
     team_reduce_values<W, NO>(S, sm.rede, v, lane, warp, val, nrm);
 }
 
-template <typename TS, int W, int KF>
+template <typename TS, int W>
 __device__ __forceinline__ void resident_quartet_propagate(const ResidentSystem &S, int t, unsigned char *smem,
                                                            int *__restrict__ status)
 {
@@ -263,7 +244,7 @@ __device__ __forceinline__ void resident_quartet_propagate(const ResidentSystem 
     const bool live = tid < Q;
     const QuartetSmem sm = quartet_carve(smem, Q, m, W);
     float4 *Vre = sm.V, *Vim = sm.V + Q;
-    QuartetRow<KF> H;
+    QuartetRow H;
     H.load(S.rq, tid, live);
     const TS *in = static_cast<const TS *>(S.psi) + static_cast<size_t>(t) * S.ts;
     size_t row[4];
@@ -340,10 +321,8 @@ __device__ __forceinline__ void resident_quartet_propagate(const ResidentSystem 
                 {
                     const float4 xr = re[H.q], xi = im[H.q];
                     const QuartetAcc o = H.apply(S.rq, re, im, xr, xi);
-                    u[0] = make_double2(o.re01.x * sj, o.im01.x * sj);
-                    u[1] = make_double2(o.re01.y * sj, o.im01.y * sj);
-                    u[2] = make_double2(o.re23.x * sj, o.im23.x * sj);
-                    u[3] = make_double2(o.re23.y * sj, o.im23.y * sj);
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) u[a] = make_double2(o.re[a] * sj, o.im[a] * sj);
                 }
                 double pa = 0.0, pb = 0.0;
                 if (live) {
