@@ -312,6 +312,17 @@ double row_sum_norm(int dim, const int *rowptr, const double *val)
     return mx;
 }
 
+// Rows per CTA of the complex64 update: halved from R while the launch has
+// fewer than 3 CTAs an SM (ctiles: trajectory tiles), up to the partials'
+// capacity.  D = 9216, 250 trajectories: 256 CTAs 17.5 us, 512 14.2 us; at D =
+// 16384 and 512 trajectories a launch has 512 already, and halving again costs
+// (98.0 to 99.2 ms for 20 steps of two such groups).
+int update_rows(int D, int R, int ctiles, int max_tiles)
+{
+    while (R > 32 && ceil_div(D, R) * ctiles < 3 * 148 && ceil_div(D, (R / 2 + 7) / 8 * 8) <= max_tiles) R = (R / 2 + 7) / 8 * 8;
+    return R;
+}
+
 // Quartets per CTA of k_lanczos_apply_d: 16, or 8 while 16 leaves under 8 CTAs
 // an SM (D = 16384, us per launch: 512 trajectories 176 with 8 or 16, 185 with
 // 32, 223 with 64).
@@ -2502,7 +2513,8 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
             }
             const int rc = for_groups(fused_c ? 1 : traj_groups(c), [&](int t0, int width, cudaStream_t gs) {
                 const size_t tm0 = static_cast<size_t>(t0) * mws;  // offset into the [t][m] T arrays
-                dim3 grid(nt, width / 64);
+                const int Ru = update_rows(D, R, width / 64, std::max(nt, ceil_div(Q, 8))), ntu = ceil_div(D, Ru);
+                dim3 grid(ntu, width / 64);
                 for (int j = 0; j < (fused_c ? 0 : m); ++j) {
                     {
                         Timed tm(c, KC_APPLY, gs);
@@ -2520,11 +2532,11 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                         k_lanczos_update<<<grid, kThreads, 0, gs>>>(
                             U + t0, Wb + j * n + t0, j > 0 ? Wb + (j - 1) * n + t0 : nullptr,
                             sc + static_cast<size_t>(j) * ldm + t0, j > 0 ? sc + static_cast<size_t>(j - 1) * ldm + t0 : nullptr,
-                            alpha + t0, Wb + (j + 1) * n + t0, part + t0, D, ldm, R);
+                            alpha + t0, Wb + (j + 1) * n + t0, part + t0, D, ldm, Ru);
                     }
                     {
                         Timed tm(c, KC_REDUCE, gs);
-                        k_lanczos_reduce<<<width / 32, dim3(32, kRedRows), 0, gs>>>(part + t0, nt, ldm, 1, j, mws,
+                        k_lanczos_reduce<<<width / 32, dim3(32, kRedRows), 0, gs>>>(part + t0, ntu, ldm, 1, j, mws,
                                                                              sc + static_cast<size_t>(j + 1) * ldm + t0,
                                                                              td + tm0, to + tm0, mdim + t0);
                     }
