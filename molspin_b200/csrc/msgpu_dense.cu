@@ -54,17 +54,19 @@ constexpr uint32_t kWaitLimit = 1u << 22;
 // The small split-correction products therefore go to their own accumulator
 // (2^-8 of the main magnitude, so their bias is negligible), and with 3 parts
 // the hi x hi product is spread over 3 K-range accumulators; the epilogue sums
-// the accumulators with round-to-nearest FP32 adds (unbiased).  TMEM: NACC x BN = 512 columns.
-template <int NS>
+// the accumulators with round-to-nearest FP32 adds (unbiased).  TMEM: NACC x BN columns,
+// 512 with the wide tile.  kHalf: a tile of half as many trajectories, for blocks whose
+// wide tiles would leave SMs idle (half_tiles).
+template <int NS, bool kHalf = false>
 struct GemmCfg {
-    static constexpr int BN = NS == 2 ? 256 : 128;       // trajectories per CTA
+    static constexpr int BN = (NS == 2 ? 256 : 128) / (kHalf ? 2 : 1);  // trajectories per CTA
     static constexpr int NHI = NS == 2 ? 1 : 3;          // hi x hi accumulators (K ranges)
     static constexpr int NACC = NHI + 1;                 // + the correction accumulator
     static constexpr int Cols = NACC * BN;               // TMEM columns (power of two, <= 512)
     static constexpr int BTile = BN * kGK * 2;           // bytes of one B part tile
     static constexpr int Stage = NS * kATile + NS * BTile;
     static constexpr int Smem = kGStages * Stage + 1024 /*align*/ + 256 /*barriers*/;
-    static_assert(Cols == 512, "TMEM split");
+    static_assert(Cols == (kHalf ? 256 : 512), "TMEM split");
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -155,14 +157,14 @@ __device__ __forceinline__ void umma_commit(uint32_t bar)
 //   out:     Mp x Dp FP32, out[n][m] = C[m][n]
 // grid = (trajectory tiles of this launch, Dp / 128), block = 128 threads;
 // the launch covers the trajectory tiles from n_tile0 on.
-template <int NS>
+template <int NS, bool kHalf>
 __global__ void __launch_bounds__(kGThreads, 1)
 k_dense_gemm(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUtensorMap ta1,
              const __grid_constant__ CUtensorMap ta2, const __grid_constant__ CUtensorMap tb0,
              const __grid_constant__ CUtensorMap tb1, const __grid_constant__ CUtensorMap tb2, float *__restrict__ out,
              int Dp, int n_tile0, int *__restrict__ status)
 {
-    using Cfg = GemmCfg<NS>;
+    using Cfg = GemmCfg<NS, kHalf>;
     constexpr int BN = Cfg::BN;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -305,13 +307,24 @@ k_dense_gemm(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CU
 // errors are the slices' truncation (2^-31 of the scale) and the FP64 state.
 constexpr int kIK = 64;              // K (int8) per stage: one 64-byte swizzle row
 constexpr int kIStages = 3;
-constexpr int kIBN = 128;            // trajectories per CTA
+constexpr int kIBN = 128;            // trajectories per CTA (half of them in the half tile)
 constexpr int kIParts = 4;           // slices per operand
 constexpr int kIATile = kGM * kIK;   // bytes of one A slice tile (8 KB)
-constexpr int kIBTile = kIBN * kIK;  // bytes of one B slice tile (8 KB)
-constexpr int kIStage = kIParts * (kIATile + kIBTile);
-constexpr int kISmem = kIStages * kIStage + 1024 /*align*/ + 256 /*barriers*/;
-constexpr int kILevels = 4;          // TMEM: 4 x 128 = 512 columns
+constexpr int kILevels = 4;
+template <bool kHalf>
+struct I8Cfg {
+    static constexpr int BN = kHalf ? kIBN / 2 : kIBN;
+    static constexpr int BTile = BN * kIK;  // bytes of one B slice tile
+    static constexpr int Stage = kIParts * (kIATile + BTile);
+    static constexpr int Smem = kIStages * Stage + 1024 /*align*/ + 256 /*barriers*/;
+    static constexpr int Cols = kILevels * BN;  // TMEM columns
+};
+
+// Half tiles while whole ones number fewer than the SMs: the tile's latency is
+// then all that counts.  int8, D = 576, 1000 trajectories: 72 whole or 144 half
+// tiles, 50 steps in 2.07 or 1.89 ms.  Where whole tiles fill the GPU, half ones
+// would read a third more from L2 for the same products.
+inline bool half_tiles(int m_tiles, int n_tiles) { return m_tiles * n_tiles < 148; }
 
 // UMMA shared-memory descriptor: K-major operand, 64-byte swizzle, rows of 64
 // bytes in 8-row (512-byte) groups: SBO = 512 B, LBO unused (1), version 1,
@@ -348,6 +361,7 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem, uint64_t a, uint64_t b, u
 //   B slices: Mp x Dp int8                          -> tensor maps tb[0..4)
 //   sa[m], sb[n]: the power-of-two scales of U's row m and trajectory n
 // grid = (trajectory tiles of this launch, Dp / 128), block = 128 threads.
+template <bool kHalf>
 __global__ void __launch_bounds__(kGThreads, 1)
 k_dense_gemm_i8(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUtensorMap ta1,
                 const __grid_constant__ CUtensorMap ta2, const __grid_constant__ CUtensorMap ta3,
@@ -356,17 +370,19 @@ k_dense_gemm_i8(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
                 const double *__restrict__ sa, const double *__restrict__ sb, double *__restrict__ out, int Dp,
                 int n_tile0, int *__restrict__ status)
 {
+    using Cfg = I8Cfg<kHalf>;
+    constexpr int BN = Cfg::BN;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char *base_ptr = smem_raw + (base - raw);
-    const uint32_t bars = base + kIStages * kIStage;  // full[3], empty[3], accum
-    uint64_t *bar_ptr = reinterpret_cast<uint64_t *>(base_ptr + kIStages * kIStage);
+    const uint32_t bars = base + kIStages * Cfg::Stage;  // full[3], empty[3], accum
+    uint64_t *bar_ptr = reinterpret_cast<uint64_t *>(base_ptr + kIStages * Cfg::Stage);
     volatile int *abort = reinterpret_cast<volatile int *>(bar_ptr + 8);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_ptr + 9);
     const uint32_t full0 = bars, empty0 = bars + 8 * kIStages, accum = bars + 16 * kIStages;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = (n_tile0 + blockIdx.x) * kIBN, m0 = blockIdx.y * kGM;
+    const int n0 = (n_tile0 + blockIdx.x) * BN, m0 = blockIdx.y * kGM;
     const int nk = Dp / kIK;
     const CUtensorMap *ta[4] = {&ta0, &ta1, &ta2, &ta3};
     const CUtensorMap *tb[4] = {&tb0, &tb1, &tb2, &tb3};
@@ -382,7 +398,7 @@ k_dense_gemm_i8(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(kILevels * kIBN));
+                     "r"(Cfg::Cols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -396,11 +412,11 @@ k_dense_gemm_i8(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
         for (int kb = 0; kb < nk; ++kb) {
             const int s = kb % kIStages, r = kb / kIStages;
             if (!mbar_wait(empty0 + 8 * s, (r & 1) ^ 1, abort)) break;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full0 + 8 * s), "r"(kIStage));
-            const uint32_t st = base + s * kIStage;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full0 + 8 * s), "r"(Cfg::Stage));
+            const uint32_t st = base + s * Cfg::Stage;
             for (int p = 0; p < kIParts; ++p) tma_load_2d(st + p * kIATile, ta[p], kb * kIK, m0, full0 + 8 * s);
             for (int q = 0; q < kIParts; ++q)
-                tma_load_2d(st + kIParts * kIATile + q * kIBTile, tb[q], kb * kIK, n0, full0 + 8 * s);
+                tma_load_2d(st + kIParts * kIATile + q * Cfg::BTile, tb[q], kb * kIK, n0, full0 + 8 * s);
             issued = kb + 1;
         }
         for (int kb = max(0, issued - kIStages); kb < issued; ++kb) {
@@ -410,13 +426,13 @@ k_dense_gemm_i8(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
         }
     } else if (threadIdx.x == 32) {
         // MMA issuer: level L = i + j accumulates a_i b_j
-        constexpr uint32_t idesc = umma_idesc_i8(kGM, kIBN);
+        constexpr uint32_t idesc = umma_idesc_i8(kGM, BN);
         uint32_t on = 0;  // bit L: level L's accumulator was written
         for (int kb = 0; kb < nk; ++kb) {
             const int s = kb % kIStages, r = kb / kIStages;
             if (!mbar_wait(full0 + 8 * s, r & 1, abort)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t st = base + s * kIStage;
+            const uint32_t st = base + s * Cfg::Stage;
 #pragma unroll
             for (int kk = 0; kk < kIK / 32; ++kk)
 #pragma unroll
@@ -425,8 +441,8 @@ k_dense_gemm_i8(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
                     for (int j = 0; j < kIParts - i; ++j) {
                         const int L = i + j;
                         const uint64_t ad = umma_desc64(st + i * kIATile + kk * 32);
-                        const uint64_t bd = umma_desc64(st + kIParts * kIATile + j * kIBTile + kk * 32);
-                        umma_i8(tmem + L * kIBN, ad, bd, idesc, (on >> L) & 1u);
+                        const uint64_t bd = umma_desc64(st + kIParts * kIATile + j * Cfg::BTile + kk * 32);
+                        umma_i8(tmem + L * BN, ad, bd, idesc, (on >> L) & 1u);
                         on |= 1u << L;
                     }
             umma_commit(empty0 + 8 * s);
@@ -447,10 +463,10 @@ k_dense_gemm_i8(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
         const uint32_t lane_base = tmem + (static_cast<uint32_t>(32 * warp) << 16);
         constexpr double w0 = 1.0 / (127.0 * 127.0), w1 = w0 / 254.0, w2 = w1 / 254.0, w3 = w2 / 254.0;
 #pragma unroll 1
-        for (int c = 0; c < kIBN; c += 16) {
+        for (int c = 0; c < BN; c += 16) {
             uint32_t v[kILevels][16];
 #pragma unroll
-            for (int L = 0; L < kILevels; ++L) tmem_ld16_issue(lane_base + static_cast<uint32_t>(L * kIBN + c), v[L]);
+            for (int L = 0; L < kILevels; ++L) tmem_ld16_issue(lane_base + static_cast<uint32_t>(L * BN + c), v[L]);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
@@ -467,7 +483,7 @@ k_dense_gemm_i8(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kILevels * kIBN));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cfg::Cols));
     }
 }
 
@@ -1097,7 +1113,9 @@ int dense_run(DenseState &st, const DenseRun &run, void *psi128, int ldm, cudaSt
     CUtensorMap ta[4], tb[4];
     std::memset(ta, 0, sizeof(ta));
     std::memset(tb, 0, sizeof(tb));
-    const int BN = i8 ? kIBN : ns == 2 ? GemmCfg<2>::BN : GemmCfg<3>::BN;
+    const int wide = i8 ? kIBN : ns == 2 ? GemmCfg<2>::BN : GemmCfg<3>::BN;
+    const bool half = half_tiles(Mp / wide, Dp / kGM);
+    const int BN = half ? wide / 2 : wide;
     void *bp = st.b_parts;
     for (int p = 0; p < ns; ++p) {
         bool okm;
@@ -1121,11 +1139,16 @@ int dense_run(DenseState &st, const DenseRun &run, void *psi128, int ldm, cudaSt
         tb[p] = tb[0];
     }
     cudaError_t e;
-    const int smem = i8 ? kISmem : ns == 2 ? GemmCfg<2>::Smem : GemmCfg<3>::Smem;
     const size_t epi_smem = (i8 ? sizeof(double) : sizeof(float)) * 2 * static_cast<size_t>(D);
-    if ((e = raise_smem_limit(reinterpret_cast<const void *>(k_dense_gemm<2>), GemmCfg<2>::Smem)) ||
-        (e = raise_smem_limit(reinterpret_cast<const void *>(k_dense_gemm<3>), GemmCfg<3>::Smem)) ||
-        (e = raise_smem_limit(reinterpret_cast<const void *>(k_dense_gemm_i8), kISmem)) ||
+    const auto gemm2 = half ? k_dense_gemm<2, true> : k_dense_gemm<2, false>;
+    const auto gemm3 = half ? k_dense_gemm<3, true> : k_dense_gemm<3, false>;
+    const auto gemm8 = half ? k_dense_gemm_i8<true> : k_dense_gemm_i8<false>;
+    const int smem = i8 ? (half ? I8Cfg<true>::Smem : I8Cfg<false>::Smem)
+                     : ns == 2 ? (half ? GemmCfg<2, true>::Smem : GemmCfg<2>::Smem)
+                               : (half ? GemmCfg<3, true>::Smem : GemmCfg<3>::Smem);
+    if ((e = raise_smem_limit(i8 ? reinterpret_cast<const void *>(gemm8)
+                                 : ns == 2 ? reinterpret_cast<const void *>(gemm2) : reinterpret_cast<const void *>(gemm3),
+                              smem)) ||
         (e = raise_smem_limit(reinterpret_cast<const void *>(i8 ? k_dense_epilogue<true> : k_dense_epilogue<false>),
                               static_cast<int>(epi_smem)))) {
         err = std::string("dense: shared memory: ") + cudaGetErrorString(e);
@@ -1216,15 +1239,15 @@ int dense_run(DenseState &st, const DenseRun &run, void *psi128, int ldm, cudaSt
     auto gemm = [&](int g, cudaStream_t sg) {
         dim3 grid(gt[g + 1] - gt[g], Dp / kGM);
         if (i8)
-            k_dense_gemm_i8<<<grid, kGThreads, smem, sg>>>(ta[0], ta[1], ta[2], ta[3], tb[0], tb[1], tb[2], tb[3],
+            gemm8<<<grid, kGThreads, smem, sg>>>(ta[0], ta[1], ta[2], ta[3], tb[0], tb[1], tb[2], tb[3],
                                                            static_cast<const double *>(st.u_scale),
                                                            static_cast<const double *>(st.b_scale),
                                                            static_cast<double *>(st.psi), Dp, gt[g], run.status);
         else if (ns == 2)
-            k_dense_gemm<2><<<grid, kGThreads, smem, sg>>>(ta[0], ta[1], ta[2], tb[0], tb[1], tb[2],
+            gemm2<<<grid, kGThreads, smem, sg>>>(ta[0], ta[1], ta[2], tb[0], tb[1], tb[2],
                                                            static_cast<float *>(st.psi), Dp, gt[g], run.status);
         else
-            k_dense_gemm<3><<<grid, kGThreads, smem, sg>>>(ta[0], ta[1], ta[2], tb[0], tb[1], tb[2],
+            gemm3<<<grid, kGThreads, smem, sg>>>(ta[0], ta[1], ta[2], tb[0], tb[1], tb[2],
                                                            static_cast<float *>(st.psi), Dp, gt[g], run.status);
     };
     if (G == 2) fork();
