@@ -320,11 +320,12 @@ struct I8Cfg {
     static constexpr int Cols = kILevels * BN;  // TMEM columns
 };
 
-// Half tiles while whole ones number fewer than the SMs: the tile's latency is
-// then all that counts.  int8, D = 576, 1000 trajectories: 72 whole or 144 half
-// tiles, 50 steps in 2.07 or 1.89 ms.  Where whole tiles fill the GPU, half ones
-// would read a third more from L2 for the same products.
-inline bool half_tiles(int m_tiles, int n_tiles) { return m_tiles * n_tiles < 148; }
+// Half tiles while all of them fit one wave: the tile's latency is then all that
+// counts.  int8, D = 576, 1000 trajectories: 72 whole or 144 half tiles, a step
+// in 41.4 or 37.8 us; D = 1024, bf16x3: 16 / 32 tiles 45.8 / 36.2 us, 64 / 128
+// tiles 49.5 / 39.7 us; bf16x6, 64 / 128 tiles 49.0 / 46.6 us.  Beyond one wave
+// the half tiles only read more: bf16x3, 128 / 256 tiles 55.8 / 60.3 us.
+inline bool half_tiles(int m_tiles, int n_tiles) { return 2 * m_tiles * n_tiles <= 148; }
 
 // UMMA shared-memory descriptor: K-major operand, 64-byte swizzle, rows of 64
 // bytes in 8-row (512-byte) groups: SBO = 512 B, LBO unused (1), version 1,

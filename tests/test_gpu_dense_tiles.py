@@ -1,6 +1,6 @@
 """Dense form with whole and half trajectory tiles at ragged shapes, against the FP64-expm oracle.
 
-A GEMM of fewer than 148 whole tiles takes half tiles; both accumulate in the same order, so the
+A GEMM whose half tiles all fit one wave (148) takes half tiles; both accumulate in the same order, so the
 shapes on either side of that limit only have to meet the forms' own error bounds per trajectory
 (bf16x3 1e-4, bf16x6 1e-5, int8x4 1e-7 over 20 steps).
 """
