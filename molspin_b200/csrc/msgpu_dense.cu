@@ -43,7 +43,7 @@ namespace {
 
 constexpr int kGM = 128;          // rows of A per CTA (TMEM lanes)
 constexpr int kGK = 64;           // K per stage: 64 BF16 = one 128-byte swizzle row
-constexpr int kGStages = 2;
+constexpr int kRing = 192 * 1024; // bytes of the operand ring, as many stages as fit
 constexpr int kGThreads = 128;    // 4 warps
 constexpr int kATile = kGM * kGK * 2;  // bytes of one A part tile (16 KB)
 constexpr uint32_t kWaitLimit = 1u << 22;
@@ -65,7 +65,8 @@ struct GemmCfg {
     static constexpr int Cols = NACC * BN;               // TMEM columns (power of two, <= 512)
     static constexpr int BTile = BN * kGK * 2;           // bytes of one B part tile
     static constexpr int Stage = NS * kATile + NS * BTile;
-    static constexpr int Smem = kGStages * Stage + 1024 /*align*/ + 256 /*barriers*/;
+    static constexpr int Stages = kRing / Stage;
+    static constexpr int Smem = Stages * Stage + 1024 /*align*/ + 256 /*barriers*/;
     static_assert(Cols == (kHalf ? 256 : 512), "TMEM split");
 };
 
@@ -105,17 +106,19 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
         : "memory");
 }
 
-// UMMA shared-memory descriptor: K-major operand, 128-byte swizzle, rows of
-// 128 bytes in 8-row (1024-byte) groups: SBO = 1024 B, LBO unused (1),
-// version 1, layout type SWIZZLE_128B (2).
+// UMMA shared-memory descriptor: K-major operand, swizzled rows of RowBytes (128
+// or 64) in 8-row groups: SBO = 8 rows, LBO unused (1), version 1, layout type
+// SWIZZLE_128B (2) or SWIZZLE_64B (4).
+template <int RowBytes>
 __device__ __forceinline__ uint64_t umma_desc(uint32_t addr)
 {
+    static_assert(RowBytes == 64 || RowBytes == 128, "one swizzle row");
     uint64_t d = 0;
     d |= static_cast<uint64_t>((addr >> 4) & 0x3FFF);
     d |= static_cast<uint64_t>(1) << 16;
-    d |= static_cast<uint64_t>(1024 >> 4) << 32;
+    d |= static_cast<uint64_t>(8 * RowBytes >> 4) << 32;
     d |= static_cast<uint64_t>(1) << 46;
-    d |= static_cast<uint64_t>(2) << 61;
+    d |= static_cast<uint64_t>(RowBytes == 128 ? 2 : 4) << 61;
     return d;
 }
 
@@ -170,11 +173,11 @@ k_dense_gemm(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CU
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;  // 1024-byte aligned ring (swizzle atoms)
     unsigned char *base_ptr = smem_raw + (base - raw);
-    const uint32_t bars = base + kGStages * Cfg::Stage;  // full[2], empty[2], accum
-    uint64_t *bar_ptr = reinterpret_cast<uint64_t *>(base_ptr + kGStages * Cfg::Stage);
-    volatile int *abort = reinterpret_cast<volatile int *>(bar_ptr + 8);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_ptr + 9);
-    const uint32_t full0 = bars, empty0 = bars + 16, accum = bars + 32;
+    const uint32_t bars = base + Cfg::Stages * Cfg::Stage;  // full, empty (a pair a stage), accum
+    uint64_t *bar_ptr = reinterpret_cast<uint64_t *>(base_ptr + Cfg::Stages * Cfg::Stage);
+    volatile int *abort = reinterpret_cast<volatile int *>(bar_ptr + 16);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_ptr + 17);
+    const uint32_t full0 = bars, empty0 = bars + 8 * Cfg::Stages, accum = bars + 16 * Cfg::Stages;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n0 = (n_tile0 + blockIdx.x) * BN, m0 = blockIdx.y * kGM;
     const int nk = Dp / kGK;
@@ -183,7 +186,7 @@ k_dense_gemm(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CU
 
     if (threadIdx.x == 0) {
         *abort = 0;
-        for (int s = 0; s < kGStages; ++s) {
+        for (int s = 0; s < Cfg::Stages; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8 * s));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty0 + 8 * s));
         }
@@ -204,7 +207,7 @@ k_dense_gemm(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CU
         // TMA producer
         int issued = 0;
         for (int kb = 0; kb < nk; ++kb) {
-            const int s = kb % kGStages, r = kb / kGStages;
+            const int s = kb % Cfg::Stages, r = kb / Cfg::Stages;
             if (!mbar_wait(empty0 + 8 * s, (r & 1) ^ 1, abort)) break;
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full0 + 8 * s),
                          "r"(Cfg::Stage));
@@ -215,8 +218,8 @@ k_dense_gemm(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CU
             issued = kb + 1;
         }
         // make sure every copy this CTA started has landed before it can exit
-        for (int kb = max(0, issued - kGStages); kb < issued; ++kb) {
-            const int s = kb % kGStages, r = kb / kGStages;
+        for (int kb = max(0, issued - Cfg::Stages); kb < issued; ++kb) {
+            const int s = kb % Cfg::Stages, r = kb / Cfg::Stages;
             for (uint32_t it = 0; it < kWaitLimit && !mbar_try(full0 + 8 * s, r & 1); ++it) {
             }
         }
@@ -226,7 +229,7 @@ k_dense_gemm(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CU
         const uint32_t corr = tmem + Cfg::NHI * BN;  // correction accumulator
         uint32_t corr_on = 0;
         for (int kb = 0; kb < nk; ++kb) {
-            const int s = kb % kGStages, r = kb / kGStages;
+            const int s = kb % Cfg::Stages, r = kb / Cfg::Stages;
             if (!mbar_wait(full0 + 8 * s, r & 1, abort)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t st = base + s * Cfg::Stage;
@@ -241,8 +244,8 @@ k_dense_gemm(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CU
 #pragma unroll
                     for (int q = 0; q < NS; ++q) {
                         if (p + q >= NS) continue;
-                        const uint64_t ad = umma_desc(st + p * kATile + kk * 32);
-                        const uint64_t bd = umma_desc(st + NS * kATile + q * Cfg::BTile + kk * 32);
+                        const uint64_t ad = umma_desc<kGK * 2>(st + p * kATile + kk * 32);
+                        const uint64_t bd = umma_desc<kGK * 2>(st + NS * kATile + q * Cfg::BTile + kk * 32);
                         if (p + q == 0) {
                             umma_bf16(hi, ad, bd, idesc, (kb == first_kb && kk == 0) ? 0u : 1u);
                         } else {
@@ -305,41 +308,32 @@ k_dense_gemm(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CU
 // below 2^31 for K <= 8192), and the epilogue combines the four levels in FP64
 // with the two scales.  The FP32 rounding of the BF16 forms is gone: the only
 // errors are the slices' truncation (2^-31 of the scale) and the FP64 state.
-constexpr int kIK = 64;              // K (int8) per stage: one 64-byte swizzle row
-constexpr int kIStages = 3;
 constexpr int kIBN = 128;            // trajectories per CTA (half of them in the half tile)
 constexpr int kIParts = 4;           // slices per operand
-constexpr int kIATile = kGM * kIK;   // bytes of one A slice tile (8 KB)
 constexpr int kILevels = 4;
+// The ring: bf16 64 K (a 128-byte row), int8 64 or, in the half tile, 128 K a stage:
+// a row of 64 bytes costs TMA as much as one of 128.  int8, D = 576, 1000
+// trajectories, half tiles, 50 steps: 64-byte rows 1.89 ms with 3 or 4 stages,
+// 128-byte rows with 2 stages 1.85 ms.  Halved rows for bf16 with twice the stages:
+// 39.0 -> 46.6 us a step at D = 1024, 1024 trajectories (half tiles).
 template <bool kHalf>
 struct I8Cfg {
     static constexpr int BN = kHalf ? kIBN / 2 : kIBN;
-    static constexpr int BTile = BN * kIK;  // bytes of one B slice tile
-    static constexpr int Stage = kIParts * (kIATile + BTile);
-    static constexpr int Smem = kIStages * Stage + 1024 /*align*/ + 256 /*barriers*/;
+    static constexpr int K = kHalf ? 128 : 64;  // K (int8) per stage: one swizzle row
+    static constexpr int ATile = kGM * K;       // bytes of one A slice tile
+    static constexpr int BTile = BN * K;        // bytes of one B slice tile
+    static constexpr int Stage = kIParts * (ATile + BTile);
+    static constexpr int Stages = kRing / Stage;
+    static constexpr int Smem = Stages * Stage + 1024 /*align*/ + 256 /*barriers*/;
     static constexpr int Cols = kILevels * BN;  // TMEM columns
 };
 
 // Half tiles while all of them fit one wave: the tile's latency is then all that
 // counts.  int8, D = 576, 1000 trajectories: 72 whole or 144 half tiles, a step
-// in 41.4 or 37.8 us; D = 1024, bf16x3: 16 / 32 tiles 45.8 / 36.2 us, 64 / 128
-// tiles 49.5 / 39.7 us; bf16x6, 64 / 128 tiles 49.0 / 46.6 us.  Beyond one wave
+// in 41.4 or 36.9 us; D = 1024, bf16x3: 16 / 32 tiles 45.8 / 34.7 us, 64 / 128
+// tiles 49.5 / 39.0 us; bf16x6, 64 / 128 tiles 49.0 / 46.6 us.  Beyond one wave
 // the half tiles only read more: bf16x3, 128 / 256 tiles 55.8 / 60.3 us.
 inline bool half_tiles(int m_tiles, int n_tiles) { return 2 * m_tiles * n_tiles <= 148; }
-
-// UMMA shared-memory descriptor: K-major operand, 64-byte swizzle, rows of 64
-// bytes in 8-row (512-byte) groups: SBO = 512 B, LBO unused (1), version 1,
-// layout type SWIZZLE_64B (4).
-__device__ __forceinline__ uint64_t umma_desc64(uint32_t addr)
-{
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((addr >> 4) & 0x3FFF);
-    d |= static_cast<uint64_t>(1) << 16;
-    d |= static_cast<uint64_t>(512 >> 4) << 32;
-    d |= static_cast<uint64_t>(1) << 46;
-    d |= static_cast<uint64_t>(4) << 61;
-    return d;
-}
 
 // kind::i8 instruction descriptor: D = S32, A = B = signed int8, both K-major.
 __host__ __device__ constexpr uint32_t umma_idesc_i8(int M, int N)
@@ -377,20 +371,20 @@ k_dense_gemm_i8(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char *base_ptr = smem_raw + (base - raw);
-    const uint32_t bars = base + kIStages * Cfg::Stage;  // full[3], empty[3], accum
-    uint64_t *bar_ptr = reinterpret_cast<uint64_t *>(base_ptr + kIStages * Cfg::Stage);
-    volatile int *abort = reinterpret_cast<volatile int *>(bar_ptr + 8);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_ptr + 9);
-    const uint32_t full0 = bars, empty0 = bars + 8 * kIStages, accum = bars + 16 * kIStages;
+    const uint32_t bars = base + Cfg::Stages * Cfg::Stage;  // full, empty (a pair a stage), accum
+    uint64_t *bar_ptr = reinterpret_cast<uint64_t *>(base_ptr + Cfg::Stages * Cfg::Stage);
+    volatile int *abort = reinterpret_cast<volatile int *>(bar_ptr + 16);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_ptr + 17);
+    const uint32_t full0 = bars, empty0 = bars + 8 * Cfg::Stages, accum = bars + 16 * Cfg::Stages;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n0 = (n_tile0 + blockIdx.x) * BN, m0 = blockIdx.y * kGM;
-    const int nk = Dp / kIK;
+    const int nk = Dp / Cfg::K;
     const CUtensorMap *ta[4] = {&ta0, &ta1, &ta2, &ta3};
     const CUtensorMap *tb[4] = {&tb0, &tb1, &tb2, &tb3};
 
     if (threadIdx.x == 0) {
         *abort = 0;
-        for (int s = 0; s < kIStages; ++s) {
+        for (int s = 0; s < Cfg::Stages; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full0 + 8 * s));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty0 + 8 * s));
         }
@@ -411,17 +405,17 @@ k_dense_gemm_i8(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
         // TMA producer
         int issued = 0;
         for (int kb = 0; kb < nk; ++kb) {
-            const int s = kb % kIStages, r = kb / kIStages;
+            const int s = kb % Cfg::Stages, r = kb / Cfg::Stages;
             if (!mbar_wait(empty0 + 8 * s, (r & 1) ^ 1, abort)) break;
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full0 + 8 * s), "r"(Cfg::Stage));
             const uint32_t st = base + s * Cfg::Stage;
-            for (int p = 0; p < kIParts; ++p) tma_load_2d(st + p * kIATile, ta[p], kb * kIK, m0, full0 + 8 * s);
+            for (int p = 0; p < kIParts; ++p) tma_load_2d(st + p * Cfg::ATile, ta[p], kb * Cfg::K, m0, full0 + 8 * s);
             for (int q = 0; q < kIParts; ++q)
-                tma_load_2d(st + kIParts * kIATile + q * Cfg::BTile, tb[q], kb * kIK, n0, full0 + 8 * s);
+                tma_load_2d(st + kIParts * Cfg::ATile + q * Cfg::BTile, tb[q], kb * Cfg::K, n0, full0 + 8 * s);
             issued = kb + 1;
         }
-        for (int kb = max(0, issued - kIStages); kb < issued; ++kb) {
-            const int s = kb % kIStages, r = kb / kIStages;
+        for (int kb = max(0, issued - Cfg::Stages); kb < issued; ++kb) {
+            const int s = kb % Cfg::Stages, r = kb / Cfg::Stages;
             for (uint32_t it = 0; it < kWaitLimit && !mbar_try(full0 + 8 * s, r & 1); ++it) {
             }
         }
@@ -430,19 +424,19 @@ k_dense_gemm_i8(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
         constexpr uint32_t idesc = umma_idesc_i8(kGM, BN);
         uint32_t on = 0;  // bit L: level L's accumulator was written
         for (int kb = 0; kb < nk; ++kb) {
-            const int s = kb % kIStages, r = kb / kIStages;
+            const int s = kb % Cfg::Stages, r = kb / Cfg::Stages;
             if (!mbar_wait(full0 + 8 * s, r & 1, abort)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t st = base + s * Cfg::Stage;
 #pragma unroll
-            for (int kk = 0; kk < kIK / 32; ++kk)
+            for (int kk = 0; kk < Cfg::K / 32; ++kk)
 #pragma unroll
                 for (int i = 0; i < kIParts; ++i)
 #pragma unroll
                     for (int j = 0; j < kIParts - i; ++j) {
                         const int L = i + j;
-                        const uint64_t ad = umma_desc64(st + i * kIATile + kk * 32);
-                        const uint64_t bd = umma_desc64(st + kIParts * kIATile + j * Cfg::BTile + kk * 32);
+                        const uint64_t ad = umma_desc<Cfg::K>(st + i * Cfg::ATile + kk * 32);
+                        const uint64_t bd = umma_desc<Cfg::K>(st + kIParts * Cfg::ATile + j * Cfg::BTile + kk * 32);
                         umma_i8(tmem + L * BN, ad, bd, idesc, (on >> L) & 1u);
                         on |= 1u << L;
                     }
@@ -982,18 +976,18 @@ bool make_map(CUtensorMap *m, const void *ptr, int rows, int cols, int box_rows)
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// 2D int8 tensor map over a rows x cols row-major matrix, box = 64 x box_rows,
-// 64-byte swizzle (the operand tiles of k_dense_gemm_i8).
-bool make_map_i8(CUtensorMap *m, const void *ptr, int rows, int cols, int box_rows)
+// 2D int8 tensor map over a rows x cols row-major matrix, box = k x box_rows with
+// swizzled rows of k bytes (the operand tiles of k_dense_gemm_i8).
+bool make_map_i8(CUtensorMap *m, const void *ptr, int rows, int cols, int box_rows, int k)
 {
     EncodeTiled enc = encoder();
     if (!enc) return false;
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols)};
-    const cuuint32_t box[2] = {static_cast<cuuint32_t>(kIK), static_cast<cuuint32_t>(box_rows)};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(k), static_cast<cuuint32_t>(box_rows)};
     const cuuint32_t estr[2] = {1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(ptr), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, k == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -1117,14 +1111,15 @@ int dense_run(DenseState &st, const DenseRun &run, void *psi128, int ldm, cudaSt
     const int wide = i8 ? kIBN : ns == 2 ? GemmCfg<2>::BN : GemmCfg<3>::BN;
     const bool half = half_tiles(Mp / wide, Dp / kGM);
     const int BN = half ? wide / 2 : wide;
+    const int ik = half ? I8Cfg<true>::K : I8Cfg<false>::K;
     void *bp = st.b_parts;
     for (int p = 0; p < ns; ++p) {
         bool okm;
         if (i8)
             okm = make_map_i8(&ta[p], static_cast<const int8_t *>(st.u_parts) + static_cast<size_t>(p) * Dp * Dp, Dp, Dp,
-                              kGM) &&
+                              kGM, ik) &&
                   make_map_i8(&tb[p], static_cast<const int8_t *>(st.b_parts) + static_cast<size_t>(p) * Mp * Dp, Mp, Dp,
-                              BN);
+                              BN, ik);
         else
             okm = make_map(&ta[p], static_cast<const __nv_bfloat16 *>(st.u_parts) + static_cast<size_t>(p) * Dp * Dp, Dp,
                            Dp, kGM) &&
