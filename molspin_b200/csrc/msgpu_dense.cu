@@ -202,6 +202,7 @@ k_dense_gemm(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CU
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    grid_wait();  // the operands are the previous kernel's
 
     if (threadIdx.x == 0) {
         // TMA producer
@@ -267,6 +268,7 @@ k_dense_gemm(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CU
         for (uint32_t it = 0; it < kWaitLimit && !mbar_try(accum, 0); ++it) {
         }
     }
+    grid_trigger();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok && !*abort) {
         const int row = m0 + 32 * warp + lane;
@@ -400,6 +402,7 @@ k_dense_gemm_i8(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    grid_wait();  // the operands are the previous kernel's
 
     if (threadIdx.x == 0) {
         // TMA producer
@@ -451,6 +454,7 @@ k_dense_gemm_i8(const __grid_constant__ CUtensorMap ta0, const __grid_constant__
         for (uint32_t it = 0; it < kWaitLimit && !mbar_try(accum, 0); ++it) {
         }
     }
+    grid_trigger();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok && !*abort) {
         const int row = m0 + 32 * warp + lane;
@@ -733,6 +737,7 @@ k_dense_epilogue(void *__restrict__ psi_v, void *__restrict__ bparts_v, double *
     __shared__ double2 s_obs[8][10];
     const int t = E.t0 + blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x < 80) s_obs[threadIdx.x / 10][threadIdx.x % 10] = E.obs_c[threadIdx.x / 10][threadIdx.x % 10];
+    grid_wait();  // the column is the GEMM's, the rest of this step's inputs the previous epilogue's
     if constexpr (kI8) {
         const double2 *col = static_cast<const double2 *>(psi_v) + static_cast<size_t>(t) * (E.Dp / 2);
         for (int i = threadIdx.x; i < E.D; i += kThreads) s_col[i] = col[i];
@@ -912,6 +917,7 @@ k_dense_epilogue(void *__restrict__ psi_v, void *__restrict__ bparts_v, double *
             }
         }
     }
+    grid_trigger();
     // trapezoid (compensated) and this time point's value, one thread per observable
     if (yield_thread) {
         const int o = threadIdx.x;
@@ -1207,6 +1213,11 @@ int dense_run(DenseState &st, const DenseRun &run, void *psi128, int ldm, cudaSt
         return s < steps ? -0.5 * std::expm1(-2.0 * (0.5 * run.st_rate) * (0.5 * (run.times[s + 1] - run.times[s])))
                          : 0.0;
     };
+    // Each kernel of a group's chain is launched before its predecessor has ended and is
+    // set up by then (launch_dependent); the GEMM lets the epilogue in after its last
+    // MMA, the epilogue the GEMM after its last operand.  D = 576, 1000 trajectories,
+    // int8: 33.3 -> 30.4 us a step; D = 1024, 1024 trajectories, bf16x3 38.9 -> 34.2,
+    // int8 49.5 -> 46.4 us; 4096 trajectories, bf16x3: the same (100 us).
     // Two stream groups when the block has at least two trajectory tiles:
     // group g owns tiles [gt[g], gt[g+1]) and runs its GEMM -> epilogue chain
     // on its own stream, so one group's epilogue overlaps the other's GEMM
@@ -1238,24 +1249,18 @@ int dense_run(DenseState &st, const DenseRun &run, void *psi128, int ldm, cudaSt
         Eg.t1 = gt[g + 1] * BN;
         Eg.prev_values = point_prev >= 0 ? run.part + g * nv + static_cast<size_t>(point_prev) * run.nobs : nullptr;
         if (i8)
-            k_dense_epilogue<true><<<Eg.t1 - Eg.t0, kEpiThreadsI8, epi_smem, ss[g]>>>(
-                st.psi, bp, static_cast<double *>(st.b_scale), Eg);
+            launch_dependent(k_dense_epilogue<true>, Eg.t1 - Eg.t0, kEpiThreadsI8, epi_smem, ss[g], st.psi, bp, st.b_scale, Eg);
         else
-            k_dense_epilogue<false><<<Eg.t1 - Eg.t0, kEpiThreads, epi_smem, ss[g]>>>(st.psi, bp, nullptr, Eg);
+            launch_dependent(k_dense_epilogue<false>, Eg.t1 - Eg.t0, kEpiThreads, epi_smem, ss[g], st.psi, bp, nullptr, Eg);
     };
     auto gemm = [&](int g, cudaStream_t sg) {
         dim3 grid(gt[g + 1] - gt[g], Dp / kGM);
         if (i8)
-            gemm8<<<grid, kGThreads, smem, sg>>>(ta[0], ta[1], ta[2], ta[3], tb[0], tb[1], tb[2], tb[3],
-                                                           static_cast<const double *>(st.u_scale),
-                                                           static_cast<const double *>(st.b_scale),
-                                                           static_cast<double *>(st.psi), Dp, gt[g], run.status);
-        else if (ns == 2)
-            gemm2<<<grid, kGThreads, smem, sg>>>(ta[0], ta[1], ta[2], tb[0], tb[1], tb[2],
-                                                           static_cast<float *>(st.psi), Dp, gt[g], run.status);
+            launch_dependent(gemm8, grid, kGThreads, smem, sg, ta[0], ta[1], ta[2], ta[3], tb[0], tb[1], tb[2], tb[3],
+                             st.u_scale, st.b_scale, st.psi, Dp, gt[g], run.status);
         else
-            gemm3<<<grid, kGThreads, smem, sg>>>(ta[0], ta[1], ta[2], tb[0], tb[1], tb[2],
-                                                           static_cast<float *>(st.psi), Dp, gt[g], run.status);
+            launch_dependent(ns == 2 ? gemm2 : gemm3, grid, kGThreads, smem, sg, ta[0], ta[1], ta[2], tb[0], tb[1], tb[2],
+                             st.psi, Dp, gt[g], run.status);
     };
     if (G == 2) fork();
     // first time point: evaluate, first half-step flip of step 0, split

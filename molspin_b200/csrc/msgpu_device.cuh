@@ -18,6 +18,29 @@
 
 namespace msgpu {
 
+// Programmatic dependent launch: a step's kernels are launched before their
+// predecessor in the stream has ended.  Up to grid_wait() a kernel sets itself up
+// and touches no global memory; the wait returns when the predecessor has ended and
+// its writes are visible.  grid_trigger() lets the successor be scheduled.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args)
+{
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Raises a kernel's dynamic shared-memory limit on the current device to at
 // least `bytes` and never lowers it.  The limit is one attribute per kernel,
 // shared by every context of the process; contexts driven from several host
