@@ -113,7 +113,7 @@ struct msgpu_ctx {
     bool tc_ok = false;        // structure present (tables valid)
     int q_tile = 0, q_tile_ldm = 0;  // autotuned quartets per CTA (and the ldm it was tuned for)
     int q_variant = 0;               // autotuned kernel variant (kApplyVariants)
-    // resident (one warp per trajectory, whole time loop per launch) form
+    // resident form (one CTA per trajectory, the whole time loop in one launch)
     int form = MSGPU_FORM_AUTO;
     DevBuf trajval, times_d, pflip_d, work_d, obs_d, dense_part;
     // dense tensor-core form
@@ -1779,8 +1779,8 @@ void launch_apply(const msgpu_ctx *c, int v, int qt, dim3 grid, cudaStream_t st,
     apply_fits(c, v, qt, &smem);
     grid.y = width / (64 * kApplyVariants[v].np);
     if (smem) raise_smem_limit(reinterpret_cast<const void *>(kApplyVariants[v].fn), static_cast<int>(smem));
-    kApplyVariants[v].fn<<<grid, kThreads, smem, st>>>(quartet_view(c), w, s, U, part, c->D / 4, c->s1, c->s2, c->ldm,
-                                                       qt);
+    launch_dependent(kApplyVariants[v].fn, grid, kThreads, smem, st, quartet_view(c), w, s, U, part, c->D / 4, c->s1,
+        c->s2, c->ldm, qt);
 }
 
 int tune_quartet_tile(msgpu_ctx *c, const float2 *w, const double *s, float2 *U, double *part)
@@ -2109,11 +2109,11 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
     double *beta0 = static_cast<double *>(c->beta0.p);
     auto yield_update = [&](double dt, int init, int row) {
         Timed tm(c, KC_YIELD);
-        k_yield<<<dim3(ldm / 32, nobs + 1), dim3(32, 32), 0, st>>>(
-            static_cast<double *>(c->qpart_obs.p), static_cast<double *>(c->qpart_nrm.p), qt, nobs, ldm, M,
-            static_cast<double *>(c->rates_d.p), dt, init, static_cast<double *>(c->prev.p),
-            static_cast<double *>(c->acc.p), static_cast<double *>(c->comp.p), beta0, sc,
-            values + static_cast<size_t>(row) * nobs, static_cast<int *>(c->status.p) + 1, static_cast<int *>(c->status.p));
+        launch_dependent(k_yield, dim3(ldm / 32, nobs + 1), dim3(32, 32), 0, st, static_cast<double *>(c->qpart_obs.p),
+            static_cast<double *>(c->qpart_nrm.p), qt, nobs, ldm, M, static_cast<double *>(c->rates_d.p), dt, init,
+            static_cast<double *>(c->prev.p), static_cast<double *>(c->acc.p), static_cast<double *>(c->comp.p), beta0,
+            sc, values + static_cast<size_t>(row) * nobs, static_cast<int *>(c->status.p) + 1,
+            static_cast<int *>(c->status.p));
     };
 
     // Evaluate the first time point and apply the first half-step flip.
@@ -2121,15 +2121,13 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
         Timed tm(c, KC_COMBINE);
         const long long sB = -1;
         if (prec == MSGPU_PREC_C128)
-            k_combine<double2, false><<<qgrid, qblock, 0, st>>>(
-                static_cast<double2 *>(c->psi128.p), nullptr, nullptr, 0, nullptr, nullptr, mws, c->s1, c->s2, Q, ldm, QR, nz,
-                steps > 0 ? g0 : -1, 0, pstep(0), sB, 0, 0.0, po, static_cast<double *>(c->qpart_obs.p),
-                static_cast<double *>(c->qpart_nrm.p));
+            launch_dependent(k_combine<double2, false>, qgrid, qblock, 0, st, static_cast<double2 *>(c->psi128.p),
+                nullptr, nullptr, 0, nullptr, nullptr, mws, c->s1, c->s2, Q, ldm, QR, nz, steps > 0 ? g0 : -1, 0,
+                pstep(0), sB, 0, 0.0, po, static_cast<double *>(c->qpart_obs.p), static_cast<double *>(c->qpart_nrm.p));
         else
-            k_combine_pp<false><<<dim3(qt, ldm / 64), qblock, 0, st>>>(
-                static_cast<float2 *>(c->basis.p), nullptr, 0, nullptr, nullptr, c->s1, c->s2, Q, ldm, QR, nz,
-                steps > 0 ? g0 : -1, 0, pstep(0), sB, 0, 0.0, po, static_cast<double *>(c->qpart_obs.p),
-                static_cast<double *>(c->qpart_nrm.p));
+            launch_dependent(k_combine_pp<false>, dim3(qt, ldm / 64), qblock, 0, st, static_cast<float2 *>(c->basis.p),
+                nullptr, 0, nullptr, nullptr, c->s1, c->s2, Q, ldm, QR, nz, steps > 0 ? g0 : -1, 0, pstep(0), sB, 0,
+                0.0, po, static_cast<double *>(c->qpart_obs.p), static_cast<double *>(c->qpart_nrm.p));
     }
     yield_update(0.0, 1, 0);
     int fused_c = 0;  // cluster size of k_lanczos_fused, 0: the four-kernel iteration
@@ -2224,6 +2222,12 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
         arn.mdim = static_cast<int *>(c->mdim.p);
         if ((e = arnoldi_scratch(arn, c->part2.p, m, ldm, st))) return cuda_fail(c, e, "Arnoldi scratch");
     }
+    // A step is a chain of short kernels, each launched before its predecessor has ended
+    // (launch_dependent), which closes most of the gap between them.  With and without, m =
+    // 16, a step: complex64 D = 9216, 250 trajectories 651 / 776 us; D = 4096 with sinks, 256
+    // trajectories 1136 / 1319 us; Taylor D = 2048, 256 trajectories 243 / 290 us; complex128
+    // D = 2048 / 8192, 256 trajectories 474 / 650, 1646 / 1797 us; D = 16384 the same.  No
+    // kernel triggers its successor early: CTAs that wait would hold places (sinks 1214 us).
     // Trajectory groups: the step's kernels work on columns [t0, t0 + width)
     // through offset pointers with the row stride ldm, so the groups share the
     // buffers.  With overlap each group has its own stream (group 0 the
@@ -2301,7 +2305,8 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                         const bool end = k == mt;
                         const int what = (end ? kTaylorEnd : kTaylorOut) | (k % 2 == 0 ? kTaylorBoth : end ? kTaylorAdd : 0);
                         Timed tm(c, KC_APPLY);
-                        k_taylor_term_q<<<gq, kThreads, 0, st>>>(pg, tmu, k == 1 ? F : cur, nxt, F, dt / (nsub * k), eta, what);
+                        launch_dependent(k_taylor_term_q, gq, kThreads, 0, st, pg, tmu, k == 1 ? F : cur, nxt, F,
+                            dt / (nsub * k), eta, what);
                         std::swap(cur, nxt);
                     }
             } else {
@@ -2311,19 +2316,20 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                 for (int sub = 0; sub < nsub; ++sub) {
                     for (int k = 1; k <= mt; ++k) {
                         Timed tm(c, KC_APPLY);
-                        k_taylor_term<<<tgrid, tblock, 0, st>>>(Hd, Kd, kappa, tmu, cur, nxt, F, dt / (nsub * k), D, ldm);
+                        launch_dependent(k_taylor_term, tgrid, tblock, 0, st, Hd, Kd, kappa, tmu, cur, nxt, F,
+                            dt / (nsub * k), D, ldm);
                         std::swap(cur, nxt);
                     }
                     Timed tm(c, KC_ORTH);
-                    k_taylor_rescale<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(F, cur, eta, n);
+                    launch_dependent(k_taylor_rescale, static_cast<unsigned>((n + 255) / 256), 256, 0, st, F, cur, eta,
+                        n);
                 }
             }
             {
                 Timed tm(c, KC_COMBINE);
-                k_combine<double2, false><<<qgrid, qblock, 0, st>>>(
-                    F, nullptr, nullptr, 0, nullptr, nullptr, mws, c->s1, c->s2, Q, ldm, QR, nz, g, 1, pstep(s),
-                    s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po, static_cast<double *>(c->qpart_obs.p),
-                    static_cast<double *>(c->qpart_nrm.p));
+                launch_dependent(k_combine<double2, false>, qgrid, qblock, 0, st, F, nullptr, nullptr, 0, nullptr,
+                    nullptr, mws, c->s1, c->s2, Q, ldm, QR, nz, g, 1, pstep(s), s + 1 < steps ? g + 1 : -1, 0,
+                    pstep(s + 1), po, static_cast<double *>(c->qpart_obs.p), static_cast<double *>(c->qpart_nrm.p));
             }
         } else if (rk4) {
             double2 *psi = static_cast<double2 *>(c->psi128.p);
@@ -2351,18 +2357,17 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                     if (int rc = refresh_quartet_values(c)) return rc;
                 Timed tm(c, KC_APPLY);
                 if (quartet_gen)
-                    k_rk4_stage_q<<<dim3(ceil_div(Q, kWarps), ldm / 32), kThreads, 0, st>>>(
-                        pg, in[stage], psi, out[stage], acc, cs[stage], ws[stage], stage + 1);
+                    launch_dependent(k_rk4_stage_q, dim3(ceil_div(Q, kWarps), ldm / 32), kThreads, 0, st, pg, in[stage],
+                        psi, out[stage], acc, cs[stage], ws[stage], stage + 1);
                 else
-                    k_rk4_stage<<<tgrid, tblock, 0, st>>>(Hd, Kd, kappa, in[stage], psi, out[stage], acc, cs[stage],
-                                                          ws[stage], stage + 1, D, ldm);
+                    launch_dependent(k_rk4_stage, tgrid, tblock, 0, st, Hd, Kd, kappa, in[stage], psi, out[stage], acc,
+                        cs[stage], ws[stage], stage + 1, D, ldm);
             }
             {
                 Timed tm(c, KC_COMBINE);
-                k_combine<double2, false><<<qgrid, qblock, 0, st>>>(
-                    psi, nullptr, nullptr, 0, nullptr, nullptr, mws, c->s1, c->s2, Q, ldm, QR, nz, g, 1, pstep(s),
-                    s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po, static_cast<double *>(c->qpart_obs.p),
-                    static_cast<double *>(c->qpart_nrm.p));
+                launch_dependent(k_combine<double2, false>, qgrid, qblock, 0, st, psi, nullptr, nullptr, 0, nullptr,
+                    nullptr, mws, c->s1, c->s2, Q, ldm, QR, nz, g, 1, pstep(s), s + 1 < steps ? g + 1 : -1, 0,
+                    pstep(s + 1), po, static_cast<double *>(c->qpart_obs.p), static_cast<double *>(c->qpart_nrm.p));
             }
         } else if (three_term) {
             // slot 0 of the basis is the state itself, w_j (j >= 1) at basis + (j - 1) n
@@ -2390,26 +2395,25 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                     const double *sj = sc + static_cast<size_t>(j) * ldm + t0;
                     {
                         Timed tm(c, KC_APPLY, gs);
-                        k_lanczos_apply_d<<<dim3(nqt, width / 32), kThreads, 0, gs>>>(Hq, slot(j) + t0, sj, U + t0, part + t0, Q,
-                                                                                      c->s1, c->s2, ldm, QT);
+                        launch_dependent(k_lanczos_apply_d, dim3(nqt, width / 32), kThreads, 0, gs, Hq, slot(j) + t0,
+                            sj, U + t0, part + t0, Q, c->s1, c->s2, ldm, QT);
                     }
                     {
                         Timed tm(c, KC_REDUCE, gs);
-                        k_lanczos_reduce<<<width / 32, dim3(32, kRedRows), 0, gs>>>(part + t0, nqt, ldm, 0, j, mws, alpha + t0,
-                                                                                    td + tm0, to + tm0, mdim + t0);
+                        launch_dependent(k_lanczos_reduce, width / 32, dim3(32, kRedRows), 0, gs, part + t0, nqt, ldm,
+                            0, j, mws, alpha + t0, td + tm0, to + tm0, mdim + t0);
                     }
                     if (j == m - 1) break;  // T_m is complete; w_m is never used
                     {
                         Timed tm(c, KC_ORTH, gs);
-                        k_lanczos_update_d<<<dim3(nt, width / 32), kThreads, 0, gs>>>(
-                            U + t0, slot(j) + t0, j > 0 ? slot(j - 1) + t0 : nullptr, sj, j > 0 ? sj - ldm : nullptr, alpha + t0,
-                            slot(j + 1) + t0, part + t0, D, ldm, R);
+                        launch_dependent(k_lanczos_update_d, dim3(nt, width / 32), kThreads, 0, gs, U + t0,
+                            slot(j) + t0, j > 0 ? slot(j - 1) + t0 : nullptr, sj, j > 0 ? sj - ldm : nullptr,
+                            alpha + t0, slot(j + 1) + t0, part + t0, D, ldm, R);
                     }
                     {
                         Timed tm(c, KC_REDUCE, gs);
-                        k_lanczos_reduce<<<width / 32, dim3(32, kRedRows), 0, gs>>>(
-                            part + t0, nt, ldm, 1, j, mws, sc + static_cast<size_t>(j + 1) * ldm + t0, td + tm0, to + tm0,
-                            mdim + t0);
+                        launch_dependent(k_lanczos_reduce, width / 32, dim3(32, kRedRows), 0, gs, part + t0, nt, ldm, 1,
+                            j, mws, sc + static_cast<size_t>(j + 1) * ldm + t0, td + tm0, to + tm0, mdim + t0);
                     }
                 }
                 {
@@ -2417,19 +2421,19 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                     const int live = std::max(0, std::min(M - t0, width));
                     int *status = static_cast<int *>(c->status.p);
                     if (dt * hn <= 128.0)
-                        k_lanczos_expm<<<ceil_div(width, 8), 256, 0, gs>>>(td + tm0, to + tm0, kappa, mdim + t0, beta0 + t0,
-                                                                           sc + t0, mws, ldm, live, dt, coef + t0, status, width);
+                        launch_dependent(k_lanczos_expm, ceil_div(width, 8), 256, 0, gs, td + tm0, to + tm0, kappa,
+                            mdim + t0, beta0 + t0, sc + t0, mws, ldm, live, dt, coef + t0, status, width);
                     else
-                        k_krylov_expm<<<ceil_div(width, expm_warps), 32 * expm_warps, expm_warps * expm_smem_warp, gs>>>(
-                            nullptr, td + tm0, to + tm0, kappa, mdim + t0, beta0 + t0, sc + t0, mws, ldm, live, dt, coef + t0,
-                            status, width);
+                        launch_dependent(k_krylov_expm, ceil_div(width, expm_warps), 32 * expm_warps,
+                            expm_warps * expm_smem_warp, gs, nullptr, td + tm0, to + tm0, kappa, mdim + t0, beta0 + t0,
+                            sc + t0, mws, ldm, live, dt, coef + t0, status, width);
                 }
                 {
                     Timed tm(c, KC_COMBINE, gs);
                     Noise gnz = nz;
                     gnz.traj_offset = static_cast<uint32_t>(t0);
-                    k_combine<double2, true><<<dim3(qt, width / 32), qblock, 0, gs>>>(
-                        psi + t0, psi + t0, Wb + t0, n, coef + t0, mdim + t0, mws, c->s1, c->s2, Q, ldm, QR, gnz, g, 1, pstep(s),
+                    launch_dependent(k_combine<double2, true>, dim3(qt, width / 32), qblock, 0, gs, psi + t0, psi + t0,
+                        Wb + t0, n, coef + t0, mdim + t0, mws, c->s1, c->s2, Q, ldm, QR, gnz, g, 1, pstep(s),
                         s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po, static_cast<double *>(c->qpart_obs.p) + t0,
                         static_cast<double *>(c->qpart_nrm.p) + t0);
                 }
@@ -2445,29 +2449,29 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                     Timed tm(c, KC_APPLY);
                     const double *sj = sc + static_cast<size_t>(j) * ldm;
                     if (quartet128)
-                        k_arnoldi_apply_q<<<dim3(ceil_div(Q, kWarps), ldm / 32), kThreads, 0, st>>>(
+                        launch_dependent(k_arnoldi_apply_q, dim3(ceil_div(Q, kWarps), ldm / 32), kThreads, 0, st,
                             QuartetD{static_cast<const int *>(c->qrow.p), static_cast<const int2 *>(c->qcolt.p),
                                      static_cast<const double2 *>(c->qval64.p), static_cast<const int *>(c->qbase.p)},
                             kappa, B.slot(j), sj, B.slot(j + 1), Q, c->s1, c->s2, ldm);
                     else
-                        k_arnoldi_apply<<<grid, kThreads, 0, st>>>(Hd, Kd, kappa, B.slot(j), sj, B.slot(j + 1), D, ldm, R);
+                        launch_dependent(k_arnoldi_apply, grid, kThreads, 0, st, Hd, Kd, kappa, B.slot(j), sj,
+                            B.slot(j + 1), D, ldm, R);
                 }
                 Timed tm(c, KC_ORTH);
                 c->launches += arnoldi_orthogonalise(B, arn, j, st) - 1;
             }
             {
                 Timed tm(c, KC_EXPM);
-                k_krylov_expm<<<ceil_div(ldm, expm_warps), 32 * expm_warps, expm_warps * expm_smem_warp, st>>>(
-                    static_cast<double2 *>(c->hess.p), nullptr, nullptr, 0.0, static_cast<int *>(c->mdim.p), beta0, sc, mws,
-                    ldm, M, dt, static_cast<double2 *>(c->coef.p), static_cast<int *>(c->status.p), ldm);
+                launch_dependent(k_krylov_expm, ceil_div(ldm, expm_warps), 32 * expm_warps, expm_warps * expm_smem_warp,
+                    st, static_cast<double2 *>(c->hess.p), nullptr, nullptr, 0.0, static_cast<int *>(c->mdim.p), beta0,
+                    sc, mws, ldm, M, dt, static_cast<double2 *>(c->coef.p), static_cast<int *>(c->status.p), ldm);
             }
             {
                 Timed tm(c, KC_COMBINE);
-                k_combine<double2, true><<<qgrid, qblock, 0, st>>>(
-                    psi, psi, Wb, n, static_cast<double2 *>(c->coef.p),
-                    static_cast<int *>(c->mdim.p), mws, c->s1, c->s2, Q, ldm, QR, nz, g, 1, pstep(s),
-                    s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po, static_cast<double *>(c->qpart_obs.p),
-                    static_cast<double *>(c->qpart_nrm.p));
+                launch_dependent(k_combine<double2, true>, qgrid, qblock, 0, st, psi, psi, Wb, n,
+                    static_cast<double2 *>(c->coef.p), static_cast<int *>(c->mdim.p), mws, c->s1, c->s2, Q, ldm, QR, nz,
+                    g, 1, pstep(s), s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po,
+                    static_cast<double *>(c->qpart_obs.p), static_cast<double *>(c->qpart_nrm.p));
             }
         } else if (arn64) {
             // complex64 Arnoldi for K = I (x) K4; one trajectory group
@@ -2486,16 +2490,16 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
             }
             {
                 Timed tm(c, KC_EXPM);
-                k_krylov_expm<<<ceil_div(ldm, expm_warps), 32 * expm_warps, expm_warps * expm_smem_warp, st>>>(
-                    static_cast<double2 *>(c->hess.p), nullptr, nullptr, 0.0, static_cast<int *>(c->mdim.p), beta0, sc,
-                    mws, ldm, M, dt, static_cast<double2 *>(c->coef.p), static_cast<int *>(c->status.p), ldm);
+                launch_dependent(k_krylov_expm, ceil_div(ldm, expm_warps), 32 * expm_warps, expm_warps * expm_smem_warp,
+                    st, static_cast<double2 *>(c->hess.p), nullptr, nullptr, 0.0, static_cast<int *>(c->mdim.p), beta0,
+                    sc, mws, ldm, M, dt, static_cast<double2 *>(c->coef.p), static_cast<int *>(c->status.p), ldm);
             }
             {
                 Timed tm(c, KC_COMBINE);
-                k_combine_pp<true><<<dim3(qt, ldm / 64), qblock, 0, st>>>(
-                    Wb, Wb, n, static_cast<double2 *>(c->coef.p), static_cast<int *>(c->mdim.p), c->s1, c->s2, Q, ldm,
-                    QR, nz, g, 1, pstep(s), s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po,
-                    static_cast<double *>(c->qpart_obs.p), static_cast<double *>(c->qpart_nrm.p));
+                launch_dependent(k_combine_pp<true>, dim3(qt, ldm / 64), qblock, 0, st, Wb, Wb, n,
+                    static_cast<double2 *>(c->coef.p), static_cast<int *>(c->mdim.p), c->s1, c->s2, Q, ldm, QR, nz, g,
+                    1, pstep(s), s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po, static_cast<double *>(c->qpart_obs.p),
+                    static_cast<double *>(c->qpart_nrm.p));
             }
         } else {
             float2 *Wb = static_cast<float2 *>(c->basis.p);  // w_0 = state
@@ -2523,37 +2527,36 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                     }
                     {
                         Timed tm(c, KC_REDUCE, gs);
-                        k_lanczos_reduce<<<width / 32, dim3(32, kRedRows), 0, gs>>>(part + t0, nqt, ldm, 0, j, mws, alpha + t0,
-                                                                             td + tm0, to + tm0, mdim + t0);
+                        launch_dependent(k_lanczos_reduce, width / 32, dim3(32, kRedRows), 0, gs, part + t0, nqt, ldm,
+                            0, j, mws, alpha + t0, td + tm0, to + tm0, mdim + t0);
                     }
                     if (j == m - 1) break;  // T_m is complete; w_m is never used
                     {
                         Timed tm(c, KC_ORTH, gs);
-                        k_lanczos_update<<<grid, kThreads, 0, gs>>>(
-                            U + t0, Wb + j * n + t0, j > 0 ? Wb + (j - 1) * n + t0 : nullptr,
-                            sc + static_cast<size_t>(j) * ldm + t0, j > 0 ? sc + static_cast<size_t>(j - 1) * ldm + t0 : nullptr,
-                            alpha + t0, Wb + (j + 1) * n + t0, part + t0, D, ldm, Ru);
+                        launch_dependent(k_lanczos_update, grid, kThreads, 0, gs, U + t0, Wb + j * n + t0,
+                            j > 0 ? Wb + (j - 1) * n + t0 : nullptr, sc + static_cast<size_t>(j) * ldm + t0,
+                            j > 0 ? sc + static_cast<size_t>(j - 1) * ldm + t0 : nullptr, alpha + t0,
+                            Wb + (j + 1) * n + t0, part + t0, D, ldm, Ru);
                     }
                     {
                         Timed tm(c, KC_REDUCE, gs);
-                        k_lanczos_reduce<<<width / 32, dim3(32, kRedRows), 0, gs>>>(part + t0, ntu, ldm, 1, j, mws,
-                                                                             sc + static_cast<size_t>(j + 1) * ldm + t0,
-                                                                             td + tm0, to + tm0, mdim + t0);
+                        launch_dependent(k_lanczos_reduce, width / 32, dim3(32, kRedRows), 0, gs, part + t0, ntu, ldm,
+                            1, j, mws, sc + static_cast<size_t>(j + 1) * ldm + t0, td + tm0, to + tm0, mdim + t0);
                     }
                 }
                 {
                     Timed tm(c, KC_EXPM, gs);
-                    k_lanczos_expm<<<ceil_div(width, 8), 256, 0, gs>>>(
-                        td + tm0, to + tm0, kappa, mdim + t0, beta0 + t0, sc + t0, mws, ldm,
-                        std::max(0, std::min(M - t0, width)), dt, coef + t0, static_cast<int *>(c->status.p), width);
+                    launch_dependent(k_lanczos_expm, ceil_div(width, 8), 256, 0, gs, td + tm0, to + tm0, kappa,
+                        mdim + t0, beta0 + t0, sc + t0, mws, ldm, std::max(0, std::min(M - t0, width)), dt, coef + t0,
+                        static_cast<int *>(c->status.p), width);
                 }
                 {
                     Timed tm(c, KC_COMBINE, gs);
                     Noise gnz = nz;
                     gnz.traj_offset = static_cast<uint32_t>(t0);
-                    k_combine_pp<true><<<dim3(qt, width / 64), qblock, 0, gs>>>(
-                        Wb + t0, Wb + t0, n, coef + t0, mdim + t0, c->s1, c->s2, Q, ldm, QR, gnz, g, 1, pstep(s),
-                        s + 1 < steps ? g + 1 : -1, 0, pstep(s + 1), po, qobs + t0, qnrm + t0);
+                    launch_dependent(k_combine_pp<true>, dim3(qt, width / 64), qblock, 0, gs, Wb + t0, Wb + t0, n,
+                        coef + t0, mdim + t0, c->s1, c->s2, Q, ldm, QR, gnz, g, 1, pstep(s), s + 1 < steps ? g + 1 : -1,
+                        0, pstep(s + 1), po, qobs + t0, qnrm + t0);
                 }
             });
             if (rc) return rc;

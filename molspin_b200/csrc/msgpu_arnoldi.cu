@@ -33,12 +33,12 @@ int orthogonalise(const ArnoldiVectors<T> &B, const ArnoldiPairK &K, const T *U,
                   cudaStream_t st)
 {
     const dim3 grid((B.Q + S.QT - 1) / S.QT, B.ldm / 32);
-    Passes<T, kPairK>::dots(j, kBatches)<<<grid, kThreads, 0, st>>>(B, K, U, S, j, 0);
+    launch_dependent(Passes<T, kPairK>::dots(j, kBatches), grid, kThreads, 0, st, B, K, U, S, j, 0);
     if (j == S.m - 1) return 1;  // w_m is never used
     const auto update = Passes<T, kPairK>::update(j, kBatches);
-    update<<<grid, kThreads, 0, st>>>(B, S, j, 0);
-    Passes<T, false>::dots(j, kBatches)<<<grid, kThreads, 0, st>>>(B, K, nullptr, S, j, 1);
-    update<<<grid, kThreads, 0, st>>>(B, S, j, 1);
+    launch_dependent(update, grid, kThreads, 0, st, B, S, j, 0);
+    launch_dependent(Passes<T, false>::dots(j, kBatches), grid, kThreads, 0, st, B, K, nullptr, S, j, 1);
+    launch_dependent(update, grid, kThreads, 0, st, B, S, j, 1);
     return 4;
 }
 

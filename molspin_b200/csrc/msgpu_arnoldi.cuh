@@ -71,6 +71,7 @@ template <typename T, int NB, bool kPairK>
 __global__ void __launch_bounds__(kThreads)
 k_arn_dots(ArnoldiVectors<T> B, ArnoldiPairK K, const T *__restrict__ U, ArnoldiScratch S, int j, int pass)
 {
+    grid_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.y * 32 + lane;
     if (pass == 1 && !S.tile_again[blockIdx.y]) return;
@@ -176,6 +177,7 @@ template <typename T, int NB>
 __global__ void __launch_bounds__(kThreads)
 k_arn_update(ArnoldiVectors<T> B, ArnoldiScratch S, int j, int pass)
 {
+    grid_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.y * 32 + lane;
     if (pass == 1 && !S.tile_again[blockIdx.y]) return;

@@ -21,12 +21,15 @@ namespace msgpu {
 // Programmatic dependent launch: a step's kernels are launched before their
 // predecessor in the stream has ended.  Up to grid_wait() a kernel sets itself up
 // and touches no global memory; the wait returns when the predecessor has ended and
-// its writes are visible.  grid_trigger() lets the successor be scheduled.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// its writes are visible.  grid_trigger() lets the successor be scheduled; without it
+// that happens as the last CTAs leave.  A kernel given to launch_dependent has the wait
+// in every CTA, before its first access to global memory.
+__device__ __forceinline__ void grid_wait() { cudaGridDependencySynchronize(); }
+__device__ __forceinline__ void grid_trigger() { cudaTriggerProgrammaticLaunchCompletion(); }
 
 template <typename... P, typename... A>
-inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args)
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                    A... args)
 {
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;

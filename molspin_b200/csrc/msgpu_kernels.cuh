@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(kThreads)
 k_arnoldi_apply(CsrD H, CsrD K, double kappa, const double2 *__restrict__ src, const double *__restrict__ scale,
                 double2 *__restrict__ W, int D, int ldm, int R)
 {
+    grid_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.y * 32 + lane;
     const int r0 = blockIdx.x * R;
@@ -168,6 +169,7 @@ __global__ void __launch_bounds__(kThreads)
 k_arnoldi_apply_q(QuartetD H, double kappa, const double2 *__restrict__ src, const double *__restrict__ scale,
                   double2 *__restrict__ W, int Q, int s1, int s2, int ldm)
 {
+    grid_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.y * 32 + lane;
     const int q = blockIdx.x * kWarps + warp;
@@ -218,6 +220,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 k_lanczos_apply_d(QuartetD H, const double2 *__restrict__ wj, const double *__restrict__ sj, double2 *__restrict__ U,
                   double *__restrict__ part, int Q, int s1, int s2, int ldm, int QT)
 {
+    grid_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.y * 32 + lane;
     const int q0 = blockIdx.x * QT;
@@ -268,6 +271,7 @@ k_lanczos_update_d(const double2 *__restrict__ U, const double2 *__restrict__ wj
                    const double *__restrict__ sj, const double *__restrict__ sjm1, const double *__restrict__ alpha,
                    double2 *__restrict__ wn, double *__restrict__ part, int D, int ldm, int R)
 {
+    grid_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.y * 32 + lane;
     const int r0 = blockIdx.x * R;
@@ -437,6 +441,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 k_lanczos_apply_compact(QuartetC H, const float2 *__restrict__ wj, const double *__restrict__ sj,
                         float2 *__restrict__ U, double *__restrict__ part, int Q, int s1, int s2, int ldm, int QT)
 {
+    grid_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.y * 64 + 2 * lane;
     const int q0 = blockIdx.x * QT;
@@ -595,6 +600,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 k_lanczos_apply_np(QuartetC H, const float2 *__restrict__ wj, const double *__restrict__ sj, float2 *__restrict__ U,
                    double *__restrict__ part, int Q, int s1, int s2, int ldm, int QT)
 {
+    grid_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tb = blockIdx.y * 64 * NP + 2 * lane;
     const int q0 = blockIdx.x * QT;
@@ -673,6 +679,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 k_lanczos_apply_cube(QuartetC H, const float2 *__restrict__ wj, const double *__restrict__ sj, float2 *__restrict__ U,
                      double *__restrict__ part, int Q, int s1, int s2, int ldm, int QT)
 {
+    grid_wait();
     extern __shared__ float4 cube[];  // [QT * 4 rows][32 lanes]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.y * 64 + 2 * lane;
@@ -741,6 +748,7 @@ k_lanczos_update(const float2 *__restrict__ U, const float2 *__restrict__ wj, co
                  const double *__restrict__ sj, const double *__restrict__ sjm1, const double *__restrict__ alpha,
                  float2 *__restrict__ wn, double *__restrict__ part, int D, int ldm, int R)
 {
+    grid_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.y * 64 + 2 * lane;
     const int r0 = blockIdx.x * R;
@@ -793,6 +801,7 @@ __global__ void __launch_bounds__(32 * kRedRows)
 k_lanczos_reduce(const double *__restrict__ part, int ntiles, int ldm, int mode, int j, int m, double *__restrict__ out,
                  double *__restrict__ tdiag, double *__restrict__ toff, int *__restrict__ mdim)
 {
+    grid_wait();
     __shared__ double red[kRedRows][33];
     const int t = blockIdx.x * 32 + threadIdx.x;
     double ps = 0.0;
@@ -831,6 +840,7 @@ __global__ void k_krylov_expm(const double2 *__restrict__ hess, const double *__
                               int ldm, int M, double dt, double2 *__restrict__ coef, int *__restrict__ status,
                               int width)
 {
+    grid_wait();
     extern __shared__ double2 smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + warp;
@@ -878,6 +888,7 @@ __global__ void __launch_bounds__(256)
 k_taylor_term(CsrD H, CsrD K, double kappa, double2 mu, const double2 *__restrict__ in, double2 *__restrict__ out,
               double2 *__restrict__ F, double scale, int D, int ldm)
 {
+    grid_wait();
     const int t = blockIdx.y * 32 + threadIdx.x;
     const int r = blockIdx.x * 8 + threadIdx.y;
     if (r >= D) return;
@@ -911,6 +922,7 @@ __global__ void __launch_bounds__(256)
 k_rk4_stage(CsrD H, CsrD K, double kappa, const double2 *__restrict__ y_in, double2 *psi, double2 *__restrict__ y_out,
             double2 *__restrict__ acc, double c, double w, int stage, int D, int ldm)
 {
+    grid_wait();
     const int t = blockIdx.y * 32 + threadIdx.x;
     const int r = blockIdx.x * 8 + threadIdx.y;
     if (r >= D) return;
@@ -941,6 +953,7 @@ k_rk4_stage(CsrD H, CsrD K, double kappa, const double2 *__restrict__ y_in, doub
 // End of a Taylor sub-step: F <- eta F (the shift e^{tau mu / s}), B <- F.
 __global__ void k_taylor_rescale(double2 *__restrict__ F, double2 *__restrict__ B, double2 eta, size_t n)
 {
+    grid_wait();
     const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double2 f = cmul(eta, F[i]);
@@ -1012,6 +1025,7 @@ constexpr int kTaylorEnd = 8;   // F *= eta, the end of a sub-step
 __global__ void __launch_bounds__(kThreads, 4)
 k_taylor_term_q(PairGenerator G, double2 mu, const double2 *in, double2 *out, double2 *F, double scale, double2 eta, int what)
 {
+    grid_wait();
     const int t = blockIdx.y * 32 + (threadIdx.x & 31);
     const int q = blockIdx.x * kWarps + (threadIdx.x >> 5);
     if (q >= G.Q) return;
@@ -1036,6 +1050,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 k_rk4_stage_q(PairGenerator G, const double2 *y_in, double2 *psi, double2 *__restrict__ y_out, double2 *__restrict__ acc,
               double c, double w, int stage)
 {
+    grid_wait();
     const int t = blockIdx.y * 32 + (threadIdx.x & 31);
     const int q = blockIdx.x * kWarps + (threadIdx.x >> 5);
     if (q >= G.Q) return;
@@ -1101,6 +1116,7 @@ k_lanczos_expm(const double *__restrict__ tdiag, const double *__restrict__ toff
                const int *__restrict__ mdim, const double *__restrict__ beta0, const double *__restrict__ vscale,
                int m, int ldm, int M, double dt, double2 *__restrict__ coef, int *__restrict__ status, int width)
 {
+    grid_wait();
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= width) return;  // whole warps leave together
@@ -1182,6 +1198,7 @@ k_combine(T *psi, const T *V0, const T *__restrict__ V, size_t vstride, const do
           int halfA, double pA, long long stepB, int halfB, double pB, PairObs po, double *__restrict__ part_obs,
           double *__restrict__ part_nrm)
 {
+    grid_wait();
     // blockDim = (32, 8): x over trajectories, y over quartets of the tile
     const int t = blockIdx.y * 32 + threadIdx.x;
     const int q0 = blockIdx.x * QR;
@@ -1256,6 +1273,7 @@ k_combine_pp(float2 *__restrict__ psi, const float2 *__restrict__ V, size_t vstr
              double pA, long long stepB, int halfB, double pB, PairObs po, double *__restrict__ part_obs,
              double *__restrict__ part_nrm)
 {
+    grid_wait();
     const int t = blockIdx.y * 64 + 2 * threadIdx.x;
     const int q0 = blockIdx.x * QR;
     double obs[2][8] = {{0, 0, 0, 0, 0, 0, 0, 0}, {0, 0, 0, 0, 0, 0, 0, 0}};
@@ -1412,6 +1430,7 @@ k_yield(const double *__restrict__ part_obs, const double *__restrict__ part_nrm
         double *__restrict__ comp, double *__restrict__ beta0, double *__restrict__ inv0, double *__restrict__ values_out,
         int *__restrict__ count, int *__restrict__ status)
 {
+    grid_wait();
     __shared__ double red[32][33];
     __shared__ int last;
     const int t = blockIdx.x * 32 + threadIdx.x, y = threadIdx.y;
