@@ -677,7 +677,7 @@ def run_batching(args):
         "clocks": clk, "e2e": None, "gpu_launches": launches,
         "routes": {"persistent": sum(not i["streamed"] for i in infos), "streamed": sum(i["streamed"] for i in infos),
                    "streamed_spmm_picks": {k: sorted(v) for k, v in picks.items()}},
-        "launch_note": "per bench step: one graph replay of the persistent k_batch launch (systems below D=2048) "
+        "launch_note": "per bench step: a resident launch per system below D=2048 on side streams "
                        "plus the streamed path's kernels for the larger systems", "cpu_baseline": None})
 
 

@@ -1,5 +1,5 @@
-// msgpu_batch.cuh -- batching form: many spin systems of uneven dimension
-// and uneven trajectory counts in ONE persistent launch.
+// msgpu_batch.cuh -- the batching form's persistent launch, for the systems
+// below the streamed route that the resident kernels do not hold.
 //
 // The launch covers every time step of every (system, trajectory) item of
 // the batch.  CTAs are persistent (a few per SM) and pull work from two

@@ -22,7 +22,7 @@ memory.
 Small systems share launches.  Requests below `pack_dim` (the batching
 form's persistent route, D < 2048) that share a time grid and Krylov
 dimension are admitted together, up to `pack_max` of them in one slot, and
-run as one persistent launch of the batching form (msgpu_batch_*) on a
+run as one batch of the batching form (msgpu_batch_*) on a
 pooled batch whose device buffers are kept between packs
 (msgpu_batch_clear).  A system's result in a batch does not depend on its
 companions, and a small request solved alone also runs as a one-system
@@ -154,7 +154,7 @@ class ServingEngine:
             return self._run(p, req)
 
     def solve_pack(self, reqs: list[Request], batch):
-        """Requests of one pack key in one persistent launch on a pooled batch
+        """Requests of one pack key in one batch on a pooled batch
         (a new one when batch is None); returns (ensemble yields per request,
         the batch to keep for the pool)."""
         from .batching import BatchB200
