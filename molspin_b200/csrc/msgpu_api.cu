@@ -21,6 +21,7 @@
 #include "msgpu_resident.h"
 #include "msgpu_spmm_tc.cuh"
 #include "msgpu_spmm_tm.cuh"
+#include "msgpu_tiles.h"
 
 using namespace msgpu;
 
@@ -289,16 +290,6 @@ int traj_groups(const msgpu_ctx *c)
     return 1;
 }
 
-// Rows per tile: keep about 64-128 row tiles per trajectory tile so that the
-// partial-sum buffers stay small and every SM has several CTAs.
-int pick_rows_per_tile(int D)
-{
-    int R = D / 64;
-    R = std::max(8, std::min(512, R));
-    R = (R + 7) / 8 * 8;
-    return R;
-}
-
 // largest absolute row sum of a CSR matrix (interleaved complex values)
 double row_sum_norm(int dim, const int *rowptr, const double *val)
 {
@@ -321,14 +312,6 @@ int update_rows(int D, int R, int ctiles, int max_tiles)
 {
     while (R > 32 && ceil_div(D, R) * ctiles < 3 * 148 && ceil_div(D, (R / 2 + 7) / 8 * 8) <= max_tiles) R = (R / 2 + 7) / 8 * 8;
     return R;
-}
-
-// Quartets per CTA of k_lanczos_apply_d: 16, or 8 while 16 leaves under 8 CTAs
-// an SM (D = 16384, us per launch: 512 trajectories 176 with 8 or 16, 185 with
-// 32, 223 with 64).
-int quartet_tile_d(int Q, int width)
-{
-    return static_cast<long long>(Q) / 16 * (width / 32) >= 8 * 148 ? 16 : 8;
 }
 
 PairObs make_pair_obs(const msgpu_ctx *c)
@@ -785,7 +768,7 @@ int ensure_workspace(msgpu_ctx *c, int prec, int m)
         if ((rc = ensure(c, c->basis, n * m * sizeof(double2), "Krylov basis")) ||
             (rc = ensure(c, c->wbuf, n * sizeof(double2), "Krylov W")) ||
             (rc = ensure(c, c->zbuf, n * sizeof(double2), "Krylov Z")) ||
-            (rc = ensure(c, c->part, static_cast<size_t>(c->ntiles) * (m + 1) * ldm * sizeof(double2), "partials")) ||
+            (rc = ensure(c, c->part, partial_rows_d(c->ntiles, m) * ldm * sizeof(double), "partials")) ||
             (rc = ensure(c, c->part2, static_cast<size_t>(3) * (m + 1) * ldm * sizeof(double2), "dots")) ||
             (rc = ensure(c, c->hess, static_cast<size_t>(ldm) * m * m * sizeof(double2), "Hessenberg")))
             return rc;
@@ -2388,9 +2371,11 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                 const double *row = c->sched_steps ? sched_row(c, g, 1) : c->hcoef.data();
                 for (int k = 0; k < c->nterms; ++k) hn += std::abs(row[k]) * c->term_norm1[k];
             }
-            const int rc = for_groups(traj_groups(c), [&](int t0, int width, cudaStream_t gs) {
+            const int G = traj_groups(c), QT = quartet_tile_d(Q, ldm / G, partial_rows_d(nt, m)), nqt = ceil_div(Q, QT);
+            if (static_cast<size_t>(std::max(nqt, nt)) * ldm * sizeof(double) > c->part.bytes)
+                return fail(c, MSGPU_ERR_STATE, "run: the tiles' partial sums exceed their buffer");
+            const int rc = for_groups(G, [&](int t0, int width, cudaStream_t gs) {
                 const size_t tm0 = static_cast<size_t>(t0) * mws;  // offset into the [t][m] T arrays
-                const int QT = quartet_tile_d(Q, width), nqt = ceil_div(Q, QT);
                 for (int j = 0; j < m; ++j) {
                     const double *sj = sc + static_cast<size_t>(j) * ldm + t0;
                     {
