@@ -184,8 +184,11 @@ inline QuartetForm quartet_form(int D, int s1, int s2, const int *h_rowptr, cons
             else if (e2only) type = same(0, 10) && same(1, 11) && same(4, 14) && same(5, 15) ? 5 : 2;
             // blocks A (x) I with the same four values share them: a nucleus' flip
             // block takes two values over all quartets, so they stay in L1 (D =
-            // 16384, 1024 trajectories complex64: 101.6 to 99.2 ms for 20 steps)
-            if (type >= 4) {
+            // 16384, 1024 trajectories complex64: 101.6 to 99.2 ms for 20 steps).  With
+            // Hamiltonian terms the values here are those of one combination, which can
+            // agree where the terms differ, and every slot is written from its own CSR
+            // entry when the coefficients change: each block keeps its own.
+            if (type >= 4 && !want_src) {
                 std::array<double, 9> key;
                 key[8] = type;
                 for (int k = 0; k < 4; ++k) {

@@ -42,3 +42,40 @@ int main()
 
 def test_three_term_partial_sums_fit_their_buffer(tmp_path):
     assert _run(tmp_path, PARTIALS) == "ok 0"
+
+
+# Two electrons (strides 8 and 4) and nuclei a (stride 2) and b (stride 1), each flipped with a value
+# of its own on the first electron: v and w.  Prints the slots the two nuclei's blocks take.
+QUARTETS = r"""
+#include <stdio.h>
+#include "msgpu_quartet.h"
+using namespace msgpu;
+int main()
+{
+    std::vector<int> rowptr(1, 0), col;
+    std::vector<double> val;
+    for (int r = 0; r < 16; ++r) {  // flip-flops of the first electron (digit 8) with a nucleus (digit 2 or 1)
+        for (int n = 2; n >= 1; --n)
+            if (((r >> 3) & 1) != ((r & n) ? 1 : 0)) {
+                col.push_back(r ^ 8 ^ n);
+                val.push_back(0.5);
+                val.push_back(0.0);
+            }
+        rowptr.push_back(static_cast<int>(col.size()));
+    }
+    for (bool terms : {false, true}) {
+        const QuartetForm f = quartet_form(16, 8, 4, rowptr.data(), col.data(), val.data(), terms);
+        // a slot's CSR entries belong to one block: as many slots as blocks of terms
+        size_t own = 0;
+        for (size_t k = 0; k < f.blk.size(); ++k)
+            for (size_t l = 0; l < k; ++l) own += f.blk[k].y == f.blk[l].y;
+        printf("%zu blocks, %s, %zu sources; ", f.blk.size(), own ? "shared" : "apart", f.src.size());
+    }
+    return 0;
+}
+"""
+
+
+def test_blocks_of_hamiltonian_terms_keep_their_own_values(tmp_path):
+    # equal values in one combination of the terms say nothing about the others
+    assert _run(tmp_path, QUARTETS) == "8 blocks, shared, 0 sources; 8 blocks, apart, 32 sources;"
