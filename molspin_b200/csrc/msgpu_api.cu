@@ -1832,11 +1832,11 @@ int msgpu_upload_hamiltonian_terms(msgpu_ctx *c, int dim, const int *rowptr, con
     if (nnz < 0) return fail(c, MSGPU_ERR_INVALID, "Hamiltonian terms: malformed row pointer");
     for (size_t i = 0; i < 2 * static_cast<size_t>(nnz) * nterms; ++i)
         if (!std::isfinite(vals[i])) return fail(c, MSGPU_ERR_NONFINITE, "Hamiltonian terms: non-finite value");
-    // a generic combination (fixed irrational-looking weights) fixes the
-    // sparsity and block structure for every combination of the terms
+    // a generic combination (term_weight) fixes the sparsity and block structure
+    // for every combination of the terms
     std::vector<double> gen(2 * static_cast<size_t>(nnz), 0.0);
     for (int t = 0; t < nterms; ++t) {
-        const double w = 1.0 + 0.7548776662466927 * (t + 1) - std::floor(0.7548776662466927 * (t + 1));
+        const double w = term_weight(t);
         for (size_t i = 0; i < gen.size(); ++i) gen[i] += w * vals[static_cast<size_t>(t) * gen.size() + i];
     }
     if (int rc = msgpu_upload_hamiltonian_csr(c, dim, rowptr, col, gen.data())) return rc;

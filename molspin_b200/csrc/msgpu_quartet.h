@@ -12,6 +12,19 @@
 
 namespace msgpu {
 
+// Weight of Hamiltonian term t (0 to 15) in the combination that fixes the sparsity
+// and block structure for every combination of the terms: 1 + the fraction of the
+// square root of a prime.  Square roots of distinct primes are independent of one
+// another and of 1 over the rationals, so values that agree or cancel here agree or
+// cancel term by term.  (Multiples of one irrational number do not do: they are an
+// arithmetic progression, up to whole numbers.)
+inline double term_weight(int t)
+{
+    static const int primes[16] = {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53};
+    const double root = std::sqrt(static_cast<double>(primes[t]));
+    return 1.0 + root - std::floor(root);
+}
+
 struct QuartetForm {
     std::vector<int> rowptr;    // Q + 1
     std::vector<int2> blk;      // {neighbour base row << 3 | type, value offset in float4}

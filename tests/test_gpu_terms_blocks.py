@@ -4,6 +4,8 @@ Nucleus a has coupling J in terms 0 and 2, nucleus b has 2J in term 1: a combina
 w0 + w2 = 2 w1 gives both the same flip blocks, the coefficients (1, 1, 0) do not.  Every form is
 compared with a context that holds the combined H: 1e-12 relative per trajectory in complex128 (the
 combination differs in summation order only), 1e-7 in complex64 (the same H rounded the same way).
+The same for one nucleus whose flip blocks depend on the second electron in such terms: they are the
+same for both of its states in that combination alone.
 """
 import numpy as np
 import pytest
@@ -29,17 +31,33 @@ def _system(couplings, field=False):
 
 def _terms():
     rest = _system({2: 0.21, 3: -0.4, 4: 0.33, 5: 0.11}, field=True)
-    mats = []
-    for s in (_system({0: J}), _system({1: 2 * J}), _system({0: J}), rest):
-        r, c, v = s.hamiltonian_csr()
-        m = sp.csr_matrix((v, c, r), shape=(256, 256))
-        m.sum_duplicates()
-        mats.append(m)
+    return (rest, *_pattern([_matrix(s) for s in (_system({0: J}), _system({1: 2 * J}), _system({0: J}), rest)]))
+
+
+def _terms_second_electron():
+    rest = _system({2: 0.21, 3: -0.4, 4: 0.33, 5: 0.11}, field=True)
+    sx = sp.csr_matrix(np.array([[0.0, 0.5], [0.5, 0.0]]))
+
+    def flip(j, up):  # j S_x(E1) I_x(N0), for one state of the second electron
+        e2 = sp.csr_matrix(np.diag([1.0, 0.0] if up else [0.0, 1.0]))
+        return sp.kron(sp.kron(sp.kron(j * sx, e2), sx), sp.identity(32)).tocsr()
+
+    return (rest, *_pattern([flip(J, True), flip(2 * J, False), flip(J, True), _matrix(rest)]))
+
+
+def _matrix(s):
+    r, c, v = s.hamiltonian_csr()
+    m = sp.csr_matrix((v, c, r), shape=(256, 256))
+    m.sum_duplicates()
+    return m
+
+
+def _pattern(mats):
     pat = sum(abs(m) for m in mats).tocsr()
     pat.sort_indices()
     rows = np.repeat(np.arange(256), np.diff(pat.indptr))
-    vals = np.stack([np.asarray(m[rows, pat.indices]).ravel() for m in mats])
-    return rest, pat.indptr.astype(np.int32), pat.indices.astype(np.int32), vals
+    vals = np.stack([np.asarray(m[rows, pat.indices]).ravel() for m in mats]).astype(np.complex128)
+    return pat.indptr.astype(np.int32), pat.indices.astype(np.int32), vals
 
 
 def _run(p, s, F, precision, propagator):
@@ -51,11 +69,12 @@ def _run(p, s, F, precision, propagator):
     return p.yields()[0]
 
 
+@pytest.mark.parametrize("terms", [_terms, _terms_second_electron])
 @pytest.mark.parametrize("form,precision,propagator,tol", [
     ("resident", "c64", "krylov", 1e-7), ("streamed", "c64", "krylov", 1e-7), ("streamed", "c128", "krylov", 1e-12),
     ("auto", "c128", "taylor", 1e-12), ("auto", "c128", "rk4", 1e-12)])
-def test_coinciding_blocks_follow_their_own_terms(form, precision, propagator, tol):
-    s, r, c, vals = _terms()
+def test_coinciding_blocks_follow_their_own_terms(form, precision, propagator, tol, terms):
+    s, r, c, vals = terms()
     F = s.trace_samples(33, 2.0)
     with hs.HSPropagatorB200(0) as p:
         p.set_form(form)

@@ -79,3 +79,31 @@ int main()
 def test_blocks_of_hamiltonian_terms_keep_their_own_values(tmp_path):
     # equal values in one combination of the terms say nothing about the others
     assert _run(tmp_path, QUARTETS) == "8 blocks, shared, 0 sources; 8 blocks, apart, 32 sources;"
+
+
+WEIGHTS = r"""
+#include <stdio.h>
+#include <math.h>
+#include "msgpu_quartet.h"
+using namespace msgpu;
+int main()
+{
+    // whole-number relations a w_i + b w_j + c w_k + d w_l = 0, |a| .. |d| <= 2
+    double least = 1.0;
+    for (int i = 0; i < 16; ++i)
+        for (int j = i + 1; j < 16; ++j)
+            for (int k = j + 1; k < 16; ++k)
+                for (int l = k + 1; l < 16; ++l)
+                    for (int n = 1; n < 625; ++n) {
+                        const int a = n % 5 - 2, b = n / 5 % 5 - 2, c = n / 25 % 5 - 2, d = n / 125 - 2;
+                        if (!a && !b && !c && !d) continue;
+                        least = fmin(least, fabs(a * term_weight(i) + b * term_weight(j) + c * term_weight(k) +
+                                                 d * term_weight(l)));
+                    }
+    printf("%s", least > 1e-9 ? "ok" : "related");  // blocks are told apart at 1e-13 of their largest value
+}
+"""
+
+
+def test_weights_of_the_terms_are_unrelated(tmp_path):
+    assert _run(tmp_path, WEIGHTS) == "ok"
