@@ -16,7 +16,7 @@ INCLUDE = os.path.join(ROOT, "include")
 LIB = os.path.join(HERE, "libmsgpu.so")
 
 SOURCES = ["msgpu_api.cu", "msgpu_resident.cu", "msgpu_resident_q.cu", "msgpu_arnoldi.cu", "msgpu_batch.cu", "msgpu_dense.cu", "msgpu_host.cpp"]
-HEADERS = ["msgpu_device.cuh", "msgpu_kernels.cuh", "msgpu_resident.h", "msgpu_resident.cuh", "msgpu_resident_q.cuh", "msgpu_quartet.h", "msgpu_tiles.h", "msgpu_arnoldi.h", "msgpu_arnoldi.cuh", "msgpu_batch.cuh", "msgpu_dense.h", "msgpu_philox.h",
+HEADERS = ["msgpu_device.cuh", "msgpu_kernels.cuh", "msgpu_resident.h", "msgpu_resident.cuh", "msgpu_resident_q.cuh", "msgpu_quartet.h", "msgpu_tiles.h", "msgpu_csr.h", "msgpu_arnoldi.h", "msgpu_arnoldi.cuh", "msgpu_batch.cuh", "msgpu_dense.h", "msgpu_philox.h",
            "msgpu_fused.cuh", "msgpu_spmm_tc.cuh", "msgpu_spmm_tm.cuh"]
 
 NVCC_FLAGS = [

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "msgpu_arnoldi.h"
+#include "msgpu_csr.h"
 #include "msgpu_dense.h"
 #include "msgpu_fused.cuh"
 #include "msgpu_kernels.cuh"
@@ -476,6 +477,10 @@ int msgpu_upload_hamiltonian_csr(msgpu_ctx *c, int dim, const int *rowptr, const
             if (!std::isfinite(v)) return fail(c, MSGPU_ERR_NONFINITE, "Hamiltonian: non-finite value");
             hi[2 * k + p] = static_cast<float>(v);
         }
+    }
+    if (repeated_columns(dim, rowptr, col)) {
+        const MergedCsr one = merge_columns(dim, rowptr, col, val, 1);
+        return msgpu_upload_hamiltonian_csr(c, dim, one.rowptr.data(), one.col.data(), one.val.data());
     }
     if (c->D != 0 && c->D != dim) {
         // dimension change invalidates state and reaction operator
@@ -967,33 +972,6 @@ bool resident_fits(const msgpu_ctx *c, int prec, int m)
     if (prec == MSGPU_PREC_C64 && !c->k_scalar) return false;
     if (c->form == MSGPU_FORM_AUTO && c->D > kResidentMaxDim) return false;
     return resident_bytes(c->D, m, prec == MSGPU_PREC_C128 ? 16 : 8) <= kResidentSmemBudget;
-}
-
-// Whether H's entries (CSR, duplicates not merged) equal their transposes'
-// conjugates to rounding: then, with K = kappa I, the Arnoldi matrix is
-// tridiagonal and the three-term recurrence gives the same Krylov step.
-bool is_hermitian(int dim, const int *rowptr, const int *col, const double *val)
-{
-    // rows are visited in order, so a sorted row's transposes come up in order too
-    std::vector<int> next(rowptr, rowptr + dim);
-    for (int r = 0; r < dim; ++r)
-        for (int k = rowptr[r]; k < rowptr[r + 1]; ++k) {
-            const int c = col[k];
-            const double re = val[2 * static_cast<size_t>(k)], im = val[2 * static_cast<size_t>(k) + 1];
-            const double tol = 4.0e-16 * (std::abs(re) + std::abs(im));
-            auto conj_at = [&](int l) {
-                return col[l] == r && std::abs(val[2 * static_cast<size_t>(l)] - re) <= tol &&
-                       std::abs(val[2 * static_cast<size_t>(l) + 1] + im) <= tol;
-            };
-            if (next[c] < rowptr[c + 1] && conj_at(next[c])) {
-                ++next[c];
-                continue;
-            }
-            bool found = false;
-            for (int l = rowptr[c]; l < rowptr[c + 1] && !found; ++l) found = conj_at(l);
-            if (!found) return false;
-        }
-    return true;
 }
 
 // complex128 runs whose recurrence is left to the library (MSGPU_REC_AUTO)
@@ -1832,6 +1810,15 @@ int msgpu_upload_hamiltonian_terms(msgpu_ctx *c, int dim, const int *rowptr, con
     if (nnz < 0) return fail(c, MSGPU_ERR_INVALID, "Hamiltonian terms: malformed row pointer");
     for (size_t i = 0; i < 2 * static_cast<size_t>(nnz) * nterms; ++i)
         if (!std::isfinite(vals[i])) return fail(c, MSGPU_ERR_NONFINITE, "Hamiltonian terms: non-finite value");
+    // entries of a row at one column become one, as in every other upload; rows and
+    // columns that the upload below refuses are left to it
+    bool in_range = rowptr[0] == 0;
+    for (int r = 0; r < dim && in_range; ++r) in_range = rowptr[r + 1] >= rowptr[r];
+    for (int k = 0; k < nnz && in_range; ++k) in_range = col[k] >= 0 && col[k] < dim;
+    if (in_range && repeated_columns(dim, rowptr, col)) {
+        const MergedCsr one = merge_columns(dim, rowptr, col, vals, nterms);
+        return msgpu_upload_hamiltonian_terms(c, dim, one.rowptr.data(), one.col.data(), nterms, one.val.data(), coef);
+    }
     // a generic combination (term_weight) fixes the sparsity and block structure
     // for every combination of the terms
     std::vector<double> gen(2 * static_cast<size_t>(nnz), 0.0);
