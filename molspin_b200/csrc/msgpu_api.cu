@@ -1051,6 +1051,7 @@ int build_quartet(msgpu_ctx *c)
 {
     if (c->q_D == c->D && c->q_s1 == c->s1 && c->q_s2 == c->s2) return MSGPU_OK;
     const int D = c->D, s1 = c->s1, s2 = c->s2, Q = D / 4;
+    c->q_D = 0;  // not valid until every array below holds it (a caller may carry on without the form)
     QuartetForm f = quartet_form(D, s1, s2, c->h_rowptr.data(), c->h_col.data(), c->h_val.data(), c->terms);
     std::vector<int> &rowptr = f.rowptr, &base = f.base, &src = f.src;
     std::vector<int2> &blks = f.blk;
@@ -1073,9 +1074,6 @@ int build_quartet(msgpu_ctx *c)
         (e = cudaMemcpyAsync(c->qbase.p, base.data(), sizeof(int) * Q, cudaMemcpyHostToDevice, c->stream)) ||
         (e = cudaStreamSynchronize(c->stream)))
         return cuda_fail(c, e, "quartet upload");
-    c->q_D = D;
-    c->q_s1 = s1;
-    c->q_s2 = s2;
     c->q_nblocks = nb;
     if (resident_q_takes(D)) c->q_slots = quartet_slots(f, s1, s2);
     ++c->q_build;
@@ -1093,6 +1091,9 @@ int build_quartet(msgpu_ctx *c)
             return cuda_fail(c, e, "quartet value map");
         if ((rc = refresh_quartet_values(c))) return rc;
     }
+    c->q_D = D;
+    c->q_s1 = s1;
+    c->q_s2 = s2;
     return MSGPU_OK;
 }
 
