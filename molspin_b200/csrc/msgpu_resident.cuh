@@ -642,10 +642,16 @@ __device__ __forceinline__ void resident_propagate(const ResidentSystem &S, int 
         }
     }
     TS *out = static_cast<TS *>(S.psi_out) + static_cast<size_t>(t) * S.ts;
+    // the observables skip the pairs of rows that none of them has a coefficient
+    // for: what is not finite there shows in the state, which stops evolving with it
+    const bool watched = steps > 0 && S.nobs > 0;
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
         const int r = tid + NT * i;
-        if (r < D) st2(out + static_cast<size_t>(r) * S.rs, ld2(x + r));
+        if (r >= D) continue;
+        const double2 z = ld2(x + r);
+        st2(out + static_cast<size_t>(r) * S.rs, z);
+        bad = bad || (watched && !(isfinite(z.x) && isfinite(z.y)));
     }
     if (own) {
         S.acc[ak] = acc;

@@ -404,7 +404,10 @@ __device__ __forceinline__ void resident_quartet_propagate(const ResidentSystem 
     TS *out = static_cast<TS *>(S.psi_out) + static_cast<size_t>(t) * S.ts;
     if (live)
 #pragma unroll
-        for (int a = 0; a < 4; ++a) st2(out + row[a], z[a]);
+        for (int a = 0; a < 4; ++a) {
+            st2(out + row[a], z[a]);
+            bad = bad || (steps > 0 && !(isfinite(z[a].x) && isfinite(z[a].y)));  // as resident_propagate
+        }
     if (own) {
         S.acc[ak] = acc;
         S.comp[ak] = comp;
