@@ -286,7 +286,7 @@ int msgpu_get_option(msgpu_ctx *ctx, int key, double *value);
  * (complex64 vectors, FP64 reductions and yield sums), Lanczos recurrence,
  * K = kappa I, Philox noise keyed by (seed, trajectory, step, half).
  * Systems of dimension below 2048 whose Krylov basis fits shared memory run
- * the resident kernels, one launch per system, all at once; the others below
+ * the resident kernels, one launch per kernel, all at once; the others below
  * 2048 share one persistent launch (replayed from a CUDA graph) in which
  * systems with dimension >= the team threshold get a whole CTA per trajectory,
  * smaller ones a warp.  msgpu_batch_tune picks that threshold and the

@@ -2,8 +2,8 @@
 // msgpu_batch_*): many radical-pair systems of uneven dimension and
 // trajectory count propagated together.  Systems below kStreamDim run the
 // resident kernels (msgpu_resident.cuh, msgpu_resident_q.cuh), a CTA per
-// trajectory with the Krylov basis in shared memory, one launch per system, all
-// launches at once on a few streams.  A system whose basis does not fit shared
+// trajectory with the Krylov basis in shared memory, one launch per kernel for all
+// its systems, all launches at once on a few streams.  A system whose basis does not fit shared
 // memory joins the persistent launch k_batch instead, replayed from a CUDA
 // graph, with the team threshold and the grid size picked by an autotuner.  A
 // large system is better served by the streamed single-system
@@ -70,7 +70,7 @@ struct msgpu_batch {
     // systems of the persistent route dropped by msgpu_batch_clear: their device
     // buffers serve the next msgpu_batch_add_system (no cudaMalloc / cudaFree per reuse)
     std::vector<BatchSystem> spare;
-    Buf sys_d, items_d, queue_d, status_d, scratch, times_d, backup;
+    Buf sys_d, items_d, queue_d, status_d, scratch, times_d, backup, many_d, first_d;
     int threshold = 512, ctas_per_sm = 2, tuned = 0;
     int sm_count = 0;
     cudaGraphExec_t graph = nullptr;
@@ -134,21 +134,51 @@ void drop_graph(msgpu_batch *b)
 
 double flip_prob(double st_rate, double h) { return -0.5 * std::expm1(-2.0 * (0.5 * st_rate) * h); }
 
-// One system's launch of a resident kernel (a CTA per trajectory).
-struct ResidentLaunch {
+// A system on the resident kernels (a CTA per trajectory).
+struct ResidentRun {
     ResidentSystem S;
-    ResidentShape shape;
+    ResidentManyShape shape;
     double cost;  // of one trajectory
 };
-constexpr size_t kResidentSmemMax = 227 * 1024;
+constexpr size_t kSmemMax = 227 * 1024;
+constexpr size_t kResidentSmemMax = kSmemMax - sizeof(ResidentSystem);  // beside the system's descriptor
 
-// Queues the resident launches, longest trajectories first, over the side
-// streams between two events on the batch's stream.
-int launch_resident(msgpu_batch *b, std::vector<ResidentLaunch> &runs)
+// Queues the resident kernels, one launch for all systems of a kernel (a launch a
+// system leaves a batch of small systems eight at a time: 500 systems of D = 64 with 8
+// trajectories, 50 steps: 41 against 3.9 ms, 64 of them with 16, 20 steps: 2.24 against
+// 0.47 ms), the longest trajectories first, over the side streams between two events on
+// the batch's stream.
+int launch_resident(msgpu_batch *b, std::vector<ResidentRun> &runs)
 {
     if (runs.empty()) return MSGPU_OK;
-    std::stable_sort(runs.begin(), runs.end(), [](const ResidentLaunch &x, const ResidentLaunch &y) { return x.cost > y.cost; });
-    const int ns = std::min<int>(8, static_cast<int>(runs.size()));
+    std::stable_sort(runs.begin(), runs.end(), [](const ResidentRun &x, const ResidentRun &y) { return x.cost > y.cost; });
+    struct Launch {
+        ResidentManyShape shape;
+        std::vector<int> runs;
+    };
+    std::vector<Launch> launches;  // by their longest trajectory
+    for (size_t i = 0; i < runs.size(); ++i) {
+        size_t k = 0;
+        while (k < launches.size() && launches[k].shape.fn != runs[i].shape.fn) ++k;
+        if (k == launches.size()) launches.push_back(Launch{runs[i].shape, {}});
+        launches[k].shape.smem = std::max(launches[k].shape.smem, runs[i].shape.smem);
+        launches[k].runs.push_back(static_cast<int>(i));
+    }
+    // every launch's systems, then every launch's first CTAs (one more than systems)
+    std::vector<ResidentSystem> sys;
+    std::vector<int> first;
+    for (const Launch &l : launches) {
+        first.push_back(0);
+        for (int i : l.runs) {
+            sys.push_back(runs[i].S);
+            first.push_back(first.back() + runs[i].S.M);
+        }
+    }
+    int rc;
+    if ((rc = upload(b, b->many_d, sys.data(), sizeof(ResidentSystem) * sys.size(), "resident systems")) ||
+        (rc = upload(b, b->first_d, first.data(), sizeof(int) * first.size(), "resident work")))
+        return rc;
+    const int ns = std::min<int>(8, static_cast<int>(launches.size()));
     cudaError_t e = cudaSuccess;
     if (!b->fork) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
     for (int k = 0; k < ns && !e; ++k)
@@ -156,12 +186,24 @@ int launch_resident(msgpu_batch *b, std::vector<ResidentLaunch> &runs)
             e = cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming);
     if (!e) e = cudaEventRecord(b->fork, b->stream);
     for (int k = 0; k < ns && !e; ++k) e = cudaStreamWaitEvent(b->side[k], b->fork, 0);
-    for (size_t i = 0; i < runs.size() && !e; ++i) {
-        const ResidentLaunch &r = runs[i];
-        if ((e = raise_smem_limit(reinterpret_cast<const void *>(r.shape.fn), static_cast<int>(r.shape.smem)))) break;
-        r.shape.fn<<<r.S.M, 32 * r.shape.warps, r.shape.smem, b->side[i % ns]>>>(r.S, static_cast<int *>(b->status_d.p));
+    int *status = static_cast<int *>(b->status_d.p);
+    size_t at_sys = 0, at = 0;  // in sys and first
+    for (size_t i = 0; i < launches.size() && !e; ++i) {
+        const ResidentManyShape &r = launches[i].shape;
+        const int n = static_cast<int>(launches[i].runs.size()), smem = static_cast<int>(r.smem);
+        const bool one = n == 1 && r.one;
+        if ((e = raise_smem_limit(one ? reinterpret_cast<const void *>(r.one) : reinterpret_cast<const void *>(r.fn), smem)))
+            break;
+        if (one)
+            r.one<<<first[at + 1], 32 * r.warps, smem, b->side[i % ns]>>>(sys[at_sys], status);
+        else
+            r.fn<<<first[at + n], 32 * r.warps, smem, b->side[i % ns]>>>(
+                static_cast<const ResidentSystem *>(b->many_d.p) + at_sys, static_cast<const int *>(b->first_d.p) + at, n,
+                status);
         ++b->launches;
         e = cudaGetLastError();
+        at_sys += n;
+        at += n + 1;
     }
     for (int k = 0; k < ns && b->join[k]; ++k) {  // joined even after an error: nothing is left running behind it
         const cudaError_t je = cudaEventRecord(b->join[k], b->side[k]);
@@ -187,7 +229,7 @@ int upload_csr(msgpu_batch *b, BatchSystem &s, const int *rowptr, const int *col
 // launches; returns the grid size through *grid.
 int prepare(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_offset, int threshold,
             int ctas_per_sm, int *grid, size_t *slice, size_t *smem, int *nlarge, int *nitems,
-            std::vector<ResidentLaunch> *resident)
+            std::vector<ResidentRun> *resident)
 {
     std::vector<ResidentSystem> desc(b->sys.size());
     std::vector<ResidentWork> large, small;
@@ -227,7 +269,7 @@ int prepare(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_of
         desc[i] = S;
         if (s.ctx) continue;  // streamed path: no work items here
         if (s.kind) {
-            ResidentShape shape = s.kind == 1 ? resident_shape_c64_state(s.D, S.m) : resident_shape_q_state(s.D, S.m);
+            const ResidentManyShape shape = s.kind == 1 ? resident_shape_many(s.D, S.m) : resident_shape_q_many(s.D, S.m);
             if (shape.fn && shape.smem <= kResidentSmemMax) {
                 if (s.kind == 1) {
                     const size_t slots = static_cast<size_t>(s.D) * s.kmax;
@@ -239,7 +281,7 @@ int prepare(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_of
                 } else {
                     S.rq = s.rq;
                 }
-                resident->push_back(ResidentLaunch{S, shape, static_cast<double>(s.D) * S.m});
+                resident->push_back(ResidentRun{S, shape, static_cast<double>(s.D) * S.m});
                 continue;
             }
         }
@@ -274,7 +316,7 @@ int prepare(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_of
     *grid = std::max(1, b->sm_count * ctas_per_sm);
     *smem = sizeof(double2) * kBatchWarps * batch_expm_words(m);
     // the Krylov dimensions that the persistent launch takes, on every route
-    if ((!items.empty() || !resident->empty()) && *smem > kResidentSmemMax)
+    if ((!items.empty() || !resident->empty()) && *smem > kSmemMax)
         return bfail(b, MSGPU_ERR_CUDA, std::string("batch: shared memory: ") + cudaGetErrorString(cudaErrorInvalidValue));
     int rc;
     if ((rc = bensure(b, b->status_d, sizeof(int), "status"))) return rc;
@@ -402,7 +444,7 @@ int run_once(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_o
 {
     int grid, nlarge, nitems;
     size_t slice, smem;
-    std::vector<ResidentLaunch> resident;
+    std::vector<ResidentRun> resident;
     if (int rc = prepare(b, ntimes, m, accumulate, step_offset, threshold, cps, &grid, &slice, &smem, &nlarge, &nitems,
                          &resident))
         return rc;
@@ -501,7 +543,7 @@ void msgpu_batch_destroy(msgpu_batch *b)
             for (Buf *x : all) brelease(b, *x);
             if (s.ctx) msgpu_destroy(s.ctx);
         }
-    Buf *all[] = {&b->sys_d, &b->items_d, &b->queue_d, &b->status_d, &b->scratch, &b->times_d, &b->backup};
+    Buf *all[] = {&b->sys_d, &b->items_d, &b->queue_d, &b->status_d, &b->scratch, &b->times_d, &b->backup, &b->many_d, &b->first_d};
     for (Buf *x : all) brelease(b, *x);
     for (int k = 0; k < 8; ++k) {
         if (b->join[k]) cudaEventDestroy(b->join[k]);
@@ -670,8 +712,8 @@ int msgpu_batch_tune(msgpu_batch *b, const double *times, int ntimes, int krylov
     bool persistent = false;  // any system on the persistent launch, which these parameters shape
     for (auto &s : b->sys) {
         const int m = std::min(krylov_dim, s.D);
-        persistent = persistent || (!s.ctx && !(s.kind && (s.kind == 1 ? resident_shape_c64_state(s.D, m).smem
-                                                                       : resident_shape_q_state(s.D, m).smem) <= kResidentSmemMax));
+        persistent = persistent || (!s.ctx && !(s.kind && (s.kind == 1 ? resident_shape_many(s.D, m).smem
+                                                                       : resident_shape_q_many(s.D, m).smem) <= kResidentSmemMax));
     }
     for (int th : thresholds)
         for (int c : cps) {

@@ -34,12 +34,14 @@ ResidentShape resident_shape_c128(int D, int m, bool lanczos)
 
 ResidentShape resident_shape_c64(int D, int m) { return resident_shape<float2, true>(D, m); }
 
-ResidentShape resident_shape_c64_state(int D, int m)
+ResidentManyShape resident_shape_many(int D, int m)
 {
-    auto make = [&](ResidentFn fn, int w) { return ResidentShape{fn, w, resident_carve<float2, true>(nullptr, D, m, w).bytes}; };
-    if (D <= 32) return make(&k_resident<float2, 1, 1, true, float2>, 1);
-    if (D <= 64) return make(&k_resident<float2, 2, 1, true, float2>, 2);
-    if (D <= 128) return make(&k_resident<float2, 4, 1, true, float2>, 4);
+    auto make = [&](ResidentManyFn fn, int w) {
+        return ResidentManyShape{fn, nullptr, w, resident_carve<float2, true>(nullptr, D, m, w).bytes};
+    };
+    if (D <= 32) return make(&k_resident_many<1>, 1);
+    if (D <= 64) return make(&k_resident_many<2>, 2);
+    if (D <= 128) return make(&k_resident_many<4>, 4);
     return make(nullptr, 0);
 }
 

@@ -669,12 +669,46 @@ template <typename T>
 constexpr int resident_min_ctas(int W) { return sizeof(T) == sizeof(float2) && W <= 16 ? 16 / W : 1; }
 
 // One launch = the whole time loop of every trajectory (one CTA each).
-template <typename T, int W, int RPT, bool kLanczos, typename TS = double2>
+template <typename T, int W, int RPT, bool kLanczos>
 __global__ void __launch_bounds__(32 * W, resident_min_ctas<T>(W))
 k_resident(const __grid_constant__ ResidentSystem S, int *__restrict__ status)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    resident_propagate<T, TS, W, RPT, kLanczos>(S, blockIdx.x, smem_raw, status);
+    resident_propagate<T, double2, W, RPT, kLanczos>(S, blockIdx.x, smem_raw, status);
+}
+
+// The system that CTA b belongs to: first[i] <= b < first[i + 1].
+__device__ __forceinline__ int system_of(const int *__restrict__ first, int nsystems, int b)
+{
+    int lo = 0, hi = nsystems;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) / 2;
+        if (__ldg(first + mid) <= b) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// Copies a system's descriptor to shared memory, where it costs no registers.
+__device__ __forceinline__ void load_system(ResidentSystem *to, const ResidentSystem *from)
+{
+    static_assert(sizeof(ResidentSystem) % 8 == 0, "copied by 8 bytes");
+    for (unsigned k = threadIdx.x; k < sizeof(ResidentSystem) / 8; k += blockDim.x)
+        reinterpret_cast<unsigned long long *>(to)[k] = __ldg(reinterpret_cast<const unsigned long long *>(from) + k);
+    __syncthreads();
+}
+
+// The same for the trajectories of many systems (the batching form).
+template <int W>
+__global__ void __launch_bounds__(32 * W, resident_min_ctas<float2>(W))
+k_resident_many(const ResidentSystem *__restrict__ systems, const int *__restrict__ first, int nsystems,
+                int *__restrict__ status)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ ResidentSystem S;
+    const int i = system_of(first, nsystems, blockIdx.x);
+    load_system(&S, systems + i);
+    resident_propagate<float2, float2, W, 1, true>(S, blockIdx.x - __ldg(first + i), smem_raw, status);
 }
 
 }  // namespace

@@ -100,19 +100,33 @@ struct ResidentShape {
     size_t smem;     // dynamic shared memory
 };
 
+// Trajectories of many systems in one launch (the batching form; complex64 on a
+// complex64 state): system i's are the CTAs from first[i] to first[i + 1].  A
+// launch for a single system takes `one` where it is there: with the descriptor in
+// shared memory a quartet step at D = 1024 takes 2 % longer than with it in the
+// kernel's arguments (512 trajectories, 10 steps 1.23 against 1.20 ms), a row step
+// at D = 64 5 % less (0.163 against 0.173 ms).
+using ResidentManyFn = void (*)(const ResidentSystem *systems, const int *first, int nsystems, int *status);
+struct ResidentManyShape {
+    ResidentManyFn fn;
+    ResidentFn one;
+    int warps;
+    size_t smem;
+};
+
 // Kernel and launch shape for dimension D and Krylov dimension m:
 // complex128 (three-term recurrence or Arnoldi), complex64 (three-term).
 ResidentShape resident_shape_c128(int D, int m, bool lanczos);
 ResidentShape resident_shape_c64(int D, int m);
-// complex64 on a complex64 state (the batching form); fn null when no shape takes it.
-ResidentShape resident_shape_c64_state(int D, int m);
+// The batching form's; fn null when no shape takes it.
+ResidentManyShape resident_shape_many(int D, int m);
 // complex64 over quartets (msgpu_resident_q.cu): dimensions it takes, its shape,
 // the device bytes of a system's ResidentQuartets and their set-up in buf from
 // the quartet form's arrays.
 struct QuartetSlots;
 bool resident_q_takes(int D);
 ResidentShape resident_shape_q(int D, int m);
-ResidentShape resident_shape_q_state(int D, int m);  // on a complex64 state
+ResidentManyShape resident_shape_q_many(int D, int m);
 size_t resident_q_bytes(int Q, const QuartetSlots &slots);
 ResidentQuartets resident_q_build(void *buf, int Q, int s1, int s2, const QuartetSlots &slots, const int *rowptr,
                                   const int2 *blk, const float4 *val, const int *base, cudaStream_t st);

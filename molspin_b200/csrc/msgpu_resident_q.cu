@@ -2,15 +2,32 @@
 
 #include "msgpu_resident_q.cuh"
 
+#include <type_traits>
+
 namespace msgpu {
 namespace {
 
+constexpr int quartet_min_ctas(int W) { return W <= 3 ? 8 / W : W <= 6 ? 2 : 1; }
+
 template <int W, typename TS>
-__global__ void __launch_bounds__(32 * W, W <= 3 ? 8 / W : W <= 6 ? 2 : 1)
+__global__ void __launch_bounds__(32 * W, quartet_min_ctas(W))
 k_resident_q(const __grid_constant__ ResidentSystem S, int *__restrict__ status)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     resident_quartet_propagate<TS, W>(S, blockIdx.x, smem_raw, status);
+}
+
+// The trajectories of many systems, as k_resident_many.
+template <int W>
+__global__ void __launch_bounds__(32 * W, quartet_min_ctas(W))
+k_resident_q_many(const ResidentSystem *__restrict__ systems, const int *__restrict__ first, int nsystems,
+                  int *__restrict__ status)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ ResidentSystem S;
+    const int i = system_of(first, nsystems, blockIdx.x);
+    load_system(&S, systems + i);
+    resident_quartet_propagate<float2, W>(S, blockIdx.x - __ldg(first + i), smem_raw, status);
 }
 
 }  // namespace
@@ -21,24 +38,38 @@ bool resident_q_takes(int D) { return D > 128 && D <= 1536; }
 
 namespace {
 
-template <typename TS>
-ResidentShape shape_q(int D, int m)
+// Warps a CTA: a thread per quartet.
+template <typename Make>
+auto shape_q(int D, int m, Make make_for)
 {
     const int Q = D / 4;
-    auto make = [&](auto fn, int w) { return ResidentShape{fn, w, quartet_carve(nullptr, Q, m, w).bytes}; };
-    if (Q <= 64) return make(&k_resident_q<2, TS>, 2);
-    if (Q <= 96) return make(&k_resident_q<3, TS>, 3);
-    if (Q <= 128) return make(&k_resident_q<4, TS>, 4);
-    if (Q <= 160) return make(&k_resident_q<5, TS>, 5);
-    if (Q <= 192) return make(&k_resident_q<6, TS>, 6);
-    if (Q <= 256) return make(&k_resident_q<8, TS>, 8);
-    return make(&k_resident_q<12, TS>, 12);
+    auto make = [&](auto w) { return make_for(w, quartet_carve(nullptr, Q, m, decltype(w)::value).bytes); };
+    if (Q <= 64) return make(std::integral_constant<int, 2>{});
+    if (Q <= 96) return make(std::integral_constant<int, 3>{});
+    if (Q <= 128) return make(std::integral_constant<int, 4>{});
+    if (Q <= 160) return make(std::integral_constant<int, 5>{});
+    if (Q <= 192) return make(std::integral_constant<int, 6>{});
+    if (Q <= 256) return make(std::integral_constant<int, 8>{});
+    return make(std::integral_constant<int, 12>{});
 }
 
 }  // namespace
 
-ResidentShape resident_shape_q(int D, int m) { return shape_q<double2>(D, m); }
-ResidentShape resident_shape_q_state(int D, int m) { return shape_q<float2>(D, m); }
+ResidentShape resident_shape_q(int D, int m)
+{
+    return shape_q(D, m, [](auto w, size_t smem) {
+        constexpr int W = decltype(w)::value;
+        return ResidentShape{&k_resident_q<W, double2>, W, smem};
+    });
+}
+
+ResidentManyShape resident_shape_q_many(int D, int m)
+{
+    return shape_q(D, m, [](auto w, size_t smem) {
+        constexpr int W = decltype(w)::value;
+        return ResidentManyShape{&k_resident_q_many<W>, &k_resident_q<W, float2>, W, smem};
+    });
+}
 
 size_t resident_q_bytes(int Q, const QuartetSlots &slots)
 {
