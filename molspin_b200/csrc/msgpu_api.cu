@@ -1075,7 +1075,7 @@ int build_quartet(msgpu_ctx *c)
         (e = cudaStreamSynchronize(c->stream)))
         return cuda_fail(c, e, "quartet upload");
     c->q_nblocks = nb;
-    if (resident_q_takes(D)) c->q_slots = quartet_slots(f, s1, s2);
+    if (resident_q_takes(D)) c->q_slots = quartet_slots(f);
     ++c->q_build;
     c->q_hrow = std::move(rowptr);
     c->q_hblk = std::move(blks);

@@ -400,7 +400,7 @@ void build_quartets(msgpu_batch *b, BatchSystem &s, const int *rowptr, const int
 {
     const int Q = s.D / 4;
     const QuartetForm f = quartet_form(s.D, s.s1, s.s2, rowptr, col, val, false);
-    const QuartetSlots slots = quartet_slots(f, s.s1, s.s2);
+    const QuartetSlots slots = quartet_slots(f);
     // one buffer: values (16-byte aligned), the resident arrays, blocks, row pointers, bases
     auto up = [](size_t n) { return (n + 15) / 16 * 16; };
     const size_t nval = up(f.val.size() * sizeof(float)), nrq = up(resident_q_bytes(Q, slots));
