@@ -55,9 +55,10 @@ struct msgpu_ctx {
     int D = 0, nnz = 0;
     DevBuf hrow, hcol, hval, hhi;
     int max_row = 0;   // most entries of a row of H
-    double h_norm1 = 0.0;            // largest absolute row sum of H (of one term)
-    std::vector<double> term_norm1;  // the same of each term (msgpu_upload_hamiltonian_terms)
-    int hermitian = -1;  // H (every term of it) equals its conjugate transpose: 1, 0, or -1 (not yet checked)
+    // of H, or of each of its terms: looked at by the first run that asks (lanczos128)
+    int hermitian = -1;         // equal to the conjugate transpose: 1, 0, or -1 (not yet looked at)
+    std::vector<double> norm1;  // largest absolute row sums
+    DevBuf props;               // both, from k_h_properties
     DevBuf ell;        // resident form: H in padded column-major order, values then columns
     std::vector<int> h_rowptr, h_col;  // host copy for the quartet-block form
     std::vector<double> h_val;
@@ -291,19 +292,6 @@ int traj_groups(const msgpu_ctx *c)
     return 1;
 }
 
-// largest absolute row sum of a CSR matrix (interleaved complex values)
-double row_sum_norm(int dim, const int *rowptr, const double *val)
-{
-    double mx = 0.0;
-    for (int r = 0; r < dim; ++r) {
-        double s = 0.0;
-        for (int k = rowptr[r]; k < rowptr[r + 1]; ++k)
-            s += std::abs(val[2 * static_cast<size_t>(k)]) + std::abs(val[2 * static_cast<size_t>(k) + 1]);
-        mx = std::max(mx, s);
-    }
-    return mx;
-}
-
 // Rows per CTA of the complex64 update: halved from R while the launch has
 // fewer than 3 CTAs an SM (ctiles: trajectory tiles), up to the partials'
 // capacity.  D = 9216, 250 trajectories: 256 CTAs 17.5 us, 512 14.2 us; at D =
@@ -361,7 +349,7 @@ void msgpu_destroy(msgpu_ctx *c)
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     collect_profile(c);
-    DevBuf *all[] = {&c->hrow, &c->hcol, &c->hval, &c->hhi, &c->ell, &c->rqbuf, &c->qrow, &c->qcolt, &c->qval, &c->qbase, &c->qval64,
+    DevBuf *all[] = {&c->hrow, &c->hcol, &c->hval, &c->hhi, &c->ell, &c->rqbuf, &c->props, &c->qrow, &c->qcolt, &c->qval, &c->qbase, &c->qval64,
                      &c->fblk, &c->fval, &c->frow, &c->fdsrc, &c->fdiag, &c->krow, &c->kcol, &c->kval, &c->bits,
                      &c->psi128, &c->basis, &c->wbuf, &c->zbuf, &c->ubuf, &c->part, &c->part2, &c->hess,
                      &c->tdiag, &c->toff, &c->coef, &c->mdim, &c->scale, &c->alpha, &c->beta0, &c->qpart_obs,
@@ -470,15 +458,19 @@ int msgpu_upload_hamiltonian_csr(msgpu_ctx *c, int dim, const int *rowptr, const
     for (int r = 0; r < dim; ++r)
         if (rowptr[r + 1] < rowptr[r]) return fail(c, MSGPU_ERR_INVALID, "Hamiltonian: row pointer not monotone");
     std::vector<float> hi(2 * static_cast<size_t>(nnz));
-    for (int k = 0; k < nnz; ++k) {
-        if (col[k] < 0 || col[k] >= dim) return fail(c, MSGPU_ERR_INVALID, "Hamiltonian: column index out of range");
-        for (int p = 0; p < 2; ++p) {
-            const double v = val[2 * k + p];
-            if (!std::isfinite(v)) return fail(c, MSGPU_ERR_NONFINITE, "Hamiltonian: non-finite value");
-            hi[2 * k + p] = static_cast<float>(v);
+    bool ascending = true;  // in every row
+    for (int r = 0; r < dim; ++r)
+        for (int k = rowptr[r], last = -1; k < rowptr[r + 1]; ++k) {
+            if (col[k] < 0 || col[k] >= dim) return fail(c, MSGPU_ERR_INVALID, "Hamiltonian: column index out of range");
+            ascending = ascending && col[k] > last;
+            last = col[k];
+            for (int p = 0; p < 2; ++p) {
+                const double v = val[2 * k + p];
+                if (!std::isfinite(v)) return fail(c, MSGPU_ERR_NONFINITE, "Hamiltonian: non-finite value");
+                hi[2 * k + p] = static_cast<float>(v);
+            }
         }
-    }
-    if (repeated_columns(dim, rowptr, col)) {
+    if (!ascending && repeated_columns(dim, rowptr, col)) {
         const MergedCsr one = merge_columns(dim, rowptr, col, val, 1);
         return msgpu_upload_hamiltonian_csr(c, dim, one.rowptr.data(), one.col.data(), one.val.data());
     }
@@ -509,7 +501,6 @@ int msgpu_upload_hamiltonian_csr(msgpu_ctx *c, int dim, const int *rowptr, const
     c->q_D = 0;  // quartet form must be rebuilt
     c->max_row = 0;
     for (int r = 0; r < dim; ++r) c->max_row = std::max(c->max_row, rowptr[r + 1] - rowptr[r]);
-    c->h_norm1 = row_sum_norm(dim, rowptr, val);
     c->hermitian = -1;
     c->terms = false;
     c->dense.have_u = false;  // a cached dense propagator belongs to the old H
@@ -667,6 +658,45 @@ __global__ void k_combine_terms(const double2 *__restrict__ terms, int nterms, T
     if (!isfinite(v.x) || !isfinite(v.y)) atomicOr(status, 2);
     val[k] = v;
     hi[k] = make_float2(static_cast<float>(v.x), static_cast<float>(v.y));
+}
+
+// Of n value arrays on one CSR pattern (one entry a column in each row): out[0]
+// counts entries that differ from their transpose's conjugate by more than
+// rounding, or have none; out[1 + t] is array t's largest absolute row sum (a
+// double's bits, which order as the values do).  A warp a row.  On the host every
+// upload of four terms of D = 16384 took 6 ms longer (16.3 against 9.8 ms).
+__global__ void __launch_bounds__(256)
+k_h_properties(const int *__restrict__ rowptr, const int *__restrict__ col, const double2 *__restrict__ val, int n,
+               size_t nnz, int D, unsigned long long *__restrict__ out)
+{
+    const int lane = threadIdx.x & 31, r = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (r >= D) return;
+    const int b = rowptr[r], e = rowptr[r + 1];
+    for (int t = 0; t < n; ++t) {
+        double s = 0.0;
+        for (int k = b + lane; k < e; k += 32) {
+            const double2 v = val[t * nnz + k];
+            s += fabs(v.x) + fabs(v.y);
+        }
+        s = warp_sum(s);
+        if (lane == 0) atomicMax(out + 1 + t, static_cast<unsigned long long>(__double_as_longlong(s)));
+    }
+    bool bad = false;
+    for (int k = b + lane; k < e; k += 32) {
+        const int c = col[k], ce = rowptr[c + 1];
+        int l = rowptr[c];
+        while (l < ce && col[l] != r) ++l;
+        if (l == ce) {
+            bad = true;
+            continue;
+        }
+        for (int t = 0; t < n; ++t) {
+            const double2 v = val[t * nnz + k], w = val[t * nnz + l];
+            const double tol = 4.0e-16 * (fabs(v.x) + fabs(v.y));
+            bad = bad || fabs(w.x - v.x) > tol || fabs(w.y + v.y) > tol;
+        }
+    }
+    if (bad) atomicAdd(out, 1ull);
 }
 
 // The resident form's copy of H: entry k of row r at r + k * D (values in the
@@ -974,12 +1004,46 @@ bool resident_fits(const msgpu_ctx *c, int prec, int m)
     return resident_bytes(c->D, m, prec == MSGPU_PREC_C128 ? 16 : 8) <= kResidentSmemBudget;
 }
 
+// Fills c->hermitian and c->norm1: on the host for a small H, which takes less than
+// a launch and its answer (20 us; 4096 entries), else from the H (its terms) on the
+// device.  Without room for the few numbers there it counts as not Hermitian, which
+// is always right.
+void look_at_hamiltonian(msgpu_ctx *c)
+{
+    if (!c->terms && c->nnz <= 4096) {
+        c->hermitian = is_hermitian(c->D, c->h_rowptr.data(), c->h_col.data(), c->h_val.data());
+        c->norm1.assign(1, row_sum_norm(c->D, c->h_rowptr.data(), c->h_val.data()));
+        return;
+    }
+    const int n = c->terms ? c->nterms : 1;
+    std::vector<unsigned long long> out(n + 1, 0);
+    const size_t bytes = out.size() * sizeof(out[0]);
+    c->hermitian = 0;
+    if (ensure(c, c->props, 17 * sizeof(out[0]), "Hamiltonian properties") != MSGPU_OK) {
+        (void)cudaGetLastError();
+        c->err.clear();
+        return;
+    }
+    auto *d = static_cast<unsigned long long *>(c->props.p);
+    if (cudaMemsetAsync(d, 0, bytes, c->stream)) return;
+    ++c->launches;
+    k_h_properties<<<ceil_div(c->D, 8), 256, 0, c->stream>>>(
+        static_cast<const int *>(c->hrow.p), static_cast<const int *>(c->hcol.p),
+        static_cast<const double2 *>(c->terms ? c->hterms.p : c->hval.p), n, c->nnz, c->D, d);
+    if (cudaGetLastError() || cudaMemcpyAsync(out.data(), d, bytes, cudaMemcpyDeviceToHost, c->stream) ||
+        cudaStreamSynchronize(c->stream))
+        return;
+    c->norm1.resize(n);
+    std::memcpy(c->norm1.data(), out.data() + 1, n * sizeof(double));
+    c->hermitian = out[0] == 0;
+}
+
 // complex128 runs whose recurrence is left to the library (MSGPU_REC_AUTO)
 // take the three-term recurrence when H is Hermitian and K = kappa I.
 bool lanczos128(msgpu_ctx *c, const msgpu_run_params *p)
 {
     if (p->precision != MSGPU_PREC_C128 || p->recurrence != MSGPU_REC_AUTO || !c->k_scalar) return false;
-    if (c->hermitian < 0) c->hermitian = is_hermitian(c->D, c->h_rowptr.data(), c->h_col.data(), c->h_val.data());
+    if (c->hermitian < 0) look_at_hamiltonian(c);
     return c->hermitian == 1;
 }
 
@@ -1813,7 +1877,7 @@ int msgpu_upload_hamiltonian_terms(msgpu_ctx *c, int dim, const int *rowptr, con
         if (!std::isfinite(vals[i])) return fail(c, MSGPU_ERR_NONFINITE, "Hamiltonian terms: non-finite value");
     // entries of a row at one column become one, as in every other upload; rows and
     // columns that the upload below refuses are left to it
-    bool in_range = rowptr[0] == 0;
+    bool in_range = rowptr[0] == 0 && col != nullptr;
     for (int r = 0; r < dim && in_range; ++r) in_range = rowptr[r + 1] >= rowptr[r];
     for (int k = 0; k < nnz && in_range; ++k) in_range = col[k] >= 0 && col[k] < dim;
     if (in_range && repeated_columns(dim, rowptr, col)) {
@@ -1838,12 +1902,6 @@ int msgpu_upload_hamiltonian_terms(msgpu_ctx *c, int dim, const int *rowptr, con
         return cuda_fail(c, e, "Hamiltonian terms upload");
     c->terms = true;
     c->nterms = nterms;
-    c->term_norm1.clear();
-    for (int t = 0; t < nterms; ++t)
-        c->term_norm1.push_back(row_sum_norm(dim, rowptr, vals + 2 * static_cast<size_t>(t) * nnz));
-    c->hermitian = 1;
-    for (int t = 0; t < nterms && c->hermitian == 1; ++t)
-        c->hermitian = is_hermitian(dim, rowptr, col, vals + 2 * static_cast<size_t>(t) * nnz);
     return msgpu_set_hamiltonian_coefficients(c, coef);
 }
 
@@ -2353,11 +2411,11 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                               static_cast<const double2 *>(c->qval64.p), static_cast<const int *>(c->qbase.p)};
             // dt |T| is below dt |H|: past 128 the squarings of the Pade form take
             // fewer steps than the sub-steps of the Taylor series
-            double hn = c->h_norm1;
+            double hn = c->norm1[0];
             if (c->terms) {
                 hn = 0.0;
                 const double *row = c->sched_steps ? sched_row(c, g, 1) : c->hcoef.data();
-                for (int k = 0; k < c->nterms; ++k) hn += std::abs(row[k]) * c->term_norm1[k];
+                for (int k = 0; k < c->nterms; ++k) hn += std::abs(row[k]) * c->norm1[k];
             }
             const int G = traj_groups(c), QT = quartet_tile_d(Q, ldm / G, partial_rows_d(nt, m)), nqt = ceil_div(Q, QT);
             if (static_cast<size_t>(std::max(nqt, nt)) * ldm * sizeof(double) > c->part.bytes)

@@ -4,6 +4,7 @@
 
 #include <stddef.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -81,6 +82,19 @@ inline bool is_hermitian(int dim, const int *rowptr, const int *col, const doubl
             if (!found) return false;
         }
     return true;
+}
+
+// Largest absolute row sum.
+inline double row_sum_norm(int dim, const int *rowptr, const double *val)
+{
+    double mx = 0.0;
+    for (int r = 0; r < dim; ++r) {
+        double s = 0.0;
+        for (int k = rowptr[r]; k < rowptr[r + 1]; ++k)
+            s += std::abs(val[2 * static_cast<size_t>(k)]) + std::abs(val[2 * static_cast<size_t>(k) + 1]);
+        mx = std::max(mx, s);
+    }
+    return mx;
 }
 
 }  // namespace msgpu
