@@ -69,6 +69,7 @@ struct msgpu_ctx {
     msgpu::QuartetSlots q_slots;      // slots of the resident quartet form
     DevBuf rqbuf;                     // ResidentQuartets of the resident form
     long long q_build = 0;            // counts quartet-form builds
+    double q_saving = 0.0;            // us that the form would have saved Taylor and RK4 runs on this H so far
     std::vector<int> q_hrow;          // host copies of the quartet form
     std::vector<int2> q_hblk;
     std::vector<float> q_hval;
@@ -499,6 +500,7 @@ int msgpu_upload_hamiltonian_csr(msgpu_ctx *c, int dim, const int *rowptr, const
     c->h_col.assign(col, col + nnz);
     c->h_val.assign(val, val + 2 * static_cast<size_t>(nnz));
     c->q_D = 0;  // quartet form must be rebuilt
+    c->q_saving = 0.0;
     c->max_row = 0;
     for (int r = 0; r < dim; ++r) c->max_row = std::max(c->max_row, rowptr[r + 1] - rowptr[r]);
     c->hermitian = -1;
@@ -1111,9 +1113,11 @@ int refresh_quartet_values(msgpu_ctx *c)
     return c->tc_build == c->q_build ? tc_tables(c) : MSGPU_OK;
 }
 
+bool quartet_ready(const msgpu_ctx *c) { return c->q_D == c->D && c->q_s1 == c->s1 && c->q_s2 == c->s2; }
+
 int build_quartet(msgpu_ctx *c)
 {
-    if (c->q_D == c->D && c->q_s1 == c->s1 && c->q_s2 == c->s2) return MSGPU_OK;
+    if (quartet_ready(c)) return MSGPU_OK;
     const int D = c->D, s1 = c->s1, s2 = c->s2, Q = D / 4;
     c->q_D = 0;  // not valid until every array below holds it (a caller may carry on without the form)
     QuartetForm f = quartet_form(D, s1, s2, c->h_rowptr.data(), c->h_col.data(), c->h_val.data(), c->terms);
@@ -2166,28 +2170,6 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
     const bool three_term = quartet128 && lanczos128(c, p);
     if (quartet128)
         if (int rc = build_quartet(c)) return rc;
-    // Taylor and RK4 with K on the electron pair run over quartet blocks (a
-    // budget without room for them keeps the CSR kernels)
-    PairGenerator pg{};
-    bool quartet_gen = false;
-    if (taylor || rk4) {
-        quartet_gen = c->k_scalar || pair_reaction(c, &pg.K, 0.0);
-        pg.pair = !c->k_scalar;
-        if (quartet_gen && build_quartet(c) != MSGPU_OK) {
-            (void)cudaGetLastError();
-            c->err.clear();
-            quartet_gen = false;
-        }
-        if (quartet_gen) {
-            pg.H = QuartetD{static_cast<const int *>(c->qrow.p), static_cast<const int2 *>(c->qcolt.p),
-                            static_cast<const double2 *>(c->qval64.p), static_cast<const int *>(c->qbase.p)};
-            pg.kappa = c->k_scalar ? c->kappa : 0.0;
-            pg.Q = Q;
-            pg.s1 = c->s1;
-            pg.s2 = c->s2;
-            pg.ldm = ldm;
-        }
-    }
     if (prec == MSGPU_PREC_C64) {
         if (int rc = build_quartet(c)) return rc;
         if (int rc = build_tc(c)) return rc;
@@ -2224,6 +2206,15 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
                 return cuda_fail(c, e, "Taylor statistics");
         }
     }
+    // statistics of a schedule row's H
+    auto schedule_stats = [&](const double *row, double *hs) {
+        hs[0] = hs[1] = hs[2] = 0.0;
+        for (int k = 0; k < c->nterms; ++k) {
+            hs[0] += row[k] * term_stats[3 * k];
+            hs[1] += row[k] * term_stats[3 * k + 1];
+            hs[2] += std::abs(row[k]) * term_stats[3 * k + 2];  // norm bound of the combination
+        }
+    };
     // shift and norm bound of G - mu I from the H statistics {tr.re, tr.im, max row sum}
     auto taylor_shift = [&](const double *hs) {
         const double2 ktr = c->k_scalar ? make_double2(c->kappa * D, 0.0) : c->k_trace;
@@ -2241,6 +2232,63 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
             return cuda_fail(c, e, "Taylor statistics");
         taylor_shift(hs);
         if (!std::isfinite(tnorm)) return fail(c, MSGPU_ERR_NONFINITE, "run: non-finite Hamiltonian norm");
+    }
+    // Sub-steps and degree of a Taylor step: theta^(mt+1)/(mt+1)! e^theta <= tol
+    // with theta = |dt| ||G - mu I||_1 / nsub <= 4
+    struct TaylorStep {
+        int nsub, mt;
+        double theta;
+    };
+    auto taylor_step = [&](double dt) {
+        TaylorStep ts;
+        ts.nsub = std::max(1, static_cast<int>(std::ceil(std::abs(dt) * tnorm / 4.0)));
+        ts.theta = std::abs(dt) * tnorm / ts.nsub;
+        ts.mt = 1;
+        for (double rem = ts.theta * ts.theta / 2.0; rem * std::exp(ts.theta) > c->taylor_tol && ts.mt < 55; ++ts.mt)
+            rem *= ts.theta / (ts.mt + 2);
+        return ts;
+    };
+    // Taylor and RK4 with K on the electron pair run over quartet blocks, once the
+    // products asked for on this H save more than the form's assembly costs (a call
+    // or two on a new H would otherwise take longer than over the CSR rows: RK4, one
+    // step, D = 16384: 5.1 against 0.28 ms).  A budget without room for them keeps
+    // the CSR kernels.
+    PairGenerator pg{};
+    bool quartet_gen = false;
+    if (taylor || rk4) {
+        quartet_gen = c->k_scalar || pair_reaction(c, &pg.K, 0.0);
+        pg.pair = !c->k_scalar;
+        if (quartet_gen && !quartet_ready(c)) {
+            // us a product saves (D = 256 to 16384, 1 to 256 trajectories: 2 to 64),
+            // and us of assembly and upload (0.06 ms at D = 256, 3.0 at D = 16384;
+            // with terms 5.3)
+            double products = 4.0 * steps;
+            if (taylor && steps > 0) {
+                if (c->sched_steps) {  // of the first step's H
+                    double hs[3];
+                    schedule_stats(sched_row(c, g0, 1), hs);
+                    taylor_shift(hs);
+                }
+                const TaylorStep ts = taylor_step(p->times[1] - p->times[0]);
+                products = std::min(1e9, static_cast<double>(ts.nsub) * ts.mt * steps);
+            }
+            c->q_saving += products * (2.0 + 5e-7 * c->nnz * ldm);
+            quartet_gen = c->q_saving >= 40.0 + (c->terms ? 12e-3 : 7e-3) * c->nnz;
+        }
+        if (quartet_gen && build_quartet(c) != MSGPU_OK) {
+            (void)cudaGetLastError();
+            c->err.clear();
+            quartet_gen = false;
+        }
+        if (quartet_gen) {
+            pg.H = QuartetD{static_cast<const int *>(c->qrow.p), static_cast<const int2 *>(c->qcolt.p),
+                            static_cast<const double2 *>(c->qval64.p), static_cast<const int *>(c->qbase.p)};
+            pg.kappa = c->k_scalar ? c->kappa : 0.0;
+            pg.Q = Q;
+            pg.s1 = c->s1;
+            pg.s2 = c->s2;
+            pg.ldm = ldm;
+        }
     }
     ArnoldiScratch arn{};
     if (arn64 || (prec == MSGPU_PREC_C128 && !taylor && !rk4 && !three_term)) {
@@ -2296,34 +2344,27 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
             const double *row = sched_row(c, g, 1);
             TermCoef cf;
             std::memset(&cf, 0, sizeof(cf));
-            double hs[3] = {0.0, 0.0, 0.0};
-            for (int k = 0; k < c->nterms; ++k) {
-                cf.c[k] = row[k];
-                if (taylor) {
-                    hs[0] += row[k] * term_stats[3 * k];
-                    hs[1] += row[k] * term_stats[3 * k + 1];
-                    hs[2] += std::abs(row[k]) * term_stats[3 * k + 2];  // norm bound of the combination
-                }
-            }
+            for (int k = 0; k < c->nterms; ++k) cf.c[k] = row[k];
             k_combine_terms<<<ceil_div(std::max(1, c->nnz), 256), 256, 0, st>>>(
                 static_cast<const double2 *>(c->hterms.p), c->nterms, cf, c->nnz, static_cast<double2 *>(c->hval.p),
                 static_cast<float2 *>(c->hhi.p), static_cast<int *>(c->status.p));
             if (prec == MSGPU_PREC_C64 || quartet128 || quartet_gen)
                 if (int rc = refresh_quartet_values(c)) return rc;
-            if (taylor) taylor_shift(hs);
+            if (taylor) {
+                double hs[3];
+                schedule_stats(row, hs);
+                taylor_shift(hs);
+            }
         }
         if ((e = cudaMemsetAsync(c->mdim.p, 0, ldm * sizeof(int), st))) return cuda_fail(c, e, "mdim reset");
         if (taylor) {
-            // exp(dt (G - mu I)) by s sub-steps of a degree-mt Taylor series
-            // (theta^(mt+1)/(mt+1)! e^theta <= tol with theta = |dt| ||G - mu I||_1 / s <= 4),
-            // each ending with F <- e^{dt mu / s} F (SpinSpace::HighamProp's loop)
+            // exp(dt (G - mu I)) by nsub sub-steps of a degree-mt Taylor series, each
+            // ending with F <- e^{dt mu / nsub} F (SpinSpace::HighamProp's loop)
             double2 *F = static_cast<double2 *>(c->psi128.p);
             double2 *cur = static_cast<double2 *>(c->wbuf.p), *nxt = static_cast<double2 *>(c->zbuf.p);
-            const int nsub = std::max(1, static_cast<int>(std::ceil(std::abs(dt) * tnorm / 4.0)));
-            const double theta = std::abs(dt) * tnorm / nsub;
-            int mt = 1;
-            for (double rem = theta * theta / 2.0; rem * std::exp(theta) > c->taylor_tol && mt < 55; ++mt)
-                rem *= theta / (mt + 2);
+            const TaylorStep ts = taylor_step(dt);
+            const int nsub = ts.nsub;
+            int mt = ts.mt;
             const double er = std::exp(dt * tmu.x / nsub), ea = dt * tmu.y / nsub;
             const double2 eta = make_double2(er * std::cos(ea), er * std::sin(ea));
             const dim3 gq(ceil_div(Q, kWarps), ldm / 32);

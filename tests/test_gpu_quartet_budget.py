@@ -14,7 +14,7 @@ from molspin_b200 import systems as S
 from tests import helpers as h
 
 pytestmark = pytest.mark.gpu
-TIMES = S.time_grid(3.0, 1.0)
+TIMES = S.time_grid(12.0, 1.0)  # enough products for Taylor and RK4 to take the quartet form
 
 
 def _open(s, terms, budget=0):

@@ -35,7 +35,7 @@ def _run(s, F, upload, precision, propagator="krylov", form="auto", recurrence=L
         p.set_electron_pair(*s.electron_strides())
         p.set_observables([(op, rate) for _, op, rate in s.observables()])
         p.set_factors(F)
-        p.propagate(S.time_grid(4.0, 1.0) if m > 4 else S.time_grid(16.0, 8.0), m, precision, propagator=propagator, recurrence=recurrence)
+        p.propagate(S.time_grid(12.0, 1.0) if m > 4 else S.time_grid(16.0, 8.0), m, precision, propagator=propagator, recurrence=recurrence)
         return p.yields()[0]
 
 
