@@ -48,14 +48,12 @@ struct BatchSystem {
     unsigned long long seed = 0;
     Buf rowptr, col, valf, obs, rates, psi, acc, comp, prev, pflip;
     // resident kernels: H in padded row order (ell: values, columns, lengths) up
-    // to D = 128, by quartets (quart) above; kind 0: neither
+    // to D = 128, by quartets (quart) above
+    enum Kind { kNone, kRows, kQuartets, kUnassembled };  // kUnassembled: quartets from the next run on
     Buf ell, quart;
-    int kind = 0, kmax = 0;
+    Kind kind = kNone;
+    int kmax = 0;
     ResidentQuartets rq{};
-    // CSR of a system on the quartet kernels, uploaded if a Krylov dimension ever
-    // needs the persistent launch
-    std::vector<int> h_rowptr, h_col;
-    std::vector<float> h_valf;
     msgpu_ctx *ctx = nullptr;  // streamed single-system path (D >= kStreamDim)
 };
 
@@ -70,7 +68,7 @@ struct msgpu_batch {
     // systems of the persistent route dropped by msgpu_batch_clear: their device
     // buffers serve the next msgpu_batch_add_system (no cudaMalloc / cudaFree per reuse)
     std::vector<BatchSystem> spare;
-    Buf sys_d, items_d, queue_d, status_d, scratch, times_d, backup, many_d, first_d;
+    Buf sys_d, items_d, queue_d, status_d, scratch, times_d, backup, many_d, first_d, jobs_d, found_d;
     int threshold = 512, ctas_per_sm = 2, tuned = 0;
     int sm_count = 0;
     cudaGraphExec_t graph = nullptr;
@@ -268,10 +266,10 @@ int prepare(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_of
         S.accumulate = accumulate;
         desc[i] = S;
         if (s.ctx) continue;  // streamed path: no work items here
-        if (s.kind) {
-            const ResidentManyShape shape = s.kind == 1 ? resident_shape_many(s.D, S.m) : resident_shape_q_many(s.D, S.m);
+        if (s.kind != BatchSystem::kNone) {
+            const ResidentManyShape shape = s.kind == BatchSystem::kRows ? resident_shape_many(s.D, S.m) : resident_shape_q_many(s.D, S.m);
             if (shape.fn && shape.smem <= kResidentSmemMax) {
-                if (s.kind == 1) {
+                if (s.kind == BatchSystem::kRows) {
                     const size_t slots = static_cast<size_t>(s.D) * s.kmax;
                     S.valf = static_cast<const float2 *>(s.ell.p);
                     S.col = reinterpret_cast<const int *>(S.valf + slots);
@@ -284,16 +282,6 @@ int prepare(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_of
                 resident->push_back(ResidentRun{S, shape, static_cast<double>(s.D) * S.m});
                 continue;
             }
-        }
-        if (s.kind && !s.h_rowptr.empty()) {
-            if (int rc = upload_csr(b, s, s.h_rowptr.data(), s.h_col.data(), s.h_valf)) return rc;
-            if (cudaStreamSynchronize(b->stream) != cudaSuccess)
-                return bfail(b, MSGPU_ERR_CUDA, "batch: Hamiltonian upload failed");
-            s.h_rowptr.clear();
-            S.rowptr = static_cast<const int *>(s.rowptr.p);
-            S.col = static_cast<const int *>(s.col.p);
-            S.valf = static_cast<const float2 *>(s.valf.p);
-            desc[i] = S;
         }
         auto &dst = s.D >= threshold ? large : small;
         for (int t = 0; t < s.M; ++t) dst.push_back(ResidentWork{static_cast<int>(i), t});
@@ -369,7 +357,7 @@ int launch(msgpu_batch *b, int grid, size_t slice, size_t smem, int nlarge, int 
 }
 
 // The resident kernels' forms of a system's H.  Without room for them in the
-// memory budget the system takes the persistent launch (kind stays 0).
+// memory budget the system takes the persistent launch (kind stays kNone).
 void build_rows(msgpu_batch *b, BatchSystem &s, const int *rowptr, const int *col, const std::vector<float> &val, int max_row)
 {
     const int D = s.D;
@@ -392,36 +380,89 @@ void build_rows(msgpu_batch *b, BatchSystem &s, const int *rowptr, const int *co
         b->err.clear();
         return;
     }
-    s.kind = 1;
+    s.kind = BatchSystem::kRows;
     s.kmax = max_row;
 }
 
 void build_quartets(msgpu_batch *b, BatchSystem &s, const int *rowptr, const int *col, const double *val)
 {
     const int Q = s.D / 4;
-    const QuartetForm f = quartet_form(s.D, s.s1, s.s2, rowptr, col, val, false);
+    const QuartetForm f = quartet_form(s.D, s.s1, s.s2, rowptr, col, val, false, false);
     const QuartetSlots slots = quartet_slots(f);
     // one buffer: values (16-byte aligned), the resident arrays, blocks, row pointers, bases
     auto up = [](size_t n) { return (n + 15) / 16 * 16; };
     const size_t nval = up(f.val.size() * sizeof(float)), nrq = up(resident_q_bytes(Q, slots));
     const size_t nblk = up(f.blk.size() * sizeof(int2)), nrow = up(f.rowptr.size() * sizeof(int)), nbase = up(Q * sizeof(int));
-    std::vector<unsigned char> buf(nval + nrq + nblk + nrow + nbase, 0);
-    std::memcpy(buf.data(), f.val.data(), f.val.size() * sizeof(float));
-    std::memcpy(buf.data() + nval + nrq, f.blk.data(), f.blk.size() * sizeof(int2));
-    std::memcpy(buf.data() + nval + nrq + nblk, f.rowptr.data(), f.rowptr.size() * sizeof(int));
-    std::memcpy(buf.data() + nval + nrq + nblk + nrow, f.base.data(), Q * sizeof(int));
-    if (upload(b, s.quart, buf.data(), buf.size(), "quartets") != MSGPU_OK) {
+    if (bensure(b, s.quart, nval + nrq + nblk + nrow + nbase, "quartets") != MSGPU_OK) {
         (void)cudaGetLastError();
         b->err.clear();
         return;
     }
+    auto put = [&](size_t at, const void *from, size_t bytes) {
+        return cudaMemcpyAsync(static_cast<unsigned char *>(s.quart.p) + at, from, bytes, cudaMemcpyHostToDevice, b->stream);
+    };
+    if (put(0, f.val.data(), f.val.size() * sizeof(float)) || put(nval + nrq, f.blk.data(), f.blk.size() * sizeof(int2)) ||
+        put(nval + nrq + nblk, f.rowptr.data(), f.rowptr.size() * sizeof(int)) ||
+        put(nval + nrq + nblk + nrow, f.base.data(), Q * sizeof(int)))
+        return;
     unsigned char *p = static_cast<unsigned char *>(s.quart.p);
     s.rq = resident_q_build(p + nval, Q, s.s1, s.s2, slots, reinterpret_cast<const int *>(p + nval + nrq + nblk),
                             reinterpret_cast<const int2 *>(p + nval + nrq), reinterpret_cast<const float4 *>(p),
                             reinterpret_cast<const int *>(p + nval + nrq + nblk + nrow), b->stream);
     if (cudaGetLastError() != cudaSuccess) return;
     ++b->launches;
-    s.kind = 2;
+    s.kind = BatchSystem::kQuartets;
+}
+
+// The quartet forms that added systems still lack, all in one launch; a system whose
+// blocks do not all get a slot there is assembled on the host from its CSR rows.
+int assemble(msgpu_batch *b)
+{
+    std::vector<QuartetJob> jobs;
+    std::vector<BatchSystem *> of;
+    for (BatchSystem &s : b->sys)
+        if (s.kind == BatchSystem::kUnassembled) {
+            jobs.push_back(QuartetJob{static_cast<const int *>(s.rowptr.p), static_cast<const int *>(s.col.p),
+                                      static_cast<const float2 *>(s.valf.p), s.quart.p, s.D, s.s1, s.s2});
+            of.push_back(&s);
+        }
+    if (jobs.empty()) return MSGPU_OK;
+    const size_t n = jobs.size();
+    std::vector<QuartetFound> found(n);
+    int rc;
+    if ((rc = upload(b, b->jobs_d, jobs.data(), n * sizeof(QuartetJob), "quartet assembly")) ||
+        (rc = bensure(b, b->found_d, n * sizeof(QuartetFound), "quartet assembly")))
+        return rc;
+    resident_q_assemble(static_cast<const QuartetJob *>(b->jobs_d.p), static_cast<int>(n),
+                        static_cast<QuartetFound *>(b->found_d.p), b->stream);
+    ++b->launches;
+    if (cudaGetLastError() ||
+        cudaMemcpyAsync(found.data(), b->found_d.p, n * sizeof(QuartetFound), cudaMemcpyDeviceToHost, b->stream) ||
+        cudaStreamSynchronize(b->stream))
+        return bfail(b, MSGPU_ERR_CUDA, "batch: quartet assembly failed");
+    for (size_t i = 0; i < n; ++i) {
+        BatchSystem &s = *of[i];
+        if (found[i].nslot >= 0) {
+            s.rq = resident_q_assembled(s.quart.p, s.D / 4, found[i]);
+            s.kind = BatchSystem::kQuartets;
+            continue;
+        }
+        std::vector<int> rowptr(s.D + 1);
+        if (cudaMemcpyAsync(rowptr.data(), s.rowptr.p, sizeof(int) * rowptr.size(), cudaMemcpyDeviceToHost, b->stream) ||
+            cudaStreamSynchronize(b->stream))
+            return bfail(b, MSGPU_ERR_CUDA, "batch: quartet assembly failed");
+        const size_t nnz = rowptr[s.D];
+        std::vector<int> col(nnz);
+        std::vector<float> valf(2 * nnz);
+        if (cudaMemcpyAsync(col.data(), s.col.p, sizeof(int) * nnz, cudaMemcpyDeviceToHost, b->stream) ||
+            cudaMemcpyAsync(valf.data(), s.valf.p, sizeof(float) * valf.size(), cudaMemcpyDeviceToHost, b->stream) ||
+            cudaStreamSynchronize(b->stream))
+            return bfail(b, MSGPU_ERR_CUDA, "batch: quartet assembly failed");
+        const std::vector<double> val(valf.begin(), valf.end());
+        s.kind = BatchSystem::kNone;
+        build_quartets(b, s, rowptr.data(), col.data(), val.data());
+    }
+    return MSGPU_OK;
 }
 
 int set_times(msgpu_batch *b, const double *times, int ntimes)
@@ -543,7 +584,8 @@ void msgpu_batch_destroy(msgpu_batch *b)
             for (Buf *x : all) brelease(b, *x);
             if (s.ctx) msgpu_destroy(s.ctx);
         }
-    Buf *all[] = {&b->sys_d, &b->items_d, &b->queue_d, &b->status_d, &b->scratch, &b->times_d, &b->backup, &b->many_d, &b->first_d};
+    Buf *all[] = {&b->sys_d, &b->items_d, &b->queue_d, &b->status_d, &b->scratch, &b->times_d, &b->backup, &b->many_d, &b->first_d,
+                  &b->jobs_d, &b->found_d};
     for (Buf *x : all) brelease(b, *x);
     for (int k = 0; k < 8; ++k) {
         if (b->join[k]) cudaEventDestroy(b->join[k]);
@@ -636,12 +678,7 @@ int msgpu_batch_add_system(msgpu_batch *b, int dim, const int *rowptr, const int
     s.seed = seed;
     const int nnz = rowptr[dim];
     std::vector<float> vf(2 * static_cast<size_t>(nnz));
-    for (int k = 0; k < nnz; ++k) {
-        if (col[k] < 0 || col[k] >= dim || !std::isfinite(val[2 * k]) || !std::isfinite(val[2 * k + 1]))
-            return -bfail(b, MSGPU_ERR_INVALID, "batch: malformed Hamiltonian");
-        vf[2 * k] = static_cast<float>(val[2 * k]);
-        vf[2 * k + 1] = static_cast<float>(val[2 * k + 1]);
-    }
+    for (size_t i = 0; i < vf.size(); ++i) vf[i] = static_cast<float>(val[i]);
     // observables in the kernel pair basis (first digit = larger stride)
     const bool swapped = stride1 < stride2;
     const int perm[4] = {0, 2, 1, 3};
@@ -653,31 +690,45 @@ int msgpu_batch_add_system(msgpu_batch *b, int dim, const int *rowptr, const int
                 op[o * 32 + 2 * (a * 4 + c)] = ops[o * 32 + 2 * (ua * 4 + uc)];
                 op[o * 32 + 2 * (a * 4 + c) + 1] = ops[o * 32 + 2 * (ua * 4 + uc) + 1];
             }
-    s.kind = 0;
+    s.kind = BatchSystem::kNone;
     int max_row = 0;
-    for (int r = 0; r < dim; ++r) max_row = std::max(max_row, rowptr[r + 1] - rowptr[r]);
+    bool ascending = true;  // a column once in every row, then
+    for (int r = 0; r < dim; ++r) {
+        max_row = std::max(max_row, rowptr[r + 1] - rowptr[r]);
+        for (int k = rowptr[r] + 1; k < rowptr[r + 1]; ++k) ascending = ascending && col[k] > col[k - 1];
+    }
     if (dim <= 128) build_rows(b, s, rowptr, col, vf, max_row);
-    else if (resident_q_takes(dim)) build_quartets(b, s, rowptr, col, val);
+    // quartets: assembled on the device from the CSR rows, or here; the CSR rows stay
+    // for a Krylov dimension whose basis does not fit shared memory
+    const bool here = resident_q_takes(dim) && (max_row > kAssembleRow || !ascending);
+    if (here && resident_shape_q_many(dim, kMaxKrylov).smem <= kResidentSmemMax) build_quartets(b, s, rowptr, col, val);
     std::vector<float> psi(2 * static_cast<size_t>(dim) * ntraj);
     for (size_t i = 0; i < psi.size(); ++i) psi[i] = static_cast<float>(factors[i]);
-    std::vector<double> zeros(static_cast<size_t>(nobs) * ntraj, 0.0);
+    const size_t sums = sizeof(double) * nobs * static_cast<size_t>(ntraj);
     int rc;
-    s.h_rowptr.clear();
-    if (s.kind == 2) {
-        s.h_rowptr.assign(rowptr, rowptr + dim + 1);
-        s.h_col.assign(col, col + nnz);
-        s.h_valf = vf;
-    }
-    // up to D = 128 a basis of any Krylov dimension fits shared memory
-    if ((s.kind == 0 && (rc = upload_csr(b, s, rowptr, col, vf))) ||
+    if ((s.kind == BatchSystem::kNone && (rc = upload_csr(b, s, rowptr, col, vf))) ||
         (rc = upload(b, s.obs, op.data(), sizeof(double) * op.size(), "observables")) ||
         (rc = upload(b, s.rates, rates, sizeof(double) * nobs, "rates")) ||
         (rc = upload(b, s.psi, psi.data(), sizeof(float) * psi.size(), "factors")) ||
-        (rc = upload(b, s.acc, zeros.data(), sizeof(double) * zeros.size(), "acc")) ||
-        (rc = upload(b, s.comp, zeros.data(), sizeof(double) * zeros.size(), "comp")) ||
-        (rc = upload(b, s.prev, zeros.data(), sizeof(double) * zeros.size(), "prev"))) {
+        (rc = bensure(b, s.acc, sums, "acc")) || (rc = bensure(b, s.comp, sums, "comp")) ||
+        (rc = bensure(b, s.prev, sums, "prev"))) {
         b->spare.push_back(s);  // its buffers are freed with the batch
         return -rc;
+    }
+    for (Buf *x : {&s.acc, &s.comp, &s.prev})
+        if (cudaMemsetAsync(x->p, 0, sums, b->stream) != cudaSuccess) {
+            b->spare.push_back(s);
+            return -bfail(b, MSGPU_ERR_CUDA, "batch: upload failed");
+        }
+    if (resident_q_takes(dim) && s.kind == BatchSystem::kNone) {
+        if (here) {
+            build_quartets(b, s, rowptr, col, val);
+        } else if (bensure(b, s.quart, resident_q_assembled_bytes(dim / 4), "quartets") == MSGPU_OK) {
+            s.kind = BatchSystem::kUnassembled;
+        } else {  // no room: the persistent launch
+            (void)cudaGetLastError();
+            b->err.clear();
+        }
     }
     if (cudaStreamSynchronize(b->stream) != cudaSuccess) {
         b->spare.push_back(s);
@@ -706,13 +757,14 @@ int msgpu_batch_tune(msgpu_batch *b, const double *times, int ntimes, int krylov
         off += s.psi.bytes;
     }
     if (int rc = set_times(b, times, ntimes)) return rc;
+    if (int rc = assemble(b)) return rc;
     const int thresholds[] = {256, 512, 1024, 2048};
     const int cps[] = {1, 2, 3, 4};
     float best = 1e30f;
     bool persistent = false;  // any system on the persistent launch, which these parameters shape
     for (auto &s : b->sys) {
         const int m = std::min(krylov_dim, s.D);
-        persistent = persistent || (!s.ctx && !(s.kind && (s.kind == 1 ? resident_shape_many(s.D, m).smem
+        persistent = persistent || (!s.ctx && !(s.kind != BatchSystem::kNone && (s.kind == BatchSystem::kRows ? resident_shape_many(s.D, m).smem
                                                                        : resident_shape_q_many(s.D, m).smem) <= kResidentSmemMax));
     }
     for (int th : thresholds)
@@ -747,6 +799,7 @@ int msgpu_batch_run(msgpu_batch *b, const double *times, int ntimes, int krylov_
         return bfail(b, MSGPU_ERR_INVALID, "batch: run needs systems, time points and krylov_dim in 1..32");
     cudaSetDevice(b->device);
     if (int rc = set_times(b, times, ntimes)) return rc;
+    if (int rc = assemble(b)) return rc;
     b->m = krylov_dim;
     return run_once(b, ntimes, krylov_dim, accumulate, step_offset, b->threshold, b->ctas_per_sm, true, &b->last_ms,
                     times);

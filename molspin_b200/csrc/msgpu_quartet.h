@@ -30,7 +30,7 @@ struct QuartetForm {
     std::vector<int2> blk;      // {neighbour base row << 3 | type, value offset in float4}
     std::vector<int> nbr;       // neighbour quartet of each block
     std::vector<float> val;     // complex values by type
-    std::vector<double> val64;  // the same in FP64
+    std::vector<double> val64;  // the same in FP64 (want64)
     std::vector<int> base;      // first row of each quartet
     std::vector<int> src;       // CSR index per value slot (want_src)
 };
@@ -186,7 +186,7 @@ inline int block_type(const double *B, unsigned nz)
 // and 16384: 0.62 and 6.4 ms with searches and divisions per entry, 0.32 and 3.6 so
 // (of which 2.7 for the entries).
 inline QuartetForm quartet_form(int D, int s1, int s2, const int *h_rowptr, const int *h_col, const double *h_val,
-                                bool want_src)
+                                bool want_src, bool want64 = true)
 {
     const int Q = D / 4, nnz = h_rowptr[D];
     const int off[4] = {0, s2, s1, s1 + s2};
@@ -195,8 +195,8 @@ inline QuartetForm quartet_form(int D, int s1, int s2, const int *h_rowptr, cons
     f.base.resize(Q);
     f.blk.reserve(nnz / 6 + Q);
     f.nbr.reserve(nnz / 6 + Q);
-    f.val.reserve(want_src ? 2 * static_cast<size_t>(nnz) : nnz / 2);
-    f.val64.reserve(f.val.capacity());
+    f.val.reserve(2 * static_cast<size_t>(nnz));  // only what is used of it is ever touched
+    if (want64) f.val64.reserve(2 * static_cast<size_t>(nnz));
     if (want_src) f.src.reserve(nnz);
     std::vector<int> place(D);  // 4 (quartet of a row) + its pair index
     for (int q = 0; q < Q; ++q) {
@@ -298,14 +298,20 @@ inline QuartetForm quartet_form(int D, int s1, int s2, const int *h_rowptr, cons
             const int n = kBlockCount[type];
             const size_t end = f.val.size();
             f.val.resize(end + 2 * n);
-            f.val64.resize(end + 2 * n);
+            float *v32 = f.val.data() + end;
             for (int k = 0; k < n; ++k) {
                 const int x = kBlockOrder[type][k];
-                for (int p = 0; p < 2; ++p) {
-                    f.val[end + 2 * k + p] = static_cast<float>(B[2 * x + p]);
-                    f.val64[end + 2 * k + p] = B[2 * x + p];
-                }
+                v32[2 * k] = static_cast<float>(B[2 * x]);
+                v32[2 * k + 1] = static_cast<float>(B[2 * x + 1]);
                 if (want_src) f.src.push_back(z.src[x]);
+            }
+            if (!want64) continue;
+            f.val64.resize(end + 2 * n);
+            double *v64 = f.val64.data() + end;
+            for (int k = 0; k < n; ++k) {
+                const int x = kBlockOrder[type][k];
+                v64[2 * k] = B[2 * x];
+                v64[2 * k + 1] = B[2 * x + 1];
             }
         }
         f.rowptr[q + 1] = static_cast<int>(f.blk.size());

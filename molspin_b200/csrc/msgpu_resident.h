@@ -131,4 +131,22 @@ size_t resident_q_bytes(int Q, const QuartetSlots &slots);
 ResidentQuartets resident_q_build(void *buf, int Q, int s1, int s2, const QuartetSlots &slots, const int *rowptr,
                                   const int2 *blk, const float4 *val, const int *base, cudaStream_t st);
 
+// The same from CSR rows on the device, one CTA a system, for an H whose blocks all
+// have a slot (rows of up to kAssembleRow entries, one a column).  buf:
+// resident_q_assembled_bytes; the view is that of a found.nslot >= 0.
+constexpr int kAssembleRow = 64;
+struct QuartetJob {
+    const int *rowptr, *col;
+    const float2 *val;
+    void *buf;
+    int D, s1, s2;
+};
+struct QuartetFound {
+    int nslot;  // -1: some block has none
+    unsigned second;
+};
+size_t resident_q_assembled_bytes(int Q);
+void resident_q_assemble(const QuartetJob *jobs, int n, QuartetFound *found, cudaStream_t st);
+ResidentQuartets resident_q_assembled(void *buf, int Q, const QuartetFound &found);
+
 }  // namespace msgpu

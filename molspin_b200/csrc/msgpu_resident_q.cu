@@ -34,7 +34,7 @@ k_resident_q_many(const ResidentSystem *__restrict__ systems, const int *__restr
 
 // Up to D = 128 the row form is as fast and leaves no thread idle; 12 warps (D =
 // 1536) is what the registers of one SM hold.
-bool resident_q_takes(int D) { return D > 128 && D <= 1536; }
+bool resident_q_takes(int D) { return D > 128 && D <= kAssembleD; }
 
 namespace {
 
@@ -86,6 +86,22 @@ ResidentQuartets resident_q_build(void *buf, int Q, int s1, int s2, const Quarte
     k_build_resident_quartets<<<(Q + 63) / 64, 64, 0, st>>>(QuartetC{rowptr, blk, val, base}, Q, s1, s2, slots, own, slot,
                                                             rest, nrest);
     return ResidentQuartets{own, slot, rest, nrest, val, Q, slots.n, slots.second};
+}
+
+size_t resident_q_assembled_bytes(int Q)
+{
+    return static_cast<size_t>(Q) * ((8 + 2 * kQuartetSlots) * sizeof(float4) + kQuartetSlots * sizeof(int2) + sizeof(int));
+}
+
+void resident_q_assemble(const QuartetJob *jobs, int n, QuartetFound *found, cudaStream_t st)
+{
+    k_assemble_quartets<<<n, kAssembleThreads, 0, st>>>(jobs, found);
+}
+
+ResidentQuartets resident_q_assembled(void *buf, int Q, const QuartetFound &found)
+{
+    const AssembledQuartets B(buf, Q);
+    return ResidentQuartets{B.own, B.slot, nullptr, B.nblk, B.val, Q, found.nslot, found.second};
 }
 
 }  // namespace msgpu

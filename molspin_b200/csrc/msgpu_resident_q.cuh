@@ -82,6 +82,159 @@ __global__ void k_build_resident_quartets(QuartetC H, int Q, int s1, int s2, Qua
     }
 }
 
+// The arrays of an assembled system in its buffer.
+struct AssembledQuartets {
+    float4 *own;   // [8][Q]
+    float4 *val;   // [kQuartetSlots][Q][2]
+    int2 *slot;    // [kQuartetSlots][Q]
+    int *nblk;     // [Q], zero
+    __host__ __device__ AssembledQuartets(void *buf, int Q)
+    {
+        own = static_cast<float4 *>(buf);
+        val = own + 8 * static_cast<size_t>(Q);
+        slot = reinterpret_cast<int2 *>(val + 2 * kQuartetSlots * static_cast<size_t>(Q));
+        nblk = reinterpret_cast<int *>(slot + kQuartetSlots * static_cast<size_t>(Q));
+    }
+};
+
+// The resident layout straight from CSR rows, one CTA a system and a row a thread:
+// the rules of quartet_slots on FP32 values (a block with equal halves is A (x) I),
+// slots for pairs of distances +-d ahead of single ones.  Systems with more than
+// kQuartetSlots slots, or a block that is of neither type, are left to the host.
+// On the host it takes 0.16 ms a system of D = 1024; here about 20 us for all
+// systems of a batch.
+constexpr int kAssembleThreads = 512, kAssembleDist = 16;
+constexpr int kAssembleD = 1536;  // what resident_q_takes
+__global__ void __launch_bounds__(kAssembleThreads)
+k_assemble_quartets(const QuartetJob *__restrict__ jobs, QuartetFound *__restrict__ found)
+{
+    const QuartetJob J = jobs[blockIdx.x];
+    const int D = J.D, Q = D / 4, s1 = J.s1, s2 = J.s2, tid = threadIdx.x, lane = tid & 31;
+    const int off[4] = {0, s2, s1, s1 + s2};
+    const AssembledQuartets B(J.buf, Q);
+    __shared__ unsigned short place[kAssembleD];     // 4 (quartet of a row) + its pair index
+    __shared__ unsigned mask[kAssembleD / 2];        // by signed distance + Q: entries 4 a + b in use
+    __shared__ signed char list[kAssembleD / 2];     // place in dist, or -1
+    __shared__ unsigned seen[kAssembleD / 4];        // by quartet: bit i, a block at dist[i]
+    __shared__ int dist[kAssembleDist], slot_of[kAssembleDist];
+    __shared__ unsigned state[kAssembleDist];        // bit 0: not of the one type it can be; bit 1: -d in the same quartet
+    __shared__ int ndist, nslot;
+    __shared__ unsigned second;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = tid; q < Q; q += kAssembleThreads) {
+        const int base = quartet_base(q, s1, s2);
+        for (int a = 0; a < 4; ++a) place[base + off[a]] = static_cast<unsigned short>(4 * q + a);
+        seen[q] = 0;
+        mask[q] = mask[Q + q] = 0;
+        B.nblk[q] = 0;
+    }
+    for (int i = tid; i < 8 * Q; i += kAssembleThreads) B.own[i] = zero;
+    for (int i = tid; i < 2 * kQuartetSlots * Q; i += kAssembleThreads) B.val[i] = zero;
+    for (int i = tid; i < kQuartetSlots * Q; i += kAssembleThreads) B.slot[i] = make_int2(i % Q, -1);
+    if (tid < kAssembleDist) state[tid] = 0;
+    __syncthreads();
+    // f(q, a, nq, b, value, row, column) for every entry that is not zero
+    auto entries = [&](auto f) {
+        for (int r = tid; r < D; r += kAssembleThreads) {
+            const int at = place[r];
+            for (int k = __ldg(J.rowptr + r); k < __ldg(J.rowptr + r + 1); ++k) {
+                const float2 v = __ldg(J.val + k);
+                if (v.x == 0.f && v.y == 0.f) continue;
+                const int c = __ldg(J.col + k), to = place[c];
+                f(at >> 2, at & 3, to >> 2, to & 3, v, r, c);
+            }
+        }
+    };
+    entries([&](int q, int a, int nq, int b, float2, int, int) {
+        const unsigned bit = 1u << (4 * a + b);
+        if (nq != q && !(mask[Q + nq - q] & bit)) atomicOr(&mask[Q + nq - q], bit);
+    });
+    __syncthreads();
+    if (tid < 32) {  // the distances in use, ascending
+        int n = 0;
+        for (int i0 = 0; i0 < 2 * Q; i0 += 32) {
+            const int i = i0 + lane;
+            const bool on = i < 2 * Q && mask[i] != 0;
+            const unsigned all = __ballot_sync(0xffffffffu, on);
+            const int at = n + __popc(all & ((1u << lane) - 1u));
+            if (i < 2 * Q) list[i] = static_cast<signed char>(on && at < kAssembleDist ? at : -1);
+            if (on && at < kAssembleDist) dist[at] = i - Q;
+            n += __popc(all);
+        }
+        if (lane == 0) ndist = n;
+    }
+    __syncthreads();
+    const bool few = ndist <= kAssembleDist;
+    // entries that couple different second (first) digits of the pair
+    constexpr unsigned kSecond = 0x5a5au, kFirst = 0x33ccu;
+    if (few)
+        entries([&](int q, int a, int nq, int b, float2 v, int r, int c) {
+            if (nq == q) return;
+            const int i = list[Q + nq - q];
+            if (!((seen[q] >> i) & 1u)) atomicOr(&seen[q], 1u << i);
+            const unsigned m = mask[Q + nq - q];
+            // on the first digit alone: the same for both of the second's states, and the reverse
+            const int step = !(m & kSecond) ? (a & 1 ? -s2 : s2) : !(m & kFirst) ? (a & 2 ? -s1 : s1) : 0;
+            bool same = false;
+            if (step != 0)
+                for (int k = __ldg(J.rowptr + r + step); k < __ldg(J.rowptr + r + step + 1) && !same; ++k) {
+                    const float2 w = __ldg(J.val + k);
+                    same = __ldg(J.col + k) == c + step && w.x == v.x && w.y == v.y;
+                }
+            if (!same) atomicOr(&state[i], 1u);
+        });
+    __syncthreads();
+    if (few)
+        for (int q = tid; q < Q; q += kAssembleThreads)
+            for (int i = 0; i < ndist; ++i) {
+                const int j = list[Q - dist[i]];
+                if (j >= 0 && ((seen[q] >> i) & 1u) && ((seen[q] >> j) & 1u)) atomicOr(&state[i], 2u);
+            }
+    __syncthreads();
+    if (tid == 0) {
+        int n = 0;
+        unsigned sec = 0;
+        bool ok = few;
+        for (int i = 0; i < ndist && ok; ++i) {
+            slot_of[i] = -1;
+            ok = !(state[i] & 1u);
+        }
+        auto is_second = [&](int i) { return (mask[Q + dist[i]] & kSecond) != 0; };
+        for (int pass = 0; pass < 2 && ok; ++pass)
+            for (int i = 0; i < ndist && ok; ++i) {
+                const int j = list[Q - dist[i]];
+                const bool pair = j >= 0 && !(state[i] & 2u) && is_second(i) == is_second(j);
+                if (slot_of[i] >= 0 || (pass == 0 && !(pair && dist[i] > 0))) continue;
+                if (n == kQuartetSlots) {
+                    ok = false;
+                    break;
+                }
+                slot_of[i] = n;
+                if (pair) slot_of[j] = n;
+                if (is_second(i)) sec |= 1u << n;
+                ++n;
+            }
+        nslot = ok ? n : -1;
+        second = sec;
+        found[blockIdx.x] = QuartetFound{nslot, sec};
+    }
+    __syncthreads();
+    if (nslot < 0) return;
+    entries([&](int q, int a, int nq, int b, float2 v, int, int) {
+        if (nq == q) {
+            reinterpret_cast<float *>(B.own + static_cast<size_t>(2 * b) * Q + q)[a] = v.x;
+            reinterpret_cast<float *>(B.own + static_cast<size_t>(2 * b + 1) * Q + q)[a] = v.y;
+            return;
+        }
+        const int k = slot_of[list[Q + nq - q]];
+        const size_t at = static_cast<size_t>(k) * Q + q;
+        B.slot[at] = make_int2(nq, static_cast<int>(2 * at));  // the same from every row of the block
+        const bool sec = (second >> k) & 1u;
+        if ((sec ? a >> 1 : a & 1) == 0)
+            reinterpret_cast<float2 *>(B.val + 2 * at)[sec ? 2 * (a & 1) + (b & 1) : 2 * (a >> 1) + (b >> 1)] = v;
+    });
+}
+
 struct QuartetAcc {
     float re[4], im[4];
 };
