@@ -1287,7 +1287,7 @@ int run_resident(msgpu_ctx *c, const msgpu_run_params *p, int prec, int m)
         return cuda_fail(c, e, "resident setup");
     const ResidentShape shape =
         quartets ? resident_shape_q(D, m)
-                 : prec == MSGPU_PREC_C64 ? resident_shape_c64(D, m) : resident_shape_c128(D, m, lanczos);
+                 : prec == MSGPU_PREC_C64 ? resident_shape_c64(D, m) : resident_shape_c128(D, m, M, lanczos);
     {
         Timed tm(c, KC_APPLY);
         if ((e = raise_smem_limit(reinterpret_cast<const void *>(shape.fn), static_cast<int>(shape.smem))))
@@ -2863,7 +2863,7 @@ extern "C" int msgpu_krylov_step_noalloc(int dim, const int *rowptr, const int *
         S.dt0 = dt;
         S.ntimes = 2;
         S.check_start = 1;
-        const ResidentShape shape = resident_shape_c128(D, m, false);
+        const ResidentShape shape = resident_shape_c128(D, m, ntraj, false);
         int h_status = 0;
         if (raise_smem_limit(reinterpret_cast<const void *>(shape.fn), static_cast<int>(shape.smem)) != cudaSuccess ||
             cudaMemsetAsync(status, 0, sizeof(int), st) != cudaSuccess)

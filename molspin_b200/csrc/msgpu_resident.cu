@@ -25,10 +25,33 @@ ResidentShape resident_shape(int D, int m)
     return make(&k_resident<T, 32, 16, kLanczos>, 32);
 }
 
+// Many trajectories at a Krylov dimension of a few: the work outside the chain of
+// products (values, exponential, barriers) counts, so half the warps with two rows a
+// thread, none of them in registers, and 16 warps an SM instead of 8.
+template <bool kLanczos>
+ResidentShape resident_shape_short(int D, int m)
+{
+    auto make = [&](auto fn, int w) {
+        return ResidentShape{fn, w, resident_carve<double2, kLanczos>(nullptr, D, m, w).bytes};
+    };
+    if (D <= 64) return make(&k_resident<double2, 1, 2, kLanczos>, 1);
+    if (D <= 128) return make(&k_resident<double2, 2, 2, kLanczos>, 2);
+    return make(&k_resident<double2, 4, 2, kLanczos>, 4);
+}
+
 }  // namespace
 
-ResidentShape resident_shape_c128(int D, int m, bool lanczos)
+// The short shape from more trajectories than the other holds at once (8 warps an SM)
+// and, with D in 33 .. 256, up to m = 6 (Arnoldi) or 2 (three-term).  B200, 16384
+// trajectories, 10 steps, ms, short / other shape: Arnoldi D = 64 m = 3 1.65 / 3.11,
+// m = 6 2.87 / 4.49, m = 8 4.21 / 5.63 (2048 trajectories 0.88 / 0.86); D = 128 m = 2
+// 2.16 / 4.21; D = 256 m = 1 2.72 / 5.22, m = 8 23.4 / 23.6; three-term D = 256 m = 1
+// 2.12 / 3.22.  256 trajectories, one wave of the other: Arnoldi D = 64 m = 3 0.23 / 0.16.
+ResidentShape resident_shape_c128(int D, int m, int M, bool lanczos)
 {
+    const int warps = D <= 64 ? 2 : D <= 128 ? 4 : 8;
+    if (D > 32 && D <= 256 && m <= (lanczos ? 2 : 6) && M > 148 * (8 / warps))
+        return lanczos ? resident_shape_short<true>(D, m) : resident_shape_short<false>(D, m);
     return lanczos ? resident_shape<double2, true>(D, m) : resident_shape<double2, false>(D, m);
 }
 

@@ -664,13 +664,18 @@ __device__ __forceinline__ void resident_propagate(const ResidentSystem &S, int 
 // CTAs per SM the register allocation must allow.  complex64 keeps 16 warps on
 // an SM (128 registers a thread): with 133 registers a scheduler holds three
 // warps, not four, and 1024 trajectories of D = 64 took 27 instead of 18 us a
-// step.
-template <typename T>
-constexpr int resident_min_ctas(int W) { return sizeof(T) == sizeof(float2) && W <= 16 ? 16 / W : 1; }
+// step.  So do the complex128 shapes of two rows a thread up to four warps, which
+// are there for many trajectories (resident_shape_c128).
+template <typename T, int RPT>
+constexpr int resident_min_ctas(int W)
+{
+    const bool full = sizeof(T) == sizeof(float2) ? W <= 16 : RPT == 2 && W <= 4;
+    return full ? 16 / W : 1;
+}
 
 // One launch = the whole time loop of every trajectory (one CTA each).
 template <typename T, int W, int RPT, bool kLanczos>
-__global__ void __launch_bounds__(32 * W, resident_min_ctas<T>(W))
+__global__ void __launch_bounds__(32 * W, resident_min_ctas<T, RPT>(W))
 k_resident(const __grid_constant__ ResidentSystem S, int *__restrict__ status)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -700,7 +705,7 @@ __device__ __forceinline__ void load_system(ResidentSystem *to, const ResidentSy
 
 // The same for the trajectories of many systems (the batching form).
 template <int W>
-__global__ void __launch_bounds__(32 * W, resident_min_ctas<float2>(W))
+__global__ void __launch_bounds__(32 * W, resident_min_ctas<float2, 1>(W))
 k_resident_many(const ResidentSystem *__restrict__ systems, const int *__restrict__ first, int nsystems,
                 int *__restrict__ status)
 {

@@ -114,9 +114,9 @@ struct ResidentManyShape {
     size_t smem;
 };
 
-// Kernel and launch shape for dimension D and Krylov dimension m:
+// Kernel and launch shape for dimension D, Krylov dimension m and M trajectories:
 // complex128 (three-term recurrence or Arnoldi), complex64 (three-term).
-ResidentShape resident_shape_c128(int D, int m, bool lanczos);
+ResidentShape resident_shape_c128(int D, int m, int M, bool lanczos);
 ResidentShape resident_shape_c64(int D, int m);
 // The batching form's; fn null when no shape takes it.
 ResidentManyShape resident_shape_many(int D, int m);
