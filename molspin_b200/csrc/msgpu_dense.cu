@@ -709,7 +709,7 @@ __device__ __forceinline__ double dense_ensemble_sum(const double *__restrict__ 
     return v;
 }
 
-// One CTA (128 threads; int8: 256) per trajectory.  The trajectory's column (2D values,
+// One CTA (128 threads; int8: 256 for few trajectories) per trajectory.  The trajectory's column (2D values,
 // re/im per row) is staged in shared memory once; flips, the norm, the
 // optional renormalisation, the pair observables and the split of the next
 // GEMM operand all work from there, and the column is written back only at
@@ -720,15 +720,17 @@ __device__ __forceinline__ double dense_ensemble_sum(const double *__restrict__ 
 //   kI8 = true:  FP64 state, four int8 slices and the column's power-of-two
 //                scale for k_dense_gemm_i8 (see k_u_split_i8 for the slicing).
 // The int8 form is bound by the latency of its FP64 chain (the norm, the scale, four
-// slices a value), so its CTA has twice the threads, the scale is read off the exponent
-// and a slice is rounded by an addition instead of two conversions: D = 576, 512
-// trajectories 13.0 -> 10.8 us.
+// slices a value), so its CTA has twice the threads while all of them are resident at
+// once (wide_epilogue), the scale is read off the exponent and a slice is rounded by an
+// addition instead of two conversions: D = 576, 512 trajectories 13.0 -> 10.8 us.  With
+// more, 128 threads leave less of an SM waiting: 8192 trajectories of D = 64, 10 steps
+// 0.82 -> 0.53 ms, 4096 of D = 576 1.01 -> 0.88, 1500 of D = 1024 0.77 -> 0.74.
 constexpr int kEpiThreads = 128, kEpiThreadsI8 = 256;
-template <bool kI8>
-__global__ void __launch_bounds__(kI8 ? kEpiThreadsI8 : kEpiThreads, kI8 ? 4 : 8)
+inline bool wide_epilogue(int trajectories) { return trajectories <= 4 * 148; }
+template <bool kI8, int kThreads = kEpiThreads>
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads)
 k_dense_epilogue(void *__restrict__ psi_v, void *__restrict__ bparts_v, double *__restrict__ bscale, DenseEpi E)
 {
-    constexpr int kThreads = kI8 ? kEpiThreadsI8 : kEpiThreads;
     using V2 = typename std::conditional<kI8, double2, float2>::type;
     extern __shared__ float4 s_col4[];  // the 2D values of the column
     V2 *s_col = reinterpret_cast<V2 *>(s_col4);
@@ -1162,8 +1164,11 @@ int dense_run(DenseState &st, const DenseRun &run, void *psi128, int ldm, cudaSt
     if ((e = raise_smem_limit(i8 ? reinterpret_cast<const void *>(gemm8)
                                  : ns == 2 ? reinterpret_cast<const void *>(gemm2) : reinterpret_cast<const void *>(gemm3),
                               smem)) ||
-        (e = raise_smem_limit(reinterpret_cast<const void *>(i8 ? k_dense_epilogue<true> : k_dense_epilogue<false>),
-                              static_cast<int>(epi_smem)))) {
+        (e = raise_smem_limit(i8 ? reinterpret_cast<const void *>(k_dense_epilogue<true>)
+                                 : reinterpret_cast<const void *>(k_dense_epilogue<false>),
+                              static_cast<int>(epi_smem))) ||
+        (i8 && (e = raise_smem_limit(reinterpret_cast<const void *>(k_dense_epilogue<true, kEpiThreadsI8>),
+                                     static_cast<int>(epi_smem))))) {
         err = std::string("dense: shared memory: ") + cudaGetErrorString(e);
         return MSGPU_ERR_CUDA;
     }
@@ -1248,8 +1253,11 @@ int dense_run(DenseState &st, const DenseRun &run, void *psi128, int ldm, cudaSt
         Eg.t0 = gt[g] * BN;
         Eg.t1 = gt[g + 1] * BN;
         Eg.prev_values = point_prev >= 0 ? run.part + g * nv + static_cast<size_t>(point_prev) * run.nobs : nullptr;
-        if (i8)
-            launch_dependent(k_dense_epilogue<true>, Eg.t1 - Eg.t0, kEpiThreadsI8, epi_smem, ss[g], st.psi, bp, st.b_scale, Eg);
+        if (i8 && wide_epilogue(Eg.t1 - Eg.t0))
+            launch_dependent(k_dense_epilogue<true, kEpiThreadsI8>, Eg.t1 - Eg.t0, kEpiThreadsI8, epi_smem, ss[g], st.psi, bp,
+                             st.b_scale, Eg);
+        else if (i8)
+            launch_dependent(k_dense_epilogue<true>, Eg.t1 - Eg.t0, kEpiThreads, epi_smem, ss[g], st.psi, bp, st.b_scale, Eg);
         else
             launch_dependent(k_dense_epilogue<false>, Eg.t1 - Eg.t0, kEpiThreads, epi_smem, ss[g], st.psi, bp, nullptr, Eg);
     };
