@@ -617,7 +617,7 @@ def run_dense(args):
 
 def run_batching(args):
     """Batching form: 64 systems of uneven dimension (64..9216) and uneven
-    trajectory counts (64..1024) advanced in one persistent graph-replayed launch."""
+    trajectory counts (64..1024) propagated together."""
     import torch
     from molspin_b200 import batching as B
     from molspin_b200 import systems as S
@@ -643,7 +643,7 @@ def run_batching(args):
     _, clk = _timed(world, stream, step, args.warmup, args.steps)
     launches = bt.launch_count() - l0[0]
     # the batch runs on its own streams: the library's time of each run (device
-    # events around the graph replay, or the wall time of the whole run when
+    # events around its launches, or the wall time of the whole run when
     # large systems take the streamed path on further streams)
     el = _max_over_ranks(sum(ms[args.warmup:]), world)
     st = bt.stats()
@@ -657,7 +657,7 @@ def run_batching(args):
             picks.setdefault(key, []).append(ws[i].system.dim)
     bt.close()
     # whole-batch HBM roofline with the minimal fused Krylov traffic (4m+1) D c per traj-step
-    # (complex64, c = 8 B); the persistent kernel keeps small systems on chip, so this is the
+    # (complex64, c = 8 B); the resident kernels keep small systems on chip, so this is the
     # bound the streamed large systems face
     bytes_per_step = sum((4 * 16 + 1) * w.system.dim * 8 * w.M for w in ws)
     peaks = _peaks()
@@ -675,9 +675,13 @@ def run_batching(args):
                      "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm if achieved else None,
                      "traffic": None, "peak_kind": "measured" if "hbm_gbs" in peaks else "fallback"},
         "clocks": clk, "e2e": None, "gpu_launches": launches,
-        "routes": {"persistent": sum(not i["streamed"] for i in infos), "streamed": sum(i["streamed"] for i in infos),
+        # up to D = 1536 the basis of 16 vectors fits a CTA's shared memory; between that and the
+        # streamed dimension a system joins the persistent launch
+        "routes": {"resident": sum(w.system.dim <= 1536 for w in ws),
+                   "persistent": sum(not i["streamed"] and w.system.dim > 1536 for i, w in zip(infos, ws)),
+                   "streamed": sum(i["streamed"] for i in infos),
                    "streamed_spmm_picks": {k: sorted(v) for k, v in picks.items()}},
-        "launch_note": "per bench step: a resident launch per system below D=2048 on side streams "
+        "launch_note": "per bench step: a resident launch per kernel for all systems up to D=1536 on side streams "
                        "plus the streamed path's kernels for the larger systems", "cpu_baseline": None})
 
 

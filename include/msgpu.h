@@ -51,8 +51,9 @@ extern "C" {
                                scalar K, else Arnoldi */
 #define MSGPU_REC_ARNOLDI 1 /* Arnoldi on G = -iH - K (as SpinSpace::ArnoldiProcess).  C64
                                takes it when K acts on the electron pair only (K = I x K4,
-                               e.g. unequal sinks on the pair's states: CGS2 with FP64 dots,
-                               FP32 storage); any other K needs C128 */
+                               e.g. unequal sinks on the pair's states: FP64 dots, FP32
+                               storage); any other K needs C128.  Classical Gram-Schmidt,
+                               repeated where a vector lost most of its norm */
 #define MSGPU_REC_LANCZOS 2 /* Lanczos on H; valid only when K is a scalar */
 
 /* Propagators. */
@@ -299,14 +300,15 @@ typedef struct msgpu_batch msgpu_batch;
 msgpu_batch *msgpu_batch_create(int device, size_t hbm_budget_bytes);
 void msgpu_batch_destroy(msgpu_batch *batch);
 const char *msgpu_batch_last_error(const msgpu_batch *batch);
-/* Returns the system index (>= 0) or -MSGPU_ERR_*.  ops: nobs 4x4 pair
+/* Returns the system index (>= 0) or -MSGPU_ERR_*.  The first run or tune
+ * after it assembles the resident kernels' forms of the added systems.  ops: nobs 4x4 pair
  * observables (as msgpu_add_pair_observable), factors: dim x ntraj
  * column-major complex (HSPreparedState factors). */
 int msgpu_batch_add_system(msgpu_batch *batch, int dim, const int *rowptr, const int *col, const double *val,
                            double kappa, int stride1, int stride2, int nobs, const double *ops, const double *rates,
                            double st_rate, unsigned long long seed, int ntraj, const double *factors);
 /* Drops every system of the batch (the team threshold and CTAs per SM of a
- * previous tune stay).  The device buffers of persistent-route systems are
+ * previous tune stay).  The device buffers of systems below dimension 2048 are
  * kept and serve the next msgpu_batch_add_system calls, so a pooled batch
  * runs one group of systems after another without allocating or freeing
  * device memory; a streamed system's context is destroyed.  Waits for the
@@ -333,8 +335,8 @@ long long msgpu_launch_count(const msgpu_ctx *ctx);
 int msgpu_spmm_choice(const msgpu_ctx *ctx, int *variant, int *tile, int *groups);
 
 /* System i of a batch: *streamed = 1 when it runs the streamed single-system
- * path on its own context (dimension >= 2048), 0 inside the persistent
- * launch; for a streamed system the SpMM its own tuner picked
+ * path on its own context (dimension >= 2048), else 0 (a resident kernel or
+ * the persistent launch); for a streamed system the SpMM its own tuner picked
  * (msgpu_spmm_choice), else -1.  No counterpart in the reference. */
 int msgpu_batch_system_info(const msgpu_batch *batch, int system, int *streamed, int *variant, int *tile, int *groups);
 

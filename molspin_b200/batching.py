@@ -5,7 +5,8 @@ one after another: the orientation loop of ``TaskHSGeneral::RunLocal``
 (RunSection/General/HS/TaskHSGeneral.cpp:347) and the RunSection step loop
 (main.cpp:651-678) each re-run the whole HSGeneral time loop.  Here every
 system below the streamed-route dimension (2048) runs a resident kernel, a CTA
-per trajectory with the Krylov basis in shared memory, all systems at once
+per trajectory with the Krylov basis in shared memory, one launch per kernel for all
+its systems
 (msgpu_batch_* in include/msgpu.h); one whose basis does not fit shared memory
 joins a persistent launch, replayed from a CUDA graph, with the team threshold
 and grid size chosen by an autotuner on the batch.  Systems at or above that
@@ -73,8 +74,8 @@ class BatchB200:
         return idx
 
     def clear(self):
-        """Drops every system; the device buffers of the persistent route are
-        kept for the next add() calls (msgpu_batch_clear)."""
+        """Drops every system; the device buffers of systems below the streamed
+        route are kept for the next add() calls (msgpu_batch_clear)."""
         self._check(L.lib.msgpu_batch_clear(self.b))
         self.systems.clear()
 
@@ -98,7 +99,7 @@ class BatchB200:
         return int(L.lib.msgpu_batch_launch_count(self.b))
 
     def system_info(self, i: int) -> dict:
-        """Route of system i (streamed or persistent) and, when streamed, the
+        """Whether system i takes the streamed route and, when it does, the
         SpMM its context's tuner picked."""
         st, v, t, g = C.c_int(0), C.c_int(0), C.c_int(0), C.c_int(0)
         self._check(L.lib.msgpu_batch_system_info(self.b, int(i), C.byref(st), C.byref(v), C.byref(t), C.byref(g)))

@@ -3,11 +3,10 @@
 // trajectory count propagated together.  Systems below kStreamDim run the
 // resident kernels (msgpu_resident.cuh, msgpu_resident_q.cuh), a CTA per
 // trajectory with the Krylov basis in shared memory, one launch per kernel for all
-// its systems, all launches at once on a few streams.  A system whose basis does not fit shared
-// memory joins the persistent launch k_batch instead, replayed from a CUDA
-// graph, with the team threshold and the grid size picked by an autotuner.  A
-// large system is better served by the streamed single-system
-// path, which advances all its trajectories in lockstep through the
+// its systems, all launches at once on a few streams.  A system whose basis does not
+// fit shared memory joins the persistent launch k_batch instead, replayed from a CUDA
+// graph, with the team threshold and the grid size picked by an autotuner.  A large
+// system is better served by the streamed single-system path, which advances all its trajectories in lockstep through the
 // quartet-block SpMM (one read of H per 64 trajectories instead of one per
 // trajectory): those systems get their own context and stream and run
 // concurrently with the persistent launch and with each other.
@@ -36,9 +35,10 @@ struct Buf {
     size_t bytes = 0;
 };
 
-// Systems of at least this dimension take the streamed single-system path
-// (measured on the 64-system benchmark batch: the persistent teams win below
-// it, the lockstep SpMM above it).
+// Systems of at least this dimension take the streamed single-system path: a
+// trajectory's basis no longer fits a CTA's shared memory there, and of the other
+// two the persistent launch wins below it and the lockstep SpMM above (the 64-system
+// benchmark batch).
 constexpr int kStreamDim = 2048;
 constexpr int kStreamWorkers = 8;  // host threads driving streamed systems
 
@@ -65,7 +65,7 @@ struct msgpu_batch {
     cudaStream_t stream = nullptr;
     std::string err;
     std::vector<BatchSystem> sys;
-    // systems of the persistent route dropped by msgpu_batch_clear: their device
+    // systems below kStreamDim dropped by msgpu_batch_clear: their device
     // buffers serve the next msgpu_batch_add_system (no cudaMalloc / cudaFree per reuse)
     std::vector<BatchSystem> spare;
     Buf sys_d, items_d, queue_d, status_d, scratch, times_d, backup, many_d, first_d, jobs_d, found_d;

@@ -20,7 +20,7 @@ keep their reservation and are destroyed only when an admission needs the
 memory.
 
 Small systems share launches.  Requests below `pack_dim` (the batching
-form's persistent route, D < 2048) that share a time grid and Krylov
+form's one-launch routes, D < 2048) that share a time grid and Krylov
 dimension are admitted together, up to `pack_max` of them in one slot, and
 run as one batch of the batching form (msgpu_batch_*) on a
 pooled batch whose device buffers are kept between packs
