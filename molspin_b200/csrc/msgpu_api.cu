@@ -2279,6 +2279,7 @@ int msgpu_run(msgpu_ctx *c, const msgpu_run_params *p)
             (void)cudaGetLastError();
             c->err.clear();
             quartet_gen = false;
+            c->q_saving = 0.0;  // not tried again at every call
         }
         if (quartet_gen) {
             pg.H = QuartetD{static_cast<const int *>(c->qrow.p), static_cast<const int2 *>(c->qcolt.p),
