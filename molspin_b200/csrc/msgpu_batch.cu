@@ -144,9 +144,13 @@ constexpr size_t kResidentSmemMax = kSmemMax - sizeof(ResidentSystem);  // besid
 // Queues the resident kernels, one launch for all systems of a kernel (a launch a
 // system leaves a batch of small systems eight at a time: 500 systems of D = 64 with 8
 // trajectories, 50 steps: 41 against 3.9 ms, 64 of them with 16, 20 steps: 2.24 against
-// 0.47 ms), the longest trajectories first, over the side streams between two events on
-// the batch's stream.
-int launch_resident(msgpu_batch *b, std::vector<ResidentRun> &runs)
+// 0.47 ms), the longest trajectories first, over side streams between two events on
+// the batch's stream.  Beside streamed systems (`streamed` of them), whose chains of
+// short kernels set the time, they take one stream, or two beside a single one: nine
+// kernels of 64 trajectories beside four systems of D = 2048 and 4096 8.6 ms with eight
+// streams, 7.7 with one; of 8 trajectories beside one system of D = 2048 5.3, 5.3 with
+// two, 6.1 with one.
+int launch_resident(msgpu_batch *b, std::vector<ResidentRun> &runs, int streamed)
 {
     if (runs.empty()) return MSGPU_OK;
     std::stable_sort(runs.begin(), runs.end(), [](const ResidentRun &x, const ResidentRun &y) { return x.cost > y.cost; });
@@ -176,7 +180,7 @@ int launch_resident(msgpu_batch *b, std::vector<ResidentRun> &runs)
     if ((rc = upload(b, b->many_d, sys.data(), sizeof(ResidentSystem) * sys.size(), "resident systems")) ||
         (rc = upload(b, b->first_d, first.data(), sizeof(int) * first.size(), "resident work")))
         return rc;
-    const int ns = std::min<int>(8, static_cast<int>(launches.size()));
+    const int ns = std::min<int>(streamed > 1 ? 1 : streamed == 1 ? 2 : 8, static_cast<int>(launches.size()));
     cudaError_t e = cudaSuccess;
     if (!b->fork) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
     for (int k = 0; k < ns && !e; ++k)
@@ -490,6 +494,10 @@ int run_once(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_o
                          &resident))
         return rc;
     const bool here = nitems > 0 || !resident.empty();
+    std::vector<int> routed;  // streamed systems (times given: a real run, not a tuning probe)
+    if (times)
+        for (size_t i = 0; i < b->sys.size(); ++i)
+            if (b->sys[i].ctx) routed.push_back(static_cast<int>(i));
     const auto w0 = std::chrono::steady_clock::now();
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
@@ -498,16 +506,11 @@ int run_once(msgpu_batch *b, int ntimes, int m, int accumulate, long long step_o
     int rc = MSGPU_OK;
     if (here && cudaMemsetAsync(b->status_d.p, 0, sizeof(int), b->stream) != cudaSuccess)
         rc = bfail(b, MSGPU_ERR_CUDA, "batch: status reset failed");
-    if (!rc) rc = launch_resident(b, resident);
+    if (!rc) rc = launch_resident(b, resident, static_cast<int>(routed.size()));
     if (!rc && nitems > 0) rc = launch(b, grid, slice, smem, nlarge, nitems, m, graph);
     if (nitems > 0) b->launches += graph ? 1 : 2;  // a replay of the captured graph, or memset + kernel
     cudaEventRecord(e1, b->stream);
-    // streamed systems (times given: a real run, not a tuning probe), each on
-    // its own context and stream, while the persistent launch runs
-    std::vector<int> routed;
-    if (times)
-        for (size_t i = 0; i < b->sys.size(); ++i)
-            if (b->sys[i].ctx) routed.push_back(static_cast<int>(i));
+    // the streamed systems, each on its own context and stream, while the others run
     std::vector<int> rcs(routed.size(), MSGPU_OK);
     if (!routed.empty() && rc == MSGPU_OK) {
         msgpu_run_params p;
