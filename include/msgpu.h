@@ -169,7 +169,9 @@ size_t msgpu_device_bytes(const msgpu_ctx *ctx);
 int msgpu_set_stream(msgpu_ctx *ctx, void *cuda_stream);
 
 /* Hamiltonian H (rad/ns) as CSR with int32 indices; val holds nnz complex
- * values.  Replaces the sp_cx_mat passed to HSPropagator::Step (HSPropagator.h:40-41). */
+ * values.  A row may hold a column more than once: the entries add up (here and
+ * in msgpu_upload_hamiltonian_terms).  Replaces the sp_cx_mat passed to
+ * HSPropagator::Step (HSPropagator.h:40-41). */
 int msgpu_upload_hamiltonian_csr(msgpu_ctx *ctx, int dim, const int *rowptr, const int *col, const double *val);
 
 
